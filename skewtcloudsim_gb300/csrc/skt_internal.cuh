@@ -105,14 +105,121 @@ __device__ __forceinline__ void note_nonfinite(Scalars* sc, double tot) {
 // the same test on one float (the wind maximum's inputs)
 __device__ __forceinline__ bool nonfinite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
 
+constexpr int kMaxPartials = 4096;
+
+// ---- dot products and maxima over the grid ---------------------------------------------------
+// A reduction keeps its sums as an unevaluated pair of floats (about 48 significant bits) from the
+// threads to the total, which becomes FP64 once. The chip's FP64 rate is about 1/60 of its FP32
+// rate: a tree of FP64 shuffles and adds held the pipe for 16 cycles per warp and add, some 2600
+// cycles for a block of 1024 threads, while the pair's five levels cost about 60 FP32 instructions
+// per warp. Products are taken exactly (fma) where FP64 took them exactly; the totals round to the
+// same FP32 step lengths (every output of the plain and mixed steps bit-identical at the sizes
+// below). A plain step at 64x32x64 went from 2.78 to 2.42 ms, at 256x128x256 from 31.1 to 28.5 ms.
+struct Sum2 {
+    float h = 0.0f, l = 0.0f;
+    // (h, l) += (b, e), two-sum on the leading parts, renormalised
+    __device__ __forceinline__ void add(float b, float e) {
+        const float s = h + b;
+        const float bv = s - h;
+        const float t = ((h - (s - bv)) + (b - bv)) + (l + e);
+        h = s + t;
+        l = t - (h - s);
+    }
+    // the exact product a * b
+    __device__ __forceinline__ void add_prod(float a, float b) {
+        const float p = __fmul_rn(a, b);  // never contracted into the sum below
+        add(p, fmaf(a, b, -p));
+    }
+    __device__ __forceinline__ double value() const { return double(h) + double(l); }
+};
+__device__ __forceinline__ Sum2 warp_sum2(Sum2 v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float h = __shfl_xor_sync(0xffffffffu, v.h, o), l = __shfl_xor_sync(0xffffffffu, v.l, o);
+        v.add(h, l);
+    }
+    return v;
+}
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float t = __shfl_xor_sync(0xffffffffu, v, o);
+        v = t > v ? t : v;
+    }
+    return v;
+}
+// the sum and the maximum (at least 0) of NTH threads with a linear thread id, in a fixed order; valid in tid 0
+template <int NTH>
+__device__ __forceinline__ void block_sum_max(Sum2& sum, float& mx, int tid) {
+    __shared__ float2 ss[NTH / 32];
+    __shared__ float sx[NTH / 32];
+    const Sum2 w = warp_sum2(sum);
+    const float m = warp_max(mx);
+    __syncthreads();
+    if ((tid & 31) == 0) {
+        ss[tid >> 5] = make_float2(w.h, w.l);
+        sx[tid >> 5] = m;
+    }
+    __syncthreads();
+    sum = Sum2();
+    mx = 0.0f;
+    if (tid < 32) {
+        if (tid < NTH / 32) {
+            sum.h = ss[tid].x;
+            sum.l = ss[tid].y;
+            mx = sx[tid] > 0.0f ? sx[tid] : 0.0f;
+        }
+        sum = warp_sum2(sum);
+        mx = warp_max(mx);
+    }
+}
+// Publishes the block's sum and maximum (each thread's own values on entry) of a grid of nb blocks
+// (bid: this block's linear index); the last block to finish reduces all partials with every thread
+// (fixed assignment, fixed tree: deterministic). True in thread 0 of that block, with the totals.
+// The arrival is one acquire-release atomic of thread 0, ordered after its own partial's stores.
+template <int NTH>
+__device__ __forceinline__ bool grid_sum_max(Scalars* sc, double* partials, int bid, int nb, int tid, Sum2 sum, float mx, double& tot,
+                                             float& mxall) {
+    __shared__ bool last;
+    float2* const psum = reinterpret_cast<float2*>(partials);
+    float* const pmax = reinterpret_cast<float*>(partials + kMaxPartials);
+    block_sum_max<NTH>(sum, mx, tid);
+    if (tid == 0) {
+        __stcg(psum + bid, make_float2(sum.h, sum.l));
+        __stcg(pmax + bid, mx);
+        unsigned t;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(t) : "l"(&sc->done_blocks) : "memory");
+        last = t == unsigned(nb) - 1u;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    Sum2 s;
+    float m = 0.0f;
+    for (int b = tid; b < nb; b += NTH) {
+        const float2 v = __ldcg(psum + b);
+        const float mb = __ldcg(pmax + b);
+        s.add(v.x, v.y);
+        m = mb > m ? mb : m;
+    }
+    block_sum_max<NTH>(s, m, tid);
+    if (tid == 0) {
+        tot = s.value();
+        mxall = m;
+        sc->done_blocks = 0;
+        note_nonfinite(sc, tot);
+    }
+    return tid == 0;
+}
+__device__ __forceinline__ int linear_block() { return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z); }
+__device__ __forceinline__ int linear_blocks() { return gridDim.x * gridDim.y * gridDim.z; }
+
 // one coarse level of the multigrid preconditioner (A-form coefficients and work vectors)
 struct MgLevel {
     int X = 0, Y = 0, Z = 0;
     float *ax = nullptr, *ay = nullptr, *az = nullptr, *aw = nullptr, *x = nullptr, *x2 = nullptr, *b = nullptr;
 };
 constexpr int kMaxMgLevels = 12;
-
-constexpr int kMaxPartials = 4096;
 
 // Kernel-level configuration (from skt_solver_cfg)
 struct SolverCfg {

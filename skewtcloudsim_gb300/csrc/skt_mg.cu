@@ -8,7 +8,7 @@
 //
 //   x64 = 0
 //   repeat: r = b - A x64 (FP64 arithmetic, FP64 norm)    until |r|/|b| <= refine_tol
-//           solve A e = r with MG-PCG in FP32 (FP64 reductions) to |r_inner| <= inner_rtol |r|
+//           solve A e = r with MG-PCG in FP32 (paired-float reductions, Sum2) to |r_inner| <= inner_rtol |r|
 //           x64 += e
 //
 // Multigrid: cell-centred, the hierarchy of the full grid (ground cells inactive: diagonal 0).
@@ -204,66 +204,16 @@ __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(LvlView L, const f
 
 constexpr int RT = 256;
 
-template <int NTH>
-__device__ __forceinline__ double bsum(double v, double* sm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x < 32) {
-        t = threadIdx.x < (NTH / 32) ? sm[threadIdx.x] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    return t;
+// a thread's compensated running sum (s, c) as the pair that the grid's reduction takes
+__device__ __forceinline__ Sum2 pair_of(float s, float c) {
+    Sum2 p;
+    p.h = s;
+    p.l = -c;
+    return p;
 }
 template <int NTH>
-__device__ __forceinline__ float bmax(float v, float* sm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float t = 0.0f;
-    if (threadIdx.x < 32) {
-        t = threadIdx.x < (NTH / 32) ? sm[threadIdx.x] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
-    }
-    return t;
-}
-// last-block reduction of per-block (sum, max) partials; true in thread 0 of the last block
-__device__ __forceinline__ bool finish(Scalars* sc, double* partials, double sum, float mx, double& tot, float& mall) {
-    __shared__ bool last;
-    __shared__ double sd[RT / 32];
-    __shared__ float sf[RT / 32];
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = sum;
-        partials[kMaxPartials + blockIdx.x] = double(mx);
-        __threadfence();
-        last = atomicAdd(&sc->done_blocks, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double s = 0.0;
-    float m = 0.0f;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += RT) {
-        s += __ldcg(partials + b);
-        const float mb = float(__ldcg(partials + kMaxPartials + b));
-        m = mb > m ? mb : m;
-    }
-    const double ts = bsum<RT>(s, sd);
-    const float tm = bmax<RT>(m, sf);
-    if (threadIdx.x == 0) {
-        tot = ts;
-        mall = tm;
-        sc->done_blocks = 0;
-        note_nonfinite(sc, ts);
-    }
-    return threadIdx.x == 0;
+__device__ __forceinline__ bool finish(Scalars* sc, double* partials, Sum2 sum, float mx, double& tot, float& mall, int tid) {
+    return grid_sum_max<NTH>(sc, partials, linear_block(), linear_blocks(), tid, sum, mx, tot, mall);
 }
 
 // ---- float-float refinement vector ----------------------------------------------------------
@@ -307,13 +257,12 @@ __device__ __forceinline__ void refine_record(Scalars* sc, double tot, float mal
     sc->inner_tol = mall;  // the inner solves reduce the max residual relative to this
 }
 
-// r = b - A (xh + xl) in float-float, |r|^2 (compensated FP32 per thread, FP64 across threads)
+// r = b - A (xh + xl) in float-float, |r|^2 (compensated FP32 per thread, paired floats across threads)
 // and max|r|; any grid
 __global__ void __launch_bounds__(RT) k_resid_ff(Grid g, const float* __restrict__ ax, const float* __restrict__ ay, const float* __restrict__ az,
                                                  const float* __restrict__ aw, const float* __restrict__ xh, const float* __restrict__ xl,
                                                  const float* __restrict__ b, float* __restrict__ r, float refine_tol, int first, Scalars* sc,
                                                  double* partials) {
-    __shared__ double smd[RT / 32];
     float acc = 0.0f, comp = 0.0f, mx = 0.0f;
     for (int c = blockIdx.x * RT + threadIdx.x; c < g.N; c += gridDim.x * RT) {
         float rv = 0.0f;
@@ -336,12 +285,9 @@ __global__ void __launch_bounds__(RT) k_resid_ff(Grid g, const float* __restrict
         acc = tt;
         mx = fmaxf(mx, fabsf(rv));
     }
-    const double bs = bsum<RT>(double(acc) - double(comp), smd);
-    __shared__ float smf[RT / 32];
-    const float bm = bmax<RT>(mx, smf);  // the block's max |r| (finish publishes thread 0's value)
     double tot;
     float mall;
-    if (finish(sc, partials, bs, bm, tot, mall)) refine_record(sc, tot, mall, refine_tol, first);
+    if (finish<RT>(sc, partials, pair_of(acc, comp), mx, tot, mall, threadIdx.x)) refine_record(sc, tot, mall, refine_tol, first);
 }
 
 // (xh, xl) += e and e = 0
@@ -361,22 +307,20 @@ __global__ void __launch_bounds__(RT) k_cast_ff(int n, const float* __restrict__
     for (int c = blockIdx.x * RT + threadIdx.x; c < n; c += gridDim.x * RT) p[c] = xh[c] + xl[c];
 }
 
-// inner CG: rho = z.r (FP64) and s = z (start), or beta = rho_new/rho and s = z + beta s
+// inner CG: rho = z.r (paired floats) and s = z (start), or beta = rho_new/rho and s = z + beta s
 template <bool START>
 __global__ void __launch_bounds__(RT) k_zr_search(int n, const float* __restrict__ z, const float* __restrict__ r, float* __restrict__ s,
                                                   Scalars* sc, double* partials) {
     if (!START && sc->converged) return;
     // pass 1 of 2: the dot product; the search update runs in k_search_mg after beta is known
-    __shared__ double smd[RT / 32];
-    double acc = 0.0;
+    Sum2 acc;
     for (int c = blockIdx.x * RT + threadIdx.x; c < n; c += gridDim.x * RT) {
-        acc += double(z[c]) * double(r[c]);
+        acc.add_prod(z[c], r[c]);
         if (START) s[c] = z[c];
     }
-    const double bs = bsum<RT>(acc, smd);
     double tot;
     float mall;
-    if (finish(sc, partials, bs, 0.0f, tot, mall)) {
+    if (finish<RT>(sc, partials, acc, 0.0f, tot, mall, threadIdx.x)) {
         if (START) {
             sc->sigma0 = tot;
             sc->converged = 0;
@@ -399,9 +343,8 @@ __global__ void __launch_bounds__(RT) k_matvec_mg(Grid g, const float* __restric
                                                   const float* __restrict__ aw, const float* __restrict__ s, float* __restrict__ As,
                                                   Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[RT / 32];
     LvlView L{g.X, g.Y, g.Z, ax, ay, az, aw};
-    double acc = 0.0;
+    Sum2 acc;
     for (int c = blockIdx.x * RT + threadIdx.x; c < g.N; c += gridDim.x * RT) {
         float v = 0.0f;
         if (aw[c] != 0.0f) {
@@ -409,12 +352,11 @@ __global__ void __launch_bounds__(RT) k_matvec_mg(Grid g, const float* __restric
             v = apply_A(L, s, xx, yy, zz, c);
         }
         As[c] = v;
-        acc += double(v) * double(s[c]);
+        acc.add_prod(v, s[c]);
     }
-    const double bs = bsum<RT>(acc, smd);
     double tot;
     float mall;
-    if (finish(sc, partials, bs, 0.0f, tot, mall)) {
+    if (finish<RT>(sc, partials, acc, 0.0f, tot, mall, threadIdx.x)) {
         sc->sigma1 = tot;
         sc->alpha = float(sc->sigma0 / tot);
     }
@@ -424,7 +366,6 @@ __global__ void __launch_bounds__(RT) k_matvec_mg(Grid g, const float* __restric
 __global__ void __launch_bounds__(RT) k_update_mg(int n, const float* __restrict__ s, const float* __restrict__ As, float* __restrict__ e,
                                                   float* __restrict__ r, float inner_rtol, int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ float smf[RT / 32];
     const float alpha = sc->alpha;
     float mx = 0.0f;
     for (int c = blockIdx.x * RT + threadIdx.x; c < n; c += gridDim.x * RT) {
@@ -434,10 +375,9 @@ __global__ void __launch_bounds__(RT) k_update_mg(int n, const float* __restrict
         const float m = fabsf(rv);
         if (m > mx) mx = m;
     }
-    const float bm = bmax<RT>(mx, smf);
     double tot;
     float mall;
-    if (finish(sc, partials, 0.0, bm, tot, mall)) {
+    if (finish<RT>(sc, partials, Sum2(), mx, tot, mall, threadIdx.x)) {
         sc->iters += 1;
         sc->outer_inner_total += 1;
         if (mall <= inner_rtol * sc->inner_tol) sc->converged = 1;
@@ -509,96 +449,6 @@ struct UIn {
         return a;
     }
 };
-
-// block-wide sum over NTH threads with a linear thread id; the total is valid in tid 0
-template <int NTH>
-__device__ __forceinline__ double bsum_t(double v, double* sm, int tid) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((tid & 31) == 0) sm[tid >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (tid < 32) {
-        t = tid < (NTH / 32) ? sm[tid] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    return t;
-}
-// last-block reduction of one FP64 partial per block of a 3D grid; true in tid 0 of the last block
-template <int NTH>
-__device__ __forceinline__ bool finish_sum(Scalars* sc, double* partials, double sum, double& tot, int tid) {
-    __shared__ bool last;
-    __shared__ double sd[NTH / 32];
-    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int nblk = gridDim.x * gridDim.y * gridDim.z;
-    if (tid == 0) {
-        partials[bid] = sum;
-        __threadfence();
-        last = atomicAdd(&sc->done_blocks, 1u) == unsigned(nblk) - 1u;
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double s = 0.0;
-    for (int b = tid; b < nblk; b += NTH) s += __ldcg(partials + b);
-    const double ts = bsum_t<NTH>(s, sd, tid);
-    if (tid == 0) {
-        tot = ts;
-        sc->done_blocks = 0;
-        note_nonfinite(sc, ts);
-    }
-    return tid == 0;
-}
-
-// finish_sum with a max as well: mx is each thread's own max, reduced over the block here
-// (partials[kMaxPartials + bid] holds the block maxima)
-template <int NTH>
-__device__ __forceinline__ bool finish_sum_max(Scalars* sc, double* partials, double sum, float mx, double& tot, float& mall, int tid) {
-    __shared__ bool last;
-    __shared__ double sd[NTH / 32];
-    __shared__ float sf[NTH / 32];
-    __shared__ float sb[NTH / 32];
-    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int nblk = gridDim.x * gridDim.y * gridDim.z;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0) sb[tid >> 5] = mx;
-    __syncthreads();
-    if (tid == 0)
-        for (int w = 1; w < NTH / 32; ++w) mx = fmaxf(mx, sb[w]);
-    if (tid == 0) {
-        partials[bid] = sum;
-        partials[kMaxPartials + bid] = double(mx);
-        __threadfence();
-        last = atomicAdd(&sc->done_blocks, 1u) == unsigned(nblk) - 1u;
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double s = 0.0;
-    float m = 0.0f;
-    for (int b = tid; b < nblk; b += NTH) {
-        s += __ldcg(partials + b);
-        m = fmaxf(m, float(__ldcg(partials + kMaxPartials + b)));
-    }
-    const double ts = bsum_t<NTH>(s, sd, tid);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __syncthreads();
-    if ((tid & 31) == 0) sf[tid >> 5] = m;
-    __syncthreads();
-    if (tid == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < NTH / 32; ++w) t = fmaxf(t, sf[w]);
-        tot = ts;
-        mall = t;
-        sc->done_blocks = 0;
-        note_nonfinite(sc, ts);
-    }
-    return tid == 0;
-}
 
 // (A u) at the four cells of a row from the z-march registers
 struct Stencil4 {
@@ -675,10 +525,9 @@ __global__ void __launch_bounds__(32 * JVY, 32 / JVY) k_mg_smooth4(int X, int Y,
         azb = cz;
     }
     if (DOT != DOT_NONE) {
-        __shared__ double smd[JVY];
-        const double bs = bsum_t<32 * JVY>(double(acc) - double(comp), smd, tid);
         double tot;
-        if (finish_sum<32 * JVY>(sc, partials, bs, tot, tid)) {
+        float mall;
+        if (finish<32 * JVY>(sc, partials, pair_of(acc, comp), 0.0f, tot, mall, tid)) {
             if (DOT == DOT_START) {
                 sc->sigma0 = tot;
                 sc->beta_f = 0.0f;
@@ -819,10 +668,9 @@ __global__ void __launch_bounds__(32 * JVY, 32 / JVY) k_mg_matvec_search4(int X,
         vc = vf;
         azb = cz;
     }
-    __shared__ double smd[JVY];
-    const double bs = bsum_t<32 * JVY>(double(acc) - double(comp), smd, tid);
     double tot;
-    if (finish_sum<32 * JVY>(sc, partials, bs, tot, tid)) {
+    float mall;
+    if (finish<32 * JVY>(sc, partials, pair_of(acc, comp), 0.0f, tot, mall, tid)) {
         sc->sigma1 = tot;
         sc->alpha = float(sc->sigma0 / tot);
     }
@@ -899,11 +747,9 @@ __global__ void __launch_bounds__(32 * JVY) k_resid_ff4(int X, int Y, int Z, int
         hc = hf; lc = lf;
         azb = cz;
     }
-    __shared__ double smd[JVY];
-    const double bs = bsum_t<32 * JVY>(double(acc) - double(comp), smd, tid);
     double tot;
     float mall;
-    if (finish_sum_max<32 * JVY>(sc, partials, bs, mx, tot, mall, tid)) refine_record(sc, tot, mall, refine_tol, first);
+    if (finish<32 * JVY>(sc, partials, pair_of(acc, comp), mx, tot, mall, tid)) refine_record(sc, tot, mall, refine_tol, first);
 }
 
 // FP16 copies of the finest level's coefficients for the V-cycle. Faces round toward zero; the
@@ -940,7 +786,6 @@ __global__ void __launch_bounds__(RT) k_mg_half(Grid g, const float* __restrict_
 __global__ void __launch_bounds__(RT) k_update_mg4(int n4, const float4* __restrict__ s, const float4* __restrict__ As, float4* __restrict__ e,
                                                    float4* __restrict__ r, float inner_rtol, int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ float smf[RT / 32];
     const float alpha = sc->alpha;
     float mx = 0.0f;
     for (int i = blockIdx.x * RT + threadIdx.x; i < n4; i += gridDim.x * RT) {
@@ -952,10 +797,9 @@ __global__ void __launch_bounds__(RT) k_update_mg4(int n4, const float4* __restr
         r[i] = rv;
         mx = fmaxf(mx, fmaxf(fmaxf(fabsf(rv.x), fabsf(rv.y)), fmaxf(fabsf(rv.z), fabsf(rv.w))));
     }
-    const float bm = bmax<RT>(mx, smf);
     double tot;
     float mall;
-    if (finish(sc, partials, 0.0, bm, tot, mall)) {
+    if (finish<RT>(sc, partials, Sum2(), mx, tot, mall, threadIdx.x)) {
         sc->iters += 1;
         sc->outer_inner_total += 1;
         if (mall <= inner_rtol * sc->inner_tol) sc->converged = 1;
@@ -963,12 +807,11 @@ __global__ void __launch_bounds__(RT) k_update_mg4(int n4, const float4* __restr
     }
 }
 
-// rho = z.r (FP64 across threads); START also sets s = z
+// rho = z.r (paired floats across threads); START also sets s = z
 template <bool START>
 __global__ void __launch_bounds__(RT) k_zr4(int n4, const float4* __restrict__ z, const float4* __restrict__ r, float4* __restrict__ s,
                                             Scalars* sc, double* partials) {
     if (!START && sc->converged) return;
-    __shared__ double smd[RT / 32];
     float acc = 0.0f, comp = 0.0f;
     for (int i = blockIdx.x * RT + threadIdx.x; i < n4; i += gridDim.x * RT) {
         const float4 zv = z[i], rv = r[i];
@@ -979,10 +822,9 @@ __global__ void __launch_bounds__(RT) k_zr4(int n4, const float4* __restrict__ z
         acc = tt;
         if (START) s[i] = zv;
     }
-    const double bs = bsum<RT>(double(acc) - double(comp), smd);
     double tot;
     float mall;
-    if (finish(sc, partials, bs, 0.0f, tot, mall)) {
+    if (finish<RT>(sc, partials, pair_of(acc, comp), 0.0f, tot, mall, threadIdx.x)) {
         if (START) {
             sc->sigma0 = tot;
             sc->converged = 0;

@@ -1,5 +1,5 @@
 // Pressure projection: boundary reset, Poisson coefficients + divergence, Jacobi-preconditioned
-// CG with FP64 reductions, pressure/density update and the velocity correction.
+// CG with paired-float reductions (Sum2), pressure/density update and the velocity correction.
 // Follows pressureProject / calculatePressureProject (Game/environment.cu:851-987).
 #include "skt_internal.cuh"
 
@@ -28,42 +28,6 @@ __device__ __forceinline__ void tile_cell(const Grid& g, const Tiles& T, int t, 
     x = tx * TX + (threadIdx.x & (TX - 1));
     y = ty * TY + (threadIdx.x / TX);
 }
-
-// fixed-order block reductions
-__device__ __forceinline__ double block_sum(double v, double* sm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sm[w] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x < 32) {
-        t = threadIdx.x < (NT / 32) ? sm[threadIdx.x] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    return t;  // valid in thread 0
-}
-__device__ __forceinline__ float block_max(float v, float* sm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sm[w] = v;
-    __syncthreads();
-    float t = 0.0f;
-    if (threadIdx.x < 32) {
-        t = threadIdx.x < (NT / 32) ? sm[threadIdx.x] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
-    }
-    return t;
-}
-
-// Publishes one block partial (sum, max) of a 1D NT-thread grid; thread 0 of the last block to
-// finish gets the totals (see publish_n). Defined after the generic reductions below.
-__device__ __forceinline__ bool publish(Scalars* sc, double* partials, double sum, float mx, double& tot, float& mxall);
 
 __device__ __forceinline__ float char_trunc(float a) {  // (char) of a float: truncate, saturate (Q3)
     const float t = truncf(a);
@@ -104,9 +68,7 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
                                               float* __restrict__ ax, float* __restrict__ ay, float* __restrict__ az, float* __restrict__ aw,
                                               float* __restrict__ r, float* __restrict__ s, float* __restrict__ pp, float* __restrict__ As,
                                               int reference, Scalars* sc, double* partials) {
-    __shared__ double smd[NT / 32];
-    __shared__ float smf[NT / 32];
-    double dsum = 0.0;
+    Sum2 dsum;
     float mx = 0.0f;
     for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
         int x, y, z;
@@ -148,15 +110,13 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
         r[c] = rv;
         const float zv = rv * precon_of(wd);
         s[c] = zv;
-        dsum += double(zv) * double(rv);
+        dsum.add_prod(zv, rv);
         const float m = (!reference || z == 0) ? fabsf(rv) : rv;
         if (m > mx) mx = m;
     }
-    const double bs = block_sum(dsum, smd);
-    const float bm = block_max(mx, smf);
     double tot;
     float mall;
-    if (publish(sc, partials, bs, bm, tot, mall)) {
+    if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
         sc->sigma0 = tot;
         sc->sigma1 = 0.0;
         sc->iters = 0;
@@ -172,8 +132,7 @@ __global__ void __launch_bounds__(NT) k_matvec(Grid g, Tiles T, const float* __r
                                                const float* __restrict__ az, const float* __restrict__ aw, const float* __restrict__ s,
                                                float* __restrict__ As, int reference, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[NT / 32];
-    double dsum = 0.0;
+    Sum2 dsum;
     for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
         int x, y, z;
         tile_cell(g, T, t, x, y, z);
@@ -194,12 +153,11 @@ __global__ void __launch_bounds__(NT) k_matvec(Grid g, Tiles T, const float* __r
         const float sc0 = s[c];
         const float out = aw[c] * sc0 + ((AL * sl + AD * sd + AB * sb + ax[c] * sr + ay[c] * su + az[c] * sf));
         As[c] = out;
-        dsum += double(out) * double(sc0);
+        dsum.add_prod(out, sc0);
     }
-    const double bs = block_sum(dsum, smd);
     double tot;
     float mall;
-    if (publish(sc, partials, bs, 0.0f, tot, mall)) {
+    if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -212,10 +170,8 @@ __global__ void __launch_bounds__(NT) k_update(Grid g, Tiles T, const float* __r
                                                const float* __restrict__ As, float* __restrict__ pp, float* __restrict__ r,
                                                int reference, float tol, int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[NT / 32];
-    __shared__ float smf[NT / 32];
     const float alpha = sc->alpha;
-    double dsum = 0.0;
+    Sum2 dsum;
     float mx = 0.0f;
     for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
         int x, y, z;
@@ -227,15 +183,13 @@ __global__ void __launch_bounds__(NT) k_update(Grid g, Tiles T, const float* __r
         const float rv = r[c] - alpha * As[c];
         r[c] = rv;
         const float zv = rv * precon_of(aw[c]);
-        dsum += double(zv) * double(rv);
+        dsum.add_prod(zv, rv);
         const float m = (!reference || z == 0) ? fabsf(rv) : rv;
         if (m > mx) mx = m;
     }
-    const double bs = block_sum(dsum, smd);
-    const float bm = block_max(mx, smf);
     double tot;
     float mall;
-    if (publish(sc, partials, bs, bm, tot, mall)) {
+    if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
         if (mall <= tol) {
@@ -267,9 +221,9 @@ __global__ void __launch_bounds__(NT) k_search(Grid g, Tiles T, const float* __r
 }
 
 // ---- vectorised PCG iteration (X % 4 == 0): float4 streams, FP32-compensated per-thread sums,
-// FP64 across threads and blocks --------------------------------------------------------------
+// paired floats across threads and blocks --------------------------------------------------------------
 
-struct Kahan {  // compensated FP32 running sum
+struct Kahan {  // compensated FP32 running sum of one thread
     float s = 0.0f, c = 0.0f;
     __device__ __forceinline__ void add(float v) {
         const float y = v - c;
@@ -277,78 +231,13 @@ struct Kahan {  // compensated FP32 running sum
         c = (t - s) - y;
         s = t;
     }
+    __device__ __forceinline__ Sum2 pair() const {
+        Sum2 p;
+        p.h = s;
+        p.l = -c;
+        return p;
+    }
 };
-
-template <int NTH>
-__device__ __forceinline__ double block_sum_n(double v, double* sm, int tid) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((tid & 31) == 0) sm[tid >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (tid < 32) {
-        t = tid < (NTH / 32) ? sm[tid] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    return t;
-}
-template <int NTH>
-__device__ __forceinline__ float block_max_n(float v, float* sm, int tid) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if ((tid & 31) == 0) sm[tid >> 5] = v;
-    __syncthreads();
-    float t = 0.0f;
-    if (tid < 32) {
-        t = tid < (NTH / 32) ? sm[tid] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
-    }
-    return t;
-}
-// publish() for any grid shape: bid = linear block id, nb = number of blocks. The last block to
-// finish reduces all partials with every thread (fixed assignment, fixed tree): deterministic.
-// Returns true in thread 0 of that block, with tot/mxall set.
-template <int NTH>
-__device__ __forceinline__ bool publish_n(Scalars* sc, double* partials, int bid, int nb, int tid, double sum, float mx, double& tot,
-                                          float& mxall) {
-    __shared__ bool last;
-    __shared__ double sms[NTH / 32];
-    __shared__ float smm[NTH / 32];
-    if (tid == 0) {
-        partials[bid] = sum;
-        partials[kMaxPartials + bid] = double(mx);
-        __threadfence();
-        const unsigned t = atomicAdd(&sc->done_blocks, 1u);
-        last = (t == unsigned(nb) - 1);
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double s = 0.0;
-    float m = 0.0f;
-    for (int b = tid; b < nb; b += NTH) {
-        s += __ldcg(partials + b);
-        const float mb = float(__ldcg(partials + kMaxPartials + b));
-        m = mb > m ? mb : m;
-    }
-    const double ts = block_sum_n<NTH>(s, sms, tid);
-    const float tm = block_max_n<NTH>(m, smm, tid);
-    if (tid == 0) {
-        tot = ts;
-        mxall = tm;
-        sc->done_blocks = 0;
-        note_nonfinite(sc, ts);
-    }
-    return tid == 0;
-}
-
-__device__ __forceinline__ bool publish(Scalars* sc, double* partials, double sum, float mx, double& tot, float& mxall) {
-    return publish_n<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, sum, mx, tot, mxall);
-}
 
 constexpr int UT = 256;
 
@@ -358,8 +247,6 @@ __global__ void __launch_bounds__(UT) k_update4(int n4, int xy4, const float4* _
                                                 const float4* __restrict__ As, float4* __restrict__ pp, float4* __restrict__ r,
                                                 int reference, float tol, int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[UT / 32];
-    __shared__ float smf[UT / 32];
     const float alpha = sc->alpha;
     Kahan acc;
     float mx = 0.0f;
@@ -383,11 +270,9 @@ __global__ void __launch_bounds__(UT) k_update4(int n4, int xy4, const float4* _
         if (m2 > mx) mx = m2;
         if (m3 > mx) mx = m3;
     }
-    const double bs = block_sum_n<UT>(double(acc.s) - double(acc.c), smd, threadIdx.x);
-    const float bm = block_max_n<UT>(mx, smf, threadIdx.x);
     double tot;
     float mall;
-    if (publish_n<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, bs, bm, tot, mall)) {
+    if (grid_sum_max<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.pair(), mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
         if (mall <= tol) {
@@ -433,7 +318,6 @@ __global__ void __launch_bounds__(MVT) k_matvec4(Grid g, int zlen, const float* 
                                                  const float* __restrict__ az, const float* __restrict__ aw, const float* __restrict__ s,
                                                  float* __restrict__ As, int reference, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[MVT / 32];
     const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
     const int y = blockIdx.y * MVY + threadIdx.y;
@@ -499,12 +383,9 @@ __global__ void __launch_bounds__(MVT) k_matvec4(Grid g, int zlen, const float* 
         scur = sf;
         azb = cz;
     }
-    const double bs = block_sum_n<MVT>(double(acc.s) - double(acc.c), smd, tid);
-    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int nb = gridDim.x * gridDim.y * gridDim.z;
     double tot;
     float mall;
-    if (publish_n<MVT>(sc, partials, bid, nb, tid, bs, 0.0f, tot, mall)) {
+    if (grid_sum_max<MVT>(sc, partials, linear_block(), linear_blocks(), tid, acc.pair(), 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -532,7 +413,6 @@ __global__ void __launch_bounds__(MVT) k_matvec_search4(Grid g, int zlen, const 
                                                         float* __restrict__ snew, float* __restrict__ As, float* __restrict__ pp,
                                                         int reference, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[MVT / 32];
     const float beta = sc->beta_f, alpha_pp = sc->alpha_pp;
     const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
@@ -612,12 +492,9 @@ __global__ void __launch_bounds__(MVT) k_matvec_search4(Grid g, int zlen, const 
         vc = vf;
         azb = cz;
     }
-    const double bs = block_sum_n<MVT>(double(acc.s) - double(acc.c), smd, tid);
-    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int nb = gridDim.x * gridDim.y * gridDim.z;
     double tot;
     float mall;
-    if (publish_n<MVT>(sc, partials, bid, nb, tid, bs, 0.0f, tot, mall)) {
+    if (grid_sum_max<MVT>(sc, partials, linear_block(), linear_blocks(), tid, acc.pair(), 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -630,8 +507,6 @@ __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4*
                                                   float4* __restrict__ r, float4* __restrict__ zout, int reference, float tol,
                                                   int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    __shared__ double smd[UT / 32];
-    __shared__ float smf[UT / 32];
     const float alpha = sc->alpha;
     Kahan acc;
     float mx = 0.0f;
@@ -654,11 +529,9 @@ __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4*
         if (m2 > mx) mx = m2;
         if (m3 > mx) mx = m3;
     }
-    const double bs = block_sum_n<UT>(double(acc.s) - double(acc.c), smd, threadIdx.x);
-    const float bm = block_max_n<UT>(mx, smf, threadIdx.x);
     double tot;
     float mall;
-    if (publish_n<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, bs, bm, tot, mall)) {
+    if (grid_sum_max<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.pair(), mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
         sc->alpha_pp = alpha;
@@ -719,7 +592,7 @@ __global__ void k_pcg_cond(cudaGraphConditionalHandle h, Scalars* sc, int loop) 
 // is the right face of the cell before (a shuffle across lanes), the back face the front face of
 // the previous plane, the down face is formed again from the row below. coef_of and the harmonic
 // mean are symmetric in their two densities (IEEE addition commutes), so every value equals
-// k_build's; z.r is summed in FP64 in a different order.
+// k_build's; z.r is summed (Sum2) in a different order.
 __device__ __forceinline__ float fcomp(const float4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); }
 __device__ __forceinline__ void fset(float4& v, int k, float a) {
     if (k == 0) v.x = a; else if (k == 1) v.y = a; else if (k == 2) v.z = a; else v.w = a;
@@ -738,8 +611,6 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
                                                 float* __restrict__ aw, float* __restrict__ r, float* __restrict__ s,
                                                 float* __restrict__ pp, float* __restrict__ As, int reference, Scalars* sc,
                                                 double* partials) {
-    __shared__ double smd[MVT / 32];
-    __shared__ float smf[MVT / 32];
     const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
     const int y = blockIdx.y * MVY + threadIdx.y;
@@ -749,7 +620,7 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
     const int X = g.X, XY = g.XY, Z = g.Z;
     const int row = x0 + y * X;
     const float4 z4 = make_float4(0, 0, 0, 0);
-    double dsum = 0.0;
+    Sum2 dsum;
     float mx = 0.0f;
     const float du_ = sky ? defU[y] : 0.0f, dw_ = sky ? defW[y] : 0.0f;
     // own plane: density and reciprocal; the back face (front face of the plane before) and w there
@@ -830,7 +701,7 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
                 const float zv = rv * precon_of(wd);
                 fset(oax, k, cR[k]); fset(oay, k, cU); fset(oaz, k, cF); fset(oaw, k, wd);
                 fset(orr, k, rv); fset(oss, k, zv);
-                dsum += double(zv) * double(rv);
+                dsum.add_prod(zv, rv);
                 const float m = (!reference || z == 0) ? fabsf(rv) : rv;
                 if (m > mx) mx = m;
                 fset(hB, k, hF); fset(cB, k, cF);
@@ -857,13 +728,9 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
         rc = rf;
         wB = wo;
     }
-    const double bs = block_sum_n<MVT>(dsum, smd, tid);
-    const float bm = block_max_n<MVT>(mx, smf, tid);
-    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int nb = gridDim.x * gridDim.y * gridDim.z;
     double tot;
     float mall;
-    if (publish_n<MVT>(sc, partials, bid, nb, tid, bs, bm, tot, mall)) {
+    if (grid_sum_max<MVT>(sc, partials, linear_block(), linear_blocks(), tid, dsum, mx, tot, mall)) {
         sc->sigma0 = tot;
         sc->sigma1 = 0.0;
         sc->iters = 0;
