@@ -570,7 +570,7 @@ skt_status skt_create(const skt_grid_desc* grid, const skt_solver_cfg* cfg, skt_
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const int nsky = 12 + 2 + 4 + 4;
     size_t bytes = al(N * 4) * nsky + al(N * 8) * 2 + al(NG * 4) * 10 + al(NG * 4) + al(NY * 4) * 6 + al(sizeof(Scalars)) +
-                   al(sizeof(double) * 2 * kMaxPartials);
+                   al(sizeof(double) * 2 * kMaxPartials) + al(pcg_grid_bytes(e));
     if (cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking) != cudaSuccess) {
         const std::string m = std::string("stream: ") + cudaGetErrorString(cudaGetLastError());
         delete h;
@@ -597,6 +597,7 @@ skt_status skt_create(const skt_grid_desc* grid, const skt_solver_cfg* cfg, skt_
     for (int i = 0; i < 6; ++i) *co[i] = (float*)take(NY * 4);
     e.sc = (Scalars*)take(sizeof(Scalars));
     e.partials = (double*)take(sizeof(double) * 2 * kMaxPartials);
+    e.grid_parts = take(pcg_grid_bytes(e));
     cudaMemsetAsync(e.pool, 0, bytes, e.stream);
     e.g.gh = e.gh;
     if (cudaMallocHost(&e.host_sc, sizeof(Scalars)) != cudaSuccess ||

@@ -77,7 +77,7 @@ struct Scalars {
     int iters;                        // PCG iterations done
     float residual;                   // last max residual
     unsigned int done_blocks;         // last-block reduction ticket
-    unsigned int done_blocks2;
+    unsigned int grid_tag;            // k_pcg_grid: the tag of its last reduction (they count on from launch to launch)
     int nsub;                         // Courant substeps of the current advection
     int status;                       // 0 ok, otherwise an skt_status
     double rnorm0;                    // mixed mode: initial residual norm
@@ -117,13 +117,13 @@ constexpr int kMaxPartials = 4096;
 // below). A plain step at 64x32x64 went from 2.78 to 2.42 ms, at 256x128x256 from 31.1 to 28.5 ms.
 struct Sum2 {
     float h = 0.0f, l = 0.0f;
-    // (h, l) += (b, e), two-sum on the leading parts, renormalised
+    // (h, l) += (b, e): two-sum on the leading parts, the rest in the low parts
     __device__ __forceinline__ void add(float b, float e) {
-        const float s = h + b;
-        const float bv = s - h;
-        const float t = ((h - (s - bv)) + (b - bv)) + (l + e);
-        h = s + t;
-        l = t - (h - s);
+        const float s = __fadd_rn(h, b);
+        const float bv = __fsub_rn(s, h);
+        const float t = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bv)), __fsub_rn(b, bv));
+        l = (l + e) + t;
+        h = s;
     }
     // the exact product a * b
     __device__ __forceinline__ void add_prod(float a, float b) {
@@ -131,24 +131,33 @@ struct Sum2 {
         add(p, fmaf(a, b, -p));
     }
     __device__ __forceinline__ double value() const { return double(h) + double(l); }
+    // the quotient of two pairs, rounded to float: a first quotient and its remainder's correction
+    __device__ __forceinline__ float over(const Sum2& d) const {
+        const float q = __fdiv_rn(h, d.h);
+        const float rem = fmaf(-q, d.h, h) + (l - q * d.l);
+        const float c = q + __fdividef(rem, d.h);
+        return isfinite(c) ? c : q;  // a zero or non-finite divisor: what the plain division gives
+    }
 };
+__device__ __forceinline__ Sum2 sum2_of(double v) {
+    Sum2 p;
+    p.h = float(v);
+    p.l = float(v - double(p.h));
+    return p;
+}
+// over the first N lanes (a power of two); every lane gets the sum of its group of N
+template <int N = 32>
 __device__ __forceinline__ Sum2 warp_sum2(Sum2 v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = N / 2; o > 0; o >>= 1) {
         const float h = __shfl_xor_sync(0xffffffffu, v.h, o), l = __shfl_xor_sync(0xffffffffu, v.l, o);
         v.add(h, l);
     }
     return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float t = __shfl_xor_sync(0xffffffffu, v, o);
-        v = t > v ? t : v;
-    }
-    return v;
-}
-// the sum and the maximum (at least 0) of NTH threads with a linear thread id, in a fixed order; valid in tid 0
+// values >= 0 (their bits order as integers)
+__device__ __forceinline__ float warp_max(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
+// the sum and the maximum (values >= 0) of NTH threads with a linear thread id, in a fixed order; valid in tid 0
 template <int NTH>
 __device__ __forceinline__ void block_sum_max(Sum2& sum, float& mx, int tid) {
     __shared__ float2 ss[NTH / 32];
@@ -167,9 +176,9 @@ __device__ __forceinline__ void block_sum_max(Sum2& sum, float& mx, int tid) {
         if (tid < NTH / 32) {
             sum.h = ss[tid].x;
             sum.l = ss[tid].y;
-            mx = sx[tid] > 0.0f ? sx[tid] : 0.0f;
+            mx = sx[tid];
         }
-        sum = warp_sum2(sum);
+        sum = warp_sum2<NTH / 32>(sum);
         mx = warp_max(mx);
     }
 }
@@ -285,6 +294,7 @@ struct Env {
     // reductions
     Scalars* sc;
     double* partials;
+    void* grid_parts = nullptr;   // k_pcg_grid's reductions: every block's partial in every block's inbox
     Scalars* host_sc = nullptr;      // pinned mirror, written by fetch_scalars
     Scalars* host_sc_dev = nullptr;  // the mirror's device-side address (mapped pinned memory)
     // host clock (environmentGPU::m_time etc.)
@@ -307,6 +317,7 @@ struct Env {
     // whose results do not depend on their grid use it; the reductions keep num_sms, so a member's
     // bits are the same inside an ensemble and alone.
     int stencil_sms = 0;
+    int pcg_grid_cap[4] = {-1, -1, -1, -1};  // k_pcg_grid: blocks resident at once per cells-per-thread variant (-1: not asked yet)
     std::string err;
     int flat = 1;  // all gh == 0
     // graph mode: the step captured once per key, the loops as conditional WHILE nodes
@@ -391,6 +402,7 @@ void launch_buoyancy(Env& e, float dtS);
 void launch_init_density(Env& e);
 void launch_new_pressure(Env& e);
 void launch_project(Env& e, float dtS);
+size_t pcg_grid_bytes(const Env& e);  // storage of grid_parts for this grid (0: the PCG is not run in one launch)
 void launch_micro(Env& e, float dt, float speed);
 void launch_ground(Env& e, float dt, float speed, float irr);
 void launch_init_state(Env& e, int noise, uint32_t seed);

@@ -586,6 +586,263 @@ __global__ void k_pcg_cond(cudaGraphConditionalHandle h, Scalars* sc, int loop) 
     cudaGraphSetConditional(h, (sc->converged == 0 && sc->status == 0) ? 1u : 0u);
 }
 
+// ---- the whole PCG in one launch (grids whose solver state fits the chip) ---------------------
+// One cooperative launch of at most one 512-thread block per SM runs every iteration. A block owns
+// K*512 consecutive cells; thread t holds cells t, t+512, ...: r, the pressure, the diagonal and
+// the direction in registers, the six face coefficients (the lower ones truncated as Q3 wants, 0
+// where there is no neighbour) in shared memory. Only the direction's halo crosses blocks: as in
+// k_matvec_search4 every block forms s_new = z + beta s_old for itself and, outside its own cells,
+// from the neighbours' z and s_old in global memory (L2), so an iteration needs two grid-wide
+// reductions and no third barrier. Each reduction is its own barrier: a block publishes its partial
+// and arrives, waits until all have arrived, and sums all partials in the same order, so every
+// block holds the same step lengths and takes the same decisions.
+// What bounds it: the two exchanges of an iteration (2 to 3 us together, the second behind a fence for
+// the direction's halo) and the block's own loads and sums. Measured per iteration, before (two
+// launches, or three for 90x51x75) and now: 32^3 12.7 and 4.7 us, 64x32x64 14 and 6.9 us, 90x51x75
+// 27 and 8.7 us, 128x64x128 over hills 30 and 12.9 us.
+// The cells of a thread depend on the grid's size alone, so a member of an ensemble gets the bits
+// of the same grid alone. Every wait is bounded; one that runs out makes the block return and
+// SKT_TIMEOUT be recorded (the other blocks' waits then run out too).
+constexpr int GCT = 512;                      // threads per block
+constexpr int kGridCells[4] = {2, 4, 8, 14};  // cells per thread of the variants (14: 200 KB of shared memory)
+constexpr unsigned kGridSpinLimit = 1u << 21;
+constexpr int kMaxGridBlocks = 256;           // blocks of the launch at most
+template <int K>
+int pcg_grid_smem(int X) { return (7 * K * GCT + 2 * X) * 4; }
+
+// one block's partial of a reduction: its sum, its maximum and the reduction's tag, read and written as one
+// 16-byte access so that a reader that sees the tag has the values with it
+struct alignas(16) GridPart {
+    float h, l, mx;
+    unsigned tag;
+};
+__device__ __forceinline__ void put_part(GridPart* p, float h, float l, float mx, unsigned tag) {
+    asm volatile("{\n\t.reg .b64 lo, hi;\n\t.reg .b128 v;\n\tmov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 v, {lo, hi};\n\t"
+                 "st.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "f"(h), "f"(l), "f"(mx), "r"(tag) : "memory");
+}
+__device__ __forceinline__ GridPart get_part(const GridPart* p) {
+    GridPart r;
+    asm volatile("{\n\t.reg .b64 lo, hi;\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%4];\n\tmov.b128 {lo, hi}, v;\n\t"
+                 "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}" : "=f"(r.h), "=f"(r.l), "=f"(r.mx), "=r"(r.tag) : "l"(p) : "memory");
+    return r;
+}
+
+// (fence.acq_rel, not __threadfence, which is the sequentially consistent fence and slower)
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Reduces sum and maximum over the grid; a barrier too: every block writes its partial into every
+// block's inbox and waits for all partials in its own, one hop through L2 (1.5 us for 128 blocks,
+// 1.1 for 32; an arrival counter and then the partials 1.8 and 1.6, one block that sums for all 2.3
+// and 1.4, every block polling one set of partials 2.9 and 1.2). The partials are summed in the same
+// order everywhere, so every thread of the grid gets the same totals. FENCE: the block's stores
+// before the reduction are visible to every block after it. Inboxes alternate by the tag's parity: a
+// block may send the next partial while another still reads these, but not the one after that.
+// False when a wait ran out.
+template <bool FENCE>
+__device__ __forceinline__ bool grid_reduce(GridPart* inbox, int nb, unsigned tag, Sum2 sum, float mx, Sum2& tot, float& mall) {
+    __shared__ float2 ws[2][GCT / 32];
+    __shared__ float wm[2][GCT / 32];
+    __shared__ float4 ts[2][kMaxGridBlocks / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, par = tag & 1u, nw = (nb + 31) >> 5;
+    sum = warp_sum2(sum);
+    mx = warp_max(mx);
+    if (lane == 0) {
+        ws[par][warp] = make_float2(sum.h, sum.l);
+        wm[par][warp] = mx;
+    }
+    __syncthreads();
+    if (warp < nw) {
+        Sum2 s;
+        s.h = ws[par][lane & (GCT / 32 - 1)].x;
+        s.l = ws[par][lane & (GCT / 32 - 1)].y;
+        s = warp_sum2<GCT / 32>(s);
+        float m = warp_max(wm[par][lane & (GCT / 32 - 1)]);
+        if (FENCE) fence_gpu();
+        bool ok = true;
+        GridPart v{0.0f, 0.0f, 0.0f, tag};
+        if (tid < nb) {
+            put_part(inbox + (size_t(par) * nb + tid) * nb + blockIdx.x, s.h, s.l, m, tag);
+            const GridPart* const mine = inbox + (size_t(par) * nb + blockIdx.x) * nb + tid;
+            v = get_part(mine);
+            for (unsigned i = 0; v.tag != tag && ok; ++i) {
+                ok = i < kGridSpinLimit;
+                v = get_part(mine);
+            }
+        }
+        if (FENCE) fence_gpu();
+        s.h = v.h;
+        s.l = v.l;
+        s = warp_sum2(s);
+        m = warp_max(v.mx);
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) ts[par][warp] = make_float4(s.h, s.l, m, ok ? 1.0f : 0.0f);
+    }
+    __syncthreads();
+    tot = Sum2();
+    mall = 0.0f;
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i < nw; ++i) {
+        const float4 t = ts[par][i];
+        tot.add(t.x, t.y);
+        mall = t.z > mall ? t.z : mall;
+        ok = ok && t.w != 0.0f;
+    }
+    return ok;
+}
+
+template <int K>
+__global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __restrict__ ax, const float* __restrict__ ay,
+                                                     const float* __restrict__ az, const float* __restrict__ aw, float* __restrict__ rg,
+                                                     float* s_even, float* s_odd, float* zg, float* __restrict__ pg, int reference,
+                                                     float tol, int max_iter, Scalars* sc, GridPart* inbox) {
+    extern __shared__ float pcg_smem[];
+    constexpr int LEN = K * GCT;
+    float* const C = pcg_smem;  // the six face coefficients
+    float* const S = pcg_smem + 6 * LEN + g.X;  // the direction with a row's halo on either side; between the phases z
+    if (sc->converged) return;  // the setup found a zero residual
+    const int tid = threadIdx.x, nb = gridDim.x, X = g.X, XY = g.XY, N = g.N;
+    const int base = blockIdx.x * LEN;
+    unsigned tag = sc->grid_tag;
+    float r[K], p[K], w[K], s[K];  // (14 cells: some spill; the pressure in global memory instead was slower, 13.8 against 12.9 us)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int l = tid + k * GCT, i = base + l;
+        float cl = 0.0f, cr = 0.0f, cd = 0.0f, cu = 0.0f, cb = 0.0f, cf = 0.0f;
+        r[k] = p[k] = w[k] = s[k] = 0.0f;
+        if (i < N) {
+            const int z = i / XY, xy = i - z * XY, y = xy / X, x = xy - y * X;
+            if (x > 0) cl = ax[i - 1];
+            if (x + 1 < X) cr = ax[i];
+            if (y > 0) cd = ay[i - X];
+            if (y + 1 < g.Y) cu = ay[i];
+            if (z > 0) cb = az[i - XY];
+            if (z + 1 < g.Z) cf = az[i];
+            if (reference) { cl = char_trunc(cl); cd = char_trunc(cd); cb = char_trunc(cb); }
+            r[k] = rg[i];
+            w[k] = aw[i];
+            s[k] = s_even[i];
+        }
+        C[l] = cl; C[LEN + l] = cr; C[2 * LEN + l] = cd; C[3 * LEN + l] = cu; C[4 * LEN + l] = cb; C[5 * LEN + l] = cf;
+    }
+    // the solver's scalars, the same in every thread; the dot products of the last iteration in shared
+    // memory (thread 0 stores them where no thread reads before the next reduction's barrier)
+    __shared__ Sum2 sigma0[2];
+    if (tid == 0) sigma0[0] = sum2_of(sc->sigma0);
+    Sum2 sigma1 = sum2_of(sc->sigma1);
+    float residual = sc->residual;
+    int done = 0, status = 0;
+    float alpha = 0.0f, beta = 0.0f;
+    int iters = 0;
+    bool ok = true;
+    const bool whole = base + LEN <= N, inner = base >= XY && base + LEN + XY <= N;
+    for (;;) {
+        // the first direction is the setup's z itself: z + 0 times itself
+        float* const snew = (iters & 1) ? s_odd : s_even;
+        const float* const sold = iters == 0 ? s_even : ((iters & 1) ? s_even : s_odd);
+        const float* const zold = iters == 0 ? s_even : zg;
+        // outside the block's cells the direction is formed from global memory: the planes before and
+        // behind for every cell (no test whether one lies inside), the rows above and below and the x
+        // neighbours from the halo. A neighbour that does not exist has coefficient 0: its index is
+        // clamped into the grid, which only the blocks at the grid's ends have to do.
+        auto form = [&](int j) { return __fmaf_rn(beta, __ldcg(sold + j), __ldcg(zold + j)); };
+        auto clamped = [&](int j) { return min(max(j, 0), N - 1); };
+        float sb[K], sf[K];
+        if (inner) {
+            const float *so = sold + base + tid, *zo = zold + base + tid;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                sb[k] = __fmaf_rn(beta, __ldcg(so - XY + k * GCT), __ldcg(zo - XY + k * GCT));
+                sf[k] = __fmaf_rn(beta, __ldcg(so + XY + k * GCT), __ldcg(zo + XY + k * GCT));
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                sb[k] = form(clamped(base + tid + k * GCT - XY));
+                sf[k] = form(clamped(base + tid + k * GCT + XY));
+            }
+        }
+        for (int h = tid; h < 2 * X; h += GCT) {
+            const int l = h < X ? h - X : LEN + h - X;
+            S[l] = form(clamped(base + l));
+        }
+        float* const sn = snew + base + tid;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int l = tid + k * GCT;
+            if (iters > 0) {
+                s[k] = __fmaf_rn(beta, s[k], S[l]);
+                if (whole || base + l < N) __stcg(sn + k * GCT, s[k]);
+            }
+            S[l] = s[k];
+        }
+        __syncthreads();
+        float As[K];
+        Kahan acc;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int l = tid + k * GCT;
+            const float o = w[k] * s[k] + ((C[l] * S[l - 1] + C[2 * LEN + l] * S[l - X] + C[4 * LEN + l] * sb[k] + C[LEN + l] * S[l + 1] +
+                                            C[3 * LEN + l] * S[l + X] + C[5 * LEN + l] * sf[k]));
+            As[k] = o;
+            acc.add(o * s[k]);
+        }
+        // (no fence: the next reads of another block's stores come after the second reduction)
+        Sum2 tot;
+        float mall;
+        ok = grid_reduce<false>(inbox, nb, ++tag, acc.pair(), 0.0f, tot, mall);
+        if (!ok) break;
+        if (!isfinite(tot.h)) { status = SKT_NAN_DETECTED; break; }
+        if (reference) tot.add(sigma1.h, sigma1.l);  // Q1
+        sigma1 = tot;
+        alpha = sigma0[iters & 1].over(sigma1);
+        Kahan zr;
+        float mx = 0.0f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int l = tid + k * GCT, i = base + l;
+            p[k] = __fmaf_rn(alpha, s[k], p[k]);
+            r[k] = r[k] - alpha * As[k];
+            const float z = r[k] * precon_of(w[k]);
+            S[l] = z;  // every read of the direction lies before the reduction's barrier
+            if (whole || i < N) __stcg(zg + base + tid + k * GCT, z);
+            zr.add(z * r[k]);
+            const float m = (!reference || i < XY) ? fabsf(r[k]) : r[k];  // Q4
+            if (m > mx) mx = m;
+        }
+        ok = grid_reduce<true>(inbox, nb, ++tag, zr.pair(), mx, tot, mall);
+        if (!ok) break;
+        beta = tot.over(sigma0[iters & 1]);
+        ++iters;
+        residual = mall;
+        if (!isfinite(tot.h)) { status = SKT_NAN_DETECTED; break; }
+        if (mall <= tol) { done = 1; break; }
+        if (iters >= max_iter) { done = 2; break; }
+        if (tid == 0) sigma0[iters & 1] = tot;
+        sigma1 = tot;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = base + tid + k * GCT;
+        if (i < N) {
+            rg[i] = r[k];
+            pg[i] = p[k];
+        }
+    }
+    if (tid == 0) {
+        if (!ok) sc->status = SKT_TIMEOUT;
+        if (blockIdx.x == 0) {
+            if (status) sc->status = status;
+            sc->alpha = alpha;
+            sc->beta_f = beta;
+            sc->residual = residual;
+            sc->iters = iters;
+            sc->converged = done;
+            sc->grid_tag = tag;
+        }
+    }
+}
+
 // k_build for flat terrain and X % 4 == 0: four cells per thread, a march along z in blocks of
 // MVY rows. Each cell's reciprocal density is formed once (the x neighbours' by shuffle, the next
 // plane's carried), and each face once: a cell forms its right, up and front faces; the left face
@@ -833,6 +1090,72 @@ __global__ void __launch_bounds__(256) k_apply_proj4(Grid g, int zlen, const flo
 
 }  // namespace
 
+namespace {
+
+template <int K>
+bool launch_pcg_grid(Env& e, int slot, int nb) {
+    const int smem = pcg_grid_smem<K>(e.g.X);
+    if (e.pcg_grid_cap[slot] < 0) {
+        // the limit set on the kernel is the device's, not this grid's need: other environments launch it too
+        int coop = 0, most = 0, per_sm = 0;
+        cudaFuncAttributes fa{};
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e.device);
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, e.device);
+        if (!coop || cudaFuncGetAttributes(&fa, k_pcg_grid<K>) != cudaSuccess || smem + int(fa.sharedSizeBytes) > most ||
+            cudaFuncSetAttribute(k_pcg_grid<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(fa.sharedSizeBytes)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid<K>, GCT, smem) != cudaSuccess) {
+            cudaGetLastError();
+            per_sm = 0;
+        }
+        e.pcg_grid_cap[slot] = per_sm * e.num_sms;
+    }
+    if (nb > e.pcg_grid_cap[slot]) return false;
+    int reference = e.cfg.semantics == 0;
+    void* args[] = {&e.g, &e.ax, &e.ay, &e.az, &e.aw, &e.r, &e.s, &e.tB, &e.tA, &e.pp, &reference, &e.cfg.pcg_tol, &e.cfg.pcg_max_iter,
+                    &e.sc, &e.grid_parts};
+    // an error is the step's to report (its check finds it)
+    (void)cudaLaunchCooperativeKernel((const void*)k_pcg_grid<K>, dim3(nb), dim3(GCT), args, smem, e.stream);
+    e.launches += 1;
+    return true;
+}
+
+// The launch shape for a grid: the variant with the fewest cells per thread that needs at most 96
+// blocks (the reductions' exchange grows with the blocks: 64x32x64 took 7.5 us an iteration as 128
+// blocks of 2 cells a thread, 7.0 as 64 of 4 and 7.6 as 32 of 8), else the fewest whose blocks fit
+// one per SM (1.09M cells on 152 SMs); nb = 0 above that, where the solver state does not fit the
+// SMs' registers and shared memory and two streaming launches per iteration are used instead.
+void pcg_grid_shape(const Env& e, int& slot, int& nb) {
+    for (const int most : {std::min(96, e.num_sms), std::min(e.num_sms, kMaxGridBlocks)})
+        for (slot = 0; slot < 4; ++slot) {
+            const int per = kGridCells[slot] * GCT;
+            nb = (e.g.N + per - 1) / per;
+            if (nb <= most) return;
+        }
+    nb = 0;
+}
+
+// The PCG in one cooperative launch; false: not taken. pcg_fused = 0 keeps its three launches per iteration.
+bool pcg_in_one_launch(Env& e) {
+    int slot, nb;
+    pcg_grid_shape(e, slot, nb);
+    if (nb == 0 || !e.cfg.pcg_fused || e.cfg.pcg_max_iter <= 0) return false;
+    ProfScope ps(e, "pcg_grid");
+    switch (slot) {
+        case 0: return launch_pcg_grid<2>(e, slot, nb);
+        case 1: return launch_pcg_grid<4>(e, slot, nb);
+        case 2: return launch_pcg_grid<8>(e, slot, nb);
+        default: return launch_pcg_grid<14>(e, slot, nb);
+    }
+}
+
+}  // namespace
+
+size_t pcg_grid_bytes(const Env& e) {
+    int slot, nb;
+    pcg_grid_shape(e, slot, nb);
+    return e.cfg.precision == 1 ? 0 : sizeof(GridPart) * 2 * size_t(nb) * nb;
+}
+
 // As = A s and s.As -> alpha (textbook operator, vectorised; X % 4 == 0)
 void launch_matvec_textbook(Env& e, const float* s, float* As) {
     const Grid& g = e.g;
@@ -873,6 +1196,13 @@ void launch_project(Env& e, float dtS) {
     }
     if (e.cfg.precision == 1) {
         mg_solve(e);
+    } else if (pcg_in_one_launch(e)) {
+        if (!e.capturing) {
+            fetch_scalars(e);
+            e.last_iters = e.host_sc->iters;
+            e.last_residual = e.host_sc->residual;
+            e.last_converged = e.host_sc->converged == 1;
+        }
     } else {
     const int chunk = 8;
     const bool vec = (g.X % 4) == 0;
