@@ -101,40 +101,38 @@ float* column_ptr(Env& e, int which) {
 // ground kernel takes irr, or in graph mode reads it from the graph's first node.
 void queue_step(Env& e, float dt, float speed, float irr) {
     const float dtS = dt * speed;
-    const bool hs = true;
     // ground, then setTempsAtGround (fused into the ground column kernel)
     launch_ground(e, dt, speed, irr);
     // theta
     launch_diffuse(e, e.th, 0, dtS);
-    e.last_nsub[0] = launch_advect(e, e.th, e.isenT, CUSTOM, CUSTOM, dtS, 0, hs);
+    e.last_nsub[0] = launch_advect(e, e.th, e.isenT, CUSTOM, CUSTOM, dtS, 0);
     // momentum
     launch_buoyancy(e, dtS);
-    launch_diffuse(e, e.u, 2, dtS);
-    launch_diffuse(e, e.v, 3, dtS);
-    launch_diffuse(e, e.w, 4, dtS);
-    e.last_nsub[1] = launch_advect(e, e.u, e.defU, CUSTOM, DIRICHLET, dtS, 1, hs);
-    e.last_nsub[2] = launch_advect(e, e.v, e.zeroY, DIRICHLET, DIRICHLET, dtS, 2, hs);
-    e.last_nsub[3] = launch_advect(e, e.w, e.defW, CUSTOM, DIRICHLET, dtS, 3, hs);
+    {
+        float* const f[3] = {e.u, e.v, e.w};
+        const int type[3] = {2, 3, 4};
+        launch_diffuse_many(e, 3, f, type, dtS);
+    }
+    e.last_nsub[1] = launch_advect(e, e.u, e.defU, CUSTOM, DIRICHLET, dtS, 1);
+    e.last_nsub[2] = launch_advect(e, e.v, e.zeroY, DIRICHLET, DIRICHLET, dtS, 2);
+    e.last_nsub[3] = launch_advect(e, e.w, e.defW, CUSTOM, DIRICHLET, dtS, 3);
     launch_init_density(e);
     launch_project(e, dtS);
     launch_new_pressure(e);
-    // moisture
-    launch_diffuse(e, e.qv, 1, dtS);
-    e.last_nsub[4] = launch_advect(e, e.qv, e.isenQv, CUSTOM, CUSTOM, dtS, 4, hs);
-    // the wind is the same for every moisture field: its substep count is computed once
-    launch_diffuse(e, e.qw, 5, dtS);
-    e.last_nsub[5] = launch_advect(e, e.qw, e.zeroY, DIRICHLET, DIRICHLET, dtS, 5, hs, true);
-    launch_diffuse(e, e.qc, 5, dtS);
-    e.last_nsub[6] = launch_advect(e, e.qc, e.zeroY, DIRICHLET, DIRICHLET, dtS, 6, hs, true);
-    // rain, snow and ice: diffuse, fall, advect each (the reference's order per species; the
-    // species do not read one another here, so the three falls run as one column march)
-    launch_diffuse(e, e.qr, 5, dtS);
-    launch_diffuse(e, e.qs, 5, dtS);
-    launch_diffuse(e, e.qi, 5, dtS);
-    launch_precip3(e, dtS);
-    e.last_nsub[7] = launch_advect(e, e.qr, e.zeroY, DIRICHLET, DIRICHLET, dtS, 7, hs, true);
-    e.last_nsub[8] = launch_advect(e, e.qs, e.zeroY, DIRICHLET, DIRICHLET, dtS, 8, hs, true);
-    e.last_nsub[9] = launch_advect(e, e.qi, e.zeroY, DIRICHLET, DIRICHLET, dtS, 9, hs, true);
+    // moisture: a field's diffusion and advection read the wind and the field alone, so the six
+    // diffuse together, then vapour, water and ice crystals are carried together, and rain, snow and
+    // ice after their fall (which reads the carried vapour); the falls run as one column march
+    {
+        float* const f[6] = {e.qv, e.qw, e.qc, e.qr, e.qs, e.qi};
+        const int type[6] = {1, 5, 5, 5, 5, 5};
+        const float* const def[6] = {e.isenQv, e.zeroY, e.zeroY, e.zeroY, e.zeroY, e.zeroY};
+        const int bc[6] = {CUSTOM, DIRICHLET, DIRICHLET, DIRICHLET, DIRICHLET, DIRICHLET};
+        launch_diffuse_many(e, 6, f, type, dtS);
+        // the wind is the same for every moisture field: its substep count is computed once
+        e.last_nsub[4] = e.last_nsub[5] = e.last_nsub[6] = launch_advect_many(e, 3, f, def, bc, bc, dtS, 4, false);
+        launch_precip3(e, dtS);
+        e.last_nsub[7] = e.last_nsub[8] = e.last_nsub[9] = launch_advect_many(e, 3, f + 3, def + 3, bc + 3, bc + 3, dtS, 7, true);
+    }
     // microphysics + latent heat
     launch_micro(e, dt, speed);
 }
@@ -1214,7 +1212,7 @@ skt_status skt_run_stage(skt_env* env, int stage, int arg, float dt, float speed
             const float* df[6] = {e.isenT, e.defU, e.zeroY, e.defW, e.isenQv, e.zeroY};
             const int sd[6] = {CUSTOM, CUSTOM, DIRICHLET, CUSTOM, CUSTOM, DIRICHLET};
             const int gd[6] = {CUSTOM, DIRICHLET, DIRICHLET, DIRICHLET, CUSTOM, DIRICHLET};
-            e.last_nsub[0] = launch_advect(e, f[arg], df[arg], sd[arg], gd[arg], dt, 0, true);
+            e.last_nsub[0] = launch_advect(e, f[arg], df[arg], sd[arg], gd[arg], dt, 0);
             break;
         }
         case 2: launch_buoyancy(e, dt); break;

@@ -394,8 +394,10 @@ struct ProfScope {
 
 // ---- launchers (defined in the kernel translation units) --------------------------------------
 void launch_diffuse(Env& e, float* f, int type, float dtS);
-int launch_advect(Env& e, float* f, const float* def, int sides, int ground, float dtS, int field_slot, bool host_sync,
-                  bool same_wind = false);
+void launch_diffuse_many(Env& e, int n, float* const* f, const int* type, float dtS);  // n fields, a launch per pass
+int launch_advect(Env& e, float* f, const float* def, int sides, int ground, float dtS, int field_slot, bool same_wind = false);
+int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, const int* sides, const int* ground, float dtS,
+                       int field_slot, bool same_wind);
 void launch_precip(Env& e, float* q, int type, float dtS);
 void launch_precip3(Env& e, float dtS);  // rain, snow and ice in one column march
 void launch_buoyancy(Env& e, float dtS);

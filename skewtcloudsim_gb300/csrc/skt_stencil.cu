@@ -14,7 +14,28 @@ namespace {
 
 constexpr int BX = 32, BY = 8;
 
-inline dim3 cell_grid(const Grid& g) { return dim3((g.X + BX - 1) / BX, (g.Y + BY - 1) / BY, g.Z); }
+inline dim3 cell_grid(const Grid& g, int fields = 1) { return dim3((g.X + BX - 1) / BX, (g.Y + BY - 1) / BY, g.Z * fields); }
+
+// One pass of a sweeping or advecting kernel over several fields at once: the fields of a launch
+// share the grid, the wind and the step, and each has its own arrays and boundary conditions. The
+// blocks of field f follow those of field f-1 along blockIdx.z. One field of a small grid does not
+// fill the GPU, and its launches cost more than its bytes: with u, v, w and the six moisture fields
+// together a step makes 60 sweeping launches instead of 200 and 32 advecting ones instead of 50: 2.13
+// to 1.40 ms at 32^3, 3.49 to 2.56 at 90x51x75, 12.9 to 12.8 for an ensemble of eight; at 512x256x512
+// both ways take the same.
+constexpr int kBatch = 6;
+struct FieldSet {
+    int n = 0;
+    const float* in[kBatch];
+    float* out[kBatch];
+    const float* def[kBatch];
+    int sides[kBatch], ground[kBatch];
+    // the field of this block, per being the blocks of one field along z. Kernels come in two forms: with
+    // one field its arrays are fixed places of the launch's arguments, and the passes of a single field
+    // stay as fast as they were (the division and the indexed arguments cost them 1 to 3 %)
+    template <bool MANY>
+    __device__ __forceinline__ int field_of(int per) const { return MANY ? int(blockIdx.z) / per : 0; }
+};
 
 // theta at a ground face seen from cell idx: potentialTempGPU(Tg-273.15, p_cell, Pg)+273.15
 // (Game/kernelSky.cu:95-100)
@@ -32,11 +53,15 @@ __device__ __forceinline__ float jacobi(float c, float l, float r, float u, floa
 
 // One Jacobi sweep of the colour-split diffusion (diffuseRedBlack Game/kernelSky.cu:43-115; both
 // colours read the same input array, Game/environment.cu:651-662).
-template <bool THETA>
-__global__ void __launch_bounds__(256) k_diffuse(Grid g, const float* __restrict__ in, float* __restrict__ out, int sides, int ground,
-                                                 const float* __restrict__ def, float k, const float* __restrict__ p,
-                                                 const float* __restrict__ Tg, const float* __restrict__ Pg) {
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
+template <bool THETA, bool MANY>
+__global__ void __launch_bounds__(256) k_diffuse(Grid g, FieldSet F, float k, const float* __restrict__ p, const float* __restrict__ Tg,
+                                                 const float* __restrict__ Pg) {
+    const int fi = F.field_of<MANY>(g.Z);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi], ground = F.ground[fi];
+    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z - fi * g.Z;
     if (x >= g.X || y >= g.Y) return;
     if (is_ground(g, x, y, z)) return;
     const int c = cidx(g, x, y, z);
@@ -89,14 +114,17 @@ __global__ void __launch_bounds__(256) k_theta_face(Grid g, const float* __restr
 }
 
 // face: theta's ground-face values per column (k_theta_face), read at the first sky row
-template <bool THETA>
-__global__ void __launch_bounds__(32 * DVY) k_diffuse4(Grid g, int zlen, const float* __restrict__ in, float* __restrict__ out, int sides,
-                                                       int ground, const float* __restrict__ def, float k,
-                                                       const float* __restrict__ face) {
+template <bool THETA, bool MANY>
+__global__ void __launch_bounds__(32 * DVY) k_diffuse4(Grid g, int zlen, int zc, FieldSet F, float k, const float* __restrict__ face) {
+    const int fi = F.field_of<MANY>(zc);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi], ground = F.ground[fi];
     const int lane = threadIdx.x;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
     const int y = blockIdx.y * DVY + threadIdx.y + 1;  // sky rows start at y = 1
-    const int zs = blockIdx.z * zlen, ze = min(zs + zlen, g.Z);
+    const int zs = (blockIdx.z - fi * zc) * zlen, ze = min(zs + zlen, g.Z);
     const bool act = x0 < g.X && y < g.Y;
     const int X = g.X, XY = g.XY;
     const int row = x0 + y * X;
@@ -429,10 +457,18 @@ __device__ __forceinline__ float4 jacobi4(float4 c, float l, float r, float4 u, 
                        jacobi(c.z, c.y, c.w, u.z, d.z, f.z, b.z, k, rinv), jacobi(c.w, c.z, r, u.w, d.w, f.w, b.w, k, rinv));
 }
 
-template <bool THETA, int R>
+struct FieldMaps {
+    CUtensorMap in[kBatch];
+};
+template <bool THETA, bool MANY, int R>
 __global__ void __launch_bounds__(32 * (R + 3), p4_min_blocks<R>())
-    k_diffuse_pair4(const __grid_constant__ CUtensorMap tin, Grid g, int zlen, float* __restrict__ out, int sides, int ground,
-                    const float* __restrict__ def, float k, const float* __restrict__ face, Scalars* __restrict__ sc) {
+    k_diffuse_pair4(const __grid_constant__ FieldMaps maps, Grid g, int zlen, int zc, FieldSet F, float k, const float* __restrict__ face,
+                    Scalars* __restrict__ sc) {
+    const int fi = F.field_of<MANY>(zc);
+    const CUtensorMap& tin = maps.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi], ground = F.ground[fi];
     extern __shared__ __align__(128) unsigned char p4_smem[];
     constexpr int NR = R + 2;
     constexpr int SLOTF = p4_slot_bytes<R>() / 4;  // floats per slot
@@ -443,7 +479,7 @@ __global__ void __launch_bounds__(32 * (R + 3), p4_min_blocks<R>())
     const int tid = threadIdx.x, lane = tid & 31, wy = tid >> 5;  // a 1D block: the warp index is warp-uniform
     const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY;
     const int bx = int(blockIdx.x) * 128, yb = 1 + int(blockIdx.y) * R;
-    const int zs = int(blockIdx.z) * zlen, ze = min(zs + zlen, Z);
+    const int zs = (int(blockIdx.z) - fi * zc) * zlen, ze = min(zs + zlen, Z);
     const int plo = max(zs - 1, 0), phi = min(ze, Z - 1);       // planes of the first sweep
     const int ilo = max(plo - 1, 0), ihi = min(phi + 1, Z - 1);  // input planes
     const float rinv = 1.0f / (1 + 6 * k);
@@ -687,11 +723,15 @@ __device__ __forceinline__ float ghost_one(const Grid& g, int x, int y, int z, i
 // One directional PPM pass (advectPPMX/Y/Z Game/kernelSky.cu:368-574) of q and of the density
 // companion (advected ones), followed by q/rho* (divideValues Game/kernelMaths.cu:38).
 // The velocity array is read as it stands when the pass starts.
-template <int AXIS>
-__global__ void __launch_bounds__(256) k_ppm(Grid g, const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ vel,
-                                             const float* __restrict__ def, int sides, int ground, const float* __restrict__ defU,
+template <int AXIS, bool MANY>
+__global__ void __launch_bounds__(256) k_ppm(Grid g, FieldSet F, const float* __restrict__ vel, const float* __restrict__ defU,
                                              const float* __restrict__ defW, float dtFull, int nsub_host, int half,
                                              const Scalars* __restrict__ sc, int slot) {
+    const int fi = F.field_of<MANY>(g.Z);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi], ground = F.ground[fi];
     int nsub = nsub_host;
     if (sc) {
         nsub = sc->nsub;
@@ -700,7 +740,7 @@ __global__ void __launch_bounds__(256) k_ppm(Grid g, const float* __restrict__ i
     const float dtSub = dtFull / float(nsub);
     const float dt = half ? dtSub * 0.5f : dtSub;
     const float cdt = dt / g.vox;
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
+    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z - fi * g.Z;
     if (x >= g.X || y >= g.Y) return;
     if (is_ground(g, x, y, z)) return;
     constexpr int ax = AXIS == 0, ay = AXIS == 1, az = AXIS == 2;
@@ -738,10 +778,15 @@ __device__ __forceinline__ float ppm_cdt(const Grid& g, float dtFull, int nsub, 
 // previous warp's cells: its flux (and q(x0-1)) is computed for 32 planes at once, one plane per
 // lane, and handed to lane 0 plane by plane, so the warp does not spend a whole flux evaluation
 // per plane on one lane.
-__global__ void __launch_bounds__(32 * DVY, 32 / DVY) k_ppm4x(Grid g, int zlen, const float* __restrict__ in, float* __restrict__ out,
-                                                    const float* __restrict__ vel, const float* __restrict__ def, int sides,
-                                                    const float* __restrict__ defU, float dtFull, int nsub_host, int half,
-                                                    const Scalars* __restrict__ sc, int slot) {
+template <bool MANY>
+__global__ void __launch_bounds__(32 * DVY, 32 / DVY) k_ppm4x(Grid g, int zlen, int zc, FieldSet F, const float* __restrict__ vel,
+                                                                   const float* __restrict__ defU, float dtFull, int nsub_host,
+                                                                   int half, const Scalars* __restrict__ sc, int slot) {
+    const int fi = F.field_of<MANY>(zc);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi];
     int nsub = nsub_host;
     if (sc) {
         nsub = sc->nsub;
@@ -752,7 +797,7 @@ __global__ void __launch_bounds__(32 * DVY, 32 / DVY) k_ppm4x(Grid g, int zlen, 
     const int xw = blockIdx.x * 128;  // the warp's first cell
     const int x0 = xw + lane * 4;
     const int y = blockIdx.y * DVY + threadIdx.y + 1;
-    const int zs = blockIdx.z * zlen, ze = min(zs + zlen, g.Z);
+    const int zs = (blockIdx.z - fi * zc) * zlen, ze = min(zs + zlen, g.Z);
     const bool wact = xw < g.X && y < g.Y;  // same for every lane of the warp
     const bool act = x0 < g.X && y < g.Y;
     const int X = g.X, XY = g.XY;
@@ -853,9 +898,14 @@ __global__ void __launch_bounds__(32 * DVY, 32 / DVY) k_ppm4x(Grid g, int zlen, 
 // keeping the window q(y-2) .. q(y+2) in registers and handing each upper-face flux on as the next
 // row's lower-face flux. Rows <= 0 are the ground ghost, rows >= Y the side ghost of the top row.
 constexpr int PY = 4;
-__global__ void __launch_bounds__(32 * PY) k_ppm4y(Grid g, int ylen, const float* __restrict__ in, float* __restrict__ out,
-                                                   const float* __restrict__ vel, const float* __restrict__ def, int sides, int ground,
-                                                   float dtFull, int nsub_host, int half, const Scalars* __restrict__ sc, int slot) {
+template <bool MANY>
+__global__ void __launch_bounds__(32 * PY) k_ppm4y(Grid g, int ylen, int yc, FieldSet F, const float* __restrict__ vel, float dtFull,
+                                                   int nsub_host, int half, const Scalars* __restrict__ sc, int slot) {
+    const int fi = F.field_of<MANY>(yc);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi], ground = F.ground[fi];
     int nsub = nsub_host;
     if (sc) {
         nsub = sc->nsub;
@@ -865,7 +915,7 @@ __global__ void __launch_bounds__(32 * PY) k_ppm4y(Grid g, int ylen, const float
     const int lane = threadIdx.x;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
     const int z = blockIdx.y * PY + threadIdx.y;
-    const int ys = 1 + blockIdx.z * ylen, ye = min(ys + ylen, g.Y);
+    const int ys = 1 + (blockIdx.z - fi * yc) * ylen, ye = min(ys + ylen, g.Y);
     if (x0 >= g.X || z >= g.Z || ys >= g.Y) return;
     const int X = g.X, Y = g.Y;
     const int base = x0 + z * g.XY;
@@ -915,10 +965,14 @@ __global__ void __launch_bounds__(32 * PY) k_ppm4y(Grid g, int ylen, const float
 // Vectorised Z pass: the z march keeps the window q(z-2) .. q(z+2) and hands each upper-face
 // flux on as the next plane's lower-face flux (computed directly at the first plane of a run; at
 // z = 0 the face velocity is the boundary value).
-__global__ void __launch_bounds__(32 * DVY) k_ppm4z(Grid g, int zlen, const float* __restrict__ in, float* __restrict__ out,
-                                                    const float* __restrict__ vel, const float* __restrict__ def, int sides,
-                                                    const float* __restrict__ defW, float dtFull, int nsub_host, int half,
-                                                    const Scalars* __restrict__ sc, int slot) {
+template <bool MANY>
+__global__ void __launch_bounds__(32 * DVY) k_ppm4z(Grid g, int zlen, int zc, FieldSet F, const float* __restrict__ vel, const float* __restrict__ defW,
+                                                    float dtFull, int nsub_host, int half, const Scalars* __restrict__ sc, int slot) {
+    const int fi = F.field_of<MANY>(zc);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi];
     int nsub = nsub_host;
     if (sc) {
         nsub = sc->nsub;
@@ -928,7 +982,7 @@ __global__ void __launch_bounds__(32 * DVY) k_ppm4z(Grid g, int zlen, const floa
     const int lane = threadIdx.x;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
     const int y = blockIdx.y * DVY + threadIdx.y + 1;
-    const int zs = blockIdx.z * zlen, ze = min(zs + zlen, g.Z);
+    const int zs = (blockIdx.z - fi * zc) * zlen, ze = min(zs + zlen, g.Z);
     if (x0 >= g.X || y >= g.Y) return;
     const int X = g.X, XY = g.XY, Z = g.Z;
     const int row = x0 + y * X;
@@ -1424,9 +1478,6 @@ __global__ void __launch_bounds__(256) k_new_pressure(Grid g, float* __restrict_
 
 namespace {
 
-// Flat terrain, X % 4 == 0: the sweeps alternate between the scratch fields and the last one
-// writes f itself, so no copy is needed (no sweep reads the array it writes, and the ground rows
-// of the scratch fields are never read). A single sweep goes through a scratch field.
 // z chunking of a march over gx x gy columns of blocks: about bps blocks per SM in the grid
 inline int z_runs(const Env& e, int gx, int gy, int bps, int& zlen) {
     int zc = std::max(1, std::min(e.g.Z, (stencil_sms(e) * bps + gx * gy - 1) / (gx * gy)));
@@ -1482,138 +1533,188 @@ bool launch_diffuse2(Env& e, int bps, const float* src, float* dst, int sides, i
 }
 
 template <bool THETA, int R>
-bool launch_diffuse_pair4(Env& e, int bps, const float* src, float* dst, int sides, int ground, const float* def, float k,
-                          const float* face) {
+bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const float* face) {
     const Grid& g = e.g;
-    CUtensorMap map;
-    if (!field_tensor_map(g, src, P4W, R + 4, &map)) return false;
+    FieldMaps maps;
+    for (int i = 0; i < F.n; ++i)
+        if (!field_tensor_map(g, F.in[i], P4W, R + 4, &maps.in[i])) return false;
     const int gx = (g.X + 127) / 128, gy = (g.Y - 1 + R - 1) / R;
     int zlen;
-    const int zc = z_runs(e, gx, gy, bps, zlen);
+    const int zc = z_runs(e, gx, gy * F.n, bps, zlen);
     constexpr int smem = p4_smem_bytes<R>();
     static bool attr = false;  // per template instance
     if (!attr) {
-        cudaFuncSetAttribute(k_diffuse_pair4<THETA, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_diffuse_pair4<THETA, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_diffuse_pair4<THETA, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         attr = true;
     }
-    k_diffuse_pair4<THETA, R><<<dim3(gx, gy, zc), 32 * (R + 3), smem, e.stream>>>(map, g, zlen, dst, sides, ground, def, k, face,
-                                                                                    e.sc);
+    const auto kernel = F.n == 1 ? k_diffuse_pair4<THETA, false, R> : k_diffuse_pair4<THETA, true, R>;
+    kernel<<<dim3(gx, gy, zc * F.n), 32 * (R + 3), smem, e.stream>>>(maps, g, zlen, zc, F, k, face, e.sc);
+    e.launches += 1;
     return true;
 }
 
 // one pass of two sweeps with the tuned kernel: k_diffuse_pair4 (float4 lanes, rows 6 or 14 per
-// block) or k_diffuse2 (one cell per lane, rows 4 or 8 per warp); false without a tensor map
+// block) or k_diffuse2 (one cell per lane, rows 4 or 8 per warp, field by field); false without a
+// tensor map
 template <bool THETA>
-bool launch_pair(Env& e, const float* src, float* dst, int sides, int ground, const float* def, float k, const float* face) {
+bool launch_pair(Env& e, const FieldSet& F, float k, const float* face) {
     const int h = e.tune.diffuse_h, bps = e.tune.diffuse2_bps;
-    switch (h) {
-        case 14: return launch_diffuse_pair4<THETA, 14>(e, bps, src, dst, sides, ground, def, k, face);
-        case 6: return launch_diffuse_pair4<THETA, 6>(e, bps, src, dst, sides, ground, def, k, face);
-        case 8: return launch_diffuse2<THETA, 8>(e, bps, src, dst, sides, ground, def, k, face);
-        default: return launch_diffuse2<THETA, 4>(e, bps, src, dst, sides, ground, def, k, face);
+    if (h == 14) return launch_diffuse_pair4<THETA, 14>(e, bps, F, k, face);
+    if (h == 6) return launch_diffuse_pair4<THETA, 6>(e, bps, F, k, face);
+    for (int i = 0; i < F.n; ++i) {
+        const bool ok = h == 8 ? launch_diffuse2<THETA, 8>(e, bps, F.in[i], F.out[i], F.sides[i], F.ground[i], F.def[i], k, face)
+                               : launch_diffuse2<THETA, 4>(e, bps, F.in[i], F.out[i], F.sides[i], F.ground[i], F.def[i], k, face);
+        if (!ok) return false;
+        e.launches += 1;
+    }
+    return true;
+}
+
+// Fields free between the stages (the advection's scratch, the solvers' vectors and coefficients):
+// what a batch of fields sweeps and advects through. (pp is not among them: it is read as the
+// projection's correction.)
+constexpr int kScratch = 13;
+float* scratch_field(const Env& e, int i) {
+    float* const xd = reinterpret_cast<float*>(e.xd);
+    float* const rd = reinterpret_cast<float*>(e.rd);
+    float* const all[kScratch] = {e.tA, e.tB, e.r, e.s, e.As, e.ax, e.ay, e.az, e.aw, xd, xd + size_t(e.g.N), rd, rd + size_t(e.g.N)};
+    return all[i];
+}
+
+// Flat terrain, X % 4 == 0: the vectorised kernels
+inline bool vec_grid(const Env& e) { return e.flat && (e.g.X % 4) == 0; }
+
+// copy the sky cells of every field's `in` to its `out`
+void copy_sky(Env& e, const FieldSet& F, const Scalars* chk, int slot) {
+    const Grid& g = e.g;
+    for (int i = 0; i < F.n; ++i) {
+        if (vec_grid(e)) {
+            const int n4 = g.N / 4;
+            k_copy_sky4<<<std::min((n4 + 255) / 256, stencil_sms(e) * 8), 256, 0, e.stream>>>(n4, g.X / 4, g.Y, (const float4*)F.in[i],
+                                                                                         (float4*)F.out[i], chk, slot);
+        } else {
+            k_copy_sky<<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, F.in[i], F.out[i], chk, slot);
+        }
+        e.launches += 1;
     }
 }
 
-void diffuse_vec(Env& e, float* f, int type, int sides, int ground, const float* def, float k, int sweeps) {
+// one sweep (two with `two`) of every field of the set
+template <bool THETA>
+void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* face) {
     const Grid& g = e.g;
+    if (!vec_grid(e)) {
+        const auto kernel = F.n == 1 ? k_diffuse<THETA, false> : k_diffuse<THETA, true>;
+        kernel<<<cell_grid(g, F.n), dim3(BX, BY), 0, e.stream>>>(g, F, k, e.p, e.Tg, e.Pg);
+        e.launches += 1;
+        return;
+    }
+    if (two && launch_pair<THETA>(e, F, k, face)) return;
     const int vx = (g.X / 4 + 31) / 32, vy = (g.Y - 1 + DVY - 1) / DVY;
     int vlen;
-    const int vz = z_runs(e, vx, vy, e.tune.diffuse_bps, vlen);
-    float* buf[3] = {e.tA, e.tB, e.As};  // As: the middle sweep of a pair when no tensor map can be made
-    const float* src = f;
-    float* face = e.g2a;  // ground scratch: free until the ground stage refills it
-    if (type == 0) {
-        k_theta_face<<<(g.X * g.Z + 255) / 256, 256, 0, e.stream>>>(g, e.p, e.Tg, e.Pg, face);
+    const int vz = z_runs(e, vx, vy * F.n, e.tune.diffuse_bps, vlen);
+    auto one = [&](const FieldSet& S) {
+        const auto kernel = S.n == 1 ? k_diffuse4<THETA, false> : k_diffuse4<THETA, true>;
+        kernel<<<dim3(vx, vy, vz * S.n), dim3(32, DVY), 0, e.stream>>>(g, vlen, vz, S, k, face);
         e.launches += 1;
+    };
+    if (!two) {
+        one(F);
+        return;
     }
-    // passes of one sweep, or (temporal blocking of depth 2) of two sweeps: an odd count starts
-    // with a single sweep
-    const bool pairs = e.tune.diffuse_depth == 2;
-    const int npass = pairs ? sweeps / 2 + sweeps % 2 : sweeps;
-    for (int q = 0; q < npass; ++q) {
-        float* dst = (q == npass - 1 && q > 0) ? f : buf[q % 2];
-        const bool two = pairs && !(q == 0 && sweeps % 2 == 1);
-        if (two) {
-            const bool ok = type == 0 ? launch_pair<true>(e, src, dst, sides, ground, def, k, face)
-                                      : launch_pair<false>(e, src, dst, sides, ground, def, k, nullptr);
-            if (!ok) {  // no tensor-map encoder: the two sweeps as two passes
-                if (type == 0) {
-                    k_diffuse4<true><<<dim3(vx, vy, vz), dim3(32, DVY), 0, e.stream>>>(g, vlen, src, buf[2], sides, ground, def, k, face);
-                    k_diffuse4<true><<<dim3(vx, vy, vz), dim3(32, DVY), 0, e.stream>>>(g, vlen, buf[2], dst, sides, ground, def, k, face);
-                } else {
-                    k_diffuse4<false><<<dim3(vx, vy, vz), dim3(32, DVY), 0, e.stream>>>(g, vlen, src, buf[2], sides, ground, def, k, nullptr);
-                    k_diffuse4<false><<<dim3(vx, vy, vz), dim3(32, DVY), 0, e.stream>>>(g, vlen, buf[2], dst, sides, ground, def, k, nullptr);
-                }
-                e.launches += 1;
-            }
-        } else if (type == 0) {
-            k_diffuse4<true><<<dim3(vx, vy, vz), dim3(32, DVY), 0, e.stream>>>(g, vlen, src, dst, sides, ground, def, k, face);
-        } else {
-            k_diffuse4<false><<<dim3(vx, vy, vz), dim3(32, DVY), 0, e.stream>>>(g, vlen, src, dst, sides, ground, def, k, nullptr);
-        }
-        e.launches += 1;
-        src = dst;
-    }
-    if (npass == 1) {
-        const int n4 = g.N / 4;
-        k_copy_sky4<<<std::min((n4 + 255) / 256, stencil_sms(e) * 8), 256, 0, e.stream>>>(n4, g.X / 4, g.Y, (const float4*)src, (float4*)f,
-                                                                                     nullptr, 0);
-        e.launches += 1;
+    for (int i = 0; i < F.n; ++i) {  // no tensor-map encoder: the two sweeps as two passes, field by field
+        FieldSet A;
+        A.n = 1;
+        A.in[0] = F.in[i];
+        A.out[0] = scratch_field(e, kScratch - 1);
+        A.def[0] = F.def[i];
+        A.sides[0] = F.sides[i];
+        A.ground[0] = F.ground[i];
+        FieldSet B = A;
+        B.in[0] = A.out[0];
+        B.out[0] = F.out[i];
+        one(A);
+        one(B);
     }
 }
 
 }  // namespace
 
-// diffuseGPU Game/environment.cu:597-673: per-type boundary table :603-638, k = 0.005*dt/vox^2
-void launch_diffuse(Env& e, float* f, int type, float dtS) {
+// diffuseGPU Game/environment.cu:597-673 of n fields at once: per-type boundary table :603-638,
+// k = 0.005*dt/vox^2. The sweeps alternate between a field and a scratch field of its own (three
+// buffers over the first passes when their number is odd), so that the last one writes the field's
+// sky cells itself: no sweep reads the array it writes, and the ground cells of the scratch fields
+// are never read.
+void launch_diffuse_many(Env& e, int n, float* const* f, const int* type, float dtS) {
     const Grid& g = e.g;
-    const float* def = nullptr;
-    int sides = NEUMANN, ground = DIRICHLET;
-    switch (type) {
-        case 0: def = e.isenT; sides = CUSTOM; ground = CUSTOM; break;
-        case 1: def = e.isenQv; sides = CUSTOM; ground = DIRICHLET; break;
-        case 2: def = e.defU; sides = CUSTOM; break;
-        case 3: def = nullptr; sides = NEUMANN; break;
-        case 4: def = e.defW; sides = CUSTOM; break;
-        default: def = e.zeroY; break;
-    }
     const float k = 0.005f * dtS / (g.vox * g.vox);
     const int sweeps = e.cfg.diffuse_sweeps;
-    ProfScope ps(e, "diffuse");
-    if (e.flat && (g.X % 4) == 0 && sweeps > 0) {
-        diffuse_vec(e, f, type, sides, ground, def, k, sweeps);
+    if (sweeps <= 0) return;
+    if (n > 1 && (n > kBatch || (long long)g.Z * n > 65535)) {  // the launch grid's z limit
+        for (int i = 0; i < n; ++i) launch_diffuse_many(e, 1, f + i, type + i, dtS);
         return;
     }
-    e.launches += sweeps + 1;
-    cudaMemcpyAsync(e.tA, f, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-    cudaMemcpyAsync(e.tB, f, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-    float* a = e.tA;
-    float* o = e.tB;
-    // general heightfield or X % 4 != 0 (or no sweeps): the scalar sweep
-    const bool vec = e.flat && (g.X % 4) == 0;
-    for (int s = 0; s < sweeps; ++s) {
-        const float* in = (s % 2 == 0) ? a : o;
-        float* out = (s % 2 == 0) ? o : a;
-        if (type == 0)
-            k_diffuse<true><<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, in, out, sides, ground, def, k, e.p, e.Tg, e.Pg);
-        else
-            k_diffuse<false><<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, in, out, sides, ground, def, k, e.p, e.Tg, e.Pg);
+    ProfScope ps(e, "diffuse");
+    FieldSet F;
+    F.n = n;
+    const bool theta = n == 1 && type[0] == 0;
+    for (int i = 0; i < n; ++i) {
+        F.def[i] = nullptr;
+        F.sides[i] = NEUMANN;
+        F.ground[i] = DIRICHLET;
+        switch (type[i]) {
+            case 0: F.def[i] = e.isenT; F.sides[i] = CUSTOM; F.ground[i] = CUSTOM; break;
+            case 1: F.def[i] = e.isenQv; F.sides[i] = CUSTOM; break;
+            case 2: F.def[i] = e.defU; F.sides[i] = CUSTOM; break;
+            case 3: break;
+            case 4: F.def[i] = e.defW; F.sides[i] = CUSTOM; break;
+            default: F.def[i] = e.zeroY; break;
+        }
     }
-    const float* res = (sweeps % 2 == 0) ? a : o;
-    if (vec) {
-        const int n4 = g.N / 4;
-        k_copy_sky4<<<std::min((n4 + 255) / 256, stencil_sms(e) * 8), 256, 0, e.stream>>>(n4, g.X / 4, g.Y, (const float4*)res, (float4*)f,
-                                                                                     nullptr, 0);
-    } else {
-        k_copy_sky<<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, res, f, nullptr, 0);
+    const float* face = nullptr;
+    if (theta && vec_grid(e)) {
+        face = e.g2a;  // ground scratch: free until the ground stage refills it
+        k_theta_face<<<(g.X * g.Z + 255) / 256, 256, 0, e.stream>>>(g, e.p, e.Tg, e.Pg, e.g2a);
+        e.launches += 1;
+    }
+    // passes of one sweep, or (temporal blocking of depth 2) of two sweeps: an odd count starts
+    // with a single sweep
+    const bool pairs = vec_grid(e) && e.tune.diffuse_depth == 2;
+    const int npass = pairs ? sweeps / 2 + sweeps % 2 : sweeps;
+    for (int q = 0; q < npass; ++q) {
+        for (int i = 0; i < n; ++i) {
+            float* const t1 = scratch_field(e, 2 * i);
+            float* const t2 = scratch_field(e, 2 * i + 1);
+            if (npass % 2 == 0 || npass == 1) {
+                F.in[i] = q % 2 == 0 ? f[i] : t1;
+                F.out[i] = q % 2 == 0 ? t1 : f[i];
+            } else {  // f, t1, t2, f, t1, f, ...
+                F.in[i] = q == 0 ? f[i] : q == 1 ? t1 : q == 2 ? t2 : (q % 2 == 1 ? f[i] : t1);
+                F.out[i] = q == 0 ? t1 : q == 1 ? t2 : q == 2 ? f[i] : (q % 2 == 1 ? t1 : f[i]);
+            }
+        }
+        const bool two = pairs && !(q == 0 && sweeps % 2 == 1);
+        if (theta) diffuse_pass<true>(e, F, two, k, face);
+        else diffuse_pass<false>(e, F, two, k, face);
+    }
+    if (npass == 1) {
+        for (int i = 0; i < n; ++i) {
+            F.in[i] = F.out[i];
+            F.out[i] = f[i];
+        }
+        copy_sky(e, F, nullptr, 0);
     }
 }
 
+void launch_diffuse(Env& e, float* f, int type, float dtS) { launch_diffuse_many(e, 1, &f, &type, dtS); }
+
 // Graph mode, advection loop: the first trip runs when the field has any substep; each trip counts
 // a substep and runs again while substeps remain. The field's count is kept for the step's stats.
-__global__ void k_adv_begin(cudaGraphConditionalHandle h, Scalars* sc, int field) {
+__global__ void k_adv_begin(cudaGraphConditionalHandle h, Scalars* sc, int field, int count) {
     sc->slot = 0;
-    if (field >= 0 && field < 10) sc->nsub_f[field] = sc->nsub;
+    for (int f = field; f < field + count; ++f)
+        if (f >= 0 && f < 10) sc->nsub_f[f] = sc->nsub;
     cudaGraphSetConditional(h, sc->nsub > 0 ? 1u : 0u);
 }
 __global__ void k_adv_next(cudaGraphConditionalHandle h, Scalars* sc, int loop) {
@@ -1622,19 +1723,25 @@ __global__ void k_adv_next(cudaGraphConditionalHandle h, Scalars* sc, int loop) 
     cudaGraphSetConditional(h, sc->slot < sc->nsub ? 1u : 0u);
 }
 
-// advectPPMWGPU Game/environment.cu:692-824. With host_sync the substep count is read back as
-// the reference does; otherwise max_substeps slots are launched and the ones beyond the device
-// count exit at once (graph capture). Returns the substep count (or -1 when not read back).
-int launch_advect(Env& e, float* f, const float* def, int sides, int ground, float dtS, int slot_id, bool host_sync,
-                  bool same_wind) {
+// advectPPMWGPU Game/environment.cu:692-824 of n fields at once (one, or several that the wind does
+// not read: the moisture fields). The substep count is read back as the reference does; in a graph
+// capture it stays on the device and the substeps run as a WHILE loop. slot_id: the first field's
+// place among the step's substep counts. same_wind: the wind has not changed since the last advection
+// (the moisture fields after the projection), so its Courant substep count (sc->nsub, and the host
+// copy) stands. Returns the substep count (-1 when it is on the device).
+int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, const int* sides, const int* ground, float dtS, int slot_id,
+                       bool same_wind) {
     const Grid& g = e.g;
+    if (n > 1 && (n > kBatch || (long long)g.Z * n > 65535)) {
+        int nsub = 0;
+        for (int i = 0; i < n; ++i) nsub = launch_advect_many(e, 1, f + i, def + i, sides + i, ground + i, dtS, slot_id + i, same_wind || i > 0);
+        return nsub;
+    }
     ProfScope ps(e, "advect");
-    // same_wind: the wind has not changed since the last advection (the moisture fields after the
-    // projection), so its Courant substep count (sc->nsub, and the host copy) stands
     if (!same_wind || e.adv_nsub < 0) {
         e.launches += 2;
         cudaMemsetAsync(&e.sc->maxbits, 0, sizeof(unsigned int), e.stream);
-        if (e.flat && (g.X % 4) == 0) {
+        if (vec_grid(e)) {
             const int n4 = g.N / 4;
             k_maxvel4<<<std::min((n4 + 255) / 256, stencil_sms(e) * 8), 256, 0, e.stream>>>(n4, g.X / 4, g.Y, g.XY / 4, (const float4*)e.u,
                                                                                       (const float4*)e.v, (const float4*)e.w,
@@ -1643,122 +1750,102 @@ int launch_advect(Env& e, float* f, const float* def, int sides, int ground, flo
             k_maxvel<<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, e.u, e.v, e.w, e.cfg.semantics == 0, e.sc);
         }
         k_nsub<<<1, 1, 0, e.stream>>>(e.sc, dtS, g.vox, float(e.cfg.max_substeps));
-        e.adv_nsub = -1;
-        if (host_sync && !e.capturing) {
+        if (!e.capturing) {
             fetch_scalars(e);
             e.adv_nsub = e.host_sc->nsub;
         } else {
             e.adv_nsub = 0;  // on the device only (sc->nsub)
         }
     }
-    int nsub = -1;
-    int slots;
-    const Scalars* chk = nullptr;
-    if (host_sync) {
-        nsub = e.adv_nsub;
-        slots = nsub;
-    } else {
-        slots = e.cfg.max_substeps;
-        chk = e.sc;
-    }
-    const dim3 grd = cell_grid(g), blk(BX, BY);
-    float* A = f;
-    float* O = e.tA;
-    const bool vec = e.flat && (g.X % 4) == 0;
+    const int nsub = e.adv_nsub;
+    const dim3 grd = cell_grid(g, n), blk(BX, BY);
+    const bool vec = vec_grid(e);
     const int gx = (g.X / 4 + 31) / 32, gy = (g.Y - 1 + DVY - 1) / DVY;
-    int zc = std::max(1, std::min(g.Z, (stencil_sms(e) * e.tune.ppm_bps + gx * gy - 1) / (gx * gy)));
-    const int zlen = (g.Z + zc - 1) / zc;
-    zc = (g.Z + zlen - 1) / zlen;
-    const dim3 vg(gx, gy, zc), vb(32, DVY);
-    // the Z pass marches: fewer, longer z chunks
-    int zc2 = std::max(1, std::min(g.Z, (stencil_sms(e) * e.tune.ppmz_bps + gx * gy - 1) / (gx * gy)));
-    const int zlen2 = (g.Z + zc2 - 1) / zc2;
-    zc2 = (g.Z + zlen2 - 1) / zlen2;
-    const dim3 vg2(gx, gy, zc2);
+    int zlen, zlen2;  // the Z pass marches: fewer, longer z chunks
+    const int zc = z_runs(e, gx, gy * n, e.tune.ppm_bps, zlen), zc2 = z_runs(e, gx, gy * n, e.tune.ppmz_bps, zlen2);
+    const dim3 vg(gx, gy, zc * n), vb(32, DVY), vg2(gx, gy, zc2 * n);
     // the Y pass marches rows in runs
     const int ygz = (g.Z + PY - 1) / PY;
-    int yc = std::max(1, std::min(g.Y - 1, (stencil_sms(e) * e.tune.ppmy_bps + gx * ygz - 1) / (gx * ygz)));
+    int yc = std::max(1, std::min(g.Y - 1, (stencil_sms(e) * e.tune.ppmy_bps + gx * ygz * n - 1) / (gx * ygz * n)));
     const int ylen = (g.Y - 1 + yc - 1) / yc;
     yc = (g.Y - 1 + ylen - 1) / ylen;
-    const dim3 yg(gx, ygz, yc), yb(32, PY);
-    const int n4 = g.N / 4;
-    const int ncopy = std::min((n4 + 255) / 256, stencil_sms(e) * 8);
+    const dim3 yg(gx, ygz, yc * n), yb(32, PY);
+    FieldSet F;
+    F.n = n;
+    for (int i = 0; i < n; ++i) {
+        F.def[i] = def[i];
+        F.sides[i] = sides[i];
+        F.ground[i] = ground[i];
+    }
     // one substep (slot i; with chk set, the kernels read the substep count from the device and
     // slots at or beyond it return at once)
     auto substep = [&](int i, const Scalars* chk) {
-        if (vec && f != e.v) {
-            // A -> O -> B -> O -> B -> A through the second scratch field: the last pass writes the
-            // field's sky cells itself (no copy). A pass reads the wind as it stands: for u (x
-            // passes) and w (z pass) that is the chain's current buffer.
-            float* B = e.tB;
-            k_ppm4x<<<vg, vb, 0, e.stream>>>(g, zlen, A, O, e.u, def, sides, e.defU, dtS, nsub, 1, chk, i);
-            k_ppm4y<<<yg, yb, 0, e.stream>>>(g, ylen, O, B, e.v, def, sides, ground, dtS, nsub, 1, chk, i);
-            k_ppm4z<<<vg2, vb, 0, e.stream>>>(g, zlen2, B, O, f == e.w ? B : e.w, def, sides, e.defW, dtS, nsub, 0, chk, i);
-            k_ppm4y<<<yg, yb, 0, e.stream>>>(g, ylen, O, B, e.v, def, sides, ground, dtS, nsub, 1, chk, i);
-            k_ppm4x<<<vg, vb, 0, e.stream>>>(g, zlen, B, A, f == e.u ? B : e.u, def, sides, e.defU, dtS, nsub, 1, chk, i);
+        auto xpass = [&](const float* vel) {
+            if (vec) (n == 1 ? k_ppm4x<false> : k_ppm4x<true>)<<<vg, vb, 0, e.stream>>>(g, zlen, zc, F, vel, e.defU, dtS, nsub, 1, chk, i);
+            else (n == 1 ? k_ppm<0, false> : k_ppm<0, true>)<<<grd, blk, 0, e.stream>>>(g, F, vel, e.defU, e.defW, dtS, nsub, 1, chk, i);
+            e.launches += 1;
+        };
+        auto ypass = [&](const float* vel) {
+            if (vec) (n == 1 ? k_ppm4y<false> : k_ppm4y<true>)<<<yg, yb, 0, e.stream>>>(g, ylen, yc, F, vel, dtS, nsub, 1, chk, i);
+            else (n == 1 ? k_ppm<1, false> : k_ppm<1, true>)<<<grd, blk, 0, e.stream>>>(g, F, vel, e.defU, e.defW, dtS, nsub, 1, chk, i);
+            e.launches += 1;
+        };
+        auto zpass = [&](const float* vel) {
+            if (vec) (n == 1 ? k_ppm4z<false> : k_ppm4z<true>)<<<vg2, vb, 0, e.stream>>>(g, zlen2, zc2, F, vel, e.defW, dtS, nsub, 0, chk, i);
+            else (n == 1 ? k_ppm<2, false> : k_ppm<2, true>)<<<grd, blk, 0, e.stream>>>(g, F, vel, e.defU, e.defW, dtS, nsub, 0, chk, i);
+            e.launches += 1;
+        };
+        // buffers of the chain: 0 the field itself, 1 and 2 its scratch fields
+        auto buf = [&](int j, int b) { return b == 0 ? f[j] : scratch_field(e, 2 * j + b - 1); };
+        auto set = [&](int from, int to) {
+            for (int j = 0; j < n; ++j) {
+                F.in[j] = buf(j, from);
+                F.out[j] = buf(j, to);
+            }
+        };
+        if (f[0] != e.v) {
+            // A -> O -> B -> O -> B -> A through the scratch fields: the last pass writes the field's
+            // sky cells itself (no copy). A pass reads the wind as it stands: for u (x passes) and w (z
+            // pass) that is the chain's current buffer.
+            set(0, 1); xpass(e.u);
+            set(1, 2); ypass(e.v);
+            set(2, 1); zpass(f[0] == e.w ? buf(0, 2) : e.w);
+            set(1, 2); ypass(e.v);
+            set(2, 0); xpass(f[0] == e.u ? buf(0, 2) : e.u);
             return;
         }
-        if (vec) {
-            k_ppm4x<<<vg, vb, 0, e.stream>>>(g, zlen, A, O, e.u, def, sides, e.defU, dtS, nsub, 1, chk, i);
-            const float* vy = e.v;
-            if (f == e.v) {
-                cudaMemcpyAsync(e.tB, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-                vy = e.tB;
-            }
-            k_ppm4y<<<yg, yb, 0, e.stream>>>(g, ylen, O, A, vy, def, sides, ground, dtS, nsub, 1, chk, i);
-            k_ppm4z<<<vg2, vb, 0, e.stream>>>(g, zlen2, A, O, e.w, def, sides, e.defW, dtS, nsub, 0, chk, i);
-            vy = e.v;
-            if (f == e.v) {
-                cudaMemcpyAsync(e.tB, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-                vy = e.tB;
-            }
-            k_ppm4y<<<yg, yb, 0, e.stream>>>(g, ylen, O, A, vy, def, sides, ground, dtS, nsub, 1, chk, i);
-            k_ppm4x<<<vg, vb, 0, e.stream>>>(g, zlen, A, O, e.u, def, sides, e.defU, dtS, nsub, 1, chk, i);
-            k_copy_sky4<<<ncopy, 256, 0, e.stream>>>(n4, g.X / 4, g.Y, (const float4*)O, (float4*)A, chk, i);
-            return;
-        }
-        // pass 1: X half, A -> O (velocity u as it stands: for f == u this is A)
-        k_ppm<0><<<grd, blk, 0, e.stream>>>(g, A, O, e.u, def, sides, ground, e.defU, e.defW, dtS, nsub, 1, chk, i);
-        // pass 2: Y half, O -> A; the velocity is v as it stands before the pass (for f == v: q0)
-        const float* vy = e.v;
-        if (f == e.v) {
-            cudaMemcpyAsync(e.tB, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-            vy = e.tB;
-        }
-        k_ppm<1><<<grd, blk, 0, e.stream>>>(g, O, A, vy, def, sides, ground, e.defU, e.defW, dtS, nsub, 1, chk, i);
-        // pass 3: Z full, A -> O
-        k_ppm<2><<<grd, blk, 0, e.stream>>>(g, A, O, e.w, def, sides, ground, e.defU, e.defW, dtS, nsub, 0, chk, i);
-        // pass 4: Y half, O -> A
-        vy = e.v;
-        if (f == e.v) {
-            cudaMemcpyAsync(e.tB, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-            vy = e.tB;
-        }
-        k_ppm<1><<<grd, blk, 0, e.stream>>>(g, O, A, vy, def, sides, ground, e.defU, e.defW, dtS, nsub, 1, chk, i);
-        // pass 5: X half, A -> O, then A = O on sky cells
-        k_ppm<0><<<grd, blk, 0, e.stream>>>(g, A, O, e.u, def, sides, ground, e.defU, e.defW, dtS, nsub, 1, chk, i);
-        k_copy_sky<<<grd, blk, 0, e.stream>>>(g, O, A, chk, i);
+        // v: the Y passes write the array they read their velocity from; the velocity is v as it
+        // stands before the pass
+        float* const vy = buf(0, 2);
+        set(0, 1); xpass(e.u);
+        cudaMemcpyAsync(vy, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
+        set(1, 0); ypass(vy);
+        set(0, 1); zpass(e.w);
+        cudaMemcpyAsync(vy, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
+        set(1, 0); ypass(vy);
+        set(0, 1); xpass(e.u);
+        set(1, 0); copy_sky(e, F, chk, i);
     };
     if (e.capturing) {
-        // graph mode: the substep count stays on the device and the substeps run as a WHILE loop
         e.adv_nsub = 0;
         graph_while(
             e, [&](cudaGraphConditionalHandle h) {
-                k_adv_begin<<<1, 1, 0, e.stream>>>(h, e.sc, slot_id);
+                k_adv_begin<<<1, 1, 0, e.stream>>>(h, e.sc, slot_id, n);
                 e.launches += 1;
             },
             [&](cudaGraphConditionalHandle h, int loop) {
-                e.launches += 6;
                 substep(0, e.sc);
                 k_adv_next<<<1, 1, 0, e.stream>>>(h, e.sc, loop);
                 e.launches += 1;
             });
         return -1;
     }
-    e.launches += 6LL * slots;
-    for (int i = 0; i < slots; ++i) substep(i, chk);
-    (void)slot_id;
+    for (int i = 0; i < nsub; ++i) substep(i, nullptr);
     return nsub;
+}
+
+int launch_advect(Env& e, float* f, const float* def, int sides, int ground, float dtS, int slot_id, bool same_wind) {
+    return launch_advect_many(e, 1, &f, &def, &sides, &ground, dtS, slot_id, same_wind);
 }
 
 // advectPrecip Game/environment.cu:826-849: substeps from the guessed fall speeds 5/1/8 m/s
@@ -1971,14 +2058,17 @@ extern "C" skt_status skt_diffuse_noalloc(int nx, int ny, int nz, float voxel, i
     // out takes the input first so its ground cells keep their values; the sweeps then alternate
     // between out and the scratch array so that the last one lands in out.
     k_copy_all<<<(int(n) + 255) / 256, 256, 0, st>>>(in_dev, out_dev, int(n));
-    const float* src = in_dev;
+    FieldSet F;
+    F.n = 1;
+    F.in[0] = in_dev;
+    F.def[0] = def;
+    F.sides[0] = sides;
+    F.ground[0] = ground;
     for (int s = 0; s < sweeps; ++s) {
-        float* dst = ((sweeps - 1 - s) % 2 == 0) ? out_dev : scratch;
-        if (field_type == 0)
-            k_diffuse<true><<<cell_grid(g), dim3(BX, BY), 0, st>>>(g, src, dst, sides, ground, def, k, p_dev, ground_T_dev, ground_p_dev);
-        else
-            k_diffuse<false><<<cell_grid(g), dim3(BX, BY), 0, st>>>(g, src, dst, sides, ground, def, k, p_dev, ground_T_dev, ground_p_dev);
-        src = dst;
+        F.out[0] = ((sweeps - 1 - s) % 2 == 0) ? out_dev : scratch;
+        if (field_type == 0) k_diffuse<true, false><<<cell_grid(g), dim3(BX, BY), 0, st>>>(g, F, k, p_dev, ground_T_dev, ground_p_dev);
+        else k_diffuse<false, false><<<cell_grid(g), dim3(BX, BY), 0, st>>>(g, F, k, p_dev, ground_T_dev, ground_p_dev);
+        F.in[0] = F.out[0];
     }
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) {

@@ -268,7 +268,7 @@ skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tun
     if (e.flat && (e.g.X % 4) == 0) {
         auto advect_once = [&]() {
             cudaMemcpyAsync(work, e.qv, n * 4, cudaMemcpyDeviceToDevice, e.stream);
-            launch_advect(e, work, e.isenQv, CUSTOM, CUSTOM, dtS, 4, true);
+            launch_advect(e, work, e.isenQv, CUSTOM, CUSTOM, dtS, 4);
         };
         e.tune = best;
         advect_once();
@@ -285,7 +285,7 @@ skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tun
                 e.tune = tr;
                 advect_once();
                 if (differs()) continue;
-                const float ms = time_ms(e, reps, [&]() { launch_advect(e, work, e.isenQv, CUSTOM, CUSTOM, dtS, 4, true); });
+                const float ms = time_ms(e, reps, [&]() { launch_advect(e, work, e.isenQv, CUSTOM, CUSTOM, dtS, 4); });
                 if (ms < pick_ms) {
                     pick_ms = ms;
                     pick = v;
