@@ -564,6 +564,7 @@ skt_status skt_create(const skt_grid_desc* grid, const skt_solver_cfg* cfg, skt_
     e.g.vox = grid->voxel;
     e.cfg = SolverCfg{c.semantics, c.diffuse_sweeps, c.pcg_tol, c.pcg_max_iter, c.max_substeps, c.precision, c.refine_tol, c.inner_max_iter,
                       c.inner_rtol, c.use_graph, c.mg_half, c.pcg_fused};
+    e.tune = default_tuning(int(n));
     const size_t N = size_t(n), NG = size_t(grid->nx) * grid->nz, NY = size_t(grid->ny);
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const int nsky = 12 + 2 + 4 + 4;

@@ -246,17 +246,32 @@ struct SolverCfg {
     int pcg_fused;       // plain: search step and pressure update fused into the operator
 };
 
-// Launch shapes of the kernels whose best shape depends on the grid and the GPU, chosen by
-// skt_autotune (skt_tune.cu) and otherwise these defaults (hand-measured at 512x256x512).
+// Launch shapes of the kernels whose best shape depends on the grid and the GPU: default_tuning at
+// skt_create, or what skt_autotune (skt_tune.cu) measures.
 struct Tuning {
-    int diffuse_depth = 1;   // sweeps per diffusion pass: 1, or 2 (temporal blocking, k_diffuse2)
-    int diffuse_h = 8;       // two-sweep kernel: k_diffuse_pair4 rows per block (6, 14), k_diffuse2 rows per warp (4, 8)
+    int diffuse_depth = 2;   // sweeps per diffusion pass: 1, or 2 (temporal blocking, k_diffuse_pair4, k_diffuse2)
+    int diffuse_h = 14;      // two-sweep kernel: k_diffuse_pair4 rows per block (6, 14), k_diffuse2 rows per warp (4, 8)
     int diffuse_bps = 32;    // k_diffuse4: blocks per SM in the grid (z-run length)
-    int diffuse2_bps = 8;    // k_diffuse2: blocks per SM in the grid (z-run length)
+    int diffuse2_bps = 8;    // k_diffuse_pair4, k_diffuse2: blocks per SM in the grid (z-run length)
     int ppm_bps = 16;        // k_ppm4x: blocks per SM (z-run length)
     int ppmz_bps = 8;        // k_ppm4z: blocks per SM (z-run length)
     int ppmy_bps = 32;       // k_ppm4y: blocks per SM (y-run length)
 };
+// The shapes by the grid's size, measured on ten grids from 32^3 to 512x256x512. Two sweeps per pass
+// are faster on every one of them (a step's diffusions 0.29 -> 0.25 ms at 32^3, 0.60 -> 0.45 at
+// 96x64x96, 3.16 -> 2.15 at 256x128x256, 20.7 -> 12.6 at 512x256x512); the low tile wins below 8M cells
+// (6 and 14 rows: 2.15 and 2.20 ms at 256x128x256, 3.48 and 3.46 at 256x192x320), and below 2M cells
+// half the blocks, whose runs would otherwise be a plane or two (0.53 and 0.54 ms at 128x64x128, 0.28
+// and 0.34 at 64x32x64). The x pass of the advection wants its longer runs up to 12M cells (a step's
+// advections 2.74 and 2.82 ms at 256x128x256, 16.9 and 16.6 at 512x256x512).
+inline Tuning default_tuning(int cells) {
+    Tuning t;
+    t.diffuse_h = cells < 8000000 ? 6 : 14;
+    t.diffuse2_bps = cells < 2000000 ? 4 : 8;
+    t.diffuse_bps = cells < 32000000 ? 16 : 32;
+    t.ppm_bps = cells < 12000000 ? 8 : 16;
+    return t;
+}
 
 // What a captured step needs at launch and afterwards: the irradiance node to update, and the
 // kernel counts (outside the loops, and per trip of each loop) to count the launches from the

@@ -1548,12 +1548,19 @@ bool launch_diffuse2(Env& e, int bps, const float* src, float* dst, int sides, i
     return true;
 }
 
+// the tensor maps of a set's inputs; a diffusion's passes read two or three sets of buffers in turn, so
+// it keeps one of these per set (encoding costs the host about as much as a launch)
+struct PassMaps {
+    FieldMaps m;
+    bool made = false;
+};
+
 template <bool THETA, int R>
-bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const float* face) {
+bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const float* face, PassMaps& maps) {
     const Grid& g = e.g;
-    FieldMaps maps;
-    for (int i = 0; i < F.n; ++i)
-        if (!field_tensor_map(g, F.in[i], P4W, R + 4, &maps.in[i])) return false;
+    for (int i = 0; i < F.n && !maps.made; ++i)
+        if (!field_tensor_map(g, F.in[i], P4W, R + 4, &maps.m.in[i])) return false;
+    maps.made = true;
     const int gx = (g.X + 127) / 128, gy = (g.Y - 1 + R - 1) / R;
     int zlen;
     const int zc = z_runs(e, gx, gy * F.n, bps, zlen);
@@ -1565,7 +1572,7 @@ bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const flo
         attr = true;
     }
     const auto kernel = F.n == 1 ? k_diffuse_pair4<THETA, false, R> : k_diffuse_pair4<THETA, true, R>;
-    kernel<<<dim3(gx, gy, zc * F.n), 32 * (R + 3), smem, e.stream>>>(maps, g, zlen, zc, F, k, face, e.sc);
+    kernel<<<dim3(gx, gy, zc * F.n), 32 * (R + 3), smem, e.stream>>>(maps.m, g, zlen, zc, F, k, face, e.sc);
     e.launches += 1;
     return true;
 }
@@ -1574,10 +1581,10 @@ bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const flo
 // block) or k_diffuse2 (one cell per lane, rows 4 or 8 per warp, field by field); false without a
 // tensor map
 template <bool THETA>
-bool launch_pair(Env& e, const FieldSet& F, float k, const float* face) {
+bool launch_pair(Env& e, const FieldSet& F, float k, const float* face, PassMaps& maps) {
     const int h = e.tune.diffuse_h, bps = e.tune.diffuse2_bps;
-    if (h == 14) return launch_diffuse_pair4<THETA, 14>(e, bps, F, k, face);
-    if (h == 6) return launch_diffuse_pair4<THETA, 6>(e, bps, F, k, face);
+    if (h == 14) return launch_diffuse_pair4<THETA, 14>(e, bps, F, k, face, maps);
+    if (h == 6) return launch_diffuse_pair4<THETA, 6>(e, bps, F, k, face, maps);
     for (int i = 0; i < F.n; ++i) {
         const bool ok = h == 8 ? launch_diffuse2<THETA, 8>(e, bps, F.in[i], F.out[i], F.sides[i], F.ground[i], F.def[i], k, face)
                                : launch_diffuse2<THETA, 4>(e, bps, F.in[i], F.out[i], F.sides[i], F.ground[i], F.def[i], k, face);
@@ -1618,7 +1625,7 @@ void copy_sky(Env& e, const FieldSet& F, const Scalars* chk, int slot) {
 
 // one sweep (two with `two`) of every field of the set
 template <bool THETA>
-void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* face) {
+void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* face, PassMaps& maps) {
     const Grid& g = e.g;
     if (!vec_grid(e)) {
         const auto kernel = F.n == 1 ? k_diffuse<THETA, false> : k_diffuse<THETA, true>;
@@ -1626,7 +1633,7 @@ void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* fac
         e.launches += 1;
         return;
     }
-    if (two && launch_pair<THETA>(e, F, k, face)) return;
+    if (two && launch_pair<THETA>(e, F, k, face, maps)) return;
     const int vx = (g.X / 4 + 31) / 32, vy = (g.Y - 1 + DVY - 1) / DVY;
     int vlen;
     const int vz = z_runs(e, vx, vy * F.n, e.tune.diffuse_bps, vlen);
@@ -1698,6 +1705,7 @@ void launch_diffuse_many(Env& e, int n, float* const* f, const int* type, float 
     // with a single sweep
     const bool pairs = vec_grid(e) && e.tune.diffuse_depth == 2;
     const int npass = pairs ? sweeps / 2 + sweeps % 2 : sweeps;
+    PassMaps maps[3];  // of the inputs f, t1, t2
     for (int q = 0; q < npass; ++q) {
         for (int i = 0; i < n; ++i) {
             float* const t1 = scratch_field(e, 2 * i);
@@ -1711,8 +1719,9 @@ void launch_diffuse_many(Env& e, int n, float* const* f, const int* type, float 
             }
         }
         const bool two = pairs && !(q == 0 && sweeps % 2 == 1);
-        if (theta) diffuse_pass<true>(e, F, two, k, face);
-        else diffuse_pass<false>(e, F, two, k, face);
+        PassMaps& pm = maps[F.in[0] == f[0] ? 0 : F.in[0] == scratch_field(e, 0) ? 1 : 2];
+        if (theta) diffuse_pass<true>(e, F, two, k, face, pm);
+        else diffuse_pass<false>(e, F, two, k, face, pm);
     }
     if (npass == 1) {
         for (int i = 0; i < n; ++i) {

@@ -191,7 +191,8 @@ skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tun
         return SKT_OK;
     }
     const size_t n = size_t(e.g.N);
-    const Tuning base = Tuning{};
+    Tuning base = default_tuning(e.g.N);
+    base.diffuse_depth = 1;  // the results every candidate must reproduce: one sweep per pass
     unsigned* count = nullptr;
     if (cudaMalloc(&count, sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
