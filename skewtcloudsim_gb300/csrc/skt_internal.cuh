@@ -71,7 +71,7 @@ constexpr int kMaxGraphLoops = 16;  // conditional loops of one captured step
 struct Scalars {
     double sigma0, sigma1, beta;      // PCG scalars (FP64)
     float alpha, beta_f;              // the FP32 step lengths applied to the vectors
-    float alpha_pp;                   // plain PCG: the step length of the pressure update still to apply
+    float alpha_of[4];                // plain PCG: the step lengths of the last four directions (their pressure updates go four at a time)
     unsigned int maxbits;             // float bits of a max-reduction (atomicMax on uint)
     int converged;                    // PCG stop flag
     int iters;                        // PCG iterations done

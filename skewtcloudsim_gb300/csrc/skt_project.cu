@@ -2,6 +2,7 @@
 // CG with paired-float reductions (Sum2), pressure/density update and the velocity correction.
 // Follows pressureProject / calculatePressureProject (Game/environment.cu:851-987).
 #include "skt_internal.cuh"
+#include "skt_tma.cuh"
 
 namespace skt {
 
@@ -33,10 +34,32 @@ __device__ __forceinline__ float char_trunc(float a) {  // (char) of a float: tr
     const float t = truncf(a);
     return fminf(fmaxf(t, -128.0f), 127.0f);
 }
-__device__ __forceinline__ float coef_of(float c, float n) {  // initAMatrix Game/kernelSky.cu:1372
-    return n == 0.0f ? 0.0f : -fmaxf(1.0f, 1.225f / (2.0f / (1.0f / c + 1.0f / n)));
+// The face coefficient -max(1, 1.225 / hm) of two cells (initAMatrix Game/kernelSky.cu:1372), hm =
+// 2 / (1/c + 1/n) the harmonic mean of their densities, from the sum of their reciprocals: 1.225 / hm
+// is 0.6125 times it, one rounding instead of two divisions' (its distance from 64 bits is the
+// smaller one).
+__device__ __forceinline__ float coef_of_sum(float s) { return -fmaxf(1.0f, 0.6125f * s); }
+// The coefficient where it is stored. Next to a whole number, where Q3's truncation turns on the last
+// bits, it comes from the reference's own two divisions, so that every truncated coefficient is the
+// reference's.
+__device__ __forceinline__ float coef_stored(float s) {
+    const float c = coef_of_sum(s), t = -c;
+    return t > 1.5f && fabsf(t - rintf(t)) <= 1e-6f * t ? -fmaxf(1.0f, __fdiv_rn(1.225f, __fdiv_rn(2.0f, s))) : c;
 }
+__device__ __forceinline__ float coef_of(float c, float n) { return n == 0.0f ? 0.0f : coef_stored(1.0f / c + 1.0f / n); }
 __device__ __forceinline__ float precon_of(float w) { return w == 0.0f ? 1.0f : 1.0f / w; }  // initPrecon :1409
+
+// The three upper faces' coefficients of a cell as Q3 has them when they are another cell's lower
+// ones, (char) of the float: their magnitudes, 0 to 128, in one word (right, up, front), and one of
+// them as a float again (the byte under the exponent of 2^23, which is then taken off: two full-rate
+// instructions, where the conversion runs at an eighth of that)
+__device__ __forceinline__ unsigned pack_trunc(float cr, float cu, float cf) {
+    return unsigned(-char_trunc(cr)) | unsigned(-char_trunc(cu)) << 8 | unsigned(-char_trunc(cf)) << 16;
+}
+template <int BYTE>
+__device__ __forceinline__ float trunc_of(unsigned w) {
+    return 8388608.0f - __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440 + BYTE));
+}
 
 // resetVelPressProj Game/kernelSky.cu:1648-1682; one thread per (x,y) marching z.
 // reference=1 returns at the first ground cell of the column (Q8).
@@ -67,7 +90,7 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
                                               const float* __restrict__ defU, const float* __restrict__ defW, float dt,
                                               float* __restrict__ ax, float* __restrict__ ay, float* __restrict__ az, float* __restrict__ aw,
                                               float* __restrict__ r, float* __restrict__ s, float* __restrict__ pp, float* __restrict__ As,
-                                              int reference, Scalars* sc, double* partials) {
+                                              int faces, int reference, Scalars* sc, double* partials) {
     Sum2 dsum;
     float mx = 0.0f;
     for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
@@ -76,9 +99,10 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
         if (x >= g.X || y >= g.Y) continue;
         const int c = cidx(g, x, y, z);
         pp[c] = 0.0f;
-        As[c] = 0.0f;
+        if (faces) As[c] = 0.0f;
         if (is_ground(g, x, y, z)) {
-            ax[c] = ay[c] = az[c] = aw[c] = 0.0f;
+            ax[c] = ay[c] = aw[c] = 0.0f;
+            if (faces) az[c] = 0.0f;
             r[c] = 0.0f;
             s[c] = 0.0f;
             continue;
@@ -92,9 +116,14 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
         const float nb = ghost(g, rho, x, y, z - 1, NEUMANN, DIRICHLET, nullptr);
         const float cr = coef_of(cur, nr), cl = coef_of(cur, nl), cu = coef_of(cur, nu);
         const float cd = coef_of(cur, nd), cf = coef_of(cur, nf), cb = coef_of(cur, nb);
-        ax[c] = cr;
-        ay[c] = cu;
-        az[c] = cf;
+        if (faces) {
+            ax[c] = cr;
+            ay[c] = cu;
+            az[c] = cf;
+        } else {
+            ax[c] = 1.0f / cur;  // the matrix-free operator's inputs
+            reinterpret_cast<unsigned*>(ay)[c] = pack_trunc(cr, cu, cf);
+        }
         float wd = 0.0f;
         wd -= cr; wd -= cl; wd -= cu; wd -= cd; wd -= cf; wd -= cb;
         aw[c] = wd;
@@ -393,116 +422,213 @@ __global__ void __launch_bounds__(MVT) k_matvec4(Grid g, int zlen, const float* 
 }
 
 // ---- fused PCG iteration (X % 4 == 0): two launches per iteration instead of three --------
-// The search step (endIteration :987-1014) and the next matrix product share one z march, and
-// the pressure update of the previous iteration (updatePandDiv :955-985, p += alpha s) rides
-// along where s_old is read anyway. The residual kernel stores z = r/diag (it forms z for z.r in
-// any case), so the operator forms s_new = z + beta s_old from two arrays wherever it needs a
-// neighbour's value. Every value is formed as in k_search4 / k_update4 (the search direction as
-// fma(beta, s_old, z), the pressure as fma(alpha, s, p)); only the dot products' summation order
-// differs.
+// The search step (endIteration :987-1014) and the next matrix product share one z march
+// (k_pcg_operator4); the residual kernel stores z = r/diag (it forms z for z.r in any case), so the
+// operator forms s_new = z + beta s_old from two arrays wherever it needs a neighbour's value. Every
+// value is formed as in k_search4 / k_update4 (the search direction as fma(beta, s_old, z), the
+// pressure as fma(alpha, s, p)); only the dot products' summation order differs.
 
-// s_new = z + beta s_old, As = A s_new, s_new.As -> alpha, and p += alpha_pp s_old. The rows
-// above and below and the next plane form their s_new from z and s_old (another warp's or
-// block's rows, read through L1/L2); the x neighbours come from the neighbouring lanes. s_old
-// and s_new are distinct buffers (a block's halo rows are another block's own rows, so s cannot
-// be updated in place).
-template <bool FLAT>
-__global__ void __launch_bounds__(MVT) k_matvec_search4(Grid g, int zlen, const float* __restrict__ ax, const float* __restrict__ ay,
-                                                        const float* __restrict__ az, const float* __restrict__ aw,
-                                                        const float* __restrict__ zv, const float* __restrict__ sold,
-                                                        float* __restrict__ snew, float* __restrict__ As, float* __restrict__ pp,
-                                                        int reference, Scalars* sc, double* partials) {
+constexpr int kDirs = 4;  // direction buffers: iteration k's direction is in buffer k % kDirs
+struct Dirs {
+    const float* d[kDirs];
+};
+
+// s_new = z + beta s_old, As = A s_new, s_new.As -> alpha. Matrix-free: a face's coefficient comes
+// from the reciprocal densities of its two cells (rinv, 0 in ground cells). REF: the lower coefficients
+// as Q3 truncates them, three bytes of a word per cell (truncating in place, with the test that keeps
+// the reference's value, cost as much as the rest of the kernel).
+// A block covers 128 x cells (a warp of four-cell lanes) by OPR rows and marches a run of z planes. The
+// four inputs stream through a ring of OPSLOTS shared-memory slots, each plane's boxes (the block's
+// cells, 4 more on either side so that the copies start on 16-byte boundaries, a row above and
+// below) filled by TMA copies of one thread, OPSLOTS planes ahead, on one mbarrier per slot; outside
+// the grid they read 0, which is the direction's value there. A lane carries its direction and
+// densities of the planes behind and at hand in registers and takes its neighbours from the slot; one
+// barrier a plane frees the slot. s_old and s_new are distinct buffers (a block's halo rows are another
+// block's own rows). FIRST: the direction is z itself.
+// What bounds it: HBM, 24 bytes a cell (20 in the textbook form) where the stored coefficients and the
+// pressure made 40: 290 us a launch at 512x512x256, 5.6 TB/s (421 before); the barrier of a plane takes
+// the rest. An iteration with its residual and a quarter of the pressure's update went from 635 to 510
+// us, at 256x256x128 from 103 to 81. Loading the planes into registers instead of the ring left the
+// lanes waiting (400 us, DRAM 48 % busy; with a plane's loads ahead and 512 threads a block 460). Tiles
+// of 16 rows with 4 or 5 slots: 516 and 518 us an iteration, 20 rows 527, 24 rows 550, 12 rows two blocks
+// per SM 531, 8 rows with 5 slots 532.
+constexpr int OPR = 8, OPT = 32 * OPR;   // rows and threads per block; two blocks per SM
+constexpr int OPW = 136;                 // box width in cells: 4 + 128 + 4
+constexpr int OPSLOTS = 4;
+constexpr int OPBOX = (OPW * (OPR + 2) * 4 + 127) / 128 * 32;  // floats per box, slots 128-byte aligned
+constexpr int op_smem_bytes() { return OPSLOTS * 4 * OPBOX * 4 + OPSLOTS * 8; }
+struct OpMaps {
+    CUtensorMap z, s, r, w;
+};
+
+template <bool FLAT, bool FIRST, bool REF>
+__global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant__ OpMaps maps, Grid g, int zlen, float* __restrict__ snew,
+                                                          float* __restrict__ As, int slot, Scalars* sc, double* partials) {
     if (sc->converged) return;
-    const float beta = sc->beta_f, alpha_pp = sc->alpha_pp;
-    const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
-    const int x0 = (blockIdx.x * 32 + lane) * 4;
-    const int y = blockIdx.y * MVY + threadIdx.y;
-    const int zs = blockIdx.z * zlen, ze = min(zs + zlen, g.Z);
-    const bool act = x0 < g.X && y < g.Y;
-    const int X = g.X, XY = g.XY;
-    const int row = x0 + y * X;
-    auto srow = [&](int c) {
-        const float4 z = ld4(zv, c), so = ld4(sold, c);
-        return make_float4(__fmaf_rn(beta, so.x, z.x), __fmaf_rn(beta, so.y, z.y), __fmaf_rn(beta, so.z, z.z), __fmaf_rn(beta, so.w, z.w));
+    extern __shared__ __align__(128) unsigned char op_smem[];
+    float* const ring = reinterpret_cast<float*>(op_smem);
+    uint64_t* const bar = reinterpret_cast<uint64_t*>(ring + OPSLOTS * 4 * OPBOX);
+    constexpr unsigned BYTES = OPW * (OPR + 2) * 4 * (2 + !FIRST + REF);
+    const float beta = sc->beta_f;
+    const int tid = threadIdx.x, lane = tid & 31, wy = tid >> 5;
+    const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY;
+    const int bx = int(blockIdx.x) * 128, yb = int(blockIdx.y) * OPR;
+    const int x0 = bx + 4 * lane, y = yb + wy;
+    const int zs = int(blockIdx.z) * zlen, ze = min(zs + zlen, Z);
+    const int p0 = max(zs - 1, 0), p1 = min(ze, Z - 1);  // planes read
+    const bool act = x0 < X && y < Y;
+    const bool below = FLAT ? y > 1 : y > 0;  // a row that may be sky lies below
+    const bool lend = x0 == 0, rend = x0 + 4 >= X, top = y + 1 >= Y;
+    const int own = (wy + 1) * OPW + 4 + 4 * lane;  // the lane's cells in a box
+
+    auto issue = [&](int q) {
+        const int s = (q - p0) % OPSLOTS;
+        float* const d = ring + s * 4 * OPBOX;
+        mbar_expect_tx(&bar[s], BYTES);
+        tma_load_3d(d, &maps.z, &bar[s], bx - 4, yb - 1, q);
+        if (!FIRST) tma_load_3d(d + OPBOX, &maps.s, &bar[s], bx - 4, yb - 1, q);
+        tma_load_3d(d + 2 * OPBOX, &maps.r, &bar[s], bx - 4, yb - 1, q);
+        if (REF) tma_load_3d(d + 3 * OPBOX, &maps.w, &bar[s], bx - 4, yb - 1, q);
     };
-    auto sone = [&](int c) { return __fmaf_rn(beta, sold[c], zv[c]); };
-    Kahan acc;
-    float4 vb = f4zero(), vc = f4zero(), azb = f4zero();
-    if (act) {
-        const int c = row + zs * XY;
-        vc = srow(c);
-        if (zs > 0) { vb = srow(c - XY); azb = ld4(az, c - XY); }
+    if (tid == 0) {
+        for (int s = 0; s < OPSLOTS; ++s) mbar_init(&bar[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();
+    int issued = p0;  // thread 0: the next plane to copy
+    if (tid == 0)
+        for (; issued <= min(p1, p0 + OPSLOTS - 1); ++issued) issue(issued);
+    bool ok = true;
+    auto wait_plane = [&](int q) {
+        const int i = q - p0, s = i % OPSLOTS;
+        const unsigned par = unsigned(i / OPSLOTS) & 1u;
+        if (!mbar_try_wait(&bar[s], par)) ok = mbar_wait(&bar[s], par) && ok;
+        return ring + s * 4 * OPBOX;
+    };
+    // the direction and the densities at an offset of a plane's slot
+    auto dir4 = [&](const float* d, int o) {
+        const float4 z = ld4(d, o);
+        if (FIRST) return z;
+        const float4 s = ld4(d + OPBOX, o);
+        return make_float4(__fmaf_rn(beta, s.x, z.x), __fmaf_rn(beta, s.y, z.y), __fmaf_rn(beta, s.z, z.z), __fmaf_rn(beta, s.w, z.w));
+    };
+    auto dir1 = [&](const float* d, int o) { return FIRST ? d[o] : __fmaf_rn(beta, d[OPBOX + o], d[o]); };
+    auto rho4 = [&](const float* d, int o) { return ld4(d + 2 * OPBOX, o); };
+    auto word4 = [&](const float* d, int o) { return *reinterpret_cast<const uint4*>(d + 3 * OPBOX + o); };
+    // the coefficient between a cell of reciprocal density a and its neighbour b; 0 where one is ground
+    auto coef = [&](float a, float b) {
+        const float c = coef_of_sum(a + b);
+        return FLAT || (a != 0.0f && b != 0.0f) ? c : 0.0f;
+    };
+
+    Kahan acc;
+    float4 vb = f4zero(), cB;
+    uint4 wb = make_uint4(0, 0, 0, 0);  // the plane before: its front faces are this plane's back ones
+    float4 rb;
+    const float* d0 = wait_plane(p0);
+    if (zs > 0) {
+        vb = dir4(d0, own);
+        rb = rho4(d0, own);
+        if (REF) wb = word4(d0, own);
+        d0 = wait_plane(zs);
+    }
+    float4 vc = dir4(d0, own), rc = rho4(d0, own);
+    if (zs == 0) rb = rc;  // outside the grid: the own density (NEUMANN)
+    cB = make_float4(coef(rc.x, rb.x), coef(rc.y, rb.y), coef(rc.z, rb.z), coef(rc.w, rb.w));
+    bool stuck = false;
     for (int z = zs; z < ze; ++z) {
-        const int c = row + z * XY;
-        float4 vf = f4zero(), vd = f4zero(), vu = f4zero(), ayd = f4zero(), cx = f4zero(), cy = f4zero(), cz = f4zero(), cw = f4zero();
-        int4 gh4 = make_int4(0, 0, 0, 0);
-        if (act) {
-            if (z + 1 < g.Z) vf = srow(c + XY);
-            if (y > 0) { vd = srow(c - X); ayd = ld4(ay, c - X); }
-            if (y + 1 < g.Y) vu = srow(c + X);
-            cx = ld4(ax, c); cy = ld4(ay, c); cz = ld4(az, c); cw = ld4(aw, c);
-            if (!FLAT) gh4 = *reinterpret_cast<const int4*>(g.gh + x0 + z * X);
-            // the previous iteration's pressure update (s_old of this row was read for vc)
-            const float4 so = ld4(sold, c);
-            float4 pv = ld4(pp, c);
-            pv.x = __fmaf_rn(alpha_pp, so.x, pv.x);
-            pv.y = __fmaf_rn(alpha_pp, so.y, pv.y);
-            pv.z = __fmaf_rn(alpha_pp, so.z, pv.z);
-            pv.w = __fmaf_rn(alpha_pp, so.w, pv.w);
-            *reinterpret_cast<float4*>(pp + c) = pv;
+        float4 vf = f4zero(), rf = rc;
+        const float* d1 = d0;
+        if (z + 1 < Z) {
+            d1 = wait_plane(z + 1);
+            vf = dir4(d1, own);
+            rf = rho4(d1, own);
         }
-        float sl = __shfl_up_sync(0xffffffffu, vc.w, 1);
-        float axl = __shfl_up_sync(0xffffffffu, cx.w, 1);
-        float sr = __shfl_down_sync(0xffffffffu, vc.x, 1);
-        if (act && lane == 0) {
-            if (x0 > 0) { sl = sone(c - 1); axl = ax[c - 1]; } else { sl = 0.0f; axl = 0.0f; }
-        }
-        if (act && (lane == 31 || x0 + 4 >= X)) sr = (x0 + 4 < X) ? sone(c + 4) : 0.0f;
-        if (act) {
-            float AL0 = axl, AL1 = cx.x, AL2 = cx.y, AL3 = cx.z;
-            float AD0 = ayd.x, AD1 = ayd.y, AD2 = ayd.z, AD3 = ayd.w;
-            float AB0 = azb.x, AB1 = azb.y, AB2 = azb.z, AB3 = azb.w;
-            if (reference) {
-                AL0 = char_trunc(AL0); AL1 = char_trunc(AL1); AL2 = char_trunc(AL2); AL3 = char_trunc(AL3);
-                AD0 = char_trunc(AD0); AD1 = char_trunc(AD1); AD2 = char_trunc(AD2); AD3 = char_trunc(AD3);
-                AB0 = char_trunc(AB0); AB1 = char_trunc(AB1); AB2 = char_trunc(AB2); AB3 = char_trunc(AB3);
+        if (y < Y) {
+            const float4 vd = dir4(d0, own - OPW), rd = rho4(d0, own - OPW), vu = dir4(d0, own + OPW);
+            const float4 ru = top ? rc : rho4(d0, own + OPW);
+            uint4 w = make_uint4(0, 0, 0, 0), wd4 = w;
+            unsigned wl = 0;
+            if (REF) {
+                w = word4(d0, own);
+                wd4 = word4(d0, own - OPW);
+                wl = reinterpret_cast<const unsigned*>(d0 + 3 * OPBOX)[own - 1];
             }
+            const float sl = dir1(d0, own - 1), sr = rend ? 0.0f : dir1(d0, own + 4);
+            const float rl = lend ? rc.x : d0[2 * OPBOX + own - 1], rr = rend ? rc.w : d0[2 * OPBOX + own + 4];
+            const float4 cR = make_float4(coef(rc.x, rc.y), coef(rc.y, rc.z), coef(rc.z, rc.w), coef(rc.w, rr));
+            auto cell = [&](float v, float r, float vl, float cL, unsigned wL, float vr, float cr, float vdn, float rdn, unsigned wD, float vup,
+                            float rup, float vbk, float& cb, unsigned wB, float vfr, float rfr) {
+                const float cU = coef(r, rup), cF = coef(r, rfr), cD = below ? coef(r, rdn) : 0.0f;
+                float wd = 0.0f;
+                wd -= cr; wd -= cL; wd -= cU; wd -= cD; wd -= cF; wd -= cb;
+                const float aL = REF ? trunc_of<0>(wL) : cL, aD = REF ? trunc_of<1>(wD) : cD, aB = REF ? trunc_of<2>(wB) : cb;
+                cb = cF;
+                return wd * v + ((aL * vl + aD * vdn + aB * vbk + cr * vr + cU * vup + cF * vfr));
+            };
             float4 o;
-            o.x = cw.x * vc.x + ((AL0 * sl + AD0 * vd.x + AB0 * vb.x + cx.x * vc.y + cy.x * vu.x + cz.x * vf.x));
-            o.y = cw.y * vc.y + ((AL1 * vc.x + AD1 * vd.y + AB1 * vb.y + cx.y * vc.z + cy.y * vu.y + cz.y * vf.y));
-            o.z = cw.z * vc.z + ((AL2 * vc.y + AD2 * vd.z + AB2 * vb.z + cx.z * vc.w + cy.z * vu.z + cz.z * vf.z));
-            o.w = cw.w * vc.w + ((AL3 * vc.z + AD3 * vd.w + AB3 * vb.w + cx.w * sr + cy.w * vu.w + cz.w * vf.w));
+            o.x = cell(vc.x, rc.x, sl, coef(rc.x, rl), wl, vc.y, cR.x, vd.x, rd.x, wd4.x, vu.x, ru.x, vb.x, cB.x, wb.x, vf.x, rf.x);
+            o.y = cell(vc.y, rc.y, vc.x, cR.x, w.x, vc.z, cR.y, vd.y, rd.y, wd4.y, vu.y, ru.y, vb.y, cB.y, wb.y, vf.y, rf.y);
+            o.z = cell(vc.z, rc.z, vc.y, cR.y, w.y, vc.w, cR.z, vd.z, rd.z, wd4.z, vu.z, ru.z, vb.z, cB.z, wb.z, vf.z, rf.z);
+            o.w = cell(vc.w, rc.w, vc.z, cR.z, w.z, sr, cR.w, vd.w, rd.w, wd4.w, vu.w, ru.w, vb.w, cB.w, wb.w, vf.w, rf.w);
             if (FLAT) {
                 if (y == 0) o = f4zero();
             } else {
-                if (y <= gh4.x) o.x = 0.0f;
-                if (y <= gh4.y) o.y = 0.0f;
-                if (y <= gh4.z) o.z = 0.0f;
-                if (y <= gh4.w) o.w = 0.0f;
+                if (rc.x == 0.0f) o.x = 0.0f;
+                if (rc.y == 0.0f) o.y = 0.0f;
+                if (rc.z == 0.0f) o.z = 0.0f;
+                if (rc.w == 0.0f) o.w = 0.0f;
             }
-            *reinterpret_cast<float4*>(snew + c) = vc;
-            *reinterpret_cast<float4*>(As + c) = o;
-            acc.add(o.x * vc.x);
-            acc.add(o.y * vc.y);
-            acc.add(o.z * vc.z);
-            acc.add(o.w * vc.w);
+            if (act) {
+                const int c = x0 + y * X + z * XY;
+                *reinterpret_cast<float4*>(snew + c) = vc;
+                *reinterpret_cast<float4*>(As + c) = o;
+                acc.add(o.x * vc.x);
+                acc.add(o.y * vc.y);
+                acc.add(o.z * vc.z);
+                acc.add(o.w * vc.w);
+            }
+            wb = w;
         }
         vb = vc;
         vc = vf;
-        azb = cz;
+        rc = rf;
+        d0 = d1;
+        // every warp has read plane z: its slot takes the plane OPSLOTS further (a stuck copy stops the block)
+        if (__syncthreads_or(!ok)) {
+            stuck = true;
+            break;
+        }
+        if (tid == 0)
+            for (; issued <= p1 && issued - OPSLOTS <= z; ++issued) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                issue(issued);
+            }
+    }
+    if (stuck) {
+        // record the timeout, then let the copies still in flight land before the block's shared memory
+        // goes away (each wait again bounded); the block's partial is still published, so that the
+        // reduction ends
+        if (tid == 0) {
+            sc->status = SKT_TIMEOUT;
+            for (int q = max(issued - OPSLOTS, p0); q < issued; ++q)
+                (void)mbar_wait(&bar[(q - p0) % OPSLOTS], unsigned((q - p0) / OPSLOTS) & 1u);
+        }
+        __syncthreads();
     }
     double tot;
     float mall;
-    if (grid_sum_max<MVT>(sc, partials, linear_block(), linear_blocks(), tid, acc.pair(), 0.0f, tot, mall)) {
-        const double s1 = reference ? sc->sigma1 + tot : tot;
+    if (grid_sum_max<OPT>(sc, partials, linear_block(), linear_blocks(), tid, acc.pair(), 0.0f, tot, mall)) {
+        const double s1 = REF ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
+        sc->alpha_of[slot] = sc->alpha;
     }
 }
 
 // r -= alpha As, z = r/diag (stored), z.r and the max residual: k_update4 without the pressure
-// update, which the next k_matvec_search4 or k_pressure_tail4 applies with alpha_pp = alpha
+// update, which k_pressure4 applies. It runs through the cells
+// backwards: the operator left the end of As and of the diagonal in L2, and finds the start of z there.
 __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4* __restrict__ aw, const float4* __restrict__ As,
                                                   float4* __restrict__ r, float4* __restrict__ zout, int reference, float tol,
                                                   int max_iter, Scalars* sc, double* partials) {
@@ -510,7 +636,7 @@ __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4*
     const float alpha = sc->alpha;
     Kahan acc;
     float mx = 0.0f;
-    for (int i = blockIdx.x * UT + threadIdx.x; i < n4; i += gridDim.x * UT) {
+    for (int i = n4 - 1 - (blockIdx.x * UT + threadIdx.x); i >= 0; i -= gridDim.x * UT) {
         const float4 a = aw[i], av = As[i];
         float4 rv = r[i];
         rv.x = rv.x - alpha * av.x; rv.y = rv.y - alpha * av.y; rv.z = rv.z - alpha * av.z; rv.w = rv.w - alpha * av.w;
@@ -534,7 +660,6 @@ __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4*
     if (grid_sum_max<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.pair(), mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
-        sc->alpha_pp = alpha;
         if (mall <= tol) {
             sc->converged = 1;
         } else if (sc->iters >= max_iter) {
@@ -547,34 +672,30 @@ __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4*
     }
 }
 
-// the last iteration's pressure update: p += alpha_pp s
-__global__ void __launch_bounds__(UT) k_pressure_tail4(int n4, const float4* __restrict__ s, float4* __restrict__ pp, const Scalars* sc) {
-    const float alpha = sc->alpha_pp;
-    for (int i = blockIdx.x * UT + threadIdx.x; i < n4; i += gridDim.x * UT) {
-        const float4 sv = s[i];
-        float4 pv = pp[i];
-        pv.x = __fmaf_rn(alpha, sv.x, pv.x);
-        pv.y = __fmaf_rn(alpha, sv.y, pv.y);
-        pv.z = __fmaf_rn(alpha, sv.z, pv.z);
-        pv.w = __fmaf_rn(alpha, sv.w, pv.w);
-        pp[i] = pv;
-    }
-}
-
-// graph mode: the last iteration's pressure update from the direction buffer of its parity
-__global__ void __launch_bounds__(UT) k_pressure_tail_sel(int n4, const float4* __restrict__ s0, const float4* __restrict__ s1,
-                                                          float4* __restrict__ pp, const Scalars* sc) {
+// The pressure updates p += alpha s (updatePandDiv :955-985), four iterations' at a time and in their
+// order: before the iteration that overwrites the oldest direction (TAIL false), and after the last one
+// to four (TAIL). The pressure is read and written once for four iterations, 6 bytes a cell and
+// iteration instead of 8 and none of them in the operator.
+template <bool TAIL>
+__global__ void __launch_bounds__(UT) k_pressure4(int n4, Dirs dirs, float4* __restrict__ pp, const Scalars* sc) {
+    if (!TAIL && sc->converged) return;  // the tail does these too
     const int it = sc->iters;
     if (it <= 0) return;
-    const float4* __restrict__ s = ((it - 1) & 1) ? s1 : s0;
-    const float alpha = sc->alpha_pp;
+    const int n = TAIL ? it - (it - 1) / kDirs * kDirs : kDirs;
+    float al[kDirs];
+#pragma unroll
+    for (int j = 0; j < kDirs; ++j) al[j] = sc->alpha_of[j];
     for (int i = blockIdx.x * UT + threadIdx.x; i < n4; i += gridDim.x * UT) {
-        const float4 sv = s[i];
         float4 pv = pp[i];
-        pv.x = __fmaf_rn(alpha, sv.x, pv.x);
-        pv.y = __fmaf_rn(alpha, sv.y, pv.y);
-        pv.z = __fmaf_rn(alpha, sv.z, pv.z);
-        pv.w = __fmaf_rn(alpha, sv.w, pv.w);
+#pragma unroll
+        for (int j = 0; j < kDirs; ++j) {
+            if (TAIL && j >= n) break;
+            const float4 sv = reinterpret_cast<const float4*>(dirs.d[j])[i];
+            pv.x = __fmaf_rn(al[j], sv.x, pv.x);
+            pv.y = __fmaf_rn(al[j], sv.y, pv.y);
+            pv.z = __fmaf_rn(al[j], sv.z, pv.z);
+            pv.w = __fmaf_rn(al[j], sv.w, pv.w);
+        }
         pp[i] = pv;
     }
 }
@@ -591,7 +712,7 @@ __global__ void k_pcg_cond(cudaGraphConditionalHandle h, Scalars* sc, int loop) 
 // K*512 consecutive cells; thread t holds cells t, t+512, ...: r, the pressure, the diagonal and
 // the direction in registers, the six face coefficients (the lower ones truncated as Q3 wants, 0
 // where there is no neighbour) in shared memory. Only the direction's halo crosses blocks: as in
-// k_matvec_search4 every block forms s_new = z + beta s_old for itself and, outside its own cells,
+// k_pcg_operator4 every block forms s_new = z + beta s_old for itself and, outside its own cells,
 // from the neighbours' z and s_old in global memory (L2), so an iteration needs two grid-wide
 // reductions and no third barrier. Each reduction is its own barrier: a block publishes its partial
 // and arrives, waits until all have arrived, and sums all partials in the same order, so every
@@ -855,12 +976,15 @@ __device__ __forceinline__ void fset(float4& v, int k, float a) {
     if (k == 0) v.x = a; else if (k == 1) v.y = a; else if (k == 2) v.z = a; else v.w = a;
 }
 __device__ __forceinline__ void face_of(float c, float rc, float n, float rn, float& h, float& coef) {
-    // hm(n) = 2/(1/c + 1/n) and coef_of(c, n) = -max(1, 1.225/hm), both 0 across a zero density
+    // hm(n) = 2/(1/c + 1/n) and coef_of(c, n), both 0 across a zero density
     if (n == 0.0f) { h = 0.0f; coef = 0.0f; return; }
     h = 2.0f / (rc + rn);
-    coef = -fmaxf(1.0f, 1.225f / h);
+    coef = coef_stored(rc + rn);
     (void)c;
 }
+// FACES: the three face coefficients are stored; otherwise, in the places of the first two,
+// what k_pcg_operator4 reads: the reciprocal densities and the truncated coefficients.
+template <bool FACES>
 __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* __restrict__ rho, const float* __restrict__ u,
                                                 const float* __restrict__ v, const float* __restrict__ w,
                                                 const float* __restrict__ defU, const float* __restrict__ defW, float dt,
@@ -963,23 +1087,30 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
                 if (m > mx) mx = m;
                 fset(hB, k, hF); fset(cB, k, cF);
             }
-            *reinterpret_cast<float4*>(ax + c) = oax;
-            *reinterpret_cast<float4*>(ay + c) = oay;
-            *reinterpret_cast<float4*>(az + c) = oaz;
+            *reinterpret_cast<float4*>(ax + c) = FACES ? oax : rc;
+            if (FACES) {
+                *reinterpret_cast<float4*>(ay + c) = oay;
+                *reinterpret_cast<float4*>(az + c) = oaz;
+                *reinterpret_cast<float4*>(As + c) = z4;
+            } else {
+                *reinterpret_cast<uint4*>(ay + c) = make_uint4(pack_trunc(oax.x, oay.x, oaz.x), pack_trunc(oax.y, oay.y, oaz.y),
+                                                               pack_trunc(oax.z, oay.z, oaz.z), pack_trunc(oax.w, oay.w, oaz.w));
+            }
             *reinterpret_cast<float4*>(aw + c) = oaw;
             *reinterpret_cast<float4*>(r + c) = orr;
             *reinterpret_cast<float4*>(s + c) = oss;
             *reinterpret_cast<float4*>(pp + c) = z4;
-            *reinterpret_cast<float4*>(As + c) = z4;
         } else if (act) {  // the ground row
             *reinterpret_cast<float4*>(ax + c) = z4;
             *reinterpret_cast<float4*>(ay + c) = z4;
-            *reinterpret_cast<float4*>(az + c) = z4;
+            if (FACES) {
+                *reinterpret_cast<float4*>(az + c) = z4;
+                *reinterpret_cast<float4*>(As + c) = z4;
+            }
             *reinterpret_cast<float4*>(aw + c) = z4;
             *reinterpret_cast<float4*>(r + c) = z4;
             *reinterpret_cast<float4*>(s + c) = z4;
             *reinterpret_cast<float4*>(pp + c) = z4;
-            *reinterpret_cast<float4*>(As + c) = z4;
         }
         pc = pf;
         rc = rf;
@@ -1092,8 +1223,9 @@ __global__ void __launch_bounds__(256) k_apply_proj4(Grid g, int zlen, const flo
 
 namespace {
 
+// whether the blocks of this launch are resident at once (asked once per environment and variant)
 template <int K>
-bool launch_pcg_grid(Env& e, int slot, int nb) {
+bool pcg_grid_fits(Env& e, int slot, int nb) {
     const int smem = pcg_grid_smem<K>(e.g.X);
     if (e.pcg_grid_cap[slot] < 0) {
         // the limit set on the kernel is the device's, not this grid's need: other environments launch it too
@@ -1109,14 +1241,16 @@ bool launch_pcg_grid(Env& e, int slot, int nb) {
         }
         e.pcg_grid_cap[slot] = per_sm * e.num_sms;
     }
-    if (nb > e.pcg_grid_cap[slot]) return false;
+    return nb <= e.pcg_grid_cap[slot];
+}
+template <int K>
+void launch_pcg_grid(Env& e, int nb) {
     int reference = e.cfg.semantics == 0;
     void* args[] = {&e.g, &e.ax, &e.ay, &e.az, &e.aw, &e.r, &e.s, &e.tB, &e.tA, &e.pp, &reference, &e.cfg.pcg_tol, &e.cfg.pcg_max_iter,
                     &e.sc, &e.grid_parts};
     // an error is the step's to report (its check finds it)
-    (void)cudaLaunchCooperativeKernel((const void*)k_pcg_grid<K>, dim3(nb), dim3(GCT), args, smem, e.stream);
+    (void)cudaLaunchCooperativeKernel((const void*)k_pcg_grid<K>, dim3(nb), dim3(GCT), args, pcg_grid_smem<K>(e.g.X), e.stream);
     e.launches += 1;
-    return true;
 }
 
 // The launch shape for a grid: the variant with the fewest cells per thread that needs at most 96
@@ -1134,18 +1268,50 @@ void pcg_grid_shape(const Env& e, int& slot, int& nb) {
     nb = 0;
 }
 
-// The PCG in one cooperative launch; false: not taken. pcg_fused = 0 keeps its three launches per iteration.
-bool pcg_in_one_launch(Env& e) {
-    int slot, nb;
+// How the plain PCG runs: in one cooperative launch where the grid fits, else matrix-free in two
+// launches per iteration (X % 4 == 0), else from stored coefficients in three (any X; pcg_fused = 0).
+enum class PcgPath { GRID, FREE, STORED };
+PcgPath pcg_path(Env& e, int& slot, int& nb, OpMaps* maps, float* const* dirs, const float* zbuf) {
     pcg_grid_shape(e, slot, nb);
-    if (nb == 0 || !e.cfg.pcg_fused || e.cfg.pcg_max_iter <= 0) return false;
-    ProfScope ps(e, "pcg_grid");
-    switch (slot) {
-        case 0: return launch_pcg_grid<2>(e, slot, nb);
-        case 1: return launch_pcg_grid<4>(e, slot, nb);
-        case 2: return launch_pcg_grid<8>(e, slot, nb);
-        default: return launch_pcg_grid<14>(e, slot, nb);
+    if (!e.cfg.pcg_fused || e.cfg.pcg_max_iter <= 0) return PcgPath::STORED;
+    if (nb > 0 && (slot == 0 ? pcg_grid_fits<2>(e, slot, nb) : slot == 1 ? pcg_grid_fits<4>(e, slot, nb)
+                   : slot == 2 ? pcg_grid_fits<8>(e, slot, nb) : pcg_grid_fits<14>(e, slot, nb)))
+        return PcgPath::GRID;
+    if (e.g.X % 4 != 0 || (long long)((e.g.X + 127) / 128) * ((e.g.Y + OPR - 1) / OPR) > kMaxPartials) return PcgPath::STORED;
+    // one set of tensor maps per direction buffer that an iteration reads; without an encoder: stored
+    for (int j = 0; j < kDirs; ++j) {
+        if (!field_tensor_map(e.g, zbuf, OPW, OPR + 2, &maps[j].z) || !field_tensor_map(e.g, dirs[j], OPW, OPR + 2, &maps[j].s) ||
+            !field_tensor_map(e.g, e.ax, OPW, OPR + 2, &maps[j].r) || !field_tensor_map(e.g, e.ay, OPW, OPR + 2, &maps[j].w))
+            return PcgPath::STORED;
     }
+    return PcgPath::FREE;
+}
+// the operator's instance (its shared memory allowed)
+template <bool FLAT, bool FIRST, bool REF>
+auto pcg_operator_of() {
+    cudaFuncSetAttribute(k_pcg_operator4<FLAT, FIRST, REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, op_smem_bytes());
+    return k_pcg_operator4<FLAT, FIRST, REF>;
+}
+template <bool FLAT>
+auto pcg_operator(bool first, bool ref) {
+    return first ? (ref ? pcg_operator_of<FLAT, true, true>() : pcg_operator_of<FLAT, true, false>())
+                 : (ref ? pcg_operator_of<FLAT, false, true>() : pcg_operator_of<FLAT, false, false>());
+}
+// z runs of the operator: the fewest planes in a row on one SM (two blocks per SM at a time; a run reads
+// a plane more on either side and fills its ring first), within the partials' storage
+int operator_runs(const Env& e, int columns, int& zlen) {
+    long long best = -1;
+    int runs = 1;
+    for (int zc = 1; zc <= e.g.Z && (long long)columns * zc <= kMaxPartials; ++zc) {
+        const int len = (e.g.Z + zc - 1) / zc;
+        const long long waves = ((long long)columns * zc + 2 * e.num_sms - 1) / (2 * e.num_sms), cost = waves * (len + 3);
+        if (best < 0 || cost < best) {
+            best = cost;
+            runs = zc;
+        }
+    }
+    zlen = (e.g.Z + runs - 1) / runs;
+    return (e.g.Z + zlen - 1) / zlen;
 }
 
 }  // namespace
@@ -1177,26 +1343,45 @@ void launch_project(Env& e, float dtS) {
     const Tiles T = tiles_of(g);
     const int ref = e.cfg.semantics == 0;
     const int nblk = std::min(std::min(T.n, e.num_sms * 4), kMaxPartials);
+    int slot = 0, gridblocks = 0;
+    // matrix-free: z = r/diag in e.tA, the directions in the free fields (the advection's scratch and
+    // the mixed solve's fields)
+    float* zbuf = e.tA;
+    float* dirs[kDirs] = {e.s, e.tB, reinterpret_cast<float*>(e.xd), reinterpret_cast<float*>(e.xd) + size_t(g.N)};
+    OpMaps maps[kDirs];
+    const PcgPath path = e.cfg.precision == 1 ? PcgPath::STORED : pcg_path(e, slot, gridblocks, maps, dirs, zbuf);
+    const bool faces = path != PcgPath::FREE;
     {
     ProfScope ps(e, "proj_setup");
     e.launches += 2;
     k_reset_vel<<<(g.XY + 127) / 128, 128, 0, e.stream>>>(g, e.u, e.v, e.w, e.defU, e.defW, ref);
+    float* z0 = faces ? e.s : zbuf;
     if (e.flat && (g.X % 4) == 0) {
         const int gx = (g.X / 4 + 31) / 32, gy = (g.Y + MVY - 1) / MVY;
         int zc = std::max(1, std::min(g.Z, (e.num_sms * 4 + gx * gy - 1) / (gx * gy)));
         while (gx * gy * zc > kMaxPartials && zc > 1) --zc;
         const int zlen = (g.Z + zc - 1) / zc;
         zc = (g.Z + zlen - 1) / zlen;
-        k_build4<<<dim3(gx, gy, zc), dim3(32, MVY), 0, e.stream>>>(g, zlen, e.rho, e.u, e.v, e.w, e.defU, e.defW, dtS, e.ax, e.ay, e.az,
-                                                                   e.aw, e.r, e.s, e.pp, e.As, ref, e.sc, e.partials);
+        const auto build = faces ? k_build4<true> : k_build4<false>;
+        build<<<dim3(gx, gy, zc), dim3(32, MVY), 0, e.stream>>>(g, zlen, e.rho, e.u, e.v, e.w, e.defU, e.defW, dtS, e.ax, e.ay, e.az, e.aw,
+                                                                e.r, z0, e.pp, e.As, ref, e.sc, e.partials);
     } else {
-        k_build<<<nblk, NT, 0, e.stream>>>(g, T, e.rho, e.u, e.v, e.w, e.defU, e.defW, dtS, e.ax, e.ay, e.az, e.aw, e.r, e.s, e.pp, e.As,
-                                          ref, e.sc, e.partials);
+        k_build<<<nblk, NT, 0, e.stream>>>(g, T, e.rho, e.u, e.v, e.w, e.defU, e.defW, dtS, e.ax, e.ay, e.az, e.aw, e.r, z0, e.pp, e.As,
+                                          faces, ref, e.sc, e.partials);
     }
     }
     if (e.cfg.precision == 1) {
         mg_solve(e);
-    } else if (pcg_in_one_launch(e)) {
+    } else if (path == PcgPath::GRID) {
+        {
+            ProfScope ps(e, "pcg_grid");
+            switch (slot) {
+                case 0: launch_pcg_grid<2>(e, gridblocks); break;
+                case 1: launch_pcg_grid<4>(e, gridblocks); break;
+                case 2: launch_pcg_grid<8>(e, gridblocks); break;
+                default: launch_pcg_grid<14>(e, gridblocks); break;
+            }
+        }
         if (!e.capturing) {
             fetch_scalars(e);
             e.last_iters = e.host_sc->iters;
@@ -1204,7 +1389,7 @@ void launch_project(Env& e, float dtS) {
             e.last_converged = e.host_sc->converged == 1;
         }
     } else {
-    const int chunk = 8;
+    const int chunk = 8;  // a multiple of kDirs: a chunk's iterations use the direction buffers as the chunk before
     const bool vec = (g.X % 4) == 0;
     // vectorised launch shapes: streams at 16 blocks/SM (several waves of the grid-stride loop:
     // 8 per SM, 1.3 waves, left the second wave a third full), the matvec's z chunks sized to fill
@@ -1220,28 +1405,23 @@ void launch_project(Env& e, float dtS) {
     const int zlen = (g.Z + zc - 1) / zc;
     zc = (g.Z + zlen - 1) / zlen;
     const dim3 mvg(gx, gy, zc);
-    // fused iterations: the search directions alternate between e.s and e.tB, z = r/diag lives in
-    // e.tA (both free during the projection: the advection's scratch); iteration k's direction is
-    // dirs[k % 2]
-    float* dirs[2] = {e.s, e.tB};
-    float* zbuf = e.tA;
-    // iteration kk of the PCG (directions alternate between the two buffers in the fused form)
+    const Dirs dp{{dirs[0], dirs[1], dirs[2], dirs[3]}};
+    const int ox = (g.X + 127) / 128, oy = (g.Y + OPR - 1) / OPR;
+    int ozlen;
+    const dim3 og(ox, oy, operator_runs(e, ox * oy, ozlen));
+    const auto op_first = e.flat ? pcg_operator<true>(true, ref) : pcg_operator<false>(true, ref);
+    const auto op_next = e.flat ? pcg_operator<true>(false, ref) : pcg_operator<false>(false, ref);
+    // iteration kk of the PCG (kk == 0: the first; others by their place in the chunks after it)
     auto iterate = [&](int kk) {
-            if (vec && e.cfg.pcg_fused) {
-                float* sd = dirs[kk & 1];
+            if (path == PcgPath::FREE) {
+                const int slot = kk % kDirs;
+                if (slot == 0 && kk > 0) {
+                    ProfScope ps(e, "pcg_update"); e.launches += 1;
+                    k_pressure4<false><<<nstream, UT, 0, e.stream>>>(n4, dp, (float4*)e.pp, e.sc);
+                }
                 { ProfScope ps(e, "pcg_matvec"); e.launches += 1;
-                  if (kk == 0) {  // the first direction is z itself (set by the build)
-                      if (e.flat) k_matvec4<true><<<mvg, mvb, 0, e.stream>>>(g, zlen, e.ax, e.ay, e.az, e.aw, sd, e.As, ref, e.sc, e.partials);
-                      else k_matvec4<false><<<mvg, mvb, 0, e.stream>>>(g, zlen, e.ax, e.ay, e.az, e.aw, sd, e.As, ref, e.sc, e.partials);
-                  } else {
-                      const float* so = dirs[(kk - 1) & 1];
-                      if (e.flat)
-                          k_matvec_search4<true><<<mvg, mvb, 0, e.stream>>>(g, zlen, e.ax, e.ay, e.az, e.aw, zbuf, so, sd, e.As, e.pp, ref,
-                                                                            e.sc, e.partials);
-                      else
-                          k_matvec_search4<false><<<mvg, mvb, 0, e.stream>>>(g, zlen, e.ax, e.ay, e.az, e.aw, zbuf, so, sd, e.As, e.pp, ref,
-                                                                             e.sc, e.partials);
-                  } }
+                  (kk == 0 ? op_first : op_next)<<<og, OPT, op_smem_bytes(), e.stream>>>(maps[(kk + kDirs - 1) % kDirs], g, ozlen, dirs[slot],
+                                                                                       e.As, slot, e.sc, e.partials); }
                 { ProfScope ps(e, "pcg_update"); e.launches += 1;
                   k_residual4<<<nstream, UT, 0, e.stream>>>(n4, g.XY / 4, (const float4*)e.aw, (const float4*)e.As, (float4*)e.r,
                                                             (float4*)zbuf, ref, e.cfg.pcg_tol, e.cfg.pcg_max_iter, e.sc, e.partials); }
@@ -1260,10 +1440,16 @@ void launch_project(Env& e, float dtS) {
                 { ProfScope ps(e, "pcg_search"); e.launches += 1; k_search<<<nblk, NT, 0, e.stream>>>(g, T, e.aw, e.r, e.s, e.sc); }
             }
     };
+    auto tail = [&]() {  // the last directions' pressure updates (no later operator launch carries them)
+        if (path != PcgPath::FREE) return;
+        ProfScope ps(e, "pcg_update");
+        e.launches += 1;
+        k_pressure4<true><<<nstream, UT, 0, e.stream>>>(n4, dp, (float4*)e.pp, e.sc);
+    };
     if (e.capturing) {
         // graph mode: iteration 0, then chunks of `chunk` iterations as a WHILE loop that runs while
-        // the solver has not stopped (an even chunk keeps the direction buffers' parity); the
-        // kernels of iterations past the stop return at once, as in the stream-ordered form
+        // the solver has not stopped; the kernels of iterations past the stop return at once, as in
+        // the stream-ordered form
         if (e.cfg.pcg_max_iter > 0) {
             iterate(0);
             graph_while(
@@ -1276,11 +1462,7 @@ void launch_project(Env& e, float dtS) {
                     k_pcg_cond<<<1, 1, 0, e.stream>>>(h, e.sc, loop);
                     e.launches += 1;
                 });
-            if (vec && e.cfg.pcg_fused) {
-                ProfScope ps(e, "pcg_update");
-                e.launches += 1;
-                k_pressure_tail_sel<<<nstream, UT, 0, e.stream>>>(n4, (const float4*)dirs[0], (const float4*)dirs[1], (float4*)e.pp, e.sc);
-            }
+            tail();
         }
     } else {
     for (int it = 0; it < e.cfg.pcg_max_iter; it += chunk) {
@@ -1289,12 +1471,7 @@ void launch_project(Env& e, float dtS) {
         fetch_scalars(e);
         if (e.host_sc->converged || e.host_sc->status != 0) break;
     }
-    if (vec && e.cfg.pcg_fused && e.host_sc->iters > 0) {
-        // the last iteration's pressure update (no later operator launch carried it)
-        ProfScope ps(e, "pcg_update");
-        e.launches += 1;
-        k_pressure_tail4<<<nstream, UT, 0, e.stream>>>(n4, (const float4*)dirs[(e.host_sc->iters - 1) & 1], (float4*)e.pp, e.sc);
-    }
+    if (e.cfg.pcg_max_iter > 0) tail();
     e.last_iters = e.host_sc->iters;
     e.last_residual = e.host_sc->residual;
     e.last_converged = e.host_sc->converged == 1;

@@ -1,8 +1,8 @@
 // Stencil kernels of the atmosphere step: diffusion, PPM advection, Courant max, sedimentation,
 // buoyancy and the equation of state.
 #include "skt_internal.cuh"
+#include "skt_tma.cuh"
 #include "../../include/skewt.h"
-#include <cuda.h>
 #include <algorithm>
 #include <mutex>
 #include <string>
@@ -187,8 +187,6 @@ constexpr int D2OUT = 28;   // cells a warp writes along x
 constexpr int D2WARPS = 8;  // warps per block, stacked in y
 constexpr int D2BW = D2OUT + 8;  // box width: 36 floats = 144 bytes
 constexpr int D2SLOTS = 6;  // ring depth (planes in flight per block)
-constexpr unsigned kMbarSpinLimit = 1u << 20;  // try_wait rounds before a wait is declared stuck
-
 template <int H>
 struct D2Rows {
     float v[H + 4];  // input rows y0-2 .. y0+H+1 (the intermediate sweep uses the first H+2)
@@ -199,36 +197,6 @@ template <int H>
 constexpr int d2_slot_bytes() { return ((D2BW * d2_box_rows<H>() * 4 + 127) / 128) * 128; }
 template <int H>
 constexpr int d2_smem_bytes() { return D2SLOTS * d2_slot_bytes<H>() + D2SLOTS * 8; }
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// a bounded wait: false when the phase did not complete within kMbarSpinLimit rounds
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-    for (unsigned i = 0; i < kMbarSpinLimit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
 
 template <bool THETA, int H>
 __global__ void __launch_bounds__(32 * D2WARPS) k_diffuse2(const __grid_constant__ CUtensorMap tin, Grid g, int zlen,
@@ -1501,11 +1469,13 @@ inline int z_runs(const Env& e, int gx, int gy, int bps, int& zlen) {
     return (e.g.Z + zlen - 1) / zlen;
 }
 
+}  // namespace
+
 // cuTensorMapEncodeTiled through the runtime's driver entry points (no link against libcuda)
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                       const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                       CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-TensorMapEncodeFn tensor_map_encoder() {
+static TensorMapEncodeFn tensor_map_encoder() {
     static TensorMapEncodeFn fn = nullptr;
     if (!fn) {
         cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
@@ -1517,7 +1487,6 @@ TensorMapEncodeFn tensor_map_encoder() {
     return fn;
 }
 
-// A field as a 3D tensor (x fastest) read in boxes of width x rows x 1 cells; false if it cannot be encoded.
 bool field_tensor_map(const Grid& g, const float* base, int width, int rows, CUtensorMap* map) {
     TensorMapEncodeFn enc = tensor_map_encoder();
     if (!enc) return false;
@@ -1528,6 +1497,8 @@ bool field_tensor_map(const Grid& g, const float* base, int width, int rows, CUt
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+namespace {
 
 template <bool THETA, int H>
 bool launch_diffuse2(Env& e, int bps, const float* src, float* dst, int sides, int ground, const float* def, float k,
