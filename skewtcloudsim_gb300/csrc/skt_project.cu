@@ -35,31 +35,38 @@ __device__ __forceinline__ float char_trunc(float a) {  // (char) of a float: tr
     return fminf(fmaxf(t, -128.0f), 127.0f);
 }
 // The face coefficient -max(1, 1.225 / hm) of two cells (initAMatrix Game/kernelSky.cu:1372), hm =
-// 2 / (1/c + 1/n) the harmonic mean of their densities, from the sum of their reciprocals: 1.225 / hm
-// is 0.6125 times it, one rounding instead of two divisions' (its distance from 64 bits is the
-// smaller one).
-__device__ __forceinline__ float coef_of_sum(float s) { return -fmaxf(1.0f, 0.6125f * s); }
-// The coefficient where it is stored. Next to a whole number, where Q3's truncation turns on the last
-// bits, it comes from the reference's own two divisions, so that every truncated coefficient is the
-// reference's.
-__device__ __forceinline__ float coef_stored(float s) {
-    const float c = coef_of_sum(s), t = -c;
-    return t > 1.5f && fabsf(t - rintf(t)) <= 1e-6f * t ? -fmaxf(1.0f, __fdiv_rn(1.225f, __fdiv_rn(2.0f, s))) : c;
+// 2 / (1/c + 1/n) the harmonic mean of their densities; 0 across a zero density (a ground cell)
+__device__ __forceinline__ float coef_of(float c, float n) {
+    return n == 0.0f ? 0.0f : -fmaxf(1.0f, 1.225f / (2.0f / (1.0f / c + 1.0f / n)));
 }
-__device__ __forceinline__ float coef_of(float c, float n) { return n == 0.0f ? 0.0f : coef_stored(1.0f / c + 1.0f / n); }
+// The same from the sum s of the reciprocal densities without its two divisions: 1.225 / hm is 0.6125 s up
+// to rounding, and differs from it by one unit in the last place at most (checked for every significand:
+// both scale with powers of two). The setup stores that difference, 0 to 2 for -1 to 1.
+__device__ __forceinline__ unsigned coef_delta(float s) {
+    return unsigned(__float_as_int(__fdiv_rn(1.225f, __fdiv_rn(2.0f, s))) - __float_as_int(0.6125f * s) + 1) & 3u;
+}
+__device__ __forceinline__ float coef_of_sum(float s, unsigned delta) {
+    return -fmaxf(1.0f, __int_as_float(__float_as_int(0.6125f * s) + int(delta) - 1));
+}
 __device__ __forceinline__ float precon_of(float w) { return w == 0.0f ? 1.0f : 1.0f / w; }  // initPrecon :1409
 
-// The three upper faces' coefficients of a cell as Q3 has them when they are another cell's lower
-// ones, (char) of the float: their magnitudes, 0 to 128, in one word (right, up, front), and one of
-// them as a float again (the byte under the exponent of 2^23, which is then taken off: two full-rate
-// instructions, where the conversion runs at an eighth of that)
-__device__ __forceinline__ unsigned pack_trunc(float cr, float cu, float cf) {
-    return unsigned(-char_trunc(cr)) | unsigned(-char_trunc(cu)) << 8 | unsigned(-char_trunc(cf)) << 16;
+// What the matrix-free operator needs of a cell besides its reciprocal density, one word: the three upper
+// faces' coefficients as Q3 has them when they are another cell's lower ones, (char) of the float, their
+// magnitudes 0 to 128 in a byte each (right, up, front), and four coef_deltas of two bits: the same
+// faces' and that of a lower face that leaves the grid (the own density on both sides).
+__device__ __forceinline__ unsigned pack_faces(float cr, float cu, float cf, float sr, float su, float sf, float sown) {
+    return unsigned(-char_trunc(cr)) | unsigned(-char_trunc(cu)) << 8 | unsigned(-char_trunc(cf)) << 16 | coef_delta(sr) << 24 |
+           coef_delta(su) << 26 | coef_delta(sf) << 28 | coef_delta(sown) << 30;
 }
+// a truncated coefficient as a float again (the byte under the exponent of 2^23, which is then taken off:
+// two full-rate instructions, where the conversion runs at an eighth of that)
 template <int BYTE>
 __device__ __forceinline__ float trunc_of(unsigned w) {
     return 8388608.0f - __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440 + BYTE));
 }
+enum { FACE_R = 24, FACE_U = 26, FACE_F = 28, FACE_OWN = 30 };  // the deltas' places
+template <int FACE>
+__device__ __forceinline__ unsigned delta_of(unsigned w) { return (w >> FACE) & 3u; }
 
 // resetVelPressProj Game/kernelSky.cu:1648-1682; one thread per (x,y) marching z.
 // reference=1 returns at the first ground cell of the column (Q8).
@@ -121,8 +128,9 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
             ay[c] = cu;
             az[c] = cf;
         } else {
-            ax[c] = 1.0f / cur;  // the matrix-free operator's inputs
-            reinterpret_cast<unsigned*>(ay)[c] = pack_trunc(cr, cu, cf);
+            const float ri = 1.0f / cur;
+            ax[c] = ri;  // the matrix-free operator's inputs
+            reinterpret_cast<unsigned*>(ay)[c] = pack_faces(cr, cu, cf, ri + 1.0f / nr, ri + 1.0f / nu, ri + 1.0f / nf, ri + ri);
         }
         float wd = 0.0f;
         wd -= cr; wd -= cl; wd -= cu; wd -= cd; wd -= cf; wd -= cb;
@@ -434,9 +442,9 @@ struct Dirs {
 };
 
 // s_new = z + beta s_old, As = A s_new, s_new.As -> alpha. Matrix-free: a face's coefficient comes
-// from the reciprocal densities of its two cells (rinv, 0 in ground cells). REF: the lower coefficients
-// as Q3 truncates them, three bytes of a word per cell (truncating in place, with the test that keeps
-// the reference's value, cost as much as the rest of the kernel).
+// from the reciprocal densities of its two cells (0 in ground cells) and its delta in the cell's word
+// (pack_faces), bit for bit the stored coefficient. REF: the lower coefficients as Q3 truncates them, from
+// the word too.
 // A block covers 128 x cells (a warp of four-cell lanes) by OPR rows and marches a run of z planes. The
 // four inputs stream through a ring of OPSLOTS shared-memory slots, each plane's boxes (the block's
 // cells, 4 more on either side so that the copies start on 16-byte boundaries, a row above and
@@ -445,10 +453,9 @@ struct Dirs {
 // densities of the planes behind and at hand in registers and takes its neighbours from the slot; one
 // barrier a plane frees the slot. s_old and s_new are distinct buffers (a block's halo rows are another
 // block's own rows). FIRST: the direction is z itself.
-// What bounds it: HBM, 24 bytes a cell (20 in the textbook form) where the stored coefficients and the
-// pressure made 40: 290 us a launch at 512x512x256, 5.6 TB/s (421 before); the barrier of a plane takes
-// the rest. An iteration with its residual and a quarter of the pressure's update went from 635 to 510
-// us, at 256x256x128 from 103 to 81. Loading the planes into registers instead of the ring left the
+// What bounds it: HBM, 24 bytes a cell where the stored coefficients and the pressure made 40 (421 us a
+// launch at 512x512x256 then, about 290 now: 5.5 TB/s); the barrier of a plane takes the rest. An iteration with its residual and a quarter of the pressure's update went from 635 to 514
+// us, at 256x256x128 from 103 to 82. Loading the planes into registers instead of the ring left the
 // lanes waiting (400 us, DRAM 48 % busy; with a plane's loads ahead and 512 threads a block 460). Tiles
 // of 16 rows with 4 or 5 slots: 516 and 518 us an iteration, 20 rows 527, 24 rows 550, 12 rows two blocks
 // per SM 531, 8 rows with 5 slots 532.
@@ -468,7 +475,7 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
     extern __shared__ __align__(128) unsigned char op_smem[];
     float* const ring = reinterpret_cast<float*>(op_smem);
     uint64_t* const bar = reinterpret_cast<uint64_t*>(ring + OPSLOTS * 4 * OPBOX);
-    constexpr unsigned BYTES = OPW * (OPR + 2) * 4 * (2 + !FIRST + REF);
+    constexpr unsigned BYTES = OPW * (OPR + 2) * 4 * (3 + !FIRST);
     const float beta = sc->beta_f;
     const int tid = threadIdx.x, lane = tid & 31, wy = tid >> 5;
     const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY;
@@ -488,7 +495,7 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
         tma_load_3d(d, &maps.z, &bar[s], bx - 4, yb - 1, q);
         if (!FIRST) tma_load_3d(d + OPBOX, &maps.s, &bar[s], bx - 4, yb - 1, q);
         tma_load_3d(d + 2 * OPBOX, &maps.r, &bar[s], bx - 4, yb - 1, q);
-        if (REF) tma_load_3d(d + 3 * OPBOX, &maps.w, &bar[s], bx - 4, yb - 1, q);
+        tma_load_3d(d + 3 * OPBOX, &maps.w, &bar[s], bx - 4, yb - 1, q);
     };
     if (tid == 0) {
         for (int s = 0; s < OPSLOTS; ++s) mbar_init(&bar[s], 1);
@@ -516,8 +523,8 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
     auto rho4 = [&](const float* d, int o) { return ld4(d + 2 * OPBOX, o); };
     auto word4 = [&](const float* d, int o) { return *reinterpret_cast<const uint4*>(d + 3 * OPBOX + o); };
     // the coefficient between a cell of reciprocal density a and its neighbour b; 0 where one is ground
-    auto coef = [&](float a, float b) {
-        const float c = coef_of_sum(a + b);
+    auto coef = [&](float a, float b, unsigned delta) {
+        const float c = coef_of_sum(a + b, delta);
         return FLAT || (a != 0.0f && b != 0.0f) ? c : 0.0f;
     };
 
@@ -529,12 +536,19 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
     if (zs > 0) {
         vb = dir4(d0, own);
         rb = rho4(d0, own);
-        if (REF) wb = word4(d0, own);
+        wb = word4(d0, own);
         d0 = wait_plane(zs);
     }
     float4 vc = dir4(d0, own), rc = rho4(d0, own);
-    if (zs == 0) rb = rc;  // outside the grid: the own density (NEUMANN)
-    cB = make_float4(coef(rc.x, rb.x), coef(rc.y, rb.y), coef(rc.z, rb.z), coef(rc.w, rb.w));
+    if (zs == 0) {  // outside the grid: the own density (NEUMANN)
+        const uint4 w = word4(d0, own);
+        rb = rc;
+        cB = make_float4(coef(rc.x, rb.x, delta_of<FACE_OWN>(w.x)), coef(rc.y, rb.y, delta_of<FACE_OWN>(w.y)),
+                         coef(rc.z, rb.z, delta_of<FACE_OWN>(w.z)), coef(rc.w, rb.w, delta_of<FACE_OWN>(w.w)));
+    } else {
+        cB = make_float4(coef(rc.x, rb.x, delta_of<FACE_F>(wb.x)), coef(rc.y, rb.y, delta_of<FACE_F>(wb.y)),
+                         coef(rc.z, rb.z, delta_of<FACE_F>(wb.z)), coef(rc.w, rb.w, delta_of<FACE_F>(wb.w)));
+    }
     bool stuck = false;
     for (int z = zs; z < ze; ++z) {
         float4 vf = f4zero(), rf = rc;
@@ -547,19 +561,17 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
         if (y < Y) {
             const float4 vd = dir4(d0, own - OPW), rd = rho4(d0, own - OPW), vu = dir4(d0, own + OPW);
             const float4 ru = top ? rc : rho4(d0, own + OPW);
-            uint4 w = make_uint4(0, 0, 0, 0), wd4 = w;
-            unsigned wl = 0;
-            if (REF) {
-                w = word4(d0, own);
-                wd4 = word4(d0, own - OPW);
-                wl = reinterpret_cast<const unsigned*>(d0 + 3 * OPBOX)[own - 1];
-            }
+            const uint4 w = word4(d0, own), wd4 = word4(d0, own - OPW);
+            const unsigned wl = reinterpret_cast<const unsigned*>(d0 + 3 * OPBOX)[own - 1];
             const float sl = dir1(d0, own - 1), sr = rend ? 0.0f : dir1(d0, own + 4);
             const float rl = lend ? rc.x : d0[2 * OPBOX + own - 1], rr = rend ? rc.w : d0[2 * OPBOX + own + 4];
-            const float4 cR = make_float4(coef(rc.x, rc.y), coef(rc.y, rc.z), coef(rc.z, rc.w), coef(rc.w, rr));
-            auto cell = [&](float v, float r, float vl, float cL, unsigned wL, float vr, float cr, float vdn, float rdn, unsigned wD, float vup,
-                            float rup, float vbk, float& cb, unsigned wB, float vfr, float rfr) {
-                const float cU = coef(r, rup), cF = coef(r, rfr), cD = below ? coef(r, rdn) : 0.0f;
+            const float4 cR = make_float4(coef(rc.x, rc.y, delta_of<FACE_R>(w.x)), coef(rc.y, rc.z, delta_of<FACE_R>(w.y)),
+                                          coef(rc.z, rc.w, delta_of<FACE_R>(w.z)), coef(rc.w, rr, delta_of<FACE_R>(w.w)));
+            const float cl = coef(rc.x, rl, lend ? delta_of<FACE_OWN>(w.x) : delta_of<FACE_R>(wl));
+            auto cell = [&](float v, float r, unsigned wo, float vl, float cL, unsigned wL, float vr, float cr, float vdn, float rdn,
+                            unsigned wD, float vup, float rup, float vbk, float& cb, unsigned wB, float vfr, float rfr) {
+                const float cU = coef(r, rup, delta_of<FACE_U>(wo)), cF = coef(r, rfr, delta_of<FACE_F>(wo));
+                const float cD = below ? coef(r, rdn, delta_of<FACE_U>(wD)) : 0.0f;
                 float wd = 0.0f;
                 wd -= cr; wd -= cL; wd -= cU; wd -= cD; wd -= cF; wd -= cb;
                 const float aL = REF ? trunc_of<0>(wL) : cL, aD = REF ? trunc_of<1>(wD) : cD, aB = REF ? trunc_of<2>(wB) : cb;
@@ -567,10 +579,10 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
                 return wd * v + ((aL * vl + aD * vdn + aB * vbk + cr * vr + cU * vup + cF * vfr));
             };
             float4 o;
-            o.x = cell(vc.x, rc.x, sl, coef(rc.x, rl), wl, vc.y, cR.x, vd.x, rd.x, wd4.x, vu.x, ru.x, vb.x, cB.x, wb.x, vf.x, rf.x);
-            o.y = cell(vc.y, rc.y, vc.x, cR.x, w.x, vc.z, cR.y, vd.y, rd.y, wd4.y, vu.y, ru.y, vb.y, cB.y, wb.y, vf.y, rf.y);
-            o.z = cell(vc.z, rc.z, vc.y, cR.y, w.y, vc.w, cR.z, vd.z, rd.z, wd4.z, vu.z, ru.z, vb.z, cB.z, wb.z, vf.z, rf.z);
-            o.w = cell(vc.w, rc.w, vc.z, cR.z, w.z, sr, cR.w, vd.w, rd.w, wd4.w, vu.w, ru.w, vb.w, cB.w, wb.w, vf.w, rf.w);
+            o.x = cell(vc.x, rc.x, w.x, sl, cl, wl, vc.y, cR.x, vd.x, rd.x, wd4.x, vu.x, ru.x, vb.x, cB.x, wb.x, vf.x, rf.x);
+            o.y = cell(vc.y, rc.y, w.y, vc.x, cR.x, w.x, vc.z, cR.y, vd.y, rd.y, wd4.y, vu.y, ru.y, vb.y, cB.y, wb.y, vf.y, rf.y);
+            o.z = cell(vc.z, rc.z, w.z, vc.y, cR.y, w.y, vc.w, cR.z, vd.z, rd.z, wd4.z, vu.z, ru.z, vb.z, cB.z, wb.z, vf.z, rf.z);
+            o.w = cell(vc.w, rc.w, w.w, vc.z, cR.z, w.z, sr, cR.w, vd.w, rd.w, wd4.w, vu.w, ru.w, vb.w, cB.w, wb.w, vf.w, rf.w);
             if (FLAT) {
                 if (y == 0) o = f4zero();
             } else {
@@ -979,11 +991,11 @@ __device__ __forceinline__ void face_of(float c, float rc, float n, float rn, fl
     // hm(n) = 2/(1/c + 1/n) and coef_of(c, n), both 0 across a zero density
     if (n == 0.0f) { h = 0.0f; coef = 0.0f; return; }
     h = 2.0f / (rc + rn);
-    coef = coef_stored(rc + rn);
+    coef = -fmaxf(1.0f, 1.225f / h);
     (void)c;
 }
 // FACES: the three face coefficients are stored; otherwise, in the places of the first two,
-// what k_pcg_operator4 reads: the reciprocal densities and the truncated coefficients.
+// what k_pcg_operator4 reads: the reciprocal densities and the words of pack_faces.
 template <bool FACES>
 __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* __restrict__ rho, const float* __restrict__ u,
                                                 const float* __restrict__ v, const float* __restrict__ w,
@@ -1093,8 +1105,11 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
                 *reinterpret_cast<float4*>(az + c) = oaz;
                 *reinterpret_cast<float4*>(As + c) = z4;
             } else {
-                *reinterpret_cast<uint4*>(ay + c) = make_uint4(pack_trunc(oax.x, oay.x, oaz.x), pack_trunc(oax.y, oay.y, oaz.y),
-                                                               pack_trunc(oax.z, oay.z, oaz.z), pack_trunc(oax.w, oay.w, oaz.w));
+                *reinterpret_cast<uint4*>(ay + c) =
+                    make_uint4(pack_faces(oax.x, oay.x, oaz.x, rc.x + rc.y, rc.x + ru.x, rc.x + rf.x, rc.x + rc.x),
+                               pack_faces(oax.y, oay.y, oaz.y, rc.y + rc.z, rc.y + ru.y, rc.y + rf.y, rc.y + rc.y),
+                               pack_faces(oax.z, oay.z, oaz.z, rc.z + rc.w, rc.z + ru.z, rc.z + rf.z, rc.z + rc.z),
+                               pack_faces(oax.w, oay.w, oaz.w, rc.w + rr, rc.w + ru.w, rc.w + rf.w, rc.w + rc.w));
             }
             *reinterpret_cast<float4*>(aw + c) = oaw;
             *reinterpret_cast<float4*>(r + c) = orr;
