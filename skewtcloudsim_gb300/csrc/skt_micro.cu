@@ -41,7 +41,7 @@ __device__ __forceinline__ void add_rates(const float (&v)[kRates], bool inside,
 // registers instead of three global arrays. RATES: also the region-summed process amounts.
 // What bounds it: the powers and exponentials of cells with condensate, and warps that hold both kinds
 // of cells; in clear air HBM (64 bytes a cell). At 512x256x512 with an eighth of the cells in cloud: 6.73
-// ms with every process forming its own powers in every cell, 2.89 with the shared terms and the exit.
+// ms with every process forming its own powers in every cell, 3.18 with the shared terms and the exit.
 template <bool RATES>
 __global__ void __launch_bounds__(256) k_micro(Grid g, float* __restrict__ qv_, float* __restrict__ qw_, float* __restrict__ qc_,
                                                float* __restrict__ qr_, float* __restrict__ qs_, float* __restrict__ qi_,
@@ -88,54 +88,47 @@ __global__ void __launch_bounds__(256) k_micro(Grid g, float* __restrict__ qv_, 
     // would take from (PSDEP is multiplied by PT1 = 0 and PSSUB limited by Qs = 0).
     if (Qw > 0.0f || Qc > 0.0f || Qr > 0.0f || Qs > 0.0f || Qi > 0.0f) {
         const Air air(t, ps, D);
-        const Slope S(slopePrecip(D, Qs, 1));
-        const float s14 = root4(S.s);
+        const float sR = slopePrecip(D, Qr, 0), sS = slopePrecip(D, Qs, 1);
         PIDW = M.FPIDW(dt, t, Qc, Qw, D, ps);
         PIHOM = M.FPIHOM(t, Qw);
         PRAUT = M.FPRAUT(Qw, QwMin, t);
         PSAUT = M.FPSAUT(t, Qc, QcMin);
-        PSDEP = M.FPSDEP(t, ps, Qv, QWI, D, air, S, s14);
+        PSDEP = M.FPSDEP(t, ps, Qv, QWI, D, air, sS);
         PSSUB = M.FPSSUB(PSDEP);
         PSDEP = fmaxf(0.0f, PSDEP);
-        // fall speeds: of rain alone where any species falls (the reference's else-if chain)
-        float UR = 0.0f;
-        const float US = 0.0f, UI = 0.0f;
-        const Slope R(slopePrecip(D, Qr, 0));
-        float r08 = 0.0f;
-        if (Qr > 0.0f || Qs > 0.0f || Qi > 0.0f) {
-            r08 = powf(R.s, 0.8f);
-            UR = 2115.0f * (M.G.Qr / (6 * r08)) * sqrtf(1.225f / D);
-            UR *= 0.01f;
-        }
+        float UR = 0.0f, US = 0.0f, UI = 0.0f;
+        if (Qr > 0.0f || Qs > 0.0f || Qi > 0.0f) fallingVelocity(Qr, Qs, Qi, D, 3, M.G.Qr, M.G.Qs, M.G.Qi, UR, US, UI);
         if (Qr > 0.0f) {
-            PIACR = M.FPIACR(Qr, Qc, air, R, r08);
-            PRACI = M.FPRACI(Qr, Qc, air, R, r08);
-            PRACW = M.FPRACW(Qr, Qw, air, R, r08);
-            PREVP = M.FPREVP(t, Qr, Qv, QWS, D, air, R, PT1);
-            PRACS = M.FPRACS(Qr, Qs, PT2, UR, US, D, S, R);
-            PSACR = M.FPSACR(Qr, Qs, UR, US, D, R, S);
-            PGFR = M.FPGFR(t, Qr, D, R);
+            const float r38 = powf(sR, 3 + 0.8f);
+            PIACR = M.FPIACR(Qr, Qc, air, sR);
+            PRACI = M.FPRACI(Qr, Qc, air, r38);
+            PRACW = M.FPRACW(Qr, Qw, air, r38);
+            PREVP = M.FPREVP(t, Qr, Qv, QWS, D, air, sR, PT1);
+            PRACS = M.FPRACS(Qr, Qs, PT2, UR, US, D, sS, sR);
+            PSACR = M.FPSACR(Qr, Qs, UR, US, D, sR, sS);
+            PGFR = M.FPGFR(t, Qr, D, sR);
         }
         if (Qs > 0.0f) {
-            PSACW = M.FPSACW(Qs, Qw, air, S, s14);
-            PSACI = M.FPSACI(t, Qs, Qc, air, S, s14);
-            PSFW = M.FPSFW(dt, t, ps, Qs, Qw, Qc, Qv, QWI, D, air);
+            const float s325 = powf(sS, 3 + 0.25f);
+            PSACW = M.FPSACW(Qs, Qw, air, s325);
+            PSACI = M.FPSACI(t, Qs, Qc, air, s325);
+            PSFW = M.FPSFW(dt, t, Qs, Qw, Qc, Qv, QWI, D, air);
             PSFI = M.FPSFI(t, Qs, Qc, Qv, QWI, air);
-            PSMLT = M.FPSMLT(t, ps, Qs, Qv, air, S, s14, PSACW, PSACR);
+            PSMLT = M.FPSMLT(t, ps, Qs, Qv, D, air, sS, PSACW, PSACR);
             PGAUT = M.FPGAUT(t, Qs, QiMin);
         }
         if (Qi > 0.0f) {
-            const Slope I(slopePrecip(D, Qi, 2));
-            const float i12 = sqrtf(I.s);
-            PGACW = M.FPGACW(Qi, Qw, I, i12, D);
-            PGACI = M.FPGACI(Qi, Qc, I, i12, D);
-            PGACR = M.FPGACR(Qi, Qr, D, UR, UI, R, I);
-            PGACS = M.FPGACS(t, Qs, Qi, D, US, UI, S, I, false);
-            const float PGACS1 = t >= 0 ? PGACS : M.FPGACS(t, Qs, Qi, D, US, UI, S, I, true);
-            PGSUB = M.FPGSUB(t, ps, Qv, QWI, Qi, D, air, I, i12);
-            PGMLT = M.FPGMLT(t, ps, Qw, Qr, Qi, Qv, D, air, I, i12, PGACW, PGACR, dtS);
+            const float sI = slopePrecip(D, Qi, 2);
+            const float i35 = powf(sI, 3.5f);
+            PGACW = M.FPGACW(Qi, Qw, i35, D);
+            PGACI = M.FPGACI(Qi, Qc, i35, D);
+            PGACR = M.FPGACR(Qi, Qr, D, UR, UI, sR, sI);
+            PGACS = M.FPGACS(t, Qs, Qi, D, US, UI, sS, sI, false);
+            const float PGACS1 = t >= 0 ? PGACS : M.FPGACS(t, Qs, Qi, D, US, UI, sS, sI, true);
+            PGSUB = M.FPGSUB(t, ps, Qv, QWI, Qi, D, air, sI);
+            PGMLT = M.FPGMLT(t, ps, Qw, Qr, Qi, Qv, D, air, sI, PGACW, PGACR, dtS);
             PGDRY = M.FPGDRY(Qw, Qc, Qr, Qs, PGACW, PGACI, PGACR, PGACS, dtS);
-            PGWET = M.FPGWET(t, ps, Qc, Qs, Qi, Qv, D, air, I, i12, PGACI, PGACS1, dtS);
+            PGWET = M.FPGWET(t, ps, Qc, Qs, Qi, Qv, D, air, sI, PGACI, PGACS1, dtS);
             PGACR1 = M.FPGACR1(Qw, Qc, Qs, Qi, PGWET, PGACW, PGACI, PGACS1, dtS);
         }
     }

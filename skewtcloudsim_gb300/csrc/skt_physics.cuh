@@ -35,13 +35,8 @@ __device__ __forceinline__ float pwater(float t) {                              
 __device__ __forceinline__ float Lwater(float t) { return (2500.8f - 2.36f * t + 0.0016f * t * t - 0.00006f * t * t * t) * 1e3f; }  // :108
 __device__ __forceinline__ float Lice(float t) { return (2834.1f - 0.29f * t - 0.004f * t * t) * 1e3f; }  // :117
 __device__ __forceinline__ float DQVair(float t, float p) { return 2.26e-5f * powf((t + 273.15f) / 273.15f, 1.94f) * (1013.25f / p); }  // :146
-// Powers of one fixed exponent are products and square and cube roots: a root is rounded once, where
-// powf forms a logarithm and an exponential and is 2 to 4 ulp off, at five to ten times the instructions.
-__device__ __forceinline__ float root4(float a) { return sqrtf(sqrtf(a)); }
-__device__ __forceinline__ float sq(float a) { return a * a; }
 __device__ __forceinline__ float ViscAir(float t) {                                                                  // :155
-    const float r = (t + 273.15f) / 273.15f;
-    return r * sqrtf(r) * ((273.15f + 111.0f) / (t + 111.0f)) * 1.716e-5f;
+    return powf((t + 273.15f) / 273.15f, 3.0f / 2.0f) * ((273.15f + 111.0f) / (t + 111.0f)) * 1.716e-5f;
 }
 __device__ __forceinline__ float slopePrecip(float D, float Q, int type) {                                              // :167
     float num;
@@ -50,7 +45,7 @@ __device__ __forceinline__ float slopePrecip(float D, float Q, int type) {      
     else if (type == 2) num = KC::PI * 0.91f * 4e-4f;
     else return 0.0f;
     const float den = fmaxf(D * Q * 0.001f, 1e-14f);
-    return root4(num / den);
+    return powf(num / den, 0.25f);
 }
 // Game/meteoformulas.cuh:219-260.  The else-if chain means type 3 ("all") computes rain only.
 __device__ __forceinline__ void fallingVelocity(float Qr, float Qs, float Qi, float dens, int type, float gR, float gS, float gI, float& UR, float& US, float& UI) {
@@ -63,11 +58,11 @@ __device__ __forceinline__ void fallingVelocity(float Qr, float Qs, float Qi, fl
         UR *= 0.01f;
     } else if (type == 1 || all) {
         float sS = slopePrecip(dens, Qs, 1);
-        US = 152.93f * (gS / (6 * root4(sS))) * sqrtf(1.225f / dens);
+        US = 152.93f * (gS / (6 * powf(sS, 0.25f))) * sqrtf(1.225f / dens);
         US *= 0.01f;
     } else if (type == 2 || all) {
         float sI = slopePrecip(dens, Qi, 2);
-        UI = (gI / (6 * sqrtf(sI))) * sqrtf(4 * KC::g * 100 * 0.91f / (3 * 0.6f * dens * 0.001f));
+        UI = (gI / (6 * powf(sI, 0.5f))) * powf(4 * KC::g * 100 * 0.91f / (3 * 0.6f * dens * 0.001f), 0.5f);
         UI *= 0.01f;
     }
 }
@@ -76,7 +71,7 @@ __device__ __forceinline__ float cvd(float t, float p, float dens) {            
     const float A = (KC::Ls / (KC::Ka * (t + 273.15f))) * (KC::Ls / (KC::Rsw * (t + 273.15f)) - 1);
     const float B = (KC::Rsw * (t + 273.15f) * p) / (2.21f * EI);
     const float N = 10000 * expf((12.96f * (ES - EI)) / (EI - 0.639f));
-    return 65.2f * ((sqrtf(N) * (ES - EI)) / (sqrtf(dens) * (A + B) * EI));
+    return 65.2f * ((powf(N, 0.5f) * (ES - EI)) / (powf(dens, 0.5f) * (A + B) * EI));
 }
 __device__ __forceinline__ float potentialTemp(float t, float pk, float pt) { return (t + 273.15f) * powf(pt / pk, KC::KAPPA) - 273.15f; }  // :299
 __device__ __forceinline__ float MLR(float t, float p) {                                                                 // :309
@@ -94,29 +89,23 @@ struct Gammas {
 
 // ---- Process rates, Game/microPhysics.cu:67-685 -----------------------------------------------
 // What several processes of a cell share, formed once per cell that holds any condensate (each process
-// formed them again under its own condition): the air's diffusivity and viscosity with the
-// ventilation term 0.31 Sc^(1/3) kv^(-1/2), and powers of the air's density.
+// formed them again under its own condition), by the same calls: every rate keeps its bits.
 struct Air {
-    float dQv, vent;   // DQVair, 0.31 Sc^(1/3) / sqrt(kv)
+    float dQv;         // DQVair
+    float Sc13, kvm;   // Sc^(1/3) and kv^(-1/2) of the ventilation terms, Sc = kv / dQv
     float dens2;       // (1.225 / D)^(1/2)
-    float dens4;       // (1.225 / D)^(1/4)
     __device__ __forceinline__ Air(float t, float ps, float D) {
         dQv = DQVair(t, ps);
         const float kv = ViscAir(t);
-        vent = 0.31f * cbrtf(kv / dQv) / sqrtf(kv);
-        dens2 = sqrtf(1.225f / D);
-        dens4 = sqrtf(dens2);
+        const float Sc = kv / dQv;
+        Sc13 = powf(Sc, 1.0f / 3.0f);
+        kvm = powf(kv, -0.5f);
+        dens2 = powf(1.225f / D, 0.5f);
     }
 };
-// a species' slope and the powers of it that its processes take
-struct Slope {
-    float s, p2, p3, p6;  // s, s^2, s^3, s^6
-    __device__ __forceinline__ explicit Slope(float v) : s(v), p2(v * v), p3(v * v * v), p6(sq(v * v * v)) {}
-};
 // the collection kernel of two falling species: 5/(a^6 b) + 2/(a^5 b^2) + 1/2/(a^4 b^3)
-__device__ __forceinline__ float collect(const Slope& a, const Slope& b) {
-    const float a4 = a.p2 * a.p2;
-    return 5 / (a.p6 * b.s) + (2 / (a4 * a.s * b.p2)) + (0.5f / (a4 * b.p3));
+__device__ __forceinline__ float collect(float a, float b) {
+    return (5 / (powf(a, 6.0f) * b) + (2 / (powf(a, 5.0f) * powf(b, 2.0f))) + (0.5f / (powf(a, 4.0f) * powf(b, 3.0f))));
 }
 struct Micro {
     Gammas G;
@@ -131,21 +120,27 @@ struct Micro {
         return 1 / (dt * sp) * (Qv - QWI) / (1 + KC::Ls / KC::Cpd * der);
     }
     __device__ float FPIMLT(float t, float Qc) const { return t >= 0 ? Qc : 0.0f; }  // :88
-    __device__ float FPIDW(float dt, float t, float Qc, float Qw, float D, float ps) const {  // :99, a = 1/2
+    __device__ float FPIDW(float dt, float t, float Qc, float Qw, float D, float ps) const {  // :99
         if (t < 0 && Qw > 0) {
+            const float a = 0.5f;
             const float quu = fmaxf(1e-12f * Ni(t) / (D * 0.001f), Qc);
-            return sq(0.5f * cvd(t, ps, D * 0.001f) * dt + sqrtf(quu)) - Qc;
+            return powf((1 - a) * cvd(t, ps, D * 0.001f) * dt + powf(quu, 1 - a), 1 / (1 - a)) - Qc;
         }
         return 0;
     }
     __device__ float FPIHOM(float t, float Qw) const { return (t < -40 && Qw > 0) ? Qw : 0.0f; }  // :115
-    // r08: the rain slope to the power 0.8
-    __device__ float FPIACR(float Qr, float Qc, const Air& A, const Slope& R, float r08) const {  // :124
-        if (Qr > 0 && Qc > 0) return (KC::PI * KC::PI * 0.3f * 8e-2f * 2115.0f * Qc * 0.99f * G.RC) / (24 * 4.19e-10f * (R.p6 * r08)) * A.dens2;
+    __device__ float FPIACR(float Qr, float Qc, const Air& A, float sR) const {  // :124
+        if (Qr > 0 && Qc > 0) {
+            const float dens = A.dens2;
+            return (KC::PI * KC::PI * 0.3f * 8e-2f * 2115.0f * Qc * 0.99f * G.RC) / (24 * 4.19e-10f * powf(sR, 6 + 0.8f)) * dens;
+        }
         return 0;
     }
-    __device__ float FPRACI(float Qr, float Qc, const Air& A, const Slope& R, float r08) const {  // :147
-        if (Qr > 0 && Qc > 0) return (KC::PI * 0.3f * 8e-2f * 2115.0f * Qc * G.R) / (4 * (R.p3 * r08)) * A.dens2;
+    __device__ float FPRACI(float Qr, float Qc, const Air& A, float r38) const {  // :147
+        if (Qr > 0 && Qc > 0) {
+            const float dens = A.dens2;
+            return (KC::PI * 0.3f * 8e-2f * 2115.0f * Qc * G.R) / (4 * r38) * dens;
+        }
         return 0;
     }
     __device__ float FPRAUT(float Qw, float QwMin, float t) const {  // :167 (note 4 / 3 is integer division in the reference)
@@ -156,58 +151,74 @@ struct Micro {
             const float disE = 0.5f * 0.5f;
             const float disp = ((1 + 3 * disE) * (1 + 4 * disE) * (1 + 5 * disE)) / ((1 + disE) * (1 + 2 * disE));
             const float L = Qw * 1.225f * 1e-3f;
-            return 1e3f * 1.1e10f * disp * (L * L * L) * (1.0f / Nc) * float(1 - expf(-(1.03e16f * (1.0f / sq(cbrtf(Nc))) * (L * L))));
+            return 1e3f * 1.1e10f * disp * (L * L * L) * powf(Nc, -1.0f) *
+                   float(1 - expf(-powf(1.03e16f * powf(Nc, -2.0f / 3.0f) * (L * L), 1.0f)));
         }
         return 0;
     }
-    __device__ float FPRACW(float Qr, float Qw, const Air& A, const Slope& R, float r08) const {  // :189
-        if (Qr > 0 && Qw > 0) return (KC::PI * 1.0f * 8e-2f * 2115.0f * Qw * G.R) / (4 * (R.p3 * r08)) * A.dens2;
+    __device__ float FPRACW(float Qr, float Qw, const Air& A, float r38) const {  // :189
+        if (Qr > 0 && Qw > 0) {
+            const float dens = A.dens2;
+            return (KC::PI * 1.0f * 8e-2f * 2115.0f * Qw * G.R) / (4 * r38) * dens;
+        }
         return 0;
     }
-    __device__ float FPREVP(float t, float Qr, float Qv, float QWS, float D, const Air& A, const Slope& R, float PT1) const {  // :210
+    __device__ float FPREVP(float t, float Qr, float Qv, float QWS, float D, const Air& air, float sR, float PT1) const {  // :210
         if (Qr > 0 && Qv / QWS < 1 && (1 - PT1) != 0) {
-            const float tK = t + 273.15f, S = Qv / QWS;
-            const float dens = root4(1.225f / (D * 0.001f));
+            const float tK = t + 273.15f, S = Qv / QWS, b = 0.8f, a = 2115.0f;
+            const float dQv = air.dQv;
+            const float dens = powf(1.225f / (D * 0.001f), 0.25f);
             return fmaxf(0.0f, -1 * 2 * KC::PI * (S - 1) * 8e-2f *
-                                   (0.78f / R.p2 + A.vent * G.ER * sqrtf(2115.0f) * dens * powf(R.s, -2.9f)) * 1 / (D * 0.001f) *
-                                   (1.0f / (KC::E0v * KC::E0v / (KC::Ka * KC::Rsw * tK * tK) + (1 / (D * 0.001f * QWS * A.dQv)))));
+                                   (0.78f * powf(sR, -2.0f) + 0.31f * air.Sc13 * G.ER * powf(a, 0.5f) *
+                                                                   air.kvm * dens * powf(sR, -((b + 5) / 2))) *
+                                   1 / (D * 0.001f) *
+                                   powf(KC::E0v * KC::E0v / (KC::Ka * KC::Rsw * tK * tK) + (1 / (D * 0.001f * QWS * dQv)), -1.0f));
         }
         return 0;
     }
-    __device__ float FPRACS(float Qr, float Qs, float PT2, float UR, float US, float D, const Slope& S, const Slope& R) const {  // :238
+    __device__ float FPRACS(float Qr, float Qs, float PT2, float UR, float US, float D, float sS, float sR) const {  // :238
         if (Qr > 0 && Qs > 0 && PT2 == 0) {
             const float size = KC::PI * KC::PI * 1.0f * 8e-2f * 3e-2f;
-            return size * fabsf(UR - US) * (0.11f / (D * 0.001f)) * collect(S, R);
+            return size * fabsf(UR - US) * (0.11f / (D * 0.001f)) *
+                   collect(sS, sR);
         }
         return 0;
     }
-    // s14: the snow slope to the power 1/4
-    __device__ float FPSACW(float Qs, float Qw, const Air& A, const Slope& S, float s14) const {  // :263
-        if (Qs > 0 && Qw > 0) return (KC::PI * 1.0f * 3e-2f * 152.93f * Qw * G.S) / (4 * (S.p3 * s14)) * A.dens2;
+    __device__ float FPSACW(float Qs, float Qw, const Air& A, float s325) const {  // :263
+        if (Qs > 0 && Qw > 0) {
+            const float dens = A.dens2;
+            return (KC::PI * 1.0f * 3e-2f * 152.93f * Qw * G.S) / (4 * s325) * dens;
+        }
         return 0;
     }
-    __device__ float FPSACR(float Qr, float Qs, float UR, float US, float D, const Slope& R, const Slope& S) const {  // :283
+    __device__ float FPSACR(float Qr, float Qs, float UR, float US, float D, float sR, float sS) const {  // :283
         if (Qr > 0 && Qs > 0) {
             const float size = KC::PI * KC::PI * 1.0f * 8e-2f * 3e-2f;
-            return size * fabsf(US - UR) * (0.99f / (D * 0.001f)) * collect(R, S);
+            return size * fabsf(US - UR) * (0.99f / (D * 0.001f)) *
+                   collect(sR, sS);
         }
         return 0;
     }
-    __device__ float FPSACI(float t, float Qs, float Qc, const Air& A, const Slope& S, float s14) const {  // :307
-        if (Qs > 0 && Qc > 0) return (KC::PI * expf(0.025f * t) * 3e-2f * 152.93f * Qc * G.S) / (4 * (S.p3 * s14)) * A.dens2;
+    __device__ float FPSACI(float t, float Qs, float Qc, const Air& A, float s325) const {  // :307
+        if (Qs > 0 && Qc > 0) {
+            const float ESI = expf(0.025f * t);
+            const float dens = A.dens2;
+            return (KC::PI * ESI * 3e-2f * 152.93f * Qc * G.S) / (4 * s325) * dens;
+        }
         return 0;
     }
     __device__ float FPSAUT(float t, float Qc, float QcMin) const {  // :327
         if (Qc - QcMin > 0 && t < 0) return 1e-3f * expf(0.025f * t) * (Qc - QcMin);
         return 0;
     }
-    __device__ float FPSFW(float dt, float t, float ps, float Qs, float Qw, float Qc, float Qv, float QWI, float D, const Air& air) const {  // :336
+    __device__ float FPSFW(float dt, float t, float Qs, float Qw, float Qc, float Qv, float QWI, float D, const Air& air) const {  // :336
         if (Qs > 0 && Qw > 0) {
             const float tK = t + 273.15f;
             const float RI50 = 5e-3f, mI50 = 4.8e-7f, mI40 = 2.46e-7f, UI50 = 100.0f;
             float Si = Qv / QWI;
+            const float X = air.dQv;
             const float A = KC::E0v / (KC::Ka * tK) * (KC::Ls * KC::Mw * 0.001f / (KC::R * tK) - 1);
-            const float B = KC::R * tK * air.dQv * KC::Mw * 0.001f * ei(t) * 1000;
+            const float B = KC::R * tK * X * KC::Mw * 0.001f * ei(t) * 1000;
             const float a1g = 206.2f * (Si - 1) / (A + B);
             const float a2g = expf(0.09f * t);
             const float dt1 = 1 / (a1g * (1 - a2g)) * (powf(mI50, 1 - a2g) - powf(mI40, 1 - a2g));
@@ -222,35 +233,37 @@ struct Micro {
             const float tK = t + 273.15f;
             const float mI50 = 4.8e-7f, mI40 = 2.46e-7f;
             float Si = Qv / QWI;
+            const float X = air.dQv;
             const float A = KC::E0v / (KC::Ka * tK) * (KC::Ls * KC::Mw * 0.001f / (KC::R * tK) - 1);
-            const float B = KC::R * tK * air.dQv * KC::Mw * 0.001f * ei(t) * 1000;
+            const float B = KC::R * tK * X * KC::Mw * 0.001f * ei(t) * 1000;
             const float a1g = 206.2f * (Si - 1) / (A + B);
             const float a2g = expf(0.09f * t);
-            if (a1g > 0) return a2g * a1g * Qc / (sqrtf(mI50) - sqrtf(mI40));
+            if (a1g > 0) return a2g * a1g * Qc / (powf(mI50, 0.5f) - powf(mI40, 0.5f));
         }
         return 0;
     }
-    // the ventilated growth of snow: 0.78 s^-2 + 0.31 Sc^(1/3) G c^(1/2) dens kv^(-1/2) s^(-21/8)
-    __device__ __forceinline__ float snow_vent(const Air& A, const Slope& S, float s14) const {
-        return 0.78f / S.p2 + A.vent * G.SS * sqrtf(152.93f) * A.dens4 / (S.p2 * sqrtf(S.s) * sqrtf(s14));
-    }
-    __device__ float FPSDEP(float t, float ps, float Qv, float QWI, float D, const Air& air, const Slope& S, float s14) const {  // :397
+    __device__ float FPSDEP(float t, float ps, float Qv, float QWI, float D, const Air& air, float sS) const {  // :397
         if (t < 0) {
-            const float tK = t + 273.15f;
+            const float tK = t + 273.15f, c = 152.93f, d = 0.25f;
+            const float dQv = air.dQv;
             float Si = Qv / QWI;
             const float A = KC::Ls * KC::Ls / (KC::Ka * KC::Rsw * tK * tK);
-            const float B = 1 / (D * 0.001f * wi(t, ps) * air.dQv);
-            return KC::PI * KC::PI * (Si - 1) / (D * 0.001f * (A + B)) * 3e-2f * snow_vent(air, S, s14);
+            const float B = 1 / (D * 0.001f * wi(t, ps) * dQv);
+            const float dens = powf(1.225f / D, 0.25f);
+            return KC::PI * KC::PI * (Si - 1) / (D * 0.001f * (A + B)) * 3e-2f *
+                   (0.78f * powf(sS, -2.0f) + 0.31f * air.Sc13 * G.SS * powf(c, 0.5f) * dens * air.kvm * powf(sS, -(d + 5) / 2));
         }
         return 0;
     }
     __device__ float FPSSUB(float PSDEP) const { return fmaxf(0.0f, -1 * PSDEP); }  // :424
-    __device__ float FPSMLT(float t, float ps, float Qs, float Qv, const Air& A, const Slope& S, float s14, float PSACW, float PSACR) const {  // :429
+    __device__ float FPSMLT(float t, float ps, float Qs, float Qv, float D, const Air& air, float sS, float PSACW, float PSACR) const {  // :429
         if (t >= 0 && Qs > 0) {
+            const float c = 152.93f, d = 0.25f;
+            const float dQv = air.dQv;
             const float Drs = ws(0.0f, ps) - Qv;
-            const float dens = A.dens4;
-            return fmaxf(0.0f, -1 * (-(2 * KC::PI / (dens * 0.001f * KC::Lf)) * (KC::Ka * t - KC::E0v * A.dQv * dens * 0.001f * Drs) * 3e-2f *
-                                        snow_vent(A, S, s14) -
+            const float dens = powf(1.225f / D, 0.25f);
+            return fmaxf(0.0f, -1 * (-(2 * KC::PI / (dens * 0.001f * KC::Lf)) * (KC::Ka * t - KC::E0v * dQv * dens * 0.001f * Drs) * 3e-2f *
+                                        (0.78f * powf(sS, -2.0f) + 0.31f * air.Sc13 * G.SS * powf(c, 0.5f) * dens * air.kvm * powf(sS, -(d + 5) / 2)) -
                                     (KC::Cvl * t / KC::Lf) * (PSACW + PSACR)));
         }
         return 0;
@@ -260,75 +273,80 @@ struct Micro {
         if (sur > 0 && t < 0) return (1e-3f * expf(0.09f * t)) * sur;
         return 0;
     }
-    __device__ float FPGFR(float t, float Qr, float D, const Slope& R) const {  // :472
-        if (Qr > 0 && t < 0) return 20 * KC::PI * KC::PI * 100.0f * 8e-2f * (0.99f / (D * 0.001f)) * (expf(0.66f * (-t)) - 1) / (R.p6 * R.s);
+    __device__ float FPGFR(float t, float Qr, float D, float sR) const {  // :472
+        if (Qr > 0 && t < 0)
+            return 20 * KC::PI * KC::PI * 100.0f * 8e-2f * (0.99f / (D * 0.001f)) * (expf(0.66f * (-t)) - 1) * powf(sR, -7.0f);
         return 0;
     }
-    __device__ float gfact(float D) const { return sqrtf(4 * KC::g * 100 * 0.91f / (3 * 0.6f * D * 0.001f)); }
-    // i12: the ice slope to the power 1/2
-    __device__ float FPGACW(float Qi, float Qw, const Slope& I, float i12, float D) const {  // :489
-        if (Qi > 0 && Qw > 0) return KC::PI * 1.0f * 4e-4f * Qw * G.I / (4 * (I.p3 * i12)) * gfact(D);
+    __device__ float gfact(float D) const { return powf(4 * KC::g * 100 * 0.91f / (3 * 0.6f * D * 0.001f), 0.5f); }
+    __device__ float FPGACW(float Qi, float Qw, float i35, float D) const {  // :489
+        if (Qi > 0 && Qw > 0) return KC::PI * 1.0f * 4e-4f * Qw * G.I / (4 * i35) * gfact(D);
         return 0;
     }
-    __device__ float FPGACI(float Qi, float Qc, const Slope& I, float i12, float D) const {  // :506
-        if (Qi > 0 && Qc > 0) return KC::PI * 1.0f * 4e-4f * Qc * G.I / (4 * (I.p3 * i12)) * gfact(D);
+    __device__ float FPGACI(float Qi, float Qc, float i35, float D) const {  // :506
+        if (Qi > 0 && Qc > 0) return KC::PI * 1.0f * 4e-4f * Qc * G.I / (4 * i35) * gfact(D);
         return 0;
     }
-    __device__ float FPGACR(float Qi, float Qr, float D, float UR, float UI, const Slope& R, const Slope& I) const {  // :523
-        if (Qi > 0 && Qr > 0) return KC::PI * KC::PI * 0.1f * 8e-2f * 4e-4f * fabsf(UI - UR) * (0.99f / (D * 0.001f)) * collect(R, I);
+    __device__ float FPGACR(float Qi, float Qr, float D, float UR, float UI, float sR, float sI) const {  // :523
+        if (Qi > 0 && Qr > 0)
+            return KC::PI * KC::PI * 0.1f * 8e-2f * 4e-4f * fabsf(UI - UR) * (0.99f / (D * 0.001f)) *
+                   collect(sR, sI);
         return 0;
     }
-    __device__ float FPGACS(float t, float Qs, float Qi, float D, float US, float UI, const Slope& S, const Slope& I, bool EGS1) const {  // :541
+    __device__ float FPGACS(float t, float Qs, float Qi, float D, float US, float UI, float sS, float sI, bool EGS1) const {  // :541
         if (Qs > 0 && Qi > 0) {
             const float EGS = (t >= 0 || EGS1) ? 1.0f : expf(0.09f * t);
-            return KC::PI * KC::PI * EGS * 3e-2f * 4e-4f * fabsf(UI - US) * (0.11f / (D * 0.001f)) * collect(S, I);
+            return KC::PI * KC::PI * EGS * 3e-2f * 4e-4f * fabsf(UI - US) * (0.11f / (D * 0.001f)) *
+                   collect(sS, sI);
         }
         return 0;
     }
     __device__ float FPGDRY(float Qw, float Qc, float Qr, float Qs, float PGACW, float PGACI, float PGACR, float PGACS, float dtS) const {  // :560
         return fminf(Qw, PGACW * dtS) + fminf(Qc, PGACI * dtS) + fminf(Qr, PGACR * dtS) + fminf(Qs, PGACS * dtS);
     }
-    // the ventilated growth of ice: 0.78 s^-2 + 0.31 Sc^(1/3) G dens kv^(-1/2) s^(-11/4)
-    __device__ __forceinline__ float ice_vent(const Air& A, const Slope& I, float i12, float dens) const {
-        return 0.78f / I.p2 + A.vent * G.RI * dens / (I.p2 * i12 * sqrtf(i12));
-    }
-    __device__ float FPGSUB(float t, float ps, float Qv, float QWI, float Qi, float D, const Air& air, const Slope& I, float i12) const {  // :572
+    __device__ float FPGSUB(float t, float ps, float Qv, float QWI, float Qi, float D, const Air& air, float sI) const {  // :572
         float Si = Qv / QWI;
         if (Qi > 0 && Si < 1) {
             const float tK = t + 273.15f;
+            const float dQv = air.dQv;
             const float A = KC::Ls * KC::Ls / (KC::Ka * KC::Rsw * tK * tK);
-            const float B = 1 / (D * 0.001f * wi(t, ps) * air.dQv);
-            const float dens = root4(4 * KC::g * 100 * 0.91f / (3 * 0.6f * D * 0.001f));
-            return fmaxf(0.0f, -1 * KC::PI * KC::PI * (Si - 1) / (D * 0.001f * (A + B)) * 4e-4f * ice_vent(air, I, i12, dens));
+            const float B = 1 / (D * 0.001f * wi(t, ps) * dQv);
+            const float dens = powf(4 * KC::g * 100 * 0.91f / (3 * 0.6f * D * 0.001f), 0.25f);
+            return fmaxf(0.0f, -1 * KC::PI * KC::PI * (Si - 1) / (D * 0.001f * (A + B)) * 4e-4f *
+                                  (0.78f * powf(sI, -2.0f) + 0.31f * air.Sc13 * G.RI * dens * air.kvm * powf(sI, -2.75f)));
         }
         return 0;
     }
-    __device__ float FPGMLT(float t, float ps, float Qw, float Qr, float Qi, float Qv, float D, const Air& A, const Slope& I, float i12, float PGACW, float PGACR, float dtS) const {  // :602
+    __device__ float FPGMLT(float t, float ps, float Qw, float Qr, float Qi, float Qv, float D, const Air& air, float sI, float PGACW, float PGACR, float dtS) const {  // :602
         if (Qi > 0) {
             const float L1 = fminf(Qw, PGACW * dtS), L2 = fminf(Qr, PGACR * dtS);
+            const float dQv = air.dQv;
             const float Drs = ws(0.0f, ps) - Qv;
-            const float dens = root4(4 * KC::g * 100 * 0.91f / (3 * 0.6f));
-            return fmaxf(0.0f, -1 * (-2 * KC::PI / (D * 0.001f * KC::Lf) * (KC::Ka * t - KC::E0v * A.dQv * D * 0.001f * Drs) * 4e-4f *
-                                        ice_vent(A, I, i12, dens) -
+            const float dens = powf(4 * KC::g * 100 * 0.91f / (3 * 0.6f), 0.25f);
+            return fmaxf(0.0f, -1 * (-2 * KC::PI / (D * 0.001f * KC::Lf) * (KC::Ka * t - KC::E0v * dQv * D * 0.001f * Drs) * 4e-4f *
+                                        (0.78f * powf(sI, -2.0f) + 0.31f * air.Sc13 * G.RI * dens * air.kvm * powf(sI, -2.75f)) -
                                     KC::Cvl * t / KC::Lf * (L1 + L2)));
         }
         return 0;
     }
-    // PGACS1: PGACS with the collection efficiency 1 (as PGACS itself is at t >= 0)
-    __device__ float FPGWET(float t, float ps, float Qc, float Qs, float Qi, float Qv, float D, const Air& A, const Slope& I, float i12, float PGACI, float PGACS1, float dtS) const {  // :632
+    __device__ float FPGWET(float t, float ps, float Qc, float Qs, float Qi, float Qv, float D, const Air& air, float sI, float PGACI, float PGACS1, float dtS) const {  // :632
         if (Qi > 0) {
             const float PGACI1 = PGACI * 10.0f;
             const float L1 = fminf(Qc, PGACI1 * dtS), L2 = fminf(Qs, PGACS1 * dtS);
+            const float dQv = air.dQv;
             const float Drs = ws(0.0f, ps) - Qv;
-            const float dens = root4(4 * KC::g * 100.0f * 0.91f / (3 * 0.6f));
-            return 2 * KC::PI * 4e-4f * (D * 0.001f * KC::E0v * A.dQv * Drs - KC::Ka * t) / (D * 0.001f * (KC::Lf + KC::Cvl * t)) *
-                       ice_vent(A, I, i12, dens) +
+            const float dens = powf(4 * KC::g * 100.0f * 0.91f / (3 * 0.6f), 0.25f);
+            return 2 * KC::PI * 4e-4f * (D * 0.001f * KC::E0v * dQv * Drs - KC::Ka * t) / (D * 0.001f * (KC::Lf + KC::Cvl * t)) *
+                       (0.78f * powf(sI, -2.0f) + 0.31f * air.Sc13 * G.RI * dens * air.kvm * powf(sI, -2.75f)) +
                    (L1 + L2) * (1 - KC::Cpi * t / (KC::Lf + KC::Cvl * t));
         }
         return 0;
     }
     __device__ float FPGACR1(float Qw, float Qc, float Qs, float Qi, float PGWET, float PGACW, float PGACI, float PGACS1, float dtS) const {  // :667
-        if (Qi > 0) return PGWET - fminf(Qw, PGACW * dtS) - fminf(Qc, PGACI * 10.0f * dtS) - fminf(Qs, PGACS1 * dtS);
+        if (Qi > 0) {
+            const float PGACI1 = PGACI * 10.0f;
+            return PGWET - fminf(Qw, PGACW * dtS) - fminf(Qc, PGACI1 * dtS) - fminf(Qs, PGACS1 * dtS);
+        }
         return 0;
     }
 
@@ -343,7 +361,7 @@ struct Micro {
             const float af = 0.45f;
             const float QG = af * k4 * tgC / h;
             const float melt = fmaxf(0.0f, QG / KC::Lf);
-            return melt * 4e-4f / sq(sI) * af / (D * 0.001f);
+            return melt * 4e-4f * powf(sI, -2.0f) * af / (D * 0.001f);
         }
         return 0;
     }
@@ -457,7 +475,7 @@ struct Micro {
             const float densW = 0.99f;
             const float Rr = Qr * D * UR;
             const float P = Rr * 3600.0f / (densW * 1000.0f) * 1000;
-            const float FFW = sqrtf(sq(P * densW / 3.6f) + sq(0.067f * powf(P, 0.846f) * wind));
+            const float FFW = sqrtf(powf(P * densW / 3.6f, 2.0f) + powf(0.067f * powf(P, 0.846f) * wind, 2.0f));
             Qf = KC::Lf * 0.001f * FFW;
             Qw = KC::Cvl * 0.001f * (0 - Tac) * FFW;
             const float k = 0.41f, z0m = 0.1f, z0h = z0m * 0.1f;

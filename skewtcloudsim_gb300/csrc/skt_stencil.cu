@@ -1139,7 +1139,7 @@ __global__ void __launch_bounds__(128) k_precip(Grid g, float* __restrict__ q, c
 // loads of the row two above are issued one iteration ahead.
 // The warps of a block share 32 columns, each a run of rows: a warp takes the values of the row above
 // its run, which belongs to the next warp, before any warp writes. One thread per column left a serial
-// chain of a whole column's powers and loads (262144 threads for 152 SMs): 1.94 and now 1.04 ms at
+// chain of a whole column's powers and loads (262144 threads for 152 SMs): 1.94 and now 1.15 ms at
 // 512x256x512, 67 and 14 us at 64x32x64. The speed of a species that a cell does not hold is not formed: its outflow is 0.
 __device__ __forceinline__ float precip_dens(float thv, float qvv, float pv, float pgc) {
     const float T = thv * powf(pv / pgc, KC::KAPPA);
