@@ -420,18 +420,22 @@ __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... P, class... A>
-void launch_next(const Env& e, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... a) {
+void launch_next(cudaStream_t st, bool chain, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... a) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = e.stream;
+    cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = e.capturing ? 0 : 1;
-    (void)cudaLaunchKernelEx(&cfg, k, P(a)...);  // an error is the step's to report
+    cfg.numAttrs = chain ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, k, P(a)...);  // an error is the caller's to report
+}
+template <class... P, class... A>
+void launch_next(const Env& e, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... a) {
+    launch_next(e.stream, !e.capturing, k, grid, block, smem, a...);
 }
 
 // ---- launchers (defined in the kernel translation units) --------------------------------------

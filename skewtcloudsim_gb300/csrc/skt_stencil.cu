@@ -4,6 +4,7 @@
 #include "skt_tma.cuh"
 #include "../../include/skewt.h"
 #include <algorithm>
+#include <climits>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -52,49 +53,140 @@ __device__ __forceinline__ float jacobi(float c, float l, float r, float u, floa
 }
 
 // One Jacobi sweep of the colour-split diffusion (diffuseRedBlack Game/kernelSky.cu:43-115; both
-// colours read the same input array, Game/environment.cu:651-662).
-template <bool THETA, bool MANY>
-__global__ void __launch_bounds__(256) k_diffuse(Grid g, FieldSet F, float k, const float* __restrict__ p, const float* __restrict__ Tg,
-                                                 const float* __restrict__ Pg) {
-    const int fi = F.field_of<MANY>(g.Z);
+// colours read the same input array, Game/environment.cu:651-662), any X and any terrain.
+// A lane owns GR rows of one x cell and marches a run of z planes: the planes behind, at hand and ahead and
+// the terrain's heights stay in registers, the next plane's loads are in flight, x neighbours come from the
+// lanes beside. Ghost values are ghost()'s: a cell's stand-in depends on where it lies only, so the march
+// hands it on. FLAT: the ground is the y = 0 layer; blocks start at row 1. face: theta's ground-face values
+// per column (k_theta_face), nullptr: formed here. keep: ground cells of out take its values.
+// What bounds it: instructions, then HBM (8 bytes a cell). A thread per cell that tested the ghost rules at
+// each neighbour took 12.7 ms for a step's diffusions at 256x128x256 with hills; the march with one row a
+// lane 8.3, with loads ahead 7.8, with four rows, which share the heights and hand each other their
+// neighbours along y, 4.8; 1.76 and 0.81 at 128x64x128, 0.83 and 0.33 at 90x51x75. Two rows and eight rows a lane
+// were 5.5 and 4.9.
+constexpr int GDY = 4, GR = 4;  // warps per block, rows per lane
+template <bool THETA, bool MANY, bool FLAT>
+__global__ void __launch_bounds__(32 * GDY) k_diffuse(Grid g, int zlen, int zc, FieldSet F, float k, const float* __restrict__ p,
+                                                      const float* __restrict__ Tg, const float* __restrict__ Pg, const float* __restrict__ face,
+                                                      const float* __restrict__ keep) {
+    after_previous();
+    const int fi = F.field_of<MANY>(zc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
     const float* __restrict__ def = F.def[fi];
     const int sides = F.sides[fi], ground = F.ground[fi];
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z - fi * g.Z;
-    if (x >= g.X || y >= g.Y) return;
-    if (is_ground(g, x, y, z)) return;
-    const int c = cidx(g, x, y, z);
-    float l = ghost(g, in, x - 1, y, z, sides, ground, def);
-    float r = ghost(g, in, x + 1, y, z, sides, ground, def);
-    float d = ghost(g, in, x, y - 1, z, sides, ground, def);
-    float u = ghost(g, in, x, y + 1, z, sides, ground, def);
-    float f = ghost(g, in, x, y, z + 1, sides, ground, def);
-    float b = ghost(g, in, x, y, z - 1, sides, ground, def);
-    if (THETA) {
-        const int idxG = x + z * g.X;
-        if (y > 0 && is_ground(g, x, y - 1, z)) d = theta_ground(p, Tg, Pg, c, idxG);
-        // lateral ground faces: only when isGroundLevel(z) holds for the reference's 16-wide tile
-        // launch (Q5, Game/kernelSky.cu:1684-1694): blockIdx.x == GHeight[threadIdx.x + z*Z] + 1
-        const bool gl = x > 0 && is_ground(g, x - 1, y, z), gr = x + 1 < g.X && is_ground(g, x + 1, y, z);
-        const bool gf = z + 1 < g.Z && is_ground(g, x, y, z + 1), gb = z > 0 && is_ground(g, x, y, z - 1);
-        if (gl | gr | gf | gb) {
-            const int bw = min(16, g.X);
-            int gi = (x % bw) + z * g.Z;
-            if (gi >= g.X * g.Z) gi = g.X * g.Z - 1;
-            const bool level = (x / bw) == g.gh[gi] + 1;
-            if (level) {
-                const int idxGL = x > 0 ? idxG - 1 : idxG, idxGR = x + 1 < g.X ? idxG + 1 : idxG;
-                const int idxGF = z + g.X < g.Z ? idxG + g.X : idxG;  // the reference compares z + X < Z
-                const int idxGB = z > 0 ? idxG - g.X : idxG;
-                if (gl) l = theta_ground(p, Tg, Pg, c, idxGL);
-                if (gr) r = theta_ground(p, Tg, Pg, c, idxGR);
-                if (gf) f = theta_ground(p, Tg, Pg, c, idxGF);
-                if (gb) b = theta_ground(p, Tg, Pg, c, idxGB);
+    const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY;
+    const int lane = threadIdx.x, xo = blockIdx.x * 32 + lane, y0 = (blockIdx.y * GDY + threadIdx.y) * GR + FLAT;
+    const int zs = (blockIdx.z - fi * zc) * zlen, ze = min(zs + zlen, Z);
+    if (y0 >= Y) return;  // a whole warp
+    const int x = min(xo, X - 1);  // the lanes beyond a row follow its last cell, the rows beyond the top the top one
+    const int rows = xo < X ? min(GR, Y - y0) : 0;
+    const float rinv = 1.0f / (1 + 6 * k);
+    const bool edge = (lane == 0 && x > 0) || (lane == 31 && x + 1 < X);  // its neighbour along x is in another warp
+    const int eo = lane == 0 ? -1 : 1;
+    const bool first = x == 0, last = x + 1 == X, sown = sides == NEUMANN;
+    int ro[GR];            // the rows' places from the first one's
+    float sv[GR], gv[GR + 1];  // what stands for a cell outside the domain (unless the own value does), for a ground cell
+#pragma unroll
+    for (int r = 0; r < GR; ++r) {
+        ro[r] = min(r, Y - 1 - y0) * X;
+        const float d = def ? def[min(y0 + r, Y - 1)] : 0.0f;
+        sv[r] = bc_val(sides, 0.0f, d);
+        gv[r + 1] = bc_val(ground, 0.0f, d);
+    }
+    gv[0] = bc_val(ground, 0.0f, def && y0 > 0 ? def[y0 - 1] : 0.0f);
+    const int yg = ground == NEUMANN ? INT_MAX - GR : y0;  // a ground cell under NEUMANN is seen with its own value
+    auto seen = [&](float v, int h, int r) { return !FLAT && yg + r <= h ? gv[r + 1] : v; };  // a cell of row r as a stencil sees it
+    auto height = [&](int i) { return FLAT ? 0 : __ldg(g.gh + i); };
+    int c = x + y0 * X + zs * XY, col = x + zs * X;
+    const bool has_down = y0 > 0, has_up = y0 + GR < Y;
+    float q[GR], n[GR], b[GR], ev[GR], up = 0.0f, down = 0.0f;
+    int hc = height(col), hn = zs + 1 < Z ? height(col + X) : hc, he = 0;
+    const int hb = zs > 0 ? height(col - X) : 0;
+    auto beside = [&](int cc, int cl) {  // what other warps hold of a plane: the rows above and below, a cell to the left or right
+        if (has_up) up = in[cc + GR * X];
+        if (has_down) down = in[cc - X];
+        if (edge) {
+            he = height(cl + eo);
+#pragma unroll
+            for (int r = 0; r < GR; ++r) ev[r] = in[cc + ro[r] + eo];
+        }
+    };
+#pragma unroll
+    for (int r = 0; r < GR; ++r) {
+        ev[r] = 0.0f;
+        q[r] = in[c + ro[r]];
+        n[r] = zs + 1 < Z ? in[c + ro[r] + XY] : 0.0f;
+        b[r] = zs > 0 ? seen(in[c + ro[r] - XY], hb, r) : (sown ? q[r] : sv[r]);
+    }
+    beside(c, col);
+    for (int z = zs; z < ze; ++z, c += XY, col += X) {
+        float n2[GR], e[GR];
+        const bool more = z + 2 <= ze && z + 2 < Z;
+        const int h2 = more ? height(col + 2 * X) : 0, hne = he;
+        const float un = up, dn = down;
+#pragma unroll
+        for (int r = 0; r < GR; ++r) {
+            n2[r] = more ? in[c + ro[r] + 2 * XY] : 0.0f;
+            e[r] = ev[r];
+        }
+        if (z + 1 < ze) beside(c + XY, col + X);
+        int hl = 0, hr = 0;
+        if (!FLAT) {
+            hl = __shfl_up_sync(0xffffffffu, hc, 1);
+            hr = __shfl_down_sync(0xffffffffu, hc, 1);
+            if (edge) (lane == 0 ? hl : hr) = hne;
+        }
+#pragma unroll
+        for (int r = 0; r < GR; ++r) {
+            const int y = y0 + r;
+            const float vc = q[r], s = sown ? vc : sv[r];
+            float l = __shfl_up_sync(0xffffffffu, vc, 1), rr = __shfl_down_sync(0xffffffffu, vc, 1);
+            if (edge) (lane == 0 ? l : rr) = e[r];
+            l = first ? s : seen(l, hl, r);
+            rr = last ? s : seen(rr, hr, r);
+            float f = z + 1 < Z ? seen(n[r], hn, r) : s, bb = b[r];
+            const float u = y + 1 < Y ? (r + 1 < GR ? q[r + 1 < GR ? r + 1 : r] : un) : s;
+            const float dv = r > 0 ? q[r > 0 ? r - 1 : 0] : dn;
+            const bool low = FLAT ? y == 1 : y > 0 && y - 1 <= hc;  // the cell below is ground
+            float d = y > 0 ? (low && ground != NEUMANN ? gv[r] : dv) : s;
+            if (r < rows && (FLAT || y > hc)) {
+                if (THETA && low) d = face ? __ldg(face + col) : theta_ground(p, Tg, Pg, c + r * X, col);
+                if (THETA && !FLAT) {
+                    // lateral ground faces: only when isGroundLevel(z) holds for the reference's 16-wide tile
+                    // launch (Q5, Game/kernelSky.cu:1684-1694): blockIdx.x == GHeight[threadIdx.x + z*Z] + 1
+                    const bool gl = !first && y <= hl, gr = !last && y <= hr;
+                    const bool gf = z + 1 < Z && y <= hn, gb = z > 0 && y <= __ldg(g.gh + col - X);
+                    if (gl | gr | gf | gb) {
+                        const int bw = min(16, X);
+                        int gi = (x % bw) + z * Z;
+                        if (gi >= X * Z) gi = X * Z - 1;
+                        const bool level = (x / bw) == g.gh[gi] + 1;
+                        if (level) {
+                            const int idxGL = x > 0 ? col - 1 : col, idxGR = x + 1 < X ? col + 1 : col;
+                            const int idxGF = z + X < Z ? col + X : col;  // the reference compares z + X < Z
+                            const int idxGB = z > 0 ? col - X : col;
+                            if (gl) l = theta_ground(p, Tg, Pg, c + r * X, idxGL);
+                            if (gr) rr = theta_ground(p, Tg, Pg, c + r * X, idxGR);
+                            if (gf) f = theta_ground(p, Tg, Pg, c + r * X, idxGF);
+                            if (gb) bb = theta_ground(p, Tg, Pg, c + r * X, idxGB);
+                        }
+                    }
+                }
+                out[c + r * X] = jacobi(vc, l, rr, u, d, f, bb, k, rinv);
+            } else if (keep && r < rows) {
+                out[c + r * X] = keep[c + r * X];
             }
         }
+#pragma unroll
+        for (int r = 0; r < GR; ++r) {
+            b[r] = seen(q[r], hc, r);
+            q[r] = n[r];
+            n[r] = n2[r];
+        }
+        hc = hn;
+        hn = h2;
     }
-    out[c] = jacobi(in[c], l, r, u, d, f, b, k, 1.0f / (1 + 6 * k));
 }
 
 // Vectorised sweep for flat terrain (ground = the y = 0 layer) and X % 4 == 0: four cells per
@@ -104,13 +196,14 @@ constexpr int DVY = 16;  // rows per block: the rows above and below come mostly
 __device__ __forceinline__ float4 ld4f(const float* p, int c) { return *reinterpret_cast<const float4*>(p + c); }
 __device__ __forceinline__ float side_val(int bc, float own, float d) { return bc == NEUMANN ? own : (bc == DIRICHLET ? 0.0f : d); }
 
-// theta's ground-face values of the first sky row (theta_ground), once per diffusion call: they
+// theta's ground-face values of every column's first sky cell (theta_ground), once per diffusion call: they
 // depend on p, Tg and Pg only, which the sweeps do not change
 __global__ void __launch_bounds__(256) k_theta_face(Grid g, const float* __restrict__ p, const float* __restrict__ Tg,
                                                     const float* __restrict__ Pg, float* __restrict__ face) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= g.X * g.Z) return;
-    face[col] = theta_ground(p, Tg, Pg, cidx(g, col % g.X, 1, col / g.X), col);
+    const int y = __ldg(g.gh + col) + 1;
+    if (y >= 0 && y < g.Y) face[col] = theta_ground(p, Tg, Pg, cidx(g, col % g.X, y, col / g.X), col);
 }
 
 // face: theta's ground-face values per column (k_theta_face), read at the first sky row
@@ -639,7 +732,8 @@ __global__ void __launch_bounds__(32 * (R + 3), p4_min_blocks<R>())
 // parabola's sign case by a select. cdt = dt/vox: the Courant number is veli*cdt (the reference
 // divides veli*dt by vox each call) and the limiter ratios use the fast divide; both change
 // results by a few ulp at most.
-__device__ __forceinline__ float ppm_flux(float veli, float vL, float vC, float vR, float cdt) {
+// The flux is the face velocity times the value returned.
+__device__ __forceinline__ float ppm_value(float veli, float vL, float vC, float vR, float cdt) {
     const float C = fminf(fmaxf(veli * cdt, -1.0f), 1.0f);
     const float qMin = fminf(vL, fminf(vC, vR));
     const float qMax = fmaxf(vL, fmaxf(vC, vR));
@@ -657,8 +751,7 @@ __device__ __forceinline__ float ppm_flux(float veli, float vL, float vC, float 
     qR = flat ? vC : qR;
     qL = flat ? vC : qL;
     const float lin = C > 0.0f ? (-qL - 2 * qR + 3 * vC) : (-2 * qL - qR + 3 * vC);
-    const float qq = qR + C * lin + C * C * (qL + qR - 2 * vC);
-    return veli * qq;
+    return qR + C * lin + C * C * (qL + qR - 2 * vC);
 }
 
 // The flux through the face between cells b (below) and c (above) with face velocity u, a below b
@@ -666,10 +759,11 @@ __device__ __forceinline__ float ppm_flux(float veli, float vL, float vC, float 
 // A cell's upper-face flux (its velocity, window q-1..q+2) and the next cell's lower-face flux
 // (the previous cell's velocity, window q-2..q+1 seen from it) are the same call, so each face is
 // computed once and handed on. For a window of ones the flux is exactly u.
-__device__ __forceinline__ float face_flux(float u, float a, float b, float c, float d, float cdt) {
+__device__ __forceinline__ float face_value(float u, float a, float b, float c, float d, float cdt) {
     const bool up = u >= 0.0f;
-    return ppm_flux(u, up ? a : d, up ? b : c, up ? c : b, cdt);
+    return ppm_value(u, up ? a : d, up ? b : c, up ? c : b, cdt);
 }
+__device__ __forceinline__ float face_flux(float u, float a, float b, float c, float d, float cdt) { return u * face_value(u, a, b, c, d, cdt); }
 
 // the advected value over the advected density companion (divideValues Game/kernelMaths.cu:38)
 __device__ __forceinline__ float ppm_update(float q, float fp, float fm, float fpo, float fmo, float cdt) {
@@ -678,24 +772,40 @@ __device__ __forceinline__ float ppm_update(float q, float fp, float fm, float f
     return nq / nr;
 }
 
-// ghost value of the density companion (a field of ones, custom value 1)
-__device__ __forceinline__ float ghost_one(const Grid& g, int x, int y, int z, int sides, int ground) {
-    if (!in_dom(g, x, y, z)) {
-        const int xc = min(max(x, 0), g.X - 1), yc = min(max(y, 0), g.Y - 1), zc = min(max(z, 0), g.Z - 1);
-        return bc_val(is_ground(g, xc, yc, zc) ? ground : sides, 1.0f, 1.0f);
-    }
-    if (is_ground(g, x, y, z)) return bc_val(ground, 1.0f, 1.0f);
-    return 1.0f;
+__device__ __forceinline__ float ppm_cdt(const Grid& g, float dtFull, int nsub, int half) {
+    const float dtSub = dtFull / float(nsub);
+    const float dt = half ? dtSub * 0.5f : dtSub;
+    return dt / g.vox;
 }
 
-// One directional PPM pass (advectPPMX/Y/Z Game/kernelSky.cu:368-574) of q and of the density
-// companion (advected ones), followed by q/rho* (divideValues Game/kernelMaths.cu:38).
-// The velocity array is read as it stands when the pass starts.
-template <int AXIS, bool MANY>
-__global__ void __launch_bounds__(256) k_ppm(Grid g, FieldSet F, const float* __restrict__ vel, const float* __restrict__ defU,
-                                             const float* __restrict__ defW, float dtFull, int nsub_host, int half,
-                                             const Scalars* __restrict__ sc, int slot) {
-    const int fi = F.field_of<MANY>(g.Z);
+// ppm_update from the faces' velocities u and values k (upper p, lower m; o: the companion's): the lower
+// flux is rounded, the upper one's product is fused into the difference
+__device__ __forceinline__ float ppm_update_of(float q, float up, float kp, float um, float km, float kpo, float kmo, float cdt) {
+    const float d = fmaf(up, kp, -__fmul_rn(um, km)), dd = fmaf(up, kpo, -__fmul_rn(um, kmo));
+    const float nq = q - cdt * d;
+    const float nr = 1.0f - cdt * dd;
+    return nq / nr;
+}
+
+// One directional PPM pass (advectPPMX/Y/Z Game/kernelSky.cu:368-574) of q and of the density companion
+// (advected ones), followed by q/rho* (divideValues Game/kernelMaths.cu:38), any X and any terrain. The
+// velocity array is read as it stands when the pass starts.
+// A window's value depends on where it lies only (ghost()'s rule), and so does a face's velocity: the lower
+// cell's where that is sky, else the boundary's value over the upper cell's own. So each face's flux is
+// formed once and serves the cells on both sides, and the companion's is the face velocity where its
+// window is all ones. FLAT: the ground is the y = 0 layer, which no thread visits.
+// What bounds it: instructions, some 90 a cell, at an eighth of the HBM rate a pass. With a thread per cell
+// that tested the ghost rules at every place of its window and formed four fluxes, a step's advections took
+// 7.56 ms at 256x128x256 with hills, now 3.94; 1.17 and 0.79 at 128x64x128; 0.60 and 0.47 at 90x51x75.
+constexpr int GXW = 28;  // X pass: cells written by a warp; two more on either side complete the windows
+constexpr int GPY = 8;   // warps per block
+
+// X pass: a lane per cell of a row, neighbours and the lower face's flux from the lanes beside; marches z
+template <bool MANY, bool FLAT>
+__global__ void __launch_bounds__(32 * GPY) k_ppm_x(Grid g, int zlen, int zc, FieldSet F, const float* __restrict__ vel,
+                                                    const float* __restrict__ defU, float dtFull, int nsub_host, int half,
+                                                    const Scalars* __restrict__ sc, int slot) {
+    const int fi = F.field_of<MANY>(zc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
     const float* __restrict__ def = F.def[fi];
@@ -705,39 +815,128 @@ __global__ void __launch_bounds__(256) k_ppm(Grid g, FieldSet F, const float* __
         nsub = sc->nsub;
         if (slot >= nsub) return;
     }
-    const float dtSub = dtFull / float(nsub);
-    const float dt = half ? dtSub * 0.5f : dtSub;
-    const float cdt = dt / g.vox;
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z - fi * g.Z;
-    if (x >= g.X || y >= g.Y) return;
-    if (is_ground(g, x, y, z)) return;
-    constexpr int ax = AXIS == 0, ay = AXIS == 1, az = AXIS == 2;
-    const int c = cidx(g, x, y, z);
-    float q[5], o[5];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-        const int off = i - 2;
-        if (off == 0) { q[i] = in[c]; o[i] = 1.0f; continue; }
-        q[i] = ghost(g, in, x + off * ax, y + off * ay, z + off * az, sides, ground, def);
-        o[i] = ghost_one(g, x + off * ax, y + off * ay, z + off * az, sides, ground);
+    const float cdt = ppm_cdt(g, dtFull, nsub, half);
+    const int lane = threadIdx.x, X = g.X, XY = g.XY;
+    const int x = blockIdx.x * GXW - 2 + lane, y = blockIdx.y * GPY + threadIdx.y + FLAT;
+    const int zs = (blockIdx.z - fi * zc) * zlen, ze = min(zs + zlen, g.Z);
+    if (y >= g.Y) return;  // a whole warp
+    const int xc = min(max(x, 0), X - 1);
+    const bool outside = x != xc, mine = lane >= 2 && lane < 2 + GXW && x < X;
+    const float dy = def ? def[y] : 0.0f, du = defU[y];
+    const float so = bc_val(sides, 1.0f, 1.0f), go = bc_val(ground, 1.0f, 1.0f);
+    auto height = [&](int i) { return FLAT ? 0 : __ldg(g.gh + i); };
+    int c = xc + y * X + zs * XY, col = xc + zs * X;
+    float qn = in[c], vn = vel[c];
+    int hn = height(col);
+    for (int z = zs; z < ze; ++z, c += XY, col += X) {
+        float q = qn;
+        const float v = vn;
+        const bool gr = !FLAT && y <= hn;
+        if (z + 1 < ze) {
+            qn = in[c + XY];
+            vn = vel[c + XY];
+            hn = height(col + X);
+        }
+        if (gr) q = bc_val(ground, q, dy);
+        else if (outside) q = bc_val(sides, q, dy);
+        const float o = gr ? go : (outside ? so : 1.0f);
+        const float l1 = __shfl_up_sync(0xffffffffu, q, 1), r1 = __shfl_down_sync(0xffffffffu, q, 1), r2 = __shfl_down_sync(0xffffffffu, q, 2);
+        const float vr = __shfl_down_sync(0xffffffffu, v, 1);
+        const float fv = outside ? bc_val(sides, vr, du) : (gr ? bc_val(ground, vr, du) : v);
+        const float k = face_value(fv, l1, q, r1, r2, cdt);
+        float ko = 1.0f;
+        if (__any_sync(0xffffffffu, o != 1.0f)) {
+            const float ol = __shfl_up_sync(0xffffffffu, o, 1), o1 = __shfl_down_sync(0xffffffffu, o, 1), o2 = __shfl_down_sync(0xffffffffu, o, 2);
+            ko = face_value(fv, ol, o, o1, o2, cdt);
+        }
+        const float um = __shfl_up_sync(0xffffffffu, fv, 1), km = __shfl_up_sync(0xffffffffu, k, 1), kmo = __shfl_up_sync(0xffffffffu, ko, 1);
+        if (mine && !gr) out[c] = ppm_update_of(q, fv, k, um, km, ko, kmo, cdt);
     }
-    const float custom = AXIS == 0 ? defU[y] : (AXIS == 1 ? 0.0f : defW[y]);
-    const float vc = vel[c];
-    const float vm = face_nb(g, vel, x, y, z, -ax, -ay, -az, sides, ground, custom);
-    const float fp = face_flux(vc, q[1], q[2], q[3], q[4], cdt), fm = face_flux(vm, q[0], q[1], q[2], q[3], cdt);
-    const float fpo = face_flux(vc, o[1], o[2], o[3], o[4], cdt), fmo = face_flux(vm, o[0], o[1], o[2], o[3], cdt);
-    out[c] = ppm_update(q[2], fp, fm, fpo, fmo, cdt);
+}
+
+// Y and Z passes: a lane per column along the axis, which it marches with the window in registers, the
+// lower face's flux handed on from the cell before
+template <int AXIS, bool MANY, bool FLAT>
+__global__ void __launch_bounds__(32 * GPY) k_ppm_march(Grid g, int tlen, int tc, FieldSet F, const float* __restrict__ vel,
+                                                        const float* __restrict__ defW, float dtFull, int nsub_host, int half,
+                                                        const Scalars* __restrict__ sc, int slot) {
+    const int fi = F.field_of<MANY>(tc);
+    const float* __restrict__ in = F.in[fi];
+    float* __restrict__ out = F.out[fi];
+    const float* __restrict__ def = F.def[fi];
+    const int sides = F.sides[fi], ground = F.ground[fi];
+    int nsub = nsub_host;
+    if (sc) {
+        nsub = sc->nsub;
+        if (slot >= nsub) return;
+    }
+    const float cdt = ppm_cdt(g, dtFull, nsub, half);
+    const int X = g.X, XY = g.XY;
+    constexpr bool YAX = AXIS == 1;
+    const int x = blockIdx.x * 32 + threadIdx.x, across = blockIdx.y * GPY + threadIdx.y + (FLAT && !YAX);  // z, or y
+    const int T = YAX ? g.Y : g.Z, step = YAX ? X : XY;
+    const int ts = (blockIdx.z - fi * tc) * tlen + (FLAT && YAX), te = min(ts + tlen, T);
+    if (x >= X || across >= (YAX ? g.Z : g.Y) || ts >= T) return;
+    const int base = YAX ? x + across * XY : x + across * X;
+    const int h0 = FLAT ? 0 : (YAX ? __ldg(g.gh + x + across * X) : 0);
+    const float dy = YAX ? 0.0f : (def ? def[across] : 0.0f), cust = YAX ? 0.0f : defW[across];
+    const float so = bc_val(sides, 1.0f, 1.0f), go = bc_val(ground, 1.0f, 1.0f);
+    const bool ones = so == 1.0f && go == 1.0f;
+    auto gr_at = [&](int t) { return YAX ? t <= h0 : (!FLAT && across <= __ldg(g.gh + x + t * X)); };
+    auto at = [&](int t) { return min(max(t, 0), T - 1); };
+    // the value and the companion at t, from what lies at at(t)
+    auto seen = [&](int t, float v, bool gr, float& o) {
+        const int k = at(t);
+        o = gr ? go : (t != k ? so : 1.0f);
+        if (!gr && t == k) return v;
+        const float d = YAX ? (def ? def[k] : 0.0f) : dy;
+        return bc_val(gr ? ground : sides, v, d);
+    };
+    float w0, w1, w2, w3, o0, o1, o2, o3, um, km, kmo;  // km, kmo: the lower face's values, um its velocity
+    bool s1, s2;  // ground at t and t + 1
+    {
+        const bool ga = gr_at(at(ts - 2)), gb = gr_at(at(ts - 1));
+        s1 = gr_at(ts);
+        s2 = gr_at(at(ts + 1));
+        w0 = seen(ts - 2, in[base + at(ts - 2) * step], ga, o0);
+        w1 = seen(ts - 1, in[base + at(ts - 1) * step], gb, o1);
+        w2 = seen(ts, in[base + ts * step], s1, o2);
+        w3 = seen(ts + 1, in[base + at(ts + 1) * step], s2, o3);
+        const float own = vel[base + ts * step];
+        const float fv = ts == 0 ? bc_val(sides, own, cust) : (gb ? bc_val(ground, own, cust) : vel[base + (ts - 1) * step]);
+        um = fv;
+        km = face_value(fv, w0, w1, w2, w3, cdt);
+        kmo = ones ? 1.0f : face_value(fv, o0, o1, o2, o3, cdt);
+    }
+    float qn = in[base + at(ts + 2) * step], vc = vel[base + ts * step];
+    bool gn = gr_at(at(ts + 2));
+    for (int t = ts; t < te; ++t) {
+        const float raw = qn, vn = vel[base + at(t + 1) * step];
+        const bool s3 = gn;
+        if (t + 1 < te) {
+            qn = in[base + at(t + 3) * step];
+            gn = gr_at(at(t + 3));
+        }
+        float o4;
+        const float w4 = seen(t + 2, raw, s3, o4);
+        const float fv = s1 ? bc_val(ground, vn, cust) : vc;
+        const float k = face_value(fv, w1, w2, w3, w4, cdt);
+        float ko = 1.0f;
+        if (!ones && (o1 != 1.0f || o2 != 1.0f || o3 != 1.0f || o4 != 1.0f)) ko = face_value(fv, o1, o2, o3, o4, cdt);
+        if (!s1) out[base + t * step] = ppm_update_of(w2, fv, k, um, km, ko, kmo, cdt);
+        um = fv;
+        km = k;
+        kmo = ko;
+        w1 = w2; w2 = w3; w3 = w4;
+        o1 = o2; o2 = o3; o3 = o4;
+        s1 = s2; s2 = s3;
+        vc = vn;
+    }
 }
 
 __device__ __forceinline__ float comp(const float4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); }
 __device__ __forceinline__ void setc(float4& v, int k, float a) {
     if (k == 0) v.x = a; else if (k == 1) v.y = a; else if (k == 2) v.z = a; else v.w = a;
-}
-
-__device__ __forceinline__ float ppm_cdt(const Grid& g, float dtFull, int nsub, int half) {
-    const float dtSub = dtFull / float(nsub);
-    const float dt = half ? dtSub * 0.5f : dtSub;
-    return dt / g.vox;
 }
 
 // Vectorised X pass (flat terrain, X % 4 == 0): a thread owns four cells of one row and marches
@@ -1599,8 +1798,14 @@ template <bool THETA>
 void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* face, PassMaps& maps) {
     const Grid& g = e.g;
     if (!vec_grid(e)) {
-        const auto kernel = F.n == 1 ? k_diffuse<THETA, false> : k_diffuse<THETA, true>;
-        kernel<<<cell_grid(g, F.n), dim3(BX, BY), 0, e.stream>>>(g, F, k, e.p, e.Tg, e.Pg);
+        const int gx = (g.X + 31) / 32, gy = (g.Y - e.flat + GDY * GR - 1) / (GDY * GR);
+        int zlen;
+        // blocks per SM: above 4M cells 16 (4.80 ms a step at 256x128x256 with hills, 5.23 at 8), below 8 (0.326 and
+        // 0.342 ms at 90x51x75)
+        const int zc = z_runs(e, gx, gy * F.n, g.N >= 4000000 ? 16 : 8, zlen);
+        const auto kernel = e.flat ? (F.n == 1 ? k_diffuse<THETA, false, true> : k_diffuse<THETA, true, true>)
+                                   : (F.n == 1 ? k_diffuse<THETA, false, false> : k_diffuse<THETA, true, false>);
+        launch_next(e, kernel, dim3(gx, gy, zc * F.n), dim3(32, GDY), 0, g, zlen, zc, F, k, e.p, e.Tg, e.Pg, face, nullptr);
         e.launches += 1;
         return;
     }
@@ -1667,7 +1872,7 @@ void launch_diffuse_many(Env& e, int n, float* const* f, const int* type, float 
         }
     }
     const float* face = nullptr;
-    if (theta && vec_grid(e)) {
+    if (theta) {
         face = e.g2a;  // ground scratch: free until the ground stage refills it
         k_theta_face<<<(g.X * g.Z + 255) / 256, 256, 0, e.stream>>>(g, e.p, e.Tg, e.Pg, e.g2a);
         e.launches += 1;
@@ -1754,8 +1959,17 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
         }
     }
     const int nsub = e.adv_nsub;
-    const dim3 grd = cell_grid(g, n), blk(BX, BY);
-    const bool vec = vec_grid(e);
+    const bool vec = vec_grid(e), flat = e.flat != 0;
+    // The general passes' grids, in blocks of eight warps per SM: above 4M cells 16 (a step's advections 3.94 ms
+    // at 256x128x256 with hills, 4.23 at 8), below 8 (0.79 and 0.81 at 128x64x128, 0.47 and 0.49 at 90x51x75)
+    const int gbps = g.N >= 4000000 ? 16 : 8;
+    int xlen, alen, tlen;
+    const int rows = g.Y - flat, gxx = (g.X + GXW - 1) / GXW, gxl = (g.X + 31) / 32, gyr = (rows + GPY - 1) / GPY, gzr = (g.Z + GPY - 1) / GPY;
+    const int xcn = z_runs(e, gxx, gyr * n, gbps, xlen), acn = z_runs(e, gxl, gyr * n, gbps, alen);
+    int tcn = std::max(1, std::min(rows, (stencil_sms(e) * gbps + gxl * gzr * n - 1) / (gxl * gzr * n)));
+    tlen = (rows + tcn - 1) / tcn;
+    tcn = (rows + tlen - 1) / tlen;
+    const dim3 gblk(32, GPY);
     const int gx = (g.X / 4 + 31) / 32, gy = (g.Y - 1 + DVY - 1) / DVY;
     int zlen, zlen2;  // the Z pass marches: fewer, longer z chunks
     const int zc = z_runs(e, gx, gy * n, e.tune.ppm_bps, zlen), zc2 = z_runs(e, gx, gy * n, e.tune.ppmz_bps, zlen2);
@@ -1778,17 +1992,25 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
     auto substep = [&](int i, const Scalars* chk) {
         auto xpass = [&](const float* vel) {
             if (vec) (n == 1 ? k_ppm4x<false> : k_ppm4x<true>)<<<vg, vb, 0, e.stream>>>(g, zlen, zc, F, vel, e.defU, dtS, nsub, 1, chk, i);
-            else (n == 1 ? k_ppm<0, false> : k_ppm<0, true>)<<<grd, blk, 0, e.stream>>>(g, F, vel, e.defU, e.defW, dtS, nsub, 1, chk, i);
+            else
+                (flat ? (n == 1 ? k_ppm_x<false, true> : k_ppm_x<true, true>) : (n == 1 ? k_ppm_x<false, false> : k_ppm_x<true, false>))
+                    <<<dim3(gxx, gyr, xcn * n), gblk, 0, e.stream>>>(g, xlen, xcn, F, vel, e.defU, dtS, nsub, 1, chk, i);
             e.launches += 1;
         };
         auto ypass = [&](const float* vel) {
             if (vec) (n == 1 ? k_ppm4y<false> : k_ppm4y<true>)<<<yg, yb, 0, e.stream>>>(g, ylen, yc, F, vel, dtS, nsub, 1, chk, i);
-            else (n == 1 ? k_ppm<1, false> : k_ppm<1, true>)<<<grd, blk, 0, e.stream>>>(g, F, vel, e.defU, e.defW, dtS, nsub, 1, chk, i);
+            else
+                (flat ? (n == 1 ? k_ppm_march<1, false, true> : k_ppm_march<1, true, true>)
+                      : (n == 1 ? k_ppm_march<1, false, false> : k_ppm_march<1, true, false>))
+                    <<<dim3(gxl, gzr, tcn * n), gblk, 0, e.stream>>>(g, tlen, tcn, F, vel, e.defW, dtS, nsub, 1, chk, i);
             e.launches += 1;
         };
         auto zpass = [&](const float* vel) {
             if (vec) (n == 1 ? k_ppm4z<false> : k_ppm4z<true>)<<<vg2, vb, 0, e.stream>>>(g, zlen2, zc2, F, vel, e.defW, dtS, nsub, 0, chk, i);
-            else (n == 1 ? k_ppm<2, false> : k_ppm<2, true>)<<<grd, blk, 0, e.stream>>>(g, F, vel, e.defU, e.defW, dtS, nsub, 0, chk, i);
+            else
+                (flat ? (n == 1 ? k_ppm_march<2, false, true> : k_ppm_march<2, true, true>)
+                      : (n == 1 ? k_ppm_march<2, false, false> : k_ppm_march<2, true, false>))
+                    <<<dim3(gxl, gyr, acn * n), gblk, 0, e.stream>>>(g, alen, acn, F, vel, e.defW, dtS, nsub, 0, chk, i);
             e.launches += 1;
         };
         // buffers of the chain: 0 the field itself, 1 and 2 its scratch fields
@@ -2051,9 +2273,17 @@ extern "C" skt_status skt_diffuse_noalloc(int nx, int ny, int nz, float voxel, i
     }
     cudaStream_t st = (cudaStream_t)stream;
     const float k = 0.005f * dt_speed / (voxel * voxel);
-    // out takes the input first so its ground cells keep their values; the sweeps then alternate
-    // between out and the scratch array so that the last one lands in out.
-    k_copy_all<<<(int(n) + 255) / 256, 256, 0, st>>>(in_dev, out_dev, int(n));
+    if (sweeps == 0) k_copy_all<<<(int(n) + 255) / 256, 256, 0, st>>>(in_dev, out_dev, int(n));
+    // The sweeps alternate between out and the scratch array so that the last one lands in out; that one
+    // takes the ground cells from the input.
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 148;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool chain = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    const int gx = (nx + 31) / 32, gy = (ny + GDY * GR - 1) / (GDY * GR);
+    int zc = std::max(1, std::min(nz, (sms * 8 + gx * gy - 1) / (gx * gy)));
+    const int zlen = (nz + zc - 1) / zc;
+    zc = (nz + zlen - 1) / zlen;
     FieldSet F;
     F.n = 1;
     F.in[0] = in_dev;
@@ -2062,8 +2292,8 @@ extern "C" skt_status skt_diffuse_noalloc(int nx, int ny, int nz, float voxel, i
     F.ground[0] = ground;
     for (int s = 0; s < sweeps; ++s) {
         F.out[0] = ((sweeps - 1 - s) % 2 == 0) ? out_dev : scratch;
-        if (field_type == 0) k_diffuse<true, false><<<cell_grid(g), dim3(BX, BY), 0, st>>>(g, F, k, p_dev, ground_T_dev, ground_p_dev);
-        else k_diffuse<false, false><<<cell_grid(g), dim3(BX, BY), 0, st>>>(g, F, k, p_dev, ground_T_dev, ground_p_dev);
+        launch_next(st, chain, field_type == 0 ? k_diffuse<true, false, false> : k_diffuse<false, false, false>, dim3(gx, gy, zc), dim3(32, GDY), 0,
+                    g, zlen, zc, F, k, p_dev, ground_T_dev, ground_p_dev, nullptr, s == sweeps - 1 ? in_dev : nullptr);
         F.in[0] = F.out[0];
     }
     const cudaError_t err = cudaGetLastError();
