@@ -413,8 +413,11 @@ struct ProfScope {
 // and its stores are visible, and then lets its own successor be placed. Nothing but the launch's own
 // latency overlaps. For chains of short kernels: the mixed projection, 220 to 650 launches, takes 1.36 ms
 // at 64x32x64 (1.95 with ordinary launches), 2.08 at 128x64x128 (2.85), 7.6 at 256x128x256 (8.9) and 43.3
-// at 512x256x512 (44.6), the coarsest level's shorter solve included. Inside a capture the launch is an
-// ordinary one: programmatic edges in a graph's loops gained nothing (ensembles 11.43 and 11.37 ms).
+// at 512x256x512 (44.6), the coarsest level's shorter solve included; a frame at 32^3 1.16 ms (1.37), three
+// substeps of one field's advection at 192x96x192 0.45 (0.55), 20 sweeps of theta at 256x128x256 0.34
+// (0.36). Inside a capture the launch is an ordinary one: programmatic edges gained a graph nothing (a
+// step at 64x32x64 1.386 ms with and without, eight members 11.51 and 11.36). A kernel that follows a copy or
+// a memset is launched in the ordinary way too.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -433,9 +436,10 @@ void launch_next(cudaStream_t st, bool chain, void (*k)(P...), dim3 grid, dim3 b
     cfg.numAttrs = chain ? 1 : 0;
     (void)cudaLaunchKernelEx(&cfg, k, P(a)...);  // an error is the caller's to report
 }
+inline bool can_chain(const Env& e) { return !e.capturing; }
 template <class... P, class... A>
 void launch_next(const Env& e, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... a) {
-    launch_next(e.stream, !e.capturing, k, grid, block, smem, a...);
+    launch_next(e.stream, can_chain(e), k, grid, block, smem, a...);
 }
 
 // ---- launchers (defined in the kernel translation units) --------------------------------------

@@ -200,6 +200,7 @@ __device__ __forceinline__ float side_val(int bc, float own, float d) { return b
 // depend on p, Tg and Pg only, which the sweeps do not change
 __global__ void __launch_bounds__(256) k_theta_face(Grid g, const float* __restrict__ p, const float* __restrict__ Tg,
                                                     const float* __restrict__ Pg, float* __restrict__ face) {
+    after_previous();
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= g.X * g.Z) return;
     const int y = __ldg(g.gh + col) + 1;
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(256) k_theta_face(Grid g, const float* __restr
 // face: theta's ground-face values per column (k_theta_face), read at the first sky row
 template <bool THETA, bool MANY>
 __global__ void __launch_bounds__(32 * DVY) k_diffuse4(Grid g, int zlen, int zc, FieldSet F, float k, const float* __restrict__ face) {
+    after_previous();
     const int fi = F.field_of<MANY>(zc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -525,6 +527,7 @@ template <bool THETA, bool MANY, int R>
 __global__ void __launch_bounds__(32 * (R + 3), p4_min_blocks<R>())
     k_diffuse_pair4(const __grid_constant__ FieldMaps maps, Grid g, int zlen, int zc, FieldSet F, float k, const float* __restrict__ face,
                     Scalars* __restrict__ sc) {
+    after_previous();
     const int fi = F.field_of<MANY>(zc);
     const CUtensorMap& tin = maps.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -805,6 +808,7 @@ template <bool MANY, bool FLAT>
 __global__ void __launch_bounds__(32 * GPY) k_ppm_x(Grid g, int zlen, int zc, FieldSet F, const float* __restrict__ vel,
                                                     const float* __restrict__ defU, float dtFull, int nsub_host, int half,
                                                     const Scalars* __restrict__ sc, int slot) {
+    after_previous();
     const int fi = F.field_of<MANY>(zc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -860,6 +864,7 @@ template <int AXIS, bool MANY, bool FLAT>
 __global__ void __launch_bounds__(32 * GPY) k_ppm_march(Grid g, int tlen, int tc, FieldSet F, const float* __restrict__ vel,
                                                         const float* __restrict__ defW, float dtFull, int nsub_host, int half,
                                                         const Scalars* __restrict__ sc, int slot) {
+    after_previous();
     const int fi = F.field_of<MANY>(tc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -949,6 +954,7 @@ template <bool MANY>
 __global__ void __launch_bounds__(32 * DVY, 32 / DVY) k_ppm4x(Grid g, int zlen, int zc, FieldSet F, const float* __restrict__ vel,
                                                                    const float* __restrict__ defU, float dtFull, int nsub_host,
                                                                    int half, const Scalars* __restrict__ sc, int slot) {
+    after_previous();
     const int fi = F.field_of<MANY>(zc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -1068,6 +1074,7 @@ constexpr int PY = 4;
 template <bool MANY>
 __global__ void __launch_bounds__(32 * PY) k_ppm4y(Grid g, int ylen, int yc, FieldSet F, const float* __restrict__ vel, float dtFull,
                                                    int nsub_host, int half, const Scalars* __restrict__ sc, int slot) {
+    after_previous();
     const int fi = F.field_of<MANY>(yc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -1135,6 +1142,7 @@ __global__ void __launch_bounds__(32 * PY) k_ppm4y(Grid g, int ylen, int yc, Fie
 template <bool MANY>
 __global__ void __launch_bounds__(32 * DVY) k_ppm4z(Grid g, int zlen, int zc, FieldSet F, const float* __restrict__ vel, const float* __restrict__ defW,
                                                     float dtFull, int nsub_host, int half, const Scalars* __restrict__ sc, int slot) {
+    after_previous();
     const int fi = F.field_of<MANY>(zc);
     const float* __restrict__ in = F.in[fi];
     float* __restrict__ out = F.out[fi];
@@ -1287,6 +1295,7 @@ __global__ void __launch_bounds__(256) k_maxvel4(int n4, int X4, int Y, int XY4,
 
 // Courant substeps from the max velocity, on the device (Game/environment.cu:726-730)
 __global__ void k_nsub(Scalars* sc, float dt, float vox, float maxsub) {
+    after_previous();
     const float maxVel = __uint_as_float(sc->maxbits);
     const float C = maxVel * dt / vox;
     sc->nsub = int(fminf(ceilf(fabsf(C)), maxsub));
@@ -1355,6 +1364,7 @@ __global__ void __launch_bounds__(32 * PRW) k_precip3(Grid g, int ylen, float* _
                                                       const float* __restrict__ th, const float* __restrict__ qv,
                                                       const float* __restrict__ p, const float* __restrict__ Pg, int mask, float dtr,
                                                       float dts, float dti, Gammas G) {
+    after_previous();
     const int col = blockIdx.x * 32 + threadIdx.x;
     const bool in = col < g.X * g.Z;
     const int x = in ? col % g.X : 0, z = in ? col / g.X : 0;
@@ -1430,6 +1440,7 @@ __global__ void __launch_bounds__(256) k_buoyancy(Grid g, float* __restrict__ v,
                                                   const float* __restrict__ qr, const float* __restrict__ qs, const float* __restrict__ qi,
                                                   const float* __restrict__ isenT, const float* __restrict__ isenQv,
                                                   const float* __restrict__ p, const float* __restrict__ Pg, float dt, float* __restrict__ dbg) {
+    after_previous();
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= g.X || y >= g.Y) return;
     if (is_ground(g, x, y, z)) return;
@@ -1541,6 +1552,7 @@ __global__ void __launch_bounds__(32 * BZ4) k_buoyancy4(Grid g, int ylen, float*
                                                         const float* __restrict__ qs, const float* __restrict__ qi,
                                                         const float* __restrict__ p, const float* __restrict__ Pg, float dt,
                                                         float* __restrict__ dbg) {
+    after_previous();
     const int lane = threadIdx.x;
     const int xw = blockIdx.x * 128, x0 = xw + lane * 4;
     const int z = blockIdx.y * BZ4 + threadIdx.y;
@@ -1632,6 +1644,7 @@ __global__ void __launch_bounds__(32 * BZ4) k_buoyancy4(Grid g, int ylen, float*
 // initDensity Game/kernelSky.cu:1432-1452
 __global__ void __launch_bounds__(256) k_init_density(Grid g, float* __restrict__ rho, const float* __restrict__ th, const float* __restrict__ p,
                                                       const float* __restrict__ qv, const float* __restrict__ Pg) {
+    after_previous();
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= g.X || y >= g.Y) return;
     if (is_ground(g, x, y, z)) return;
@@ -1644,6 +1657,7 @@ __global__ void __launch_bounds__(256) k_init_density(Grid g, float* __restrict_
 // calculateNewPressure Game/kernelSky.cu:1454-1474
 __global__ void __launch_bounds__(256) k_new_pressure(Grid g, float* __restrict__ p, const float* __restrict__ rho, const float* __restrict__ th,
                                                       const float* __restrict__ qv, const float* __restrict__ Pg) {
+    after_previous();
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= g.X || y >= g.Y) return;
     if (is_ground(g, x, y, z)) return;
@@ -1742,7 +1756,7 @@ bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const flo
         attr = true;
     }
     const auto kernel = F.n == 1 ? k_diffuse_pair4<THETA, false, R> : k_diffuse_pair4<THETA, true, R>;
-    kernel<<<dim3(gx, gy, zc * F.n), 32 * (R + 3), smem, e.stream>>>(maps.m, g, zlen, zc, F, k, face, e.sc);
+    launch_next(e, kernel, dim3(gx, gy, zc * F.n), 32 * (R + 3), smem, maps.m, g, zlen, zc, F, k, face, e.sc);
     e.launches += 1;
     return true;
 }
@@ -1815,7 +1829,7 @@ void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* fac
     const int vz = z_runs(e, vx, vy * F.n, e.tune.diffuse_bps, vlen);
     auto one = [&](const FieldSet& S) {
         const auto kernel = S.n == 1 ? k_diffuse4<THETA, false> : k_diffuse4<THETA, true>;
-        kernel<<<dim3(vx, vy, vz * S.n), dim3(32, DVY), 0, e.stream>>>(g, vlen, vz, S, k, face);
+        launch_next(e, kernel, dim3(vx, vy, vz * S.n), dim3(32, DVY), 0, g, vlen, vz, S, k, face);
         e.launches += 1;
     };
     if (!two) {
@@ -1874,7 +1888,7 @@ void launch_diffuse_many(Env& e, int n, float* const* f, const int* type, float 
     const float* face = nullptr;
     if (theta) {
         face = e.g2a;  // ground scratch: free until the ground stage refills it
-        k_theta_face<<<(g.X * g.Z + 255) / 256, 256, 0, e.stream>>>(g, e.p, e.Tg, e.Pg, e.g2a);
+        launch_next(e, k_theta_face, (g.X * g.Z + 255) / 256, 256, 0, g, e.p, e.Tg, e.Pg, e.g2a);
         e.launches += 1;
     }
     // passes of one sweep, or (temporal blocking of depth 2) of two sweeps: an odd count starts
@@ -1950,7 +1964,7 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
         } else {
             k_maxvel<<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, e.u, e.v, e.w, e.cfg.semantics == 0, e.sc);
         }
-        k_nsub<<<1, 1, 0, e.stream>>>(e.sc, dtS, g.vox, float(e.cfg.max_substeps));
+        launch_next(e, k_nsub, 1, 1, 0, e.sc, dtS, g.vox, float(e.cfg.max_substeps));
         if (!e.capturing) {
             fetch_scalars(e);
             e.adv_nsub = e.host_sc->nsub;
@@ -1990,27 +2004,31 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
     // one substep (slot i; with chk set, the kernels read the substep count from the device and
     // slots at or beyond it return at once)
     auto substep = [&](int i, const Scalars* chk) {
+        // chain: the pass follows a kernel (not a copy)
         auto xpass = [&](const float* vel) {
-            if (vec) (n == 1 ? k_ppm4x<false> : k_ppm4x<true>)<<<vg, vb, 0, e.stream>>>(g, zlen, zc, F, vel, e.defU, dtS, nsub, 1, chk, i);
+            if (vec) launch_next(e, n == 1 ? k_ppm4x<false> : k_ppm4x<true>, vg, vb, 0, g, zlen, zc, F, vel, e.defU, dtS, nsub, 1, chk, i);
             else
-                (flat ? (n == 1 ? k_ppm_x<false, true> : k_ppm_x<true, true>) : (n == 1 ? k_ppm_x<false, false> : k_ppm_x<true, false>))
-                    <<<dim3(gxx, gyr, xcn * n), gblk, 0, e.stream>>>(g, xlen, xcn, F, vel, e.defU, dtS, nsub, 1, chk, i);
+                launch_next(e, flat ? (n == 1 ? k_ppm_x<false, true> : k_ppm_x<true, true>) : (n == 1 ? k_ppm_x<false, false> : k_ppm_x<true, false>),
+                            dim3(gxx, gyr, xcn * n), gblk, 0, g, xlen, xcn, F, vel, e.defU, dtS, nsub, 1, chk, i);
             e.launches += 1;
         };
-        auto ypass = [&](const float* vel) {
-            if (vec) (n == 1 ? k_ppm4y<false> : k_ppm4y<true>)<<<yg, yb, 0, e.stream>>>(g, ylen, yc, F, vel, dtS, nsub, 1, chk, i);
+        auto ypass = [&](const float* vel, bool chain) {
+            chain = chain && can_chain(e);
+            if (vec) launch_next(e.stream, chain, n == 1 ? k_ppm4y<false> : k_ppm4y<true>, yg, yb, 0, g, ylen, yc, F, vel, dtS, nsub, 1, chk, i);
             else
-                (flat ? (n == 1 ? k_ppm_march<1, false, true> : k_ppm_march<1, true, true>)
-                      : (n == 1 ? k_ppm_march<1, false, false> : k_ppm_march<1, true, false>))
-                    <<<dim3(gxl, gzr, tcn * n), gblk, 0, e.stream>>>(g, tlen, tcn, F, vel, e.defW, dtS, nsub, 1, chk, i);
+                launch_next(e.stream, chain,
+                            flat ? (n == 1 ? k_ppm_march<1, false, true> : k_ppm_march<1, true, true>)
+                                 : (n == 1 ? k_ppm_march<1, false, false> : k_ppm_march<1, true, false>),
+                            dim3(gxl, gzr, tcn * n), gblk, 0, g, tlen, tcn, F, vel, e.defW, dtS, nsub, 1, chk, i);
             e.launches += 1;
         };
         auto zpass = [&](const float* vel) {
-            if (vec) (n == 1 ? k_ppm4z<false> : k_ppm4z<true>)<<<vg2, vb, 0, e.stream>>>(g, zlen2, zc2, F, vel, e.defW, dtS, nsub, 0, chk, i);
+            if (vec) launch_next(e, n == 1 ? k_ppm4z<false> : k_ppm4z<true>, vg2, vb, 0, g, zlen2, zc2, F, vel, e.defW, dtS, nsub, 0, chk, i);
             else
-                (flat ? (n == 1 ? k_ppm_march<2, false, true> : k_ppm_march<2, true, true>)
-                      : (n == 1 ? k_ppm_march<2, false, false> : k_ppm_march<2, true, false>))
-                    <<<dim3(gxl, gyr, acn * n), gblk, 0, e.stream>>>(g, alen, acn, F, vel, e.defW, dtS, nsub, 0, chk, i);
+                launch_next(e,
+                            flat ? (n == 1 ? k_ppm_march<2, false, true> : k_ppm_march<2, true, true>)
+                                 : (n == 1 ? k_ppm_march<2, false, false> : k_ppm_march<2, true, false>),
+                            dim3(gxl, gyr, acn * n), gblk, 0, g, alen, acn, F, vel, e.defW, dtS, nsub, 0, chk, i);
             e.launches += 1;
         };
         // buffers of the chain: 0 the field itself, 1 and 2 its scratch fields
@@ -2026,9 +2044,9 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
             // sky cells itself (no copy). A pass reads the wind as it stands: for u (x passes) and w (z
             // pass) that is the chain's current buffer.
             set(0, 1); xpass(e.u);
-            set(1, 2); ypass(e.v);
+            set(1, 2); ypass(e.v, true);
             set(2, 1); zpass(f[0] == e.w ? buf(0, 2) : e.w);
-            set(1, 2); ypass(e.v);
+            set(1, 2); ypass(e.v, true);
             set(2, 0); xpass(f[0] == e.u ? buf(0, 2) : e.u);
             return;
         }
@@ -2037,10 +2055,10 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
         float* const vy = buf(0, 2);
         set(0, 1); xpass(e.u);
         cudaMemcpyAsync(vy, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-        set(1, 0); ypass(vy);
+        set(1, 0); ypass(vy, false);
         set(0, 1); zpass(e.w);
         cudaMemcpyAsync(vy, e.v, sizeof(float) * size_t(g.N), cudaMemcpyDeviceToDevice, e.stream);
-        set(1, 0); ypass(vy);
+        set(1, 0); ypass(vy, false);
         set(0, 1); xpass(e.u);
         set(1, 0); copy_sky(e, F, chk, i);
     };
@@ -2098,7 +2116,7 @@ void launch_precip3(Env& e, float dtS) {
     for (int s = 0; s < passes; ++s) {
         const int mask = (sub[0] > s ? 1 : 0) | (sub[1] > s ? 2 : 0) | (sub[2] > s ? 4 : 0);
         e.launches += 1;
-        k_precip3<<<(cols + 31) / 32, dim3(32, PRW), 0, e.stream>>>(g, (g.Y - 1 + PRW - 1) / PRW, e.qr, e.qs, e.qi, e.th, e.qv, e.p, e.Pg,
+        launch_next(e, k_precip3, (cols + 31) / 32, dim3(32, PRW), 0, g, (g.Y - 1 + PRW - 1) / PRW, e.qr, e.qs, e.qi, e.th, e.qv, e.p, e.Pg,
                                                                     mask, dts[0], dts[1], dts[2], e.gam);
     }
 }
@@ -2113,20 +2131,20 @@ void launch_buoyancy(Env& e, float dtS) {
         int yc = std::max(1, std::min(g.Y - 1, (stencil_sms(e) * 8 + gx * gz - 1) / (gx * gz)));
         const int ylen = (g.Y - 1 + yc - 1) / yc;
         yc = (g.Y - 1 + ylen - 1) / ylen;
-        k_buoyancy4<<<dim3(gx, gz, yc), dim3(32, BZ4), 0, e.stream>>>(g, ylen, e.v, e.th, e.qv, e.qr, e.qs, e.qi, e.p, e.Pg, dtS, dbg);
+        launch_next(e, k_buoyancy4, dim3(gx, gz, yc), dim3(32, BZ4), 0, g, ylen, e.v, e.th, e.qv, e.qr, e.qs, e.qi, e.p, e.Pg, dtS, dbg);
         return;
     }
-    k_buoyancy<<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, e.v, e.th, e.qv, e.qr, e.qs, e.qi, e.isenT, e.isenQv, e.p, e.Pg, dtS, dbg);
+    launch_next(e, k_buoyancy, cell_grid(g), dim3(BX, BY), 0, g, e.v, e.th, e.qv, e.qr, e.qs, e.qi, e.isenT, e.isenQv, e.p, e.Pg, dtS, dbg);
 }
 void launch_init_density(Env& e) {
     ProfScope ps(e, "eos");
     e.launches += 1;
-    k_init_density<<<cell_grid(e.g), dim3(BX, BY), 0, e.stream>>>(e.g, e.rho, e.th, e.p, e.qv, e.Pg);
+    launch_next(e, k_init_density, cell_grid(e.g), dim3(BX, BY), 0, e.g, e.rho, e.th, e.p, e.qv, e.Pg);
 }
 void launch_new_pressure(Env& e) {
     ProfScope ps(e, "eos");
     e.launches += 1;
-    k_new_pressure<<<cell_grid(e.g), dim3(BX, BY), 0, e.stream>>>(e.g, e.p, e.rho, e.th, e.qv, e.Pg);
+    launch_next(e, k_new_pressure, cell_grid(e.g), dim3(BX, BY), 0, e.g, e.p, e.rho, e.th, e.qv, e.Pg);
 }
 
 // ---------------------------------------------------------------------------------------------
