@@ -1233,34 +1233,49 @@ __global__ void __launch_bounds__(256) k_copy_sky4(int n4, int X4, int Y, const 
 
 // Max over sky cells of three fields (getMaxDivergence Game/kernelSky.cu:910-953 applied to
 // u, v and w into one slot). reference=1: |a| at z=0, signed a for z>=1, floored at 0.
-__global__ void __launch_bounds__(256) k_maxvel(Grid g, const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
-                                                int reference, Scalars* __restrict__ sc) {
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
-    float m = 0.0f;
-    bool bad = false;
-    if (x < g.X && y < g.Y && !is_ground(g, x, y, z)) {
-        const int c = cidx(g, x, y, z);
-        const bool absv = !reference || z == 0;
-        float v0 = a0[c], v1 = a1[c], v2 = a2[c];
-        bad = nonfinite(v0) | nonfinite(v1) | nonfinite(v2);
-        if (absv) { v0 = fabsf(v0); v1 = fabsf(v1); v2 = fabsf(v2); }
-        if (v0 > m) m = v0;
-        if (v1 > m) m = v1;
-        if (v2 > m) m = v2;
-    }
+// A lane marches a run of z planes; one atomic per block (one per warp, each of 32 cells, took 24 us at
+// 128x64x128, now 6).
+__device__ __forceinline__ void note_max(float m, bool bad, int tid, Scalars* sc) {  // 256 threads
+    __shared__ float sm[8];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float t = __shfl_xor_sync(0xffffffffu, m, o);
         if (t > m) m = t;
     }
-    if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(&sc->maxbits, __float_as_uint(m));
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) sc->status = SKT_NAN_DETECTED;  // a NaN or Inf wind
+    if ((tid & 31) == 0) sm[tid >> 5] = m;
+    if (__any_sync(0xffffffffu, bad) && (tid & 31) == 0) sc->status = SKT_NAN_DETECTED;  // a NaN or Inf wind
+    __syncthreads();
+    if (tid == 0) {
+        float b = 0.0f;
+        for (int w = 0; w < 8; ++w) b = sm[w] > b ? sm[w] : b;
+        if (b > 0.0f) atomicMax(&sc->maxbits, __float_as_uint(b));
+    }
+}
+__global__ void __launch_bounds__(256) k_maxvel(Grid g, int zlen, const float* __restrict__ a0, const float* __restrict__ a1,
+                                                const float* __restrict__ a2, int reference, Scalars* __restrict__ sc) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    const int zs = blockIdx.z * zlen, ze = min(zs + zlen, g.Z);
+    float m = 0.0f;
+    bool bad = false;
+    if (x < g.X && y < g.Y) {
+#pragma unroll 4
+        for (int z = zs; z < ze; ++z) {
+            const int c = cidx(g, x, y, z);
+            float v0 = a0[c], v1 = a1[c], v2 = a2[c];
+            if (is_ground(g, x, y, z)) continue;
+            bad |= nonfinite(v0) | nonfinite(v1) | nonfinite(v2);
+            if (!reference || z == 0) { v0 = fabsf(v0); v1 = fabsf(v1); v2 = fabsf(v2); }
+            if (v0 > m) m = v0;
+            if (v1 > m) m = v1;
+            if (v2 > m) m = v2;
+        }
+    }
+    note_max(m, bad, threadIdx.y * 32 + threadIdx.x, sc);
 }
 
 // flat terrain: the same max over rows y >= 1, as float4 streams with one atomic per block
 __global__ void __launch_bounds__(256) k_maxvel4(int n4, int X4, int Y, int XY4, const float4* __restrict__ a0, const float4* __restrict__ a1,
                                                  const float4* __restrict__ a2, int reference, Scalars* __restrict__ sc) {
-    __shared__ float sm[8];
     float m = 0.0f;
     bool bad = false;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < n4; i += gridDim.x * 256) {
@@ -1278,19 +1293,7 @@ __global__ void __launch_bounds__(256) k_maxvel4(int n4, int X4, int Y, int XY4,
             if (e3 > m) m = e3;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float t = __shfl_xor_sync(0xffffffffu, m, o);
-        if (t > m) m = t;
-    }
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) sc->status = SKT_NAN_DETECTED;  // a NaN or Inf wind
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float b = 0.0f;
-        for (int w = 0; w < 8; ++w) b = sm[w] > b ? sm[w] : b;
-        if (b > 0.0f) atomicMax(&sc->maxbits, __float_as_uint(b));
-    }
+    note_max(m, bad, threadIdx.x, sc);
 }
 
 // Courant substeps from the max velocity, on the device (Game/environment.cu:726-730)
@@ -1962,7 +1965,10 @@ int launch_advect_many(Env& e, int n, float* const* f, const float* const* def, 
                                                                                       (const float4*)e.v, (const float4*)e.w,
                                                                                       e.cfg.semantics == 0, e.sc);
         } else {
-            k_maxvel<<<cell_grid(g), dim3(BX, BY), 0, e.stream>>>(g, e.u, e.v, e.w, e.cfg.semantics == 0, e.sc);
+            const int mx = (g.X + 31) / 32, my = (g.Y + 7) / 8;
+            int mlen;
+            const int mz = z_runs(e, mx, my, 8, mlen);
+            k_maxvel<<<dim3(mx, my, mz), dim3(32, 8), 0, e.stream>>>(g, mlen, e.u, e.v, e.w, e.cfg.semantics == 0, e.sc);
         }
         launch_next(e, k_nsub, 1, 1, 0, e.sc, dtS, g.vox, float(e.cfg.max_substeps));
         if (!e.capturing) {
