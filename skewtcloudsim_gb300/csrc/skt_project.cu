@@ -196,68 +196,159 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
     }
 }
 
-// As = A s and s.As (applyAGPU Game/kernelSky.cu:719-778 + dotProductGPU :675-717).
-// reference=1: lower coefficients pass through a char (Q3) and the denominator keeps
-// accumulating (Q1).
-__global__ void __launch_bounds__(NT) k_matvec(Grid g, Tiles T, const float* __restrict__ ax, const float* __restrict__ ay,
-                                               const float* __restrict__ az, const float* __restrict__ aw, const float* __restrict__ s,
-                                               float* __restrict__ As, int reference, Scalars* sc, double* partials) {
+// As = A s and s.As (applyAGPU Game/kernelSky.cu:719-778 + dotProductGPU :675-717), any X.
+// reference=1: lower coefficients pass through a char (Q3) and the denominator keeps accumulating (Q1).
+// A lane owns MR rows of one x cell and marches a run of z planes with the planes of s in registers and the
+// next plane's loads in flight; x neighbours come from the lanes beside. Ground cells hold s = 0 and
+// coefficients 0, as does the face to one, so no neighbour is tested. Blocks take their (x, y, z run) tiles
+// in turn, whatever their number.
+// What bounds it: HBM (24 bytes a cell) and the loads' instructions. A thread per cell that asked the
+// heights about every neighbour took 77 us at 251x118x275, now
+// 52; one or two rows a lane 62 and 65, eight warps a block 58.
+constexpr int MR = 4, MW = 4;  // rows per lane, warps per block
+struct Runs {
+    int nx, ny, n, zlen;  // tiles along x and y, all of them, planes per tile
+};
+inline Runs matvec_runs(const Grid& g, int sms) {
+    Runs t;
+    t.nx = (g.X + 31) / 32;
+    t.ny = (g.Y + MR * MW - 1) / (MR * MW);
+    int zc = std::max(1, std::min(g.Z, (sms * 8 + t.nx * t.ny - 1) / (t.nx * t.ny)));
+    t.zlen = (g.Z + zc - 1) / zc;
+    t.n = t.nx * t.ny * ((g.Z + t.zlen - 1) / t.zlen);
+    return t;
+}
+__global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float* __restrict__ ax, const float* __restrict__ ay,
+                                                    const float* __restrict__ az, const float* __restrict__ aw, const float* __restrict__ s,
+                                                    float* __restrict__ As, int reference, Scalars* sc, double* partials) {
     if (sc->converged) return;
+    const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY, lane = threadIdx.x;
     Sum2 dsum;
+    struct Plane {
+        float cx[MR], cy[MR], cz[MR], cw[MR], es[MR], ea[MR], up, down, cd;
+    };
     for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
-        int x, y, z;
-        tile_cell(g, T, t, x, y, z);
-        if (x >= g.X || y >= g.Y) continue;
-        const int c = cidx(g, x, y, z);
-        if (is_ground(g, x, y, z)) continue;  // As of ground cells stays 0
-        const bool hl = x > 0 && !is_ground(g, x - 1, y, z);
-        const bool hr = x + 1 < g.X && !is_ground(g, x + 1, y, z);
-        const bool hd = y > 0 && !is_ground(g, x, y - 1, z);
-        const bool hu = y + 1 < g.Y;
-        const bool hb = z > 0 && !is_ground(g, x, y, z - 1);
-        const bool hf = z + 1 < g.Z && !is_ground(g, x, y, z + 1);
-        const float sl = hl ? s[c - 1] : 0.0f, sr = hr ? s[c + 1] : 0.0f;
-        const float sd = hd ? s[c - g.X] : 0.0f, su = hu ? s[c + g.X] : 0.0f;
-        const float sb = hb ? s[c - g.XY] : 0.0f, sf = hf ? s[c + g.XY] : 0.0f;
-        float AL = hl ? ax[c - 1] : 0.0f, AD = hd ? ay[c - g.X] : 0.0f, AB = hb ? az[c - g.XY] : 0.0f;
-        if (reference) { AL = char_trunc(AL); AD = char_trunc(AD); AB = char_trunc(AB); }
-        const float sc0 = s[c];
-        const float out = aw[c] * sc0 + ((AL * sl + AD * sd + AB * sb + ax[c] * sr + ay[c] * su + az[c] * sf));
-        As[c] = out;
-        dsum.add_prod(out, sc0);
+        const int xo = (t % T.nx) * 32 + lane, y0 = ((t / T.nx) % T.ny * MW + threadIdx.y) * MR;
+        const int zs = t / (T.nx * T.ny) * T.zlen, ze = min(zs + T.zlen, Z);
+        if (y0 >= Y) continue;  // a whole warp
+        const int x = min(xo, X - 1);  // the lanes beyond a row follow its last cell, the rows beyond the top the top one
+        const int rows = xo < X ? min(MR, Y - y0) : 0;
+        const bool el = lane == 0 && x > 0, er = lane == 31 && x + 1 < X, first = x == 0, last = x + 1 == X;
+        int ro[MR];
+#pragma unroll
+        for (int r = 0; r < MR; ++r) ro[r] = min(r, Y - 1 - y0) * X;
+        int c = x + y0 * X + zs * XY;
+        auto load = [&](int cc, Plane& P) {
+            P.up = y0 + MR < Y ? s[cc + MR * X] : 0.0f;
+            P.down = y0 > 0 ? s[cc - X] : 0.0f;
+            P.cd = y0 > 0 ? ay[cc - X] : 0.0f;
+#pragma unroll
+            for (int r = 0; r < MR; ++r) {
+                const int q = cc + ro[r];
+                P.cx[r] = ax[q]; P.cy[r] = ay[q]; P.cz[r] = az[q]; P.cw[r] = aw[q];
+                P.es[r] = el || er ? s[q + (el ? -1 : 1)] : 0.0f;
+                P.ea[r] = el ? ax[q - 1] : 0.0f;
+            }
+        };
+        float q[MR], n[MR], b[MR], zb[MR];
+        Plane P;
+        load(c, P);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+            q[r] = s[c + ro[r]];
+            n[r] = zs + 1 < Z ? s[c + ro[r] + XY] : 0.0f;
+            b[r] = zs > 0 ? s[c + ro[r] - XY] : 0.0f;
+            zb[r] = zs > 0 ? az[c + ro[r] - XY] : 0.0f;
+        }
+        for (int z = zs; z < ze; ++z, c += XY) {
+            Plane N;
+            float n2[MR];
+            if (z + 1 < ze) load(c + XY, N);
+#pragma unroll
+            for (int r = 0; r < MR; ++r) n2[r] = z + 2 <= ze && z + 2 < Z ? s[c + ro[r] + 2 * XY] : 0.0f;
+#pragma unroll
+            for (int r = 0; r < MR; ++r) {
+                const float v = q[r];
+                float sl = __shfl_up_sync(0xffffffffu, v, 1), sr = __shfl_down_sync(0xffffffffu, v, 1), AL = __shfl_up_sync(0xffffffffu, P.cx[r], 1);
+                if (el) { sl = P.es[r]; AL = P.ea[r]; }
+                if (er) sr = P.es[r];
+                if (first) sl = AL = 0.0f;
+                if (last) sr = 0.0f;
+                const float sd = r > 0 ? q[r > 0 ? r - 1 : 0] : P.down;
+                float AD = r > 0 ? P.cy[r > 0 ? r - 1 : 0] : P.cd, AB = zb[r];
+                const float su = y0 + r + 1 < Y ? (r + 1 < MR ? q[r + 1 < MR ? r + 1 : r] : P.up) : 0.0f;
+                if (reference) { AL = char_trunc(AL); AD = char_trunc(AD); AB = char_trunc(AB); }
+                const float ld = fmaf(AL, sl, __fmul_rn(AD, sd));
+                const float out = fmaf(P.cw[r], v, fmaf(P.cz[r], n[r], fmaf(P.cy[r], su, fmaf(P.cx[r], sr, fmaf(AB, b[r], ld)))));
+                if (r < rows && P.cw[r] != 0.0f) {  // As of ground cells stays 0
+                    As[c + r * X] = out;
+                    dsum.add_prod(out, v);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < MR; ++r) {
+                b[r] = q[r];
+                q[r] = n[r];
+                n[r] = n2[r];
+                zb[r] = P.cz[r];
+            }
+            P = N;
+        }
     }
     double tot;
     float mall;
-    if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, 0.0f, tot, mall)) {
+    if (grid_sum_max<32 * MW>(sc, partials, blockIdx.x, gridDim.x, threadIdx.y * 32 + lane, dsum, 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
     }
 }
 
+// The arrays as float4 streams and a scalar rest (any X; ground cells hold 0, which every formula keeps):
+// fn(value, place) for value in float4 or float form
+template <class F4, class F1>
+__device__ __forceinline__ void stream4(int n, F4 four, F1 one) {
+    const int n4 = n / 4, t = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int i = t; i < n4; i += gridDim.x * blockDim.x) four(i);
+    if (t < n - 4 * n4) one(4 * n4 + t);
+}
+
 // p += alpha s; r -= alpha As (updatePandDiv :955-985), then the stop test on the max residual
-// (getMaxDivergence, Q4 in reference mode), z = r/diag and z.r for the next search direction.
-__global__ void __launch_bounds__(NT) k_update(Grid g, Tiles T, const float* __restrict__ aw, const float* __restrict__ s,
+// (getMaxDivergence, Q4 in reference mode: |r| on the z = 0 plane only), z = r/diag and z.r for the next search
+// direction. HBM-bound, 28 bytes a cell: 115 us at 251x118x275 cell by cell in tiles, 41 as float4 streams.
+__global__ void __launch_bounds__(NT) k_update(int n, int XY, const float* __restrict__ aw, const float* __restrict__ s,
                                                const float* __restrict__ As, float* __restrict__ pp, float* __restrict__ r,
                                                int reference, float tol, int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
     const float alpha = sc->alpha;
     Sum2 dsum;
     float mx = 0.0f;
-    for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
-        int x, y, z;
-        tile_cell(g, T, t, x, y, z);
-        if (x >= g.X || y >= g.Y) continue;
-        if (is_ground(g, x, y, z)) continue;
-        const int c = cidx(g, x, y, z);
-        pp[c] += alpha * s[c];
-        const float rv = r[c] - alpha * As[c];
-        r[c] = rv;
-        const float zv = rv * precon_of(aw[c]);
+    auto cell = [&](float a, float sv, float av, float& pv, float& rv, int c) {
+        pv += alpha * sv;
+        rv = rv - alpha * av;
+        const float zv = rv * precon_of(a);
         dsum.add_prod(zv, rv);
-        const float m = (!reference || z == 0) ? fabsf(rv) : rv;
+        const float m = (!reference || c < XY) ? fabsf(rv) : rv;
         if (m > mx) mx = m;
-    }
+    };
+    stream4(n,
+            [&](int i) {
+                const float4 a = reinterpret_cast<const float4*>(aw)[i], sv = reinterpret_cast<const float4*>(s)[i];
+                const float4 av = reinterpret_cast<const float4*>(As)[i];
+                float4 pv = reinterpret_cast<float4*>(pp)[i], rv = reinterpret_cast<float4*>(r)[i];
+                cell(a.x, sv.x, av.x, pv.x, rv.x, 4 * i);
+                cell(a.y, sv.y, av.y, pv.y, rv.y, 4 * i + 1);
+                cell(a.z, sv.z, av.z, pv.z, rv.z, 4 * i + 2);
+                cell(a.w, sv.w, av.w, pv.w, rv.w, 4 * i + 3);
+                reinterpret_cast<float4*>(pp)[i] = pv;
+                reinterpret_cast<float4*>(r)[i] = rv;
+            },
+            [&](int c) {
+                float pv = pp[c], rv = r[c];
+                cell(aw[c], s[c], As[c], pv, rv, c);
+                pp[c] = pv;
+                r[c] = rv;
+            });
     double tot;
     float mall;
     if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
@@ -275,20 +366,22 @@ __global__ void __launch_bounds__(NT) k_update(Grid g, Tiles T, const float* __r
     }
 }
 
-// s = z + beta s (endIteration :987-1014), z recomputed from r and the diagonal
-__global__ void __launch_bounds__(NT) k_search(Grid g, Tiles T, const float* __restrict__ aw, const float* __restrict__ r,
-                                               float* __restrict__ s, const Scalars* sc) {
+// s = z + beta s (endIteration :987-1014), z recomputed from r and the diagonal; 16 bytes a cell, 72 us at
+// 251x118x275 in tiles, now 24
+__global__ void __launch_bounds__(NT) k_search(int n, const float* __restrict__ aw, const float* __restrict__ r, float* __restrict__ s,
+                                               const Scalars* sc) {
     if (sc->converged) return;
     const float beta = sc->beta_f;
-    for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
-        int x, y, z;
-        tile_cell(g, T, t, x, y, z);
-        if (x >= g.X || y >= g.Y) continue;
-        if (is_ground(g, x, y, z)) continue;
-        const int c = cidx(g, x, y, z);
-        const float zv = r[c] * precon_of(aw[c]);
-        s[c] = zv + beta * s[c];
-    }
+    auto cell = [&](float a, float rv, float sv) {
+        return fmaf(beta, sv, __fmul_rn(rv, precon_of(a)));
+    };
+    stream4(n,
+            [&](int i) {
+                const float4 a = reinterpret_cast<const float4*>(aw)[i], rv = reinterpret_cast<const float4*>(r)[i];
+                const float4 sv = reinterpret_cast<float4*>(s)[i];
+                reinterpret_cast<float4*>(s)[i] = make_float4(cell(a.x, rv.x, sv.x), cell(a.y, rv.y, sv.y), cell(a.z, rv.z, sv.z), cell(a.w, rv.w, sv.w));
+            },
+            [&](int c) { s[c] = cell(aw[c], r[c], s[c]); });
 }
 
 // ---- vectorised PCG iteration (X % 4 == 0): float4 streams, FP32-compensated per-thread sums,
@@ -1446,6 +1539,8 @@ void launch_project(Env& e, float dtS) {
     // the GPU
     const int n4 = g.N / 4;
     const int nstream = std::min(std::min((n4 + UT - 1) / UT, e.num_sms * 16), kMaxPartials);
+    const int nany = std::max(1, std::min(std::min((n4 + NT - 1) / NT, e.num_sms * 16), kMaxPartials));
+    const Runs MT = matvec_runs(g, e.num_sms);
     const dim3 mvb(32, MVY);
     const int gx = (g.X / 4 + 31) / 32, gy = (g.Y + MVY - 1) / MVY;
     // about 6 blocks of 1024 threads per SM in the operator's grid (one resident at a time): at
@@ -1485,9 +1580,9 @@ void launch_project(Env& e, float dtS) {
                 { ProfScope ps(e, "pcg_search"); e.launches += 1;
                   k_search4<<<nstream, UT, 0, e.stream>>>(n4, (const float4*)e.aw, (const float4*)e.r, (float4*)e.s, e.sc); }
             } else {
-                { ProfScope ps(e, "pcg_matvec"); e.launches += 1; k_matvec<<<nblk, NT, 0, e.stream>>>(g, T, e.ax, e.ay, e.az, e.aw, e.s, e.As, ref, e.sc, e.partials); }
-                { ProfScope ps(e, "pcg_update"); e.launches += 1; k_update<<<nblk, NT, 0, e.stream>>>(g, T, e.aw, e.s, e.As, e.pp, e.r, ref, e.cfg.pcg_tol, e.cfg.pcg_max_iter, e.sc, e.partials); }
-                { ProfScope ps(e, "pcg_search"); e.launches += 1; k_search<<<nblk, NT, 0, e.stream>>>(g, T, e.aw, e.r, e.s, e.sc); }
+                { ProfScope ps(e, "pcg_matvec"); e.launches += 1; k_matvec<<<std::min(MT.n, kMaxPartials), dim3(32, MW), 0, e.stream>>>(g, MT, e.ax, e.ay, e.az, e.aw, e.s, e.As, ref, e.sc, e.partials); }
+                { ProfScope ps(e, "pcg_update"); e.launches += 1; k_update<<<nany, NT, 0, e.stream>>>(g.N, g.XY, e.aw, e.s, e.As, e.pp, e.r, ref, e.cfg.pcg_tol, e.cfg.pcg_max_iter, e.sc, e.partials); }
+                { ProfScope ps(e, "pcg_search"); e.launches += 1; k_search<<<nany, NT, 0, e.stream>>>(g.N, e.aw, e.r, e.s, e.sc); }
             }
     };
     auto tail = [&]() {  // the last directions' pressure updates (no later operator launch carries them)
