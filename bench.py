@@ -45,8 +45,8 @@ METRIC = "cell-steps/s at 512x512x256, mixed vs plain PCG at 1e-5 rel err; % HBM
 # Algorithmic bytes per cell per launch of each profiled stage (FP32 fields; each array counted
 # once per launch; neighbour re-reads excluded).
 STAGE_BYTES = {
-    "pcg_matvec": 40.0,   # fused: z, s_old, aw, ax, ay, az read; p read+write; s_new, As write
-    "pcg_update": 20.0,   # fused: r read+write; As, aw read; z write
+    "pcg_matvec": 40.0,   # stored coefficients: z, s_old, aw, ax, ay, az read; p read+write; s_new, As write
+    "pcg_update": 20.0,   # r read+write; As, aw read; z write
     "pcg_search": 16.0,   # unfused (--pcg-fused 0): r, aw read; s read+write
     "diffuse": 8.0,       # per sweep: in read, out write
     "advect": 12.0,       # per pass: q, vel read; out write
@@ -61,13 +61,24 @@ STAGE_BYTES = {
 }
 
 
-# DRAM traffic per cell of one launch of the plain PCG's kernels: ncu dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch at 512x256x256 (33554432 cells), k_matvec_search4 and
-# k_residual4. Every array is streamed once per launch, so the traffic grows with the cells and is
-# scaled to the launch size here.
+# The matrix-free plain PCG (the default above about a million cells, nx % 4 == 0): the operator reads z,
+# s_old, the reciprocal density and one word and writes s_new and As; the residual's 20 B and, every
+# fourth iteration, the pressure's 24 B (four directions read, p read+write) share a profile stage of
+# five launches in four iterations. 24 + 20 + 6 = 50 B an iteration.
+FREE_BYTES = {"pcg_matvec": 24.0, "pcg_update": (4 * 20.0 + 24.0) / 5}
+FREE_ITERATION_BYTES = 50.0
+
+# DRAM traffic per cell of one launch: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at
+# 512x256x256 (33554432 cells). Every array is streamed once per launch, so the traffic grows with the
+# cells and is scaled to the launch size here. With stored coefficients, then matrix-free
+# (k_pcg_operator4, and the mean of four k_residual4 and one k_pressure4).
 MEASURED_TRAFFIC_PER_CELL = {
     "pcg_matvec": (981.662976 + 375.963392) * 1e6 / 33554432,
     "pcg_update": (402.723840 + 224.641536) * 1e6 / 33554432,
+}
+FREE_TRAFFIC_PER_CELL = {
+    "pcg_matvec": (554.915328 + 234.966016) * 1e6 / 33554432,
+    "pcg_update": (4 * (402.703104 + 219.609088) + 671.106048 + 112.221696) / 5 * 1e6 / 33554432,
 }
 
 
@@ -268,8 +279,9 @@ def stage_bytes(diffuse_depth=1):
 
 def step_bytes(mode, pcg_iters, outer, diffuse_depth=1):
     """Algorithmic bytes per cell-step of the whole step as the library moves them: the stages
-    (stage_bytes) plus the pressure solve. Plain Jacobi-PCG: 60 B per iteration (the operator with
-    the search step and the pressure update 40 B, the residual update with z = r/diag 20 B). Mixed:
+    (stage_bytes) plus the pressure solve. Plain Jacobi-PCG with stored coefficients: 60 B per iteration
+    (the operator with the search step and the pressure update 40 B, the residual update with
+    z = r/diag 20 B). Mixed:
     per inner iteration the operator + search (32 B), the update (24 B) and the V-cycle (93 B: four
     finest-level passes of 16-24.5 B with FP16 coefficients plus the coarser levels), per
     refinement step the float-float residual (32 B) and the correction (20 B)."""
@@ -296,8 +308,8 @@ def mode_config(args, mode):
 def scope_step_bytes(mode, pcg_iters, outer):
     """The scope table's algorithmic model of a cell-step: 2558 B of stages plus 52 B per Jacobi-PCG
     iteration (matrix-free: the operator's coefficients formed from the density, 4 B, instead of
-    four stored coefficient arrays, 16 B) plus 40 B per refinement step. The library streams the
-    stored coefficients (60 B per plain iteration, 1.15x the model's 52 B)."""
+    four stored coefficient arrays, 16 B) plus 40 B per refinement step. The library's own matrix-free
+    iteration moves 50 B (the pressure four iterations at a time)."""
     assert mode != "mixed"  # the model has no term for the V-cycle
     return 2558.0 + 52.0 * pcg_iters
 
@@ -501,31 +513,31 @@ def main():
     dname, d = dom
     per_launch_ms = d["ms"] / max(d["kernels"], 1)
     peak, peak_kind = measured_peak()
-    bpc = STAGE_BYTES.get(dname)
+    # the library's own rule (above the one-launch PCG's size, float4 rows) for the matrix-free iteration
+    free = head["mode"] != "mixed" and args.pcg_fused and init.nx % 4 == 0 and "pcg_matvec" in prof
+    bpc = FREE_BYTES[dname] if free and dname in FREE_BYTES else STAGE_BYTES.get(dname)
     roofline = None
     if bpc:
         achieved = bpc * cells / (per_launch_ms / 1e3) / 1e9
-        tpc = MEASURED_TRAFFIC_PER_CELL.get(dname) if (head["mode"] == "plain" and args.pcg_fused) else None
+        tpc = FREE_TRAFFIC_PER_CELL.get(dname) if (head["mode"] == "plain" and free) else None
         roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                     "frac": round(achieved / peak, 4), "traffic": int(tpc * cells) if tpc else None, "kernel": dname,
                     "bytes_per_cell": bpc, "launch_us": round(per_launch_ms * 1e3, 2), "peak_source": peak_kind}
         if tpc:
             roofline["traffic_source"] = ("ncu DRAM bytes read + written by one launch at 512x256x256, scaled to this "
-                                          "launch's cells (bytes per launch)")
+                                          "launch's cells (bytes per launch; pcg_update: the mean of its kernels)")
     step_ms_prof = sum(v["ms"] for v in prof.values())
     depth = head["tuning"].get("diffuse_depth", 1)
-    bstep = step_bytes(head["mode"], head["pcg_iters"], head["outer"], depth)
+    bstep = stage_bytes(depth) + FREE_ITERATION_BYTES * head["pcg_iters"] if free else step_bytes(head["mode"], head["pcg_iters"], head["outer"], depth)
     step_model = {"bytes_per_cell_step": bstep, "achieved_gbs": round(bstep * head["value"] / 1e9, 1),
                   "frac": round(bstep * head["value"] / 1e9 / peak, 4), "peak_source": peak_kind,
                   "model": (f"the library's own bytes: {stage_bytes(depth):.0f} B of stages (diffusion at {depth} sweep(s) per "
-                            "pass) + 60 B per plain PCG iteration (stored coefficients)")}
+                            "pass) + " + ("50 B per plain PCG iteration (matrix-free)" if free else "60 B per plain PCG iteration (stored coefficients)"))}
     if head["mode"] != "mixed":
         sb = scope_step_bytes(head["mode"], head["pcg_iters"], head["outer"])
         step_model["scope_model"] = {
             "bytes_per_cell_step": sb, "frac": round(sb * head["value"] / 1e9 / peak, 4),
-            "model": "2558 B of stages + 52 B per matrix-free Jacobi-PCG iteration; the library streams four stored "
-                     "coefficient arrays (16 B) where the model reads the density (4 B): 60 / 52 = 1.15x the "
-                     "model's solver bytes"}
+            "model": "2558 B of stages + 52 B per matrix-free Jacobi-PCG iteration (the library's own moves 50 B)"}
 
     # ---- end to end through the C ABI from host buffers (headline mode) -------------------
     e2e = None
@@ -603,15 +615,15 @@ def main():
                                      f"{head['residual']:.3g} > 1e-5), as the reference's does")
     if "plain_textbook" in res:
         t = res["plain_textbook"]
+        tdepth = t["tuning"].get("diffuse_depth", 1)
+        tbytes = stage_bytes(tdepth) + FREE_ITERATION_BYTES * t["pcg_iters"] if free else step_bytes("plain", t["pcg_iters"], 0, tdepth)
         out["plain_textbook"] = {
             "value": t["value"], "ms_per_step": t["ms_per_step"], "semantics": "textbook",
             "pcg_iters_per_step": t["pcg_iters"], "converged": t["converged"], "max_residual": t["residual"],
             "pcg_max_iter": t["pcg_max_iter"], "gpu_launches": t["launches"], "clocks": t["clocks"],
             "note": "the plain Jacobi-PCG on the textbook (symmetric) operator the mixed mode solves, run without the "
                     "iteration cap to the reference's stop test max |r| <= 1e-5",
-            "step_roofline": {"bytes_per_cell_step": step_bytes("plain", t["pcg_iters"], 0, t["tuning"].get("diffuse_depth", 1)),
-                              "frac": round(step_bytes("plain", t["pcg_iters"], 0, t["tuning"].get("diffuse_depth", 1)) * t["value"]
-                                            / 1e9 / peak, 4),
+            "step_roofline": {"bytes_per_cell_step": tbytes, "frac": round(tbytes * t["value"] / 1e9 / peak, 4),
                               "scope_model_frac": round(scope_step_bytes("plain", t["pcg_iters"], 0) * t["value"] / 1e9 / peak, 4)},
             "profile_ms": {k: round(v["ms"], 3) for k, v in t["prof"].items()}}
     if "mixed" in res and head["mode"] != "mixed":

@@ -87,9 +87,10 @@ typedef struct {
                            skt_step call. Not used while per-stage profiling is on. 0: launches
                            issued stream-ordered, the loop counts read back by the host. */
     int mg_half;        /* MIXED: the V-cycle smooths with FP16 copies of the finest coefficients */
-    int pcg_fused;      /* PLAIN, nx % 4 == 0: two launches per iteration (search step and pressure
-                           update fused into the operator's march) instead of three; same values up
-                           to the dot products' summation order */
+    int pcg_fused;      /* PLAIN: 1 the whole solve in one launch up to about a million cells, above that
+                           (nx % 4 == 0) two launches per iteration with the search step fused into a
+                           matrix-free operator and the pressure updated every fourth one; 0 three
+                           launches per iteration; same values up to the dot products' summation order */
 } skt_solver_cfg;
 
 typedef struct {
@@ -287,7 +288,8 @@ skt_status skt_set_tuning(skt_env* env, const skt_tuning* t);
  * name and grid in that file (and no SKT_TUNE_FORCE), the entry is applied; otherwise every
  * candidate shape is timed on scratch copies of the environment's own fields (a few hundred
  * milliseconds at 512x256x512), candidates whose results differ from the default shapes' in any
- * bit are rejected, the fastest are applied and, with cache_path set, written to the cache (a JSON
+ * bit are rejected, the grid size's own shapes give way only to ones at least 3 % faster, and the
+ * choice is applied and, with cache_path set, written to the cache (a JSON
  * object, one entry per line). Call between steps; the fields are not changed. Allocates one small
  * device counter while measuring. */
 skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tuning* out);

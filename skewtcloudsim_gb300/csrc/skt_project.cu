@@ -581,8 +581,8 @@ struct Dirs {
 // barrier a plane frees the slot. s_old and s_new are distinct buffers (a block's halo rows are another
 // block's own rows). FIRST: the direction is z itself.
 // What bounds it: HBM, 24 bytes a cell where the stored coefficients and the pressure made 40 (421 us a
-// launch at 512x512x256 then, about 290 now: 5.5 TB/s); the barrier of a plane takes the rest. An iteration with its residual and a quarter of the pressure's update went from 635 to 514
-// us, at 256x256x128 from 103 to 82. Loading the planes into registers instead of the ring left the
+// launch at 512x512x256 then, 247 now: 6.5 TB/s, 23.5 bytes of DRAM traffic a cell). An iteration with its
+// residual and a quarter of the pressure's update went from 635 to 514 us, at 256x256x128 from 103 to 82. Loading the planes into registers instead of the ring left the
 // lanes waiting (400 us, DRAM 48 % busy; with a plane's loads ahead and 512 threads a block 460). Tiles
 // of 16 rows with 4 or 5 slots: 516 and 518 us an iteration, 20 rows 527, 24 rows 550, 12 rows two blocks
 // per SM 531, 8 rows with 5 slots 532.
