@@ -203,6 +203,73 @@ __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(LvlView L, const f
     for (int i = threadIdx.x; i < n; i += kCoarseThreads) x[i] = xa[i];
 }
 
+// The same where a thread can own kCoarseRun cells of a column along z (levels of up to 2048 cells, and more with
+// a few planes): the own values and the neighbour along z stay in registers, a cell reads five values from
+// shared memory instead of seven, and every load stands before the sweep's first store. A projection takes
+// 1.24 ms at 64x32x64 (1.33 with k_mg_coarse), 7.38 at 256x128x256 (7.57); runs of four cells 1.30 and 7.46, of
+// eight, too few warps for the latency, 1.44 and 7.61. Larger levels have more cells a thread than registers for
+// this form.
+constexpr int kCoarseRun = 2, kCoarseRunThreads = 1024;
+__global__ void __launch_bounds__(kCoarseRunThreads) k_mg_coarse_run(LvlView L, const float* __restrict__ b, float* __restrict__ x, const int* skip) {
+    after_previous();
+    if (skip && *skip) return;
+    extern __shared__ float sm[];
+    const int X = L.X, Y = L.Y, Z = L.Z, XY = X * Y, n = XY * Z;
+    const bool on = int(threadIdx.x) < XY * ((Z + kCoarseRun - 1) / kCoarseRun);
+    const int col = on ? threadIdx.x % XY : 0, z0 = on ? threadIdx.x / XY * kCoarseRun : 0;
+    const int nk = on ? min(kCoarseRun, Z - z0) : 0, c0 = col + XY * z0, xx = col % X, yy = col / X;
+    float* xa = sm + XY;
+    float* xb = xa + n + 2 * XY;
+    float cw[kCoarseRun], cl[kCoarseRun], cr[kCoarseRun], cd[kCoarseRun], cu[kCoarseRun], bv[kCoarseRun], cz[kCoarseRun + 1], v[kCoarseRun];
+    cz[0] = on && z0 > 0 ? L.az[c0 - XY] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kCoarseRun; ++k) {
+        const bool in = k < nk;
+        const int c = in ? c0 + k * XY : 0;
+        v[k] = 0.0f;
+        cw[k] = in ? L.aw[c] : 0.0f;
+        bv[k] = in ? b[c] : 0.0f;
+        cl[k] = (in && xx > 0) ? L.ax[c - 1] : 0.0f;
+        cr[k] = (in && xx + 1 < X) ? L.ax[c] : 0.0f;
+        cd[k] = (in && yy > 0) ? L.ay[c - X] : 0.0f;
+        cu[k] = (in && yy + 1 < Y) ? L.ay[c] : 0.0f;
+        cz[k + 1] = (in && z0 + k + 1 < Z) ? L.az[c] : 0.0f;
+    }
+    for (int i = threadIdx.x; i < 2 * (n + 2 * XY); i += blockDim.x) sm[i] = 0.0f;
+    __syncthreads();
+    for (int it = 0; it < kCoarseSweeps; ++it) {
+        const float* const q = xa + c0;
+        const float bottom = on ? q[-XY] : 0.0f, top = nk == kCoarseRun ? q[kCoarseRun * XY] : 0.0f;
+        float nl[kCoarseRun], nr[kCoarseRun], nd[kCoarseRun], nu[kCoarseRun], w[kCoarseRun];
+#pragma unroll
+        for (int k = 0; k < kCoarseRun; ++k) {  // every load before the first store
+            const float* const p = q + (k < nk ? k : 0) * XY;
+            nl[k] = p[-1]; nr[k] = p[1]; nd[k] = p[-X]; nu[k] = p[X];
+        }
+#pragma unroll
+        for (int k = 0; k < kCoarseRun; ++k) {
+            const float d = cw[k], xc = v[k];
+            float a = fmaf(d, xc, __fmul_rn(cl[k], nl[k]));
+            a = fmaf(cr[k], nr[k], a);
+            a = fmaf(cd[k], nd[k], a);
+            a = fmaf(cu[k], nu[k], a);
+            a = fmaf(cz[k], k > 0 ? v[k > 0 ? k - 1 : 0] : bottom, a);
+            a = fmaf(cz[k + 1], k + 1 < kCoarseRun ? v[k + 1 < kCoarseRun ? k + 1 : k] : top, a);
+            w[k] = d == 0.0f ? 0.0f : fmaf(kOmega, __fdividef(bv[k] - a, d), xc);
+        }
+#pragma unroll
+        for (int k = 0; k < kCoarseRun; ++k) {
+            v[k] = w[k];
+            if (k < nk) xb[c0 + k * XY] = w[k];
+        }
+        __syncthreads();
+        float* t = xa; xa = xb; xb = t;
+    }
+#pragma unroll
+    for (int k = 0; k < kCoarseRun; ++k)
+        if (k < nk) x[c0 + k * XY] = v[k];
+}
+
 // ---- refinement / CG helpers (1D over all cells) ---------------------------------------------
 
 constexpr int RT = 256;
@@ -876,6 +943,7 @@ bool mg_allocate(Env& e) {
     }
     if (X * Y * Z > kCoarseMax) return false;  // no level small enough for the one-block solve
     cudaFuncSetAttribute(k_mg_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoarseSmemMax);
+    cudaFuncSetAttribute(k_mg_coarse_run, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoarseSmemMax);
     const size_t hbytes = al(size_t(g.N) * 2) * 4;
     bytes += hbytes;
     if (cudaMalloc(&e.mg_pool, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
@@ -962,8 +1030,9 @@ void vcycle_vec(Env& e, int l, const CT* ax, const CT* ay, const CT* az, const C
 bool vcycle(Env& e, int l, const float* b, float* x, float* x2, const int* skip, int dot) {
     const LvlView L = view(e, l);
     if (l == e.mg_levels) {
-        const int n = L.X * L.Y * L.Z;
-        launch_next(e, k_mg_coarse, 1, kCoarseThreads, coarse_smem(L.X, L.Y, L.Z), L, b, x, skip);
+        const int runs = L.X * L.Y * ((L.Z + kCoarseRun - 1) / kCoarseRun);
+        if (runs <= kCoarseRunThreads) launch_next(e, k_mg_coarse_run, 1, (runs + 31) / 32 * 32, coarse_smem(L.X, L.Y, L.Z), L, b, x, skip);
+        else launch_next(e, k_mg_coarse, 1, kCoarseThreads, coarse_smem(L.X, L.Y, L.Z), L, b, x, skip);
         e.launches += 1;
         return false;
     }

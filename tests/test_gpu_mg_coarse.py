@@ -1,4 +1,4 @@
-"""The V-cycle's coarsest level (k_mg_coarse), where it can go wrong: a grid that has no coarser level, at
+"""The V-cycle's coarsest level (k_mg_coarse_run, k_mg_coarse), where it can go wrong: a grid that has no coarser level, at
 the largest size the kernel takes, with one of its planes in two and so the largest zero planes around the
 iterate (more shared memory than a launch has by default), coarsest levels whose cells end inside a warp,
 terrain. The mixed projection against the FP64 oracle solved to 1e-13: relative L2 1e-6 on u, w, p and rho
@@ -18,6 +18,7 @@ pytestmark = pytest.mark.gpu
     (16, 8, 16, 0), (32, 16, 8, 0),   # the coarsest level alone, 2048 and 4096 cells
     (64, 32, 2, 0),                   # two planes of 2048
     (32, 16, 16, 0), (40, 24, 56, 0), (72, 40, 72, 0),
+    (24, 16, 30, 1),                  # an odd number of planes, half a run at the end
     (128, 64, 64, 1),
 ])
 def test_coarsest_level_matches_fp64(gpu_lib, x, y, z, hills):
