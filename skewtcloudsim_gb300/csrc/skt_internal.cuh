@@ -332,6 +332,7 @@ struct Env {
     // whose results do not depend on their grid use it; the reductions keep num_sms, so a member's
     // bits are the same inside an ensemble and alone.
     int stencil_sms = 0;
+    unsigned big_smem = 0;  // two-sweep kernels whose shared-memory limit is raised on this environment's device (allow_smem)
     int pcg_grid_cap[4] = {-1, -1, -1, -1};  // k_pcg_grid: blocks resident at once per cells-per-thread variant (-1: not asked yet)
     std::string err;
     int flat = 1;  // all gh == 0

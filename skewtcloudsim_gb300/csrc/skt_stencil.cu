@@ -1716,6 +1716,20 @@ bool field_tensor_map(const Grid& g, const float* base, int width, int rows, CUt
 
 namespace {
 
+// Raises a kernel's dynamic shared-memory limit where this environment has not yet (bit: the kernel's place
+// in Env::big_smem). The limit belongs to the device's context, and every environment has its own device,
+// so nothing about it is kept process-wide. False: the kernel cannot have that much.
+template <class K>
+bool allow_smem(Env& e, int bit, K kernel, int bytes) {
+    if (e.big_smem >> bit & 1u) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    e.big_smem |= 1u << bit;
+    return true;
+}
+
 template <bool THETA, int H>
 bool launch_diffuse2(Env& e, int bps, const float* src, float* dst, int sides, int ground, const float* def, float k,
                      const float* face) {
@@ -1726,11 +1740,7 @@ bool launch_diffuse2(Env& e, int bps, const float* src, float* dst, int sides, i
     int zlen;
     const int zc = z_runs(e, gx, gy, bps, zlen);
     constexpr int smem = d2_smem_bytes<H>();
-    static bool attr = false;  // per template instance
-    if (!attr) {
-        cudaFuncSetAttribute(k_diffuse2<THETA, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr = true;
-    }
+    if (!allow_smem(e, 0 + (H == 8 ? 2 : 0) + THETA, k_diffuse2<THETA, H>, smem)) return false;
     k_diffuse2<THETA, H><<<dim3(gx, gy, zc), dim3(32, D2WARPS), smem, e.stream>>>(map, g, zlen, dst, sides, ground, def, k, face, e.sc);
     return true;
 }
@@ -1752,13 +1762,8 @@ bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const flo
     int zlen;
     const int zc = z_runs(e, gx, gy * F.n, bps, zlen);
     constexpr int smem = p4_smem_bytes<R>();
-    static bool attr = false;  // per template instance
-    if (!attr) {
-        cudaFuncSetAttribute(k_diffuse_pair4<THETA, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        cudaFuncSetAttribute(k_diffuse_pair4<THETA, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr = true;
-    }
     const auto kernel = F.n == 1 ? k_diffuse_pair4<THETA, false, R> : k_diffuse_pair4<THETA, true, R>;
+    if (!allow_smem(e, 4 + (R == 14 ? 4 : 0) + (F.n == 1 ? 2 : 0) + THETA, kernel, smem)) return false;
     launch_next(e, kernel, dim3(gx, gy, zc * F.n), 32 * (R + 3), smem, maps.m, g, zlen, zc, F, k, face, e.sc);
     e.launches += 1;
     return true;
@@ -1766,7 +1771,7 @@ bool launch_diffuse_pair4(Env& e, int bps, const FieldSet& F, float k, const flo
 
 // one pass of two sweeps with the tuned kernel: k_diffuse_pair4 (float4 lanes, rows 6 or 14 per
 // block) or k_diffuse2 (one cell per lane, rows 4 or 8 per warp, field by field); false without a
-// tensor map
+// tensor map or the shared memory
 template <bool THETA>
 bool launch_pair(Env& e, const FieldSet& F, float k, const float* face, PassMaps& maps) {
     const int h = e.tune.diffuse_h, bps = e.tune.diffuse2_bps;
@@ -1839,7 +1844,7 @@ void diffuse_pass(Env& e, const FieldSet& F, bool two, float k, const float* fac
         one(F);
         return;
     }
-    for (int i = 0; i < F.n; ++i) {  // no tensor-map encoder: the two sweeps as two passes, field by field
+    for (int i = 0; i < F.n; ++i) {  // no tensor-map encoder or no shared memory: the two sweeps as two passes, field by field
         FieldSet A;
         A.n = 1;
         A.in[0] = F.in[i];
