@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "skt_physics.cuh"
+#include "skt_sum.hpp"
 #include "../../include/skewt.h"
 
 namespace skt {
@@ -108,115 +109,128 @@ __device__ __forceinline__ bool nonfinite(float v) { return (__float_as_uint(v) 
 constexpr int kMaxPartials = 4096;
 
 // ---- dot products and maxima over the grid ---------------------------------------------------
-// A reduction keeps its sums as an unevaluated pair of floats (about 48 significant bits) from the
-// threads to the total, which becomes FP64 once. The chip's FP64 rate is about 1/60 of its FP32
-// rate: a tree of FP64 shuffles and adds held the pipe for 16 cycles per warp and add, some 2600
-// cycles for a block of 1024 threads, while the pair's five levels cost about 60 FP32 instructions
-// per warp. Products are taken exactly (fma) where FP64 took them exactly; the totals round to the
-// same FP32 step lengths (every output of the plain and mixed steps bit-identical at the sizes
-// below). A plain step at 64x32x64 went from 2.78 to 2.42 ms, at 256x128x256 from 31.1 to 28.5 ms.
-struct Sum2 {
-    float h = 0.0f, l = 0.0f;
-    // (h, l) += (b, e): two-sum on the leading parts, the rest in the low parts
-    __device__ __forceinline__ void add(float b, float e) {
-        const float s = __fadd_rn(h, b);
-        const float bv = __fsub_rn(s, h);
-        const float t = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bv)), __fsub_rn(b, bv));
-        l = (l + e) + t;
-        h = s;
-    }
-    // the exact product a * b
-    __device__ __forceinline__ void add_prod(float a, float b) {
-        const float p = __fmul_rn(a, b);  // never contracted into the sum below
-        add(p, fmaf(a, b, -p));
-    }
-    __device__ __forceinline__ double value() const { return double(h) + double(l); }
-    // the quotient of two pairs, rounded to float: a first quotient and its remainder's correction
-    __device__ __forceinline__ float over(const Sum2& d) const {
-        const float q = __fdiv_rn(h, d.h);
-        const float rem = fmaf(-q, d.h, h) + (l - q * d.l);
-        const float c = q + __fdividef(rem, d.h);
-        return isfinite(c) ? c : q;  // a zero or non-finite divisor: what the plain division gives
-    }
-};
-__device__ __forceinline__ Sum2 sum2_of(double v) {
-    Sum2 p;
-    p.h = float(v);
-    p.l = float(v - double(p.h));
-    return p;
+// The totals have FP64's range and at least its precision on every level: a thread's sum (skt_sum.hpp, or
+// the compensated FP32 sum of the vectorised kernels), a warp's exact total in whole numbers, FP64 from the
+// warps to the grid. The chip's FP64 rate is about 1/60 of its FP32 rate and an FP64 add takes 65 cycles, so
+// FP64 stays with a few lanes of a block: a tree of FP64 shuffles in every warp held the pipe for 16 cycles
+// per warp and add, some 2600 for a block of 1024 threads; the cuts and integer reductions cost about 45
+// instructions per warp.
+template <bool T>
+__device__ __forceinline__ WarpSum warp_sum(Sum v) {
+    normalise<T>(v);
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(v.h) & 0x7fffffffu) >> 23;
+    WarpSum w{0, 0, 0, max(top, 48u)};
+    if (top == 255u) return w;
+    int a, b, c;
+    cut<T>(v, w.e, a, b, c);
+    w.a = __reduce_add_sync(0xffffffffu, a);
+    w.b = __reduce_add_sync(0xffffffffu, b);
+    w.c = __reduce_add_sync(0xffffffffu, c);
+    return w;
 }
-// over the first N lanes (a power of two); every lane gets the sum of its group of N
+// FP64 over the first N lanes (a power of two); every lane gets the sum of its group of N
 template <int N = 32>
-__device__ __forceinline__ Sum2 warp_sum2(Sum2 v) {
+__device__ __forceinline__ double warp_sum64(double v) {
 #pragma unroll
-    for (int o = N / 2; o > 0; o >>= 1) {
-        const float h = __shfl_xor_sync(0xffffffffu, v.h, o), l = __shfl_xor_sync(0xffffffffu, v.l, o);
-        v.add(h, l);
-    }
+    for (int o = N / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+// The total of 2^K lanes' values (the others hold 0), in every lane, by integer reductions: what it loses lies
+// below 2^-51 of the largest value (an FP64 tree's bound is K 2^-53 of all values together). An FP64 add takes
+// 65 cycles, five levels with their shuffles 450.
+template <int K>
+__device__ __forceinline__ Fixed lanes_total(const Fixed& f) {
+    const bool some = f.v != 0 || f.u == kNotFinite;
+    const int u = int(__reduce_max_sync(0xffffffffu, unsigned(some ? f.u + 2048 : 0))) - 2048;
+    int hi = 0, mid = 0, lo = 0;
+    if (some) split(f, u, hi, mid, lo);
+    hi = __reduce_add_sync(0xffffffffu, hi);
+    mid = __reduce_add_sync(0xffffffffu, mid);
+    lo = __reduce_add_sync(0xffffffffu, lo);
+    return joined<K>(hi, mid, lo, u);
+}
+// a block's total from its 2^K warps' sums, warp w's in ws[w]; far (FAR): what a warp holds outside FP32's
+// range, which is nothing as a rule
+template <int K, bool FAR>
+__device__ __forceinline__ Fixed warps_total(const int4* ws, const double* far, int lane) {
+    int4 w = make_int4(0, 0, 0, 48);
+    if (lane < 1 << K) w = ws[lane];
+    Fixed f = lanes_total<K>(fixed_of(WarpSum{w.x, w.y, w.z, unsigned(w.w)}));
+    if (FAR) {
+        const double d = lane < 1 << K ? far[lane] : 0.0;
+        if (__any_sync(0xffffffffu, d != 0.0)) f = fixed_of(value(f) + warp_sum64(d));
+    }
+    return f;
+}
+// what the lanes hold outside FP32's range: nothing, as a rule
+__device__ __forceinline__ double warp_far(double v) { return __any_sync(0xffffffffu, v != 0.0) ? warp_sum64(v) : 0.0; }
+constexpr int log2_of(int n) { return n > 1 ? 1 + log2_of(n / 2) : 0; }
 // values >= 0 (their bits order as integers)
 __device__ __forceinline__ float warp_max(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
-// the sum and the maximum (values >= 0) of NTH threads with a linear thread id, in a fixed order; valid in tid 0
-template <int NTH>
-__device__ __forceinline__ void block_sum_max(Sum2& sum, float& mx, int tid) {
-    __shared__ float2 ss[NTH / 32];
-    __shared__ float sx[NTH / 32];
-    const Sum2 w = warp_sum2(sum);
-    const float m = warp_max(mx);
-    __syncthreads();
-    if ((tid & 31) == 0) {
-        ss[tid >> 5] = make_float2(w.h, w.l);
-        sx[tid >> 5] = m;
-    }
-    __syncthreads();
-    sum = Sum2();
-    mx = 0.0f;
-    if (tid < 32) {
-        if (tid < NTH / 32) {
-            sum.h = ss[tid].x;
-            sum.l = ss[tid].y;
-            mx = sx[tid];
-        }
-        sum = warp_sum2<NTH / 32>(sum);
-        mx = warp_max(mx);
-    }
-}
-// Publishes the block's sum and maximum (each thread's own values on entry) of a grid of nb blocks
-// (bid: this block's linear index); the last block to finish reduces all partials with every thread
-// (fixed assignment, fixed tree: deterministic). True in thread 0 of that block, with the totals.
-// The arrival is one acquire-release atomic of thread 0, ordered after its own partial's stores.
-template <int NTH>
-__device__ __forceinline__ bool grid_sum_max(Scalars* sc, double* partials, int bid, int nb, int tid, Sum2 sum, float mx, double& tot,
+// Publishes the block's sum and maximum (each thread's own values on entry; maxima >= 0) of a grid of nb
+// blocks (bid: this block's linear index, tid: the thread's of NTH); the last block to finish reduces all
+// partials (fixed assignment, fixed tree: deterministic). True in thread 0 of that block, with the totals.
+// The arrival is one acquire-release atomic of thread 0, ordered after its own partial's stores. FAR: sums of
+// Sum::add_prod, with a third and an FP64 part. Once per kernel.
+template <int NTH, bool FAR>
+__device__ __forceinline__ bool grid_sum_max(Scalars* sc, double* partials, int bid, int nb, int tid, const Sum& sum, float mx, double& tot,
                                              float& mxall) {
+    constexpr int W = NTH / 32, LT = NTH < 256 ? NTH : 256;  // warps; threads that sum the partials: their FP64 adds share one pipe
     __shared__ bool last;
-    float2* const psum = reinterpret_cast<float2*>(partials);
+    __shared__ int4 ws[W];
+    __shared__ float wx[W];
+    __shared__ double wd[FAR || W < LT / 32 ? W : LT / 32];
     float* const pmax = reinterpret_cast<float*>(partials + kMaxPartials);
-    block_sum_max<NTH>(sum, mx, tid);
-    if (tid == 0) {
-        __stcg(psum + bid, make_float2(sum.h, sum.l));
-        __stcg(pmax + bid, mx);
-        unsigned t;
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(t) : "l"(&sc->done_blocks) : "memory");
-        last = t == unsigned(nb) - 1u;
+    const int lane = tid & 31, warp = tid >> 5;
+    {
+        const WarpSum w = warp_sum<FAR>(sum);
+        const float m = warp_max(mx);
+        const double f = FAR ? warp_far(sum.far) : 0.0;
+        if (lane == 0) {
+            ws[warp] = make_int4(w.a, w.b, w.c, int(w.e));
+            wx[warp] = m;
+            if (FAR) wd[warp] = f;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const double s = value(warps_total<log2_of(W), FAR>(ws, wd, lane));
+        const float m = warp_max(lane < W ? wx[lane < W ? lane : 0] : 0.0f);
+        if (lane == 0) {
+            __stcg(partials + bid, s);
+            __stcg(pmax + bid, m);
+            unsigned t;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(t) : "l"(&sc->done_blocks) : "memory");
+            last = t == unsigned(nb) - 1u;
+        }
     }
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    Sum2 s;
-    float m = 0.0f;
-    for (int b = tid; b < nb; b += NTH) {
-        const float2 v = __ldcg(psum + b);
-        const float mb = __ldcg(pmax + b);
-        s.add(v.x, v.y);
-        m = mb > m ? mb : m;
+    if (tid < LT) {
+        double s = 0.0;
+        float m = 0.0f;
+        for (int b = tid; b < nb; b += LT) {
+            s += __ldcg(partials + b);
+            const float mb = __ldcg(pmax + b);
+            m = mb > m ? mb : m;
+        }
+        s = value(lanes_total<5>(fixed_of(s)));
+        m = warp_max(m);
+        if (lane == 0) {
+            wd[warp] = s;
+            wx[warp] = m;
+        }
     }
-    block_sum_max<NTH>(s, m, tid);
-    if (tid == 0) {
-        tot = s.value();
-        mxall = m;
-        sc->done_blocks = 0;
-        note_nonfinite(sc, tot);
+    __syncthreads();
+    if (warp == 0) {
+        constexpr int LW = LT / 32;
+        tot = warp_sum64<LW>(lane < LW ? wd[lane < LW ? lane : 0] : 0.0);
+        mxall = warp_max(lane < LW ? wx[lane < LW ? lane : 0] : 0.0f);
+        if (lane == 0) {
+            sc->done_blocks = 0;
+            note_nonfinite(sc, tot);
+        }
     }
     return tid == 0;
 }

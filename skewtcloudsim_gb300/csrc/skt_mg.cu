@@ -8,7 +8,7 @@
 //
 //   x64 = 0
 //   repeat: r = b - A x64 (FP64 arithmetic, FP64 norm)    until |r|/|b| <= refine_tol
-//           solve A e = r with MG-PCG in FP32 (paired-float reductions, Sum2) to |r_inner| <= inner_rtol |r|
+//           solve A e = r with MG-PCG in FP32 (FP64 reductions) to |r_inner| <= inner_rtol |r|
 //           x64 += e
 //
 // Multigrid: cell-centred, the hierarchy of the full grid (ground cells inactive: diagonal 0).
@@ -274,16 +274,9 @@ __global__ void __launch_bounds__(kCoarseRunThreads) k_mg_coarse_run(LvlView L, 
 
 constexpr int RT = 256;
 
-// a thread's compensated running sum (s, c) as the pair that the grid's reduction takes
-__device__ __forceinline__ Sum2 pair_of(float s, float c) {
-    Sum2 p;
-    p.h = s;
-    p.l = -c;
-    return p;
-}
-template <int NTH>
-__device__ __forceinline__ bool finish(Scalars* sc, double* partials, Sum2 sum, float mx, double& tot, float& mall, int tid) {
-    return grid_sum_max<NTH>(sc, partials, linear_block(), linear_blocks(), tid, sum, mx, tot, mall);
+template <int NTH, bool FAR>
+__device__ __forceinline__ bool finish(Scalars* sc, double* partials, const Sum& sum, float mx, double& tot, float& mall, int tid) {
+    return grid_sum_max<NTH, FAR>(sc, partials, linear_block(), linear_blocks(), tid, sum, mx, tot, mall);
 }
 
 // ---- float-float refinement vector ----------------------------------------------------------
@@ -327,7 +320,7 @@ __device__ __forceinline__ void refine_record(Scalars* sc, double tot, float mal
     sc->inner_tol = mall;  // the inner solves reduce the max residual relative to this
 }
 
-// r = b - A (xh + xl) in float-float, |r|^2 (compensated FP32 per thread, paired floats across threads)
+// r = b - A (xh + xl) in float-float, |r|^2 (compensated FP32 per thread, FP64 across warps)
 // and max|r|; any grid
 __global__ void __launch_bounds__(RT) k_resid_ff(Grid g, const float* __restrict__ ax, const float* __restrict__ ay, const float* __restrict__ az,
                                                  const float* __restrict__ aw, const float* __restrict__ xh, const float* __restrict__ xl,
@@ -357,7 +350,7 @@ __global__ void __launch_bounds__(RT) k_resid_ff(Grid g, const float* __restrict
     }
     double tot;
     float mall;
-    if (finish<RT>(sc, partials, pair_of(acc, comp), mx, tot, mall, threadIdx.x)) refine_record(sc, tot, mall, refine_tol, first);
+    if (finish<RT, false>(sc, partials, sum_of(acc, comp), mx, tot, mall, threadIdx.x)) refine_record(sc, tot, mall, refine_tol, first);
 }
 
 // (xh, xl) += e and e = 0
@@ -377,20 +370,20 @@ __global__ void __launch_bounds__(RT) k_cast_ff(int n, const float* __restrict__
     for (int c = blockIdx.x * RT + threadIdx.x; c < n; c += gridDim.x * RT) p[c] = xh[c] + xl[c];
 }
 
-// inner CG: rho = z.r (paired floats) and s = z (start), or beta = rho_new/rho and s = z + beta s
+// inner CG: rho = z.r (exact products, FP64) and s = z (start), or beta = rho_new/rho and s = z + beta s
 template <bool START>
 __global__ void __launch_bounds__(RT) k_zr_search(int n, const float* __restrict__ z, const float* __restrict__ r, float* __restrict__ s,
                                                   Scalars* sc, double* partials) {
     if (!START && sc->converged) return;
     // pass 1 of 2: the dot product; the search update runs in k_search_mg after beta is known
-    Sum2 acc;
+    Sum acc;
     for (int c = blockIdx.x * RT + threadIdx.x; c < n; c += gridDim.x * RT) {
         acc.add_prod(z[c], r[c]);
         if (START) s[c] = z[c];
     }
     double tot;
     float mall;
-    if (finish<RT>(sc, partials, acc, 0.0f, tot, mall, threadIdx.x)) {
+    if (finish<RT, true>(sc, partials, acc, 0.0f, tot, mall, threadIdx.x)) {
         if (START) {
             sc->sigma0 = tot;
             sc->converged = 0;
@@ -414,7 +407,7 @@ __global__ void __launch_bounds__(RT) k_matvec_mg(Grid g, const float* __restric
                                                   Scalars* sc, double* partials) {
     if (sc->converged) return;
     LvlView L{g.X, g.Y, g.Z, ax, ay, az, aw};
-    Sum2 acc;
+    Sum acc;
     for (int c = blockIdx.x * RT + threadIdx.x; c < g.N; c += gridDim.x * RT) {
         float v = 0.0f;
         if (aw[c] != 0.0f) {
@@ -426,7 +419,7 @@ __global__ void __launch_bounds__(RT) k_matvec_mg(Grid g, const float* __restric
     }
     double tot;
     float mall;
-    if (finish<RT>(sc, partials, acc, 0.0f, tot, mall, threadIdx.x)) {
+    if (finish<RT, true>(sc, partials, acc, 0.0f, tot, mall, threadIdx.x)) {
         sc->sigma1 = tot;
         sc->alpha = float(sc->sigma0 / tot);
     }
@@ -447,7 +440,7 @@ __global__ void __launch_bounds__(RT) k_update_mg(int n, const float* __restrict
     }
     double tot;
     float mall;
-    if (finish<RT>(sc, partials, Sum2(), mx, tot, mall, threadIdx.x)) {
+    if (finish<RT, false>(sc, partials, Sum(), mx, tot, mall, threadIdx.x)) {
         sc->iters += 1;
         sc->outer_inner_total += 1;
         if (mall <= inner_rtol * sc->inner_tol) sc->converged = 1;
@@ -598,7 +591,7 @@ __global__ void __launch_bounds__(32 * JVY, 32 / JVY) k_mg_smooth4(int X, int Y,
     if (DOT != DOT_NONE) {
         double tot;
         float mall;
-        if (finish<32 * JVY>(sc, partials, pair_of(acc, comp), 0.0f, tot, mall, tid)) {
+        if (finish<32 * JVY, false>(sc, partials, sum_of(acc, comp), 0.0f, tot, mall, tid)) {
             if (DOT == DOT_START) {
                 sc->sigma0 = tot;
                 sc->beta_f = 0.0f;
@@ -743,7 +736,7 @@ __global__ void __launch_bounds__(32 * JVY, 32 / JVY) k_mg_matvec_search4(int X,
     }
     double tot;
     float mall;
-    if (finish<32 * JVY>(sc, partials, pair_of(acc, comp), 0.0f, tot, mall, tid)) {
+    if (finish<32 * JVY, false>(sc, partials, sum_of(acc, comp), 0.0f, tot, mall, tid)) {
         sc->sigma1 = tot;
         sc->alpha = float(sc->sigma0 / tot);
     }
@@ -822,7 +815,7 @@ __global__ void __launch_bounds__(32 * JVY) k_resid_ff4(int X, int Y, int Z, int
     }
     double tot;
     float mall;
-    if (finish<32 * JVY>(sc, partials, pair_of(acc, comp), mx, tot, mall, tid)) refine_record(sc, tot, mall, refine_tol, first);
+    if (finish<32 * JVY, false>(sc, partials, sum_of(acc, comp), mx, tot, mall, tid)) refine_record(sc, tot, mall, refine_tol, first);
 }
 
 // FP16 copies of the finest level's coefficients for the V-cycle. Faces round toward zero; the
@@ -873,7 +866,7 @@ __global__ void __launch_bounds__(RT) k_update_mg4(int n4, const float4* __restr
     }
     double tot;
     float mall;
-    if (finish<RT>(sc, partials, Sum2(), mx, tot, mall, threadIdx.x)) {
+    if (finish<RT, false>(sc, partials, Sum(), mx, tot, mall, threadIdx.x)) {
         sc->iters += 1;
         sc->outer_inner_total += 1;
         if (mall <= inner_rtol * sc->inner_tol) sc->converged = 1;
@@ -881,7 +874,7 @@ __global__ void __launch_bounds__(RT) k_update_mg4(int n4, const float4* __restr
     }
 }
 
-// rho = z.r (paired floats across threads); START also sets s = z
+// rho = z.r (FP64 across warps); START also sets s = z
 template <bool START>
 __global__ void __launch_bounds__(RT) k_zr4(int n4, const float4* __restrict__ z, const float4* __restrict__ r, float4* __restrict__ s,
                                             Scalars* sc, double* partials) {
@@ -898,7 +891,7 @@ __global__ void __launch_bounds__(RT) k_zr4(int n4, const float4* __restrict__ z
     }
     double tot;
     float mall;
-    if (finish<RT>(sc, partials, pair_of(acc, comp), 0.0f, tot, mall, threadIdx.x)) {
+    if (finish<RT, false>(sc, partials, sum_of(acc, comp), 0.0f, tot, mall, threadIdx.x)) {
         if (START) {
             sc->sigma0 = tot;
             sc->converged = 0;

@@ -1,5 +1,5 @@
 // Pressure projection: boundary reset, Poisson coefficients + divergence, Jacobi-preconditioned
-// CG with paired-float reductions (Sum2), pressure/density update and the velocity correction.
+// CG with FP64 reductions, pressure/density update and the velocity correction.
 // Follows pressureProject / calculatePressureProject (Game/environment.cu:851-987).
 #include "skt_internal.cuh"
 #include "skt_tma.cuh"
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
                                               float* __restrict__ ax, float* __restrict__ ay, float* __restrict__ az, float* __restrict__ aw,
                                               float* __restrict__ r, float* __restrict__ s, float* __restrict__ pp, float* __restrict__ As,
                                               int faces, int reference, Scalars* sc, double* partials) {
-    Sum2 dsum;
+    Sum dsum;
     float mx = 0.0f;
     for (int t = blockIdx.x; t < T.n; t += gridDim.x) {
         int x, y, z;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
     }
     double tot;
     float mall;
-    if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
+    if (grid_sum_max<NT, true>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
         sc->sigma0 = tot;
         sc->sigma1 = 0.0;
         sc->iters = 0;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float*
                                                     float* __restrict__ As, int reference, Scalars* sc, double* partials) {
     if (sc->converged) return;
     const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY, lane = threadIdx.x;
-    Sum2 dsum;
+    Sum dsum;
     struct Plane {
         float cx[MR], cy[MR], cz[MR], cw[MR], es[MR], ea[MR], up, down, cd;
     };
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float*
     }
     double tot;
     float mall;
-    if (grid_sum_max<32 * MW>(sc, partials, blockIdx.x, gridDim.x, threadIdx.y * 32 + lane, dsum, 0.0f, tot, mall)) {
+    if (grid_sum_max<32 * MW, true>(sc, partials, blockIdx.x, gridDim.x, threadIdx.y * 32 + lane, dsum, 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(NT) k_update(int n, int XY, const float* __res
                                                int reference, float tol, int max_iter, Scalars* sc, double* partials) {
     if (sc->converged) return;
     const float alpha = sc->alpha;
-    Sum2 dsum;
+    Sum dsum;
     float mx = 0.0f;
     auto cell = [&](float a, float sv, float av, float& pv, float& rv, int c) {
         pv += alpha * sv;
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(NT) k_update(int n, int XY, const float* __res
             });
     double tot;
     float mall;
-    if (grid_sum_max<NT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
+    if (grid_sum_max<NT, true>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, dsum, mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
         if (mall <= tol) {
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(NT) k_search(int n, const float* __restrict__ 
 }
 
 // ---- vectorised PCG iteration (X % 4 == 0): float4 streams, FP32-compensated per-thread sums,
-// paired floats across threads and blocks --------------------------------------------------------------
+// FP64 across warps and blocks --------------------------------------------------------------
 
 struct Kahan {  // compensated FP32 running sum of one thread
     float s = 0.0f, c = 0.0f;
@@ -395,12 +395,7 @@ struct Kahan {  // compensated FP32 running sum of one thread
         c = (t - s) - y;
         s = t;
     }
-    __device__ __forceinline__ Sum2 pair() const {
-        Sum2 p;
-        p.h = s;
-        p.l = -c;
-        return p;
-    }
+    __device__ __forceinline__ Sum sum() const { return sum_of(s, c); }
 };
 
 constexpr int UT = 256;
@@ -436,7 +431,7 @@ __global__ void __launch_bounds__(UT) k_update4(int n4, int xy4, const float4* _
     }
     double tot;
     float mall;
-    if (grid_sum_max<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.pair(), mx, tot, mall)) {
+    if (grid_sum_max<UT, false>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.sum(), mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
         if (mall <= tol) {
@@ -549,7 +544,7 @@ __global__ void __launch_bounds__(MVT) k_matvec4(Grid g, int zlen, const float* 
     }
     double tot;
     float mall;
-    if (grid_sum_max<MVT>(sc, partials, linear_block(), linear_blocks(), tid, acc.pair(), 0.0f, tot, mall)) {
+    if (grid_sum_max<MVT, false>(sc, partials, linear_block(), linear_blocks(), tid, acc.sum(), 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -757,7 +752,7 @@ __global__ void __launch_bounds__(OPT, 2) k_pcg_operator4(const __grid_constant_
     }
     double tot;
     float mall;
-    if (grid_sum_max<OPT>(sc, partials, linear_block(), linear_blocks(), tid, acc.pair(), 0.0f, tot, mall)) {
+    if (grid_sum_max<OPT, false>(sc, partials, linear_block(), linear_blocks(), tid, acc.sum(), 0.0f, tot, mall)) {
         const double s1 = REF ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -796,7 +791,7 @@ __global__ void __launch_bounds__(UT) k_residual4(int n4, int xy4, const float4*
     }
     double tot;
     float mall;
-    if (grid_sum_max<UT>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.pair(), mx, tot, mall)) {
+    if (grid_sum_max<UT, false>(sc, partials, blockIdx.x, gridDim.x, threadIdx.x, acc.sum(), mx, tot, mall)) {
         sc->iters += 1;
         sc->residual = mall;
         if (mall <= tol) {
@@ -870,88 +865,109 @@ constexpr int kMaxGridBlocks = 256;           // blocks of the launch at most
 template <int K>
 int pcg_grid_smem(int X) { return (7 * K * GCT + 2 * X) * 4; }
 
-// one block's partial of a reduction: its sum, its maximum and the reduction's tag, read and written as one
-// 16-byte access so that a reader that sees the tag has the values with it
+// one block's partial of a reduction: its sum (Fixed's number), its maximum, and in one word the low 20 bits of
+// the reduction's tag and the sum's unit; read and written as one 16-byte access so that a reader that sees
+// the tag has the values with it
 struct alignas(16) GridPart {
-    float h, l, mx;
-    unsigned tag;
+    long long v;
+    float mx;
+    unsigned word;
 };
-__device__ __forceinline__ void put_part(GridPart* p, float h, float l, float mx, unsigned tag) {
-    asm volatile("{\n\t.reg .b64 lo, hi;\n\t.reg .b128 v;\n\tmov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 v, {lo, hi};\n\t"
-                 "st.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "f"(h), "f"(l), "f"(mx), "r"(tag) : "memory");
+__device__ __forceinline__ unsigned part_word(unsigned tag, int u) { return tag << 12 | unsigned(u + 2048); }
+__device__ __forceinline__ void put_part(GridPart* p, long long v, float mx, unsigned word) {
+    asm volatile("{\n\t.reg .b64 hi;\n\t.reg .b128 v;\n\tmov.b64 hi, {%2, %3};\n\tmov.b128 v, {%1, hi};\n\t"
+                 "st.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "l"(v), "f"(mx), "r"(word) : "memory");
 }
 __device__ __forceinline__ GridPart get_part(const GridPart* p) {
     GridPart r;
-    asm volatile("{\n\t.reg .b64 lo, hi;\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%4];\n\tmov.b128 {lo, hi}, v;\n\t"
-                 "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}" : "=f"(r.h), "=f"(r.l), "=f"(r.mx), "=r"(r.tag) : "l"(p) : "memory");
+    asm volatile("{\n\t.reg .b64 hi;\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%3];\n\tmov.b128 {%0, hi}, v;\n\t"
+                 "mov.b64 {%1, %2}, hi;\n\t}" : "=l"(r.v), "=f"(r.mx), "=r"(r.word) : "l"(p) : "memory");
     return r;
 }
 
 // (fence.acq_rel, not __threadfence, which is the sequentially consistent fence and slower)
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
+// what the threads of a block share of the solver's scalars; thread 0 writes between a reduction's barriers
+enum GridState { GRID_GO, GRID_DONE, GRID_CAP, GRID_NAN, GRID_STUCK };
+struct GridScalars {
+    double sigma0, sigma1;  // the dot products of the last iteration
+    float len, residual;    // the step length that the last reduction gave, the last max residual
+    int state;
+};
+
 // Reduces sum and maximum over the grid; a barrier too: every block writes its partial into every
 // block's inbox and waits for all partials in its own, one hop through L2 (1.5 us for 128 blocks,
 // 1.1 for 32; an arrival counter and then the partials 1.8 and 1.6, one block that sums for all 2.3
 // and 1.4, every block polling one set of partials 2.9 and 1.2). The partials are summed in the same
-// order everywhere, so every thread of the grid gets the same totals. FENCE: the block's stores
-// before the reduction are visible to every block after it. Inboxes alternate by the tag's parity: a
-// block may send the next partial while another still reads these, but not the one after that.
-// False when a wait ran out.
-template <bool FENCE>
-__device__ __forceinline__ bool grid_reduce(GridPart* inbox, int nb, unsigned tag, Sum2 sum, float mx, Sum2& tot, float& mall) {
-    __shared__ float2 ws[2][GCT / 32];
-    __shared__ float wm[2][GCT / 32];
-    __shared__ float4 ts[2][kMaxGridBlocks / 32];
+// order everywhere, so every block gets the same totals; its first warp forms the step length from
+// them in fin(total, maximum, whether no wait ran out), one lane of which stores. The FP64 work is the
+// polling warps' and the first one's alone. FENCE: the block's stores before the reduction are visible to
+// every block after it. Inboxes alternate by the tag's parity: a block may send the next partial while
+// another still reads these, but not the one after that.
+template <bool FENCE, bool EXACT, class Fin>
+__device__ __forceinline__ void grid_reduce(GridPart* inbox, int nb, unsigned tag, const Sum& sum, float mx, Fin fin) {
+    constexpr int W = GCT / 32, B = kMaxGridBlocks / 32;
+    __shared__ int4 ws[W];
+    __shared__ float wm[W], tm[B];
+    __shared__ double wf[W], ts[B];
+    __shared__ int tk[B];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, par = tag & 1u, nw = (nb + 31) >> 5;
-    sum = warp_sum2(sum);
-    mx = warp_max(mx);
-    if (lane == 0) {
-        ws[par][warp] = make_float2(sum.h, sum.l);
-        wm[par][warp] = mx;
+    {
+        const WarpSum v = warp_sum<EXACT>(sum);
+        const float m = warp_max(mx);
+        const double f = EXACT ? warp_far(sum.far) : 0.0;
+        if (lane == 0) {
+            ws[warp] = make_int4(v.a, v.b, v.c, int(v.e));
+            wm[warp] = m;
+            if (EXACT) wf[warp] = f;
+        }
     }
     __syncthreads();
+    double tot = 0.0;
+    float mall = 0.0f;
+    bool ok = true;
     if (warp < nw) {
-        Sum2 s;
-        s.h = ws[par][lane & (GCT / 32 - 1)].x;
-        s.l = ws[par][lane & (GCT / 32 - 1)].y;
-        s = warp_sum2<GCT / 32>(s);
-        float m = warp_max(wm[par][lane & (GCT / 32 - 1)]);
+        const Fixed s = warps_total<log2_of(W), EXACT>(ws, wf, lane);
+        const float m = warp_max(lane < W ? wm[lane % W] : 0.0f);
         if (FENCE) fence_gpu();
-        bool ok = true;
-        GridPart v{0.0f, 0.0f, 0.0f, tag};
+        GridPart v{0, 0.0f, part_word(tag, -2048)};
         if (tid < nb) {
-            put_part(inbox + (size_t(par) * nb + tid) * nb + blockIdx.x, s.h, s.l, m, tag);
+            put_part(inbox + (size_t(par) * nb + tid) * nb + blockIdx.x, s.v, m, part_word(tag, s.u));
             const GridPart* const mine = inbox + (size_t(par) * nb + blockIdx.x) * nb + tid;
             v = get_part(mine);
-            for (unsigned i = 0; v.tag != tag && ok; ++i) {
+            for (unsigned i = 0; (v.word ^ tag << 12) >> 12 && ok; ++i) {
                 ok = i < kGridSpinLimit;
                 v = get_part(mine);
             }
         }
         if (FENCE) fence_gpu();
-        s.h = v.h;
-        s.l = v.l;
-        s = warp_sum2(s);
-        m = warp_max(v.mx);
+        tot = value(lanes_total<5>(Fixed{v.v, int(v.word & 0xfffu) - 2048}));
+        mall = warp_max(v.mx);
         ok = __all_sync(0xffffffffu, ok);
-        if (lane == 0) ts[par][warp] = make_float4(s.h, s.l, m, ok ? 1.0f : 0.0f);
     }
+    if (nw > 1) {
+        if (warp < nw && lane == 0) {
+            ts[warp] = tot;
+            tm[warp] = mall;
+            tk[warp] = ok;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const bool in = lane < nw;
+            tot = in ? ts[in ? lane : 0] : 0.0;
+            for (int o = 1; o < nw; o <<= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+            mall = warp_max(in ? tm[in ? lane : 0] : 0.0f);
+            ok = __all_sync(0xffffffffu, !in || tk[in ? lane : 0]);
+        }
+    }
+    if (warp == 0) fin(tot, mall, ok);
     __syncthreads();
-    tot = Sum2();
-    mall = 0.0f;
-    bool ok = true;
-#pragma unroll 1
-    for (int i = 0; i < nw; ++i) {
-        const float4 t = ts[par][i];
-        tot.add(t.x, t.y);
-        mall = t.z > mall ? t.z : mall;
-        ok = ok && t.w != 0.0f;
-    }
-    return ok;
 }
 
-template <int K>
+// EXACT: the dot products' terms as k_matvec and k_update take them (X % 4 != 0), exact products summed to
+// FP64's precision; otherwise as k_matvec4 and k_update4 do, FP32 products summed with compensation.
+template <int K, bool EXACT>
 __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __restrict__ ax, const float* __restrict__ ay,
                                                      const float* __restrict__ az, const float* __restrict__ aw, float* __restrict__ rg,
                                                      float* s_even, float* s_odd, float* zg, float* __restrict__ pg, int reference,
@@ -985,16 +1001,14 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
         }
         C[l] = cl; C[LEN + l] = cr; C[2 * LEN + l] = cd; C[3 * LEN + l] = cu; C[4 * LEN + l] = cb; C[5 * LEN + l] = cf;
     }
-    // the solver's scalars, the same in every thread; the dot products of the last iteration in shared
-    // memory (thread 0 stores them where no thread reads before the next reduction's barrier)
-    __shared__ Sum2 sigma0[2];
-    if (tid == 0) sigma0[0] = sum2_of(sc->sigma0);
-    Sum2 sigma1 = sum2_of(sc->sigma1);
-    float residual = sc->residual;
-    int done = 0, status = 0;
+    __shared__ GridScalars G;
+    if (tid == 0) {
+        G.sigma0 = sc->sigma0;
+        G.sigma1 = sc->sigma1;
+        G.residual = sc->residual;
+    }
     float alpha = 0.0f, beta = 0.0f;
     int iters = 0;
-    bool ok = true;
     const bool whole = base + LEN <= N, inner = base >= XY && base + LEN + XY <= N;
     for (;;) {
         // the first direction is the setup's z itself: z + 0 times itself
@@ -1039,24 +1053,31 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
         __syncthreads();
         float As[K];
         Kahan acc;
+        Sum exact;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int l = tid + k * GCT;
             const float o = w[k] * s[k] + ((C[l] * S[l - 1] + C[2 * LEN + l] * S[l - X] + C[4 * LEN + l] * sb[k] + C[LEN + l] * S[l + 1] +
                                             C[3 * LEN + l] * S[l + X] + C[5 * LEN + l] * sf[k]));
             As[k] = o;
-            acc.add(o * s[k]);
+            if (EXACT) exact.add_prod(o, s[k]);
+            else acc.add(o * s[k]);
         }
         // (no fence: the next reads of another block's stores come after the second reduction)
-        Sum2 tot;
-        float mall;
-        ok = grid_reduce<false>(inbox, nb, ++tag, acc.pair(), 0.0f, tot, mall);
-        if (!ok) break;
-        if (!isfinite(tot.h)) { status = SKT_NAN_DETECTED; break; }
-        if (reference) tot.add(sigma1.h, sigma1.l);  // Q1
-        sigma1 = tot;
-        alpha = sigma0[iters & 1].over(sigma1);
+        grid_reduce<false, EXACT>(inbox, nb, ++tag, EXACT ? exact : acc.sum(), 0.0f, [&](double tot, float, bool ok) {
+            const double s1 = reference ? G.sigma1 + tot : tot;  // Q1
+            const float a = quotient(G.sigma0, s1);
+            __syncwarp();
+            if (tid == 0) {
+                G.sigma1 = s1;
+                G.len = a;
+                G.state = !ok ? GRID_STUCK : !isfinite(tot) ? GRID_NAN : GRID_GO;
+            }
+        });
+        if (G.state != GRID_GO) break;
+        alpha = G.len;
         Kahan zr;
+        Sum zx;
         float mx = 0.0f;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
@@ -1066,21 +1087,27 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
             const float z = r[k] * precon_of(w[k]);
             S[l] = z;  // every read of the direction lies before the reduction's barrier
             if (whole || i < N) __stcg(zg + base + tid + k * GCT, z);
-            zr.add(z * r[k]);
+            if (EXACT) zx.add_prod(z, r[k]);
+            else zr.add(z * r[k]);
             const float m = (!reference || i < XY) ? fabsf(r[k]) : r[k];  // Q4
             if (m > mx) mx = m;
         }
-        ok = grid_reduce<true>(inbox, nb, ++tag, zr.pair(), mx, tot, mall);
-        if (!ok) break;
-        beta = tot.over(sigma0[iters & 1]);
+        grid_reduce<true, EXACT>(inbox, nb, ++tag, EXACT ? zx : zr.sum(), mx, [&](double tot, float mall, bool ok) {
+            const float b = quotient(tot, G.sigma0);
+            __syncwarp();
+            if (tid == 0) {
+                G.sigma0 = G.sigma1 = tot;
+                G.len = b;
+                G.residual = mall;
+                G.state = !ok ? GRID_STUCK : !isfinite(tot) ? GRID_NAN : mall <= tol ? GRID_DONE : iters + 1 >= max_iter ? GRID_CAP : GRID_GO;
+            }
+        });
+        if (G.state == GRID_STUCK) break;
         ++iters;
-        residual = mall;
-        if (!isfinite(tot.h)) { status = SKT_NAN_DETECTED; break; }
-        if (mall <= tol) { done = 1; break; }
-        if (iters >= max_iter) { done = 2; break; }
-        if (tid == 0) sigma0[iters & 1] = tot;
-        sigma1 = tot;
+        beta = G.len;
+        if (G.state != GRID_GO) break;
     }
+    const int state = G.state;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         const int i = base + tid + k * GCT;
@@ -1090,14 +1117,14 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
         }
     }
     if (tid == 0) {
-        if (!ok) sc->status = SKT_TIMEOUT;
+        if (state == GRID_STUCK) sc->status = SKT_TIMEOUT;
         if (blockIdx.x == 0) {
-            if (status) sc->status = status;
+            if (state == GRID_NAN) sc->status = SKT_NAN_DETECTED;
             sc->alpha = alpha;
             sc->beta_f = beta;
-            sc->residual = residual;
+            sc->residual = G.residual;
             sc->iters = iters;
-            sc->converged = done;
+            sc->converged = state == GRID_DONE ? 1 : state == GRID_CAP ? 2 : 0;
             sc->grid_tag = tag;
         }
     }
@@ -1109,7 +1136,7 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
 // is the right face of the cell before (a shuffle across lanes), the back face the front face of
 // the previous plane, the down face is formed again from the row below. coef_of and the harmonic
 // mean are symmetric in their two densities (IEEE addition commutes), so every value equals
-// k_build's; z.r is summed (Sum2) in a different order.
+// k_build's; z.r is summed in a different order.
 __device__ __forceinline__ float fcomp(const float4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); }
 __device__ __forceinline__ void fset(float4& v, int k, float a) {
     if (k == 0) v.x = a; else if (k == 1) v.y = a; else if (k == 2) v.z = a; else v.w = a;
@@ -1140,7 +1167,7 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
     const int X = g.X, XY = g.XY, Z = g.Z;
     const int row = x0 + y * X;
     const float4 z4 = make_float4(0, 0, 0, 0);
-    Sum2 dsum;
+    Sum dsum;
     float mx = 0.0f;
     const float du_ = sky ? defU[y] : 0.0f, dw_ = sky ? defW[y] : 0.0f;
     // own plane: density and reciprocal; the back face (front face of the plane before) and w there
@@ -1260,7 +1287,7 @@ __global__ void __launch_bounds__(MVT) k_build4(Grid g, int zlen, const float* _
     }
     double tot;
     float mall;
-    if (grid_sum_max<MVT>(sc, partials, linear_block(), linear_blocks(), tid, dsum, mx, tot, mall)) {
+    if (grid_sum_max<MVT, true>(sc, partials, linear_block(), linear_blocks(), tid, dsum, mx, tot, mall)) {
         sc->sigma0 = tot;
         sc->sigma1 = 0.0;
         sc->iters = 0;
@@ -1365,6 +1392,10 @@ __global__ void __launch_bounds__(256) k_apply_proj4(Grid g, int zlen, const flo
 
 namespace {
 
+template <int K>
+const void* pcg_grid_kernel(const Env& e) {
+    return e.g.X % 4 != 0 ? (const void*)k_pcg_grid<K, true> : (const void*)k_pcg_grid<K, false>;
+}
 // whether the blocks of this launch are resident at once (asked once per environment and variant)
 template <int K>
 bool pcg_grid_fits(Env& e, int slot, int nb) {
@@ -1373,11 +1404,12 @@ bool pcg_grid_fits(Env& e, int slot, int nb) {
         // the limit set on the kernel is the device's, not this grid's need: other environments launch it too
         int coop = 0, most = 0, per_sm = 0;
         cudaFuncAttributes fa{};
+        const void* const kernel = pcg_grid_kernel<K>(e);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e.device);
         cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, e.device);
-        if (!coop || cudaFuncGetAttributes(&fa, k_pcg_grid<K>) != cudaSuccess || smem + int(fa.sharedSizeBytes) > most ||
-            cudaFuncSetAttribute(k_pcg_grid<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(fa.sharedSizeBytes)) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid<K>, GCT, smem) != cudaSuccess) {
+        if (!coop || cudaFuncGetAttributes(&fa, kernel) != cudaSuccess || smem + int(fa.sharedSizeBytes) > most ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(fa.sharedSizeBytes)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, GCT, smem) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 0;
         }
@@ -1391,7 +1423,7 @@ void launch_pcg_grid(Env& e, int nb) {
     void* args[] = {&e.g, &e.ax, &e.ay, &e.az, &e.aw, &e.r, &e.s, &e.tB, &e.tA, &e.pp, &reference, &e.cfg.pcg_tol, &e.cfg.pcg_max_iter,
                     &e.sc, &e.grid_parts};
     // an error is the step's to report (its check finds it)
-    (void)cudaLaunchCooperativeKernel((const void*)k_pcg_grid<K>, dim3(nb), dim3(GCT), args, pcg_grid_smem<K>(e.g.X), e.stream);
+    (void)cudaLaunchCooperativeKernel(pcg_grid_kernel<K>(e), dim3(nb), dim3(GCT), args, pcg_grid_smem<K>(e.g.X), e.stream);
     e.launches += 1;
 }
 
