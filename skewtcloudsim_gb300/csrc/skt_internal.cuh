@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "skt_physics.cuh"
+#include "skt_rules.hpp"
 #include "skt_sum.hpp"
 #include "../../include/skewt.h"
 

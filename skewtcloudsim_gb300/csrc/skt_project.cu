@@ -1125,7 +1125,7 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
             sc->residual = G.residual;
             sc->iters = iters;
             sc->converged = state == GRID_DONE ? 1 : state == GRID_CAP ? 2 : 0;
-            sc->grid_tag = tag;
+            sc->grid_tag = tag_after(tag, state == GRID_STUCK);
         }
     }
 }
