@@ -76,18 +76,18 @@ __global__ void __launch_bounds__(256) k_reset_faces(Grid g, float* __restrict__
                                                      const float* __restrict__ defU, const float* __restrict__ defW) {
     after_previous();
     const int X = g.X, Y = g.Y, Z = g.Z;
-    int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < X * Y) {
-        if (i >= X) w[i + (Z - 1) * g.XY] = defW[i / X];
+    unsigned i = blockIdx.x * 256u + threadIdx.x;  // may exceed 2^31 (far_faces)
+    if (i < unsigned(X * Y)) {
+        if (i >= unsigned(X)) w[int(i) + (Z - 1) * g.XY] = defW[int(i) / X];
         return;
     }
-    i -= X * Y;
-    if (i < X * Z) {
-        if (Y > 1) v[cidx(g, i % X, Y - 1, i / X)] = 0.0f;
+    i -= unsigned(X * Y);
+    if (i < unsigned(X * Z)) {
+        if (Y > 1) v[cidx(g, int(i) % X, Y - 1, int(i) / X)] = 0.0f;
         return;
     }
-    i -= X * Z;
-    if (i < Y * Z && i % Y > 0) u[cidx(g, X - 1, i % Y, i / Y)] = defU[i % Y];
+    i -= unsigned(X * Z);
+    if (i < unsigned(Y * Z) && int(i) % Y > 0) u[cidx(g, X - 1, int(i) % Y, int(i) / Y)] = defU[int(i) % Y];
 }
 // Over terrain: one thread per (x,y) marching z, RVZ planes' heights loaded at a time (one at a time
 // 63 us at 128x64x128, now 19)
@@ -1435,8 +1435,7 @@ void launch_pcg_grid(Env& e, int nb) {
 void pcg_grid_shape(const Env& e, int& slot, int& nb) {
     for (const int most : {std::min(96, e.num_sms), std::min(e.num_sms, kMaxGridBlocks)})
         for (slot = 0; slot < 4; ++slot) {
-            const int per = kGridCells[slot] * GCT;
-            nb = (e.g.N + per - 1) / per;
+            nb = blocks_for(e.g.N, kGridCells[slot] * GCT);
             if (nb <= most) return;
         }
     nb = 0;
@@ -1528,7 +1527,7 @@ void launch_project(Env& e, float dtS) {
     {
     ProfScope ps(e, "proj_setup");
     e.launches += 2;
-    if (e.flat) launch_next(e, k_reset_faces, (g.X * (g.Y + g.Z) + g.Y * g.Z + 255) / 256, 256, 0, g, e.u, e.v, e.w, e.defU, e.defW);
+    if (e.flat) launch_next(e, k_reset_faces, far_faces(g.X, g.Y, g.Z) / 256u + 1u, 256, 0, g, e.u, e.v, e.w, e.defU, e.defW);
     else launch_next(e, k_reset_vel, (g.XY + 127) / 128, 128, 0, g, e.u, e.v, e.w, e.defU, e.defW, ref);
     float* z0 = faces ? e.s : zbuf;
     if (e.flat && (g.X % 4) == 0) {

@@ -10,4 +10,11 @@ namespace skt {
 // that no partial of an abandoned launch is taken for one of the next.
 constexpr unsigned tag_after(unsigned tag, bool stuck) { return stuck ? tag + 1 : tag; }
 
+// blocks of `per` cells for a grid of n (any n >= 1 that an int holds)
+constexpr int blocks_for(int n, int per) { return (n - 1) / per + 1; }
+
+// The faces on the far sides, those of x = X-1, y = Y-1 and z = Z-1: up to 1.5 * 2^31 of them on a grid below
+// 2^31 cells with two rows and one plane
+constexpr unsigned far_faces(int X, int Y, int Z) { return unsigned(X) * unsigned(Y) + unsigned(X) * unsigned(Z) + unsigned(Y) * unsigned(Z); }
+
 }  // namespace skt
