@@ -241,8 +241,8 @@ skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tun
     struct Cand { int depth, h, bps; };
     std::vector<Cand> cands;
     for (int bps : {16, 32, 64}) cands.push_back({1, base.diffuse_h, bps});
-    if (e.flat && (e.g.X % 4) == 0 && e.cfg.diffuse_sweeps >= 2)
-    {
+    const bool pairs = e.flat && (e.g.X % 4) == 0 && e.cfg.diffuse_sweeps >= 2;
+    if (pairs) {
         for (int bps : {2, 4, 8}) cands.push_back({2, 14, bps});
         for (int bps : {4, 8}) cands.push_back({2, 6, bps});
         for (int h : {4, 8})
@@ -253,7 +253,7 @@ skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tun
     // the size's own shape goes first and stands unless another one beats it clearly
     const Tuning own = default_tuning(e.g.N);
     auto is_own = [&](const Cand& c) {
-        return c.depth == own.diffuse_depth && (c.depth == 1 ? c.bps == own.diffuse_bps : c.h == own.diffuse_h && c.bps == own.diffuse2_bps);
+        return c.depth == (pairs ? own.diffuse_depth : 1) && (c.depth == 1 ? c.bps == own.diffuse_bps : c.h == own.diffuse_h && c.bps == own.diffuse2_bps);
     };
     std::stable_partition(cands.begin(), cands.end(), is_own);
     float own_ms = 1e30f;
@@ -280,6 +280,9 @@ skt_status skt_autotune(skt_env* env, const char* cache_path, int flags, skt_tun
             best.diffuse2_bps = tr.diffuse2_bps;
         }
     }
+    // terrain or an x no multiple of four sweeps without the two-sweep kernel: its depth was not measured, and the
+    // size's own stands for when the terrain is flat (an edit, a cache read on another terrain)
+    if (!pairs) best.diffuse_depth = own.diffuse_depth;
     // ---- PPM passes: each march's run length in turn (the water-vapour advection) ----
     float adv_ms = 0.0f;
     if (e.flat && (e.g.X % 4) == 0) {
