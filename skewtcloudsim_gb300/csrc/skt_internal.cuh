@@ -272,19 +272,21 @@ struct Tuning {
     int ppmz_bps = 8;        // k_ppm4z: blocks per SM (z-run length)
     int ppmy_bps = 32;       // k_ppm4y: blocks per SM (y-run length)
 };
-// The shapes by the grid's size, measured on ten grids from 32^3 to 512x256x512. Two sweeps per pass
+// The shapes by the grid's size, measured on twenty grids from 32^3 to 512x256x512. Two sweeps per pass
 // are faster on every one of them (a step's diffusions 0.29 -> 0.25 ms at 32^3, 0.60 -> 0.45 at
-// 96x64x96, 3.16 -> 2.15 at 256x128x256, 20.7 -> 12.6 at 512x256x512); the low tile wins below 8M cells
-// (6 and 14 rows: 2.15 and 2.20 ms at 256x128x256, 3.48 and 3.46 at 256x192x320), and below 2M cells
-// half the blocks, whose runs would otherwise be a plane or two (0.53 and 0.54 ms at 128x64x128, 0.28
-// and 0.34 at 64x32x64). The x pass of the advection wants its longer runs up to 12M cells (a step's
-// advections 2.74 and 2.82 ms at 256x128x256, 16.9 and 16.6 at 512x256x512).
+// 96x64x96, 3.16 -> 2.15 at 256x128x256, 20.7 -> 12.6 at 512x256x512); the low tile wins below 14M cells (a
+// step with 6 and 14 rows: 1.63 and 1.71 ms at 192x128x192, 2.08 and 2.13 at 256x128x256, 2.47 and 2.48 at
+// 256x160x256, 3.52 and 3.55 at 320x128x320, 4.31 and 4.21 at 320x160x320, 5.90 and 5.77 at 384x192x384), and
+// below 2M cells half the blocks, whose runs would otherwise be a plane or two (0.53 and 0.54 ms at
+// 128x64x128, 0.28 and 0.34 at 64x32x64). The x pass of the advection wants its longer runs up to 24M cells (a
+// step's advections in 8 and 16 blocks an SM 2.25 and 2.35 ms at 256x128x256, 3.79 and 3.84 at 320x128x320,
+// 4.50 and 4.60 at 384x128x384, 6.58 and 6.60 at 384x192x384, 16.9 and 16.6 at 512x256x512).
 inline Tuning default_tuning(int cells) {
     Tuning t;
-    t.diffuse_h = cells < 8000000 ? 6 : 14;
+    t.diffuse_h = cells < 14000000 ? 6 : 14;
     t.diffuse2_bps = cells < 2000000 ? 4 : 8;
     t.diffuse_bps = cells < 32000000 ? 16 : 32;
-    t.ppm_bps = cells < 12000000 ? 8 : 16;
+    t.ppm_bps = cells < 24000000 ? 8 : 16;
     return t;
 }
 
