@@ -45,9 +45,11 @@ METRIC = "cell-steps/s at 512x512x256, mixed vs plain PCG at 1e-5 rel err; % HBM
 # Algorithmic bytes per cell per launch of each profiled stage (FP32 fields; each array counted
 # once per launch; neighbour re-reads excluded).
 STAGE_BYTES = {
-    "pcg_matvec": 40.0,   # stored coefficients: z, s_old, aw, ax, ay, az read; p read+write; s_new, As write
+    # a two-launch PCG iteration with stored coefficients, the model of step_bytes; the library's own
+    # iterations are PLAIN_FORMS'
+    "pcg_matvec": 40.0,   # z, s_old, aw, ax, ay, az read; p read+write; s_new, As write
     "pcg_update": 20.0,   # r read+write; As, aw read; z write
-    "pcg_search": 16.0,   # unfused (--pcg-fused 0): r, aw read; s read+write
+    "pcg_search": 16.0,   # r, aw read; s read+write
     "diffuse": 8.0,       # per sweep: in read, out write
     "advect": 12.0,       # per pass: q, vel read; out write
     "micro": 64.0,        # 6 Q + th read/write, rho, p read (fused addHeat)
@@ -61,17 +63,30 @@ STAGE_BYTES = {
 }
 
 
-# The matrix-free plain PCG (the default above about a million cells, nx % 4 == 0): the operator reads z,
-# s_old, the reciprocal density and one word and writes s_new and As; the residual's 20 B and, every
-# fourth iteration, the pressure's 24 B (four directions read, p read+write) share a profile stage of
-# five launches in four iterations. 24 + 20 + 6 = 50 B an iteration.
-FREE_BYTES = {"pcg_matvec": 24.0, "pcg_update": (4 * 20.0 + 24.0) / 5}
-FREE_ITERATION_BYTES = 50.0
+# The plain PCG's three forms: bytes per cell of a launch of each profiled stage, and of an iteration.
+# Matrix-free (above about a million cells, nx % 4 == 0): the operator reads z, s_old, the reciprocal density
+# and one word and writes s_new and As (24 B); the residual's 20 B and, every fourth iteration, the pressure's
+# 24 B (four directions read, p read+write) share a stage of five launches in four iterations. Three launches
+# (--pcg-fused 0, or any nx above a million cells): s, ax, ay, az, aw read and As written; s, As, aw read, p
+# and r read+write; r, aw read and s read+write. One launch (up to about a million cells): the solver's state
+# stays on the chip, and HBM bounds none of it.
+PLAIN_FORMS = {
+    "matrix-free": ({"pcg_matvec": 24.0, "pcg_update": (4 * 20.0 + 24.0) / 5}, 50.0),
+    "three launches": ({"pcg_matvec": 24.0, "pcg_update": 28.0, "pcg_search": 16.0}, 68.0),
+    "one launch": ({}, 0.0),
+}
+
+
+def plain_form(stages):
+    """Which of PLAIN_FORMS a plain step ran, by the stages that the library profiled."""
+    return "one launch" if "pcg_grid" in stages else "three launches" if "pcg_search" in stages else "matrix-free"
+
 
 # DRAM traffic per cell of one launch: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at
 # 512x256x256 (33554432 cells). Every array is streamed once per launch, so the traffic grows with the
-# cells and is scaled to the launch size here. With stored coefficients, then matrix-free
-# (k_pcg_operator4, and the mean of four k_residual4 and one k_pressure4).
+# cells and is scaled to the launch size here. First of the stored-coefficient model's launches (a check of
+# its bytes), then of the matrix-free form's (k_pcg_operator4, and the mean of four k_residual4 and one
+# k_pressure4).
 MEASURED_TRAFFIC_PER_CELL = {
     "pcg_matvec": (981.662976 + 375.963392) * 1e6 / 33554432,
     "pcg_update": (402.723840 + 224.641536) * 1e6 / 33554432,
@@ -278,16 +293,27 @@ def stage_bytes(diffuse_depth=1):
 
 
 def step_bytes(mode, pcg_iters, outer, diffuse_depth=1):
-    """Algorithmic bytes per cell-step of the whole step as the library moves them: the stages
-    (stage_bytes) plus the pressure solve. Plain Jacobi-PCG with stored coefficients: 60 B per iteration
-    (the operator with the search step and the pressure update 40 B, the residual update with
-    z = r/diag 20 B). Mixed:
+    """Algorithmic bytes per cell-step of the whole step: the stages (stage_bytes) plus the pressure
+    solve. Plain: a model with stored coefficients in two launches, 60 B per iteration (the operator with
+    the search step and the pressure update 40 B, the residual update with z = r/diag 20 B); what the
+    library moves is plain_step_bytes. Mixed, as the library moves them:
     per inner iteration the operator + search (32 B), the update (24 B) and the V-cycle (93 B: four
     finest-level passes of 16-24.5 B with FP16 coefficients plus the coarser levels), per
     refinement step the float-float residual (32 B) and the correction (20 B)."""
     if mode == "plain":
         return stage_bytes(diffuse_depth) + 60.0 * pcg_iters
     return stage_bytes(diffuse_depth) + (32.0 + 24.0 + 93.0) * pcg_iters + 52.0 * max(outer, 1)
+
+
+def sweeps_per_pass(tuning, nx, ground_height):
+    """The diffusion's sweeps per pass: the shapes' depth where the two-sweep kernel runs (flat terrain,
+    nx % 4 == 0), else one."""
+    return tuning.get("diffuse_depth", 1) if nx % 4 == 0 and not np.any(ground_height) else 1
+
+
+def plain_step_bytes(form, pcg_iters, diffuse_depth=1):
+    """Bytes per cell-step of a plain step as the library moves them, by the PCG's form (PLAIN_FORMS)."""
+    return stage_bytes(diffuse_depth) + PLAIN_FORMS[form][1] * pcg_iters
 
 
 # plain_textbook: the plain Jacobi-PCG on the textbook (symmetric) operator the mixed mode solves,
@@ -472,7 +498,8 @@ def main():
     ap.add_argument("--semantics", type=int, default=0)
     ap.add_argument("--mg-half", type=int, default=1, help="mixed: FP16 finest-level coefficients in the V-cycle")
     ap.add_argument("--pcg-fused", type=int, default=1,
-                    help="plain: 1 = two launches per PCG iteration (search step fused into the operator), 0 = three")
+                    help="plain: 1 = the PCG in one launch up to about a million cells, above that (nx %% 4 == 0) matrix-free in "
+                         "two launches per iteration; 0 = three launches per iteration from stored coefficients")
     ap.add_argument("--graph", type=int, default=1,
                     help="1 = each step one launch of the captured CUDA graph (device-side loops), 0 = stream-ordered")
     ap.add_argument("--ensemble-runner", default="graph", choices=["graph", "threads"],
@@ -513,13 +540,12 @@ def main():
     dname, d = dom
     per_launch_ms = d["ms"] / max(d["kernels"], 1)
     peak, peak_kind = measured_peak()
-    # the library's own rule (above the one-launch PCG's size, float4 rows) for the matrix-free iteration
-    free = head["mode"] != "mixed" and args.pcg_fused and init.nx % 4 == 0 and "pcg_matvec" in prof
-    bpc = FREE_BYTES[dname] if free and dname in FREE_BYTES else STAGE_BYTES.get(dname)
+    form = None if head["mode"] == "mixed" else plain_form(prof)
+    bpc = PLAIN_FORMS[form][0].get(dname) if form and dname.startswith("pcg_") else STAGE_BYTES.get(dname)
     roofline = None
     if bpc:
         achieved = bpc * cells / (per_launch_ms / 1e3) / 1e9
-        tpc = FREE_TRAFFIC_PER_CELL.get(dname) if (head["mode"] == "plain" and free) else None
+        tpc = FREE_TRAFFIC_PER_CELL.get(dname) if form == "matrix-free" else None
         roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                     "frac": round(achieved / peak, 4), "traffic": int(tpc * cells) if tpc else None, "kernel": dname,
                     "bytes_per_cell": bpc, "launch_us": round(per_launch_ms * 1e3, 2), "peak_source": peak_kind}
@@ -527,12 +553,14 @@ def main():
             roofline["traffic_source"] = ("ncu DRAM bytes read + written by one launch at 512x256x256, scaled to this "
                                           "launch's cells (bytes per launch; pcg_update: the mean of its kernels)")
     step_ms_prof = sum(v["ms"] for v in prof.values())
-    depth = head["tuning"].get("diffuse_depth", 1)
-    bstep = stage_bytes(depth) + FREE_ITERATION_BYTES * head["pcg_iters"] if free else step_bytes(head["mode"], head["pcg_iters"], head["outer"], depth)
+    depth = sweeps_per_pass(head["tuning"], init.nx, init.ground_height)
+    bstep = plain_step_bytes(form, head["pcg_iters"], depth) if form else step_bytes(head["mode"], head["pcg_iters"], head["outer"], depth)
+    solver = {None: "149 B per inner MG-PCG iteration + 52 B per refinement step", "one launch": "the plain PCG on the chip"}.get(
+        form, f"{PLAIN_FORMS[form][1]:.0f} B per plain PCG iteration ({form})" if form else "")
     step_model = {"bytes_per_cell_step": bstep, "achieved_gbs": round(bstep * head["value"] / 1e9, 1),
                   "frac": round(bstep * head["value"] / 1e9 / peak, 4), "peak_source": peak_kind,
                   "model": (f"the library's own bytes: {stage_bytes(depth):.0f} B of stages (diffusion at {depth} sweep(s) per "
-                            "pass) + " + ("50 B per plain PCG iteration (matrix-free)" if free else "60 B per plain PCG iteration (stored coefficients)"))}
+                            "pass) + " + solver)}
     if head["mode"] != "mixed":
         sb = scope_step_bytes(head["mode"], head["pcg_iters"], head["outer"])
         step_model["scope_model"] = {
@@ -615,8 +643,8 @@ def main():
                                      f"{head['residual']:.3g} > 1e-5), as the reference's does")
     if "plain_textbook" in res:
         t = res["plain_textbook"]
-        tdepth = t["tuning"].get("diffuse_depth", 1)
-        tbytes = stage_bytes(tdepth) + FREE_ITERATION_BYTES * t["pcg_iters"] if free else step_bytes("plain", t["pcg_iters"], 0, tdepth)
+        tdepth = sweeps_per_pass(t["tuning"], init.nx, init.ground_height)
+        tbytes = plain_step_bytes(plain_form(t["prof"]), t["pcg_iters"], tdepth)
         out["plain_textbook"] = {
             "value": t["value"], "ms_per_step": t["ms_per_step"], "semantics": "textbook",
             "pcg_iters_per_step": t["pcg_iters"], "converged": t["converged"], "max_residual": t["residual"],
@@ -628,12 +656,11 @@ def main():
             "profile_ms": {k: round(v["ms"], 3) for k, v in t["prof"].items()}}
     if "mixed" in res and head["mode"] != "mixed":
         m = res["mixed"]
+        mbytes = step_bytes("mixed", m["pcg_iters"], m["outer"], sweeps_per_pass(m["tuning"], init.nx, init.ground_height))
         out["mixed"] = {"value": m["value"], "ms_per_step": m["ms_per_step"], "speedup_vs_plain": round(m["value"] / head["value"], 3),
                         "semantics": m["semantics"], "inner_iters_per_step": m["pcg_iters"], "refine_steps": m["outer"],
                         "converged": m["converged"], "rel_residual": m["residual"], "gpu_launches": m["launches"],
-                        "step_roofline": {"bytes_per_cell_step": step_bytes("mixed", m["pcg_iters"], m["outer"], m["tuning"].get("diffuse_depth", 1)),
-                                          "frac": round(step_bytes("mixed", m["pcg_iters"], m["outer"], m["tuning"].get("diffuse_depth", 1))
-                                                        * m["value"] / 1e9 / peak, 4)},
+                        "step_roofline": {"bytes_per_cell_step": mbytes, "frac": round(mbytes * m["value"] / 1e9 / peak, 4)},
                         "clocks": m["clocks"], "profile_ms": {k: round(v["ms"], 3) for k, v in m["prof"].items()}}
         if "plain_textbook" in res:
             out["mixed"]["speedup_vs_plain_textbook"] = round(m["value"] / res["plain_textbook"]["value"], 3)
