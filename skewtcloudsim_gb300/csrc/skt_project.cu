@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(NT) k_build(Grid g, Tiles T, const float* __re
 // in turn, whatever their number.
 // What bounds it: HBM (24 bytes a cell) and the loads' instructions. A thread per cell that asked the
 // heights about every neighbour took 77 us at 251x118x275, now
-// 52; one or two rows a lane 62 and 65, eight warps a block 58.
+// 59 (52 with the sums in pairs of floats; then one or two rows a lane 62 and 65, eight warps a block 58).
 constexpr int MR = 4, MW = 4;  // rows per lane, warps per block
 struct Runs {
     int nx, ny, n, zlen;  // tiles along x and y, all of them, planes per tile
@@ -218,12 +218,20 @@ inline Runs matvec_runs(const Grid& g, int sms) {
     t.n = t.nx * t.ny * ((g.Z + t.zlen - 1) / t.zlen);
     return t;
 }
-__global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float* __restrict__ ax, const float* __restrict__ ay,
+__global__ void __launch_bounds__(32 * MW, 4) k_matvec(Grid g, Runs T, const float* __restrict__ ax, const float* __restrict__ ay,
                                                     const float* __restrict__ az, const float* __restrict__ aw, const float* __restrict__ s,
                                                     float* __restrict__ As, int reference, Scalars* sc, double* partials) {
     if (sc->converged) return;
     const int X = g.X, Y = g.Y, Z = g.Z, XY = g.XY, lane = threadIdx.x;
-    Sum dsum;
+    // the thread's sum waits in shared memory: four blocks an SM leave the march 128 registers and none for it
+    // (141 registers and three blocks 69 us at 251x118x275, spills 62, this 59)
+    constexpr int NTH = 32 * MW;
+    __shared__ float part[3][NTH];
+    __shared__ double far[NTH];
+    const int tid = threadIdx.y * 32 + lane;
+    volatile float* const mine = &part[0][tid];
+    mine[0] = mine[NTH] = mine[2 * NTH] = 0.0f;
+    far[tid] = 0.0;
     struct Plane {
         float cx[MR], cy[MR], cz[MR], cw[MR], es[MR], ea[MR], up, down, cd;
     };
@@ -262,7 +270,7 @@ __global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float*
         }
         for (int z = zs; z < ze; ++z, c += XY) {
             Plane N;
-            float n2[MR];
+            float n2[MR], o[MR];
             if (z + 1 < ze) load(c + XY, N);
 #pragma unroll
             for (int r = 0; r < MR; ++r) n2[r] = z + 2 <= ze && z + 2 < Z ? s[c + ro[r] + 2 * XY] : 0.0f;
@@ -280,11 +288,15 @@ __global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float*
                 if (reference) { AL = char_trunc(AL); AD = char_trunc(AD); AB = char_trunc(AB); }
                 const float ld = fmaf(AL, sl, __fmul_rn(AD, sd));
                 const float out = fmaf(P.cw[r], v, fmaf(P.cz[r], n[r], fmaf(P.cy[r], su, fmaf(P.cx[r], sr, fmaf(AB, b[r], ld)))));
-                if (r < rows && P.cw[r] != 0.0f) {  // As of ground cells stays 0
-                    As[c + r * X] = out;
-                    dsum.add_prod(out, v);
-                }
+                const bool sky = r < rows && P.cw[r] != 0.0f;
+                if (sky) As[c + r * X] = out;  // As of ground cells stays 0
+                o[r] = sky ? out : 0.0f;
             }
+            Sum dsum;
+            dsum.h = mine[0]; dsum.l = mine[NTH]; dsum.t = mine[2 * NTH];
+            dsum.add_prods(o, q);
+            mine[0] = dsum.h; mine[NTH] = dsum.l; mine[2 * NTH] = dsum.t;
+            if (dsum.far != 0.0) far[tid] += dsum.far;
 #pragma unroll
             for (int r = 0; r < MR; ++r) {
                 b[r] = q[r];
@@ -297,7 +309,10 @@ __global__ void __launch_bounds__(32 * MW) k_matvec(Grid g, Runs T, const float*
     }
     double tot;
     float mall;
-    if (grid_sum_max<32 * MW, true>(sc, partials, blockIdx.x, gridDim.x, threadIdx.y * 32 + lane, dsum, 0.0f, tot, mall)) {
+    Sum dsum;
+    dsum.h = mine[0]; dsum.l = mine[NTH]; dsum.t = mine[2 * NTH];
+    dsum.far = far[tid];
+    if (grid_sum_max<NTH, true>(sc, partials, blockIdx.x, gridDim.x, tid, dsum, 0.0f, tot, mall)) {
         const double s1 = reference ? sc->sigma1 + tot : tot;
         sc->sigma1 = s1;
         sc->alpha = float(sc->sigma0 / s1);
@@ -315,7 +330,7 @@ __device__ __forceinline__ void stream4(int n, F4 four, F1 one) {
 
 // p += alpha s; r -= alpha As (updatePandDiv :955-985), then the stop test on the max residual
 // (getMaxDivergence, Q4 in reference mode: |r| on the z = 0 plane only), z = r/diag and z.r for the next search
-// direction. HBM-bound, 28 bytes a cell: 115 us at 251x118x275 cell by cell in tiles, 41 as float4 streams.
+// direction. HBM-bound, 28 bytes a cell: 115 us at 251x118x275 cell by cell in tiles, 43 as float4 streams.
 __global__ void __launch_bounds__(NT) k_update(int n, int XY, const float* __restrict__ aw, const float* __restrict__ s,
                                                const float* __restrict__ As, float* __restrict__ pp, float* __restrict__ r,
                                                int reference, float tol, int max_iter, Scalars* sc, double* partials) {
@@ -326,28 +341,28 @@ __global__ void __launch_bounds__(NT) k_update(int n, int XY, const float* __res
     auto cell = [&](float a, float sv, float av, float& pv, float& rv, int c) {
         pv += alpha * sv;
         rv = rv - alpha * av;
-        const float zv = rv * precon_of(a);
-        dsum.add_prod(zv, rv);
         const float m = (!reference || c < XY) ? fabsf(rv) : rv;
         if (m > mx) mx = m;
+        return rv * precon_of(a);
     };
     stream4(n,
             [&](int i) {
                 const float4 a = reinterpret_cast<const float4*>(aw)[i], sv = reinterpret_cast<const float4*>(s)[i];
                 const float4 av = reinterpret_cast<const float4*>(As)[i];
                 float4 pv = reinterpret_cast<float4*>(pp)[i], rv = reinterpret_cast<float4*>(r)[i];
-                cell(a.x, sv.x, av.x, pv.x, rv.x, 4 * i);
-                cell(a.y, sv.y, av.y, pv.y, rv.y, 4 * i + 1);
-                cell(a.z, sv.z, av.z, pv.z, rv.z, 4 * i + 2);
-                cell(a.w, sv.w, av.w, pv.w, rv.w, 4 * i + 3);
+                const float z0 = cell(a.x, sv.x, av.x, pv.x, rv.x, 4 * i), z1 = cell(a.y, sv.y, av.y, pv.y, rv.y, 4 * i + 1);
+                const float z2 = cell(a.z, sv.z, av.z, pv.z, rv.z, 4 * i + 2), z3 = cell(a.w, sv.w, av.w, pv.w, rv.w, 4 * i + 3);
                 reinterpret_cast<float4*>(pp)[i] = pv;
                 reinterpret_cast<float4*>(r)[i] = rv;
+                const float z[4] = {z0, z1, z2, z3}, q[4] = {rv.x, rv.y, rv.z, rv.w};
+                dsum.add_prods(z, q);
             },
             [&](int c) {
                 float pv = pp[c], rv = r[c];
-                cell(aw[c], s[c], As[c], pv, rv, c);
+                const float z = cell(aw[c], s[c], As[c], pv, rv, c);
                 pp[c] = pv;
                 r[c] = rv;
+                dsum.add_prod(z, rv);
             });
     double tot;
     float mall;
@@ -852,9 +867,11 @@ __global__ void k_pcg_cond(cudaGraphConditionalHandle h, Scalars* sc, int loop) 
 // and arrives, waits until all have arrived, and sums all partials in the same order, so every
 // block holds the same step lengths and takes the same decisions.
 // What bounds it: the two exchanges of an iteration (2 to 3 us together, the second behind a fence for
-// the direction's halo) and the block's own loads and sums. Measured per iteration, before (two
-// launches, or three for 90x51x75) and now: 32^3 12.7 and 4.7 us, 64x32x64 14 and 6.9 us, 90x51x75
-// 27 and 8.7 us, 128x64x128 over hills 30 and 12.9 us.
+// the direction's halo) and the block's own loads and sums. Measured per iteration, with streaming launches
+// (two, or three for 90x51x75) and in one: 32^3 12.7 and 5.3 us, 64x32x64 14 and 6.9 us, 90x51x75 27 and
+// 9.4 us, 128x64x128 30 and 12.5 us. Sums in pairs of floats, FP32's range and products: 4.8, 7.2, 8.8 and
+// 12.9 us; FP64 trees and divisions in their place 5.5 at 32^3, exact products tested one by one 10.6 at
+// 90x51x75.
 // The cells of a thread depend on the grid's size alone, so a member of an ensemble gets the bits
 // of the same grid alone. Every wait is bounded; one that runs out makes the block return and
 // SKT_TIMEOUT be recorded (the other blocks' waits then run out too).
@@ -889,7 +906,7 @@ __device__ __forceinline__ GridPart get_part(const GridPart* p) {
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 // what the threads of a block share of the solver's scalars; thread 0 writes between a reduction's barriers
-enum GridState { GRID_GO, GRID_DONE, GRID_CAP, GRID_NAN, GRID_STUCK };
+enum GridState { GRID_GO, GRID_DONE, GRID_CAP, GRID_NAN, GRID_STUCK, GRID_FAR };
 struct GridScalars {
     double sigma0, sigma1;  // the dot products of the last iteration
     float len, residual;    // the step length that the last reduction gave, the last max residual
@@ -902,25 +919,25 @@ struct GridScalars {
 // and 1.4, every block polling one set of partials 2.9 and 1.2). The partials are summed in the same
 // order everywhere, so every block gets the same totals; its first warp forms the step length from
 // them in fin(total, maximum, whether no wait ran out), one lane of which stores. The FP64 work is the
-// polling warps' and the first one's alone. FENCE: the block's stores before the reduction are visible to
+// polling warps' and the first one's alone. THIRD: sums of Sum::add_near; FAR: sums of Sum::add_far. FENCE: the block's stores before the reduction are visible to
 // every block after it. Inboxes alternate by the tag's parity: a block may send the next partial while
 // another still reads these, but not the one after that.
-template <bool FENCE, bool EXACT, class Fin>
+template <bool FENCE, bool THIRD, bool FAR, class Fin>
 __device__ __forceinline__ void grid_reduce(GridPart* inbox, int nb, unsigned tag, const Sum& sum, float mx, Fin fin) {
     constexpr int W = GCT / 32, B = kMaxGridBlocks / 32;
     __shared__ int4 ws[W];
     __shared__ float wm[W], tm[B];
-    __shared__ double wf[W], ts[B];
+    __shared__ double wf[FAR ? W : 1], ts[B];
     __shared__ int tk[B];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, par = tag & 1u, nw = (nb + 31) >> 5;
     {
-        const WarpSum v = warp_sum<EXACT>(sum);
+        const WarpSum v = warp_sum<THIRD>(sum);
         const float m = warp_max(mx);
-        const double f = EXACT ? warp_far(sum.far) : 0.0;
+        const double f = FAR ? warp_far(sum.far) : 0.0;
         if (lane == 0) {
             ws[warp] = make_int4(v.a, v.b, v.c, int(v.e));
             wm[warp] = m;
-            if (EXACT) wf[warp] = f;
+            if (FAR) wf[warp] = f;
         }
     }
     __syncthreads();
@@ -928,7 +945,7 @@ __device__ __forceinline__ void grid_reduce(GridPart* inbox, int nb, unsigned ta
     float mall = 0.0f;
     bool ok = true;
     if (warp < nw) {
-        const Fixed s = warps_total<log2_of(W), EXACT>(ws, wf, lane);
+        const Fixed s = warps_total<log2_of(W), FAR>(ws, wf, lane);
         const float m = warp_max(lane < W ? wm[lane % W] : 0.0f);
         if (FENCE) fence_gpu();
         GridPart v{0, 0.0f, part_word(tag, -2048)};
@@ -1060,25 +1077,32 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
             const float o = w[k] * s[k] + ((C[l] * S[l - 1] + C[2 * LEN + l] * S[l - X] + C[4 * LEN + l] * sb[k] + C[LEN + l] * S[l + 1] +
                                             C[3 * LEN + l] * S[l + X] + C[5 * LEN + l] * sf[k]));
             As[k] = o;
-            if (EXACT) exact.add_prod(o, s[k]);
-            else acc.add(o * s[k]);
+            if (!EXACT) acc.add(o * s[k]);
         }
+        if (EXACT) exact.add_near(As, s);
         // (no fence: the next reads of another block's stores come after the second reduction)
-        grid_reduce<false, EXACT>(inbox, nb, ++tag, EXACT ? exact : acc.sum(), 0.0f, [&](double tot, float, bool ok) {
+        auto operator_done = [&](double tot, float, bool ok, bool again) {
             const double s1 = reference ? G.sigma1 + tot : tot;  // Q1
             const float a = quotient(G.sigma0, s1);
             __syncwarp();
             if (tid == 0) {
-                G.sigma1 = s1;
+                G.state = !ok ? GRID_STUCK : again && !Sum::total_holds(tot) ? GRID_FAR : !isfinite(tot) ? GRID_NAN : GRID_GO;
+                if (G.state != GRID_FAR) G.sigma1 = s1;
                 G.len = a;
-                G.state = !ok ? GRID_STUCK : !isfinite(tot) ? GRID_NAN : GRID_GO;
             }
-        });
+        };
+        grid_reduce<false, EXACT, false>(inbox, nb, ++tag, EXACT ? exact : acc.sum(), 0.0f,
+                                         [&](double tot, float m, bool ok) { operator_done(tot, m, ok, EXACT); });
+        if (EXACT && G.state == GRID_FAR) {  // the same for every block
+            Sum far;
+            far.add_far(As, s);
+            grid_reduce<false, false, true>(inbox, nb, ++tag, far, 0.0f, [&](double tot, float m, bool ok) { operator_done(tot, m, ok, false); });
+        }
         if (G.state != GRID_GO) break;
         alpha = G.len;
         Kahan zr;
         Sum zx;
-        float mx = 0.0f;
+        float zs[K], mx = 0.0f;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int l = tid + k * GCT, i = base + l;
@@ -1087,21 +1111,30 @@ __global__ void __launch_bounds__(GCT, 1) k_pcg_grid(Grid g, const float* __rest
             const float z = r[k] * precon_of(w[k]);
             S[l] = z;  // every read of the direction lies before the reduction's barrier
             if (whole || i < N) __stcg(zg + base + tid + k * GCT, z);
-            if (EXACT) zx.add_prod(z, r[k]);
+            if (EXACT) zs[k] = z;
             else zr.add(z * r[k]);
             const float m = (!reference || i < XY) ? fabsf(r[k]) : r[k];  // Q4
             if (m > mx) mx = m;
         }
-        grid_reduce<true, EXACT>(inbox, nb, ++tag, EXACT ? zx : zr.sum(), mx, [&](double tot, float mall, bool ok) {
+        if (EXACT) zx.add_near(zs, r);
+        auto residual_done = [&](double tot, float mall, bool ok, bool again) {
             const float b = quotient(tot, G.sigma0);
             __syncwarp();
             if (tid == 0) {
-                G.sigma0 = G.sigma1 = tot;
+                G.state = !ok ? GRID_STUCK : again && !Sum::total_holds(tot) ? GRID_FAR : !isfinite(tot) ? GRID_NAN : mall <= tol ? GRID_DONE
+                          : iters + 1 >= max_iter ? GRID_CAP : GRID_GO;
+                if (G.state != GRID_FAR) G.sigma0 = G.sigma1 = tot;
                 G.len = b;
                 G.residual = mall;
-                G.state = !ok ? GRID_STUCK : !isfinite(tot) ? GRID_NAN : mall <= tol ? GRID_DONE : iters + 1 >= max_iter ? GRID_CAP : GRID_GO;
             }
-        });
+        };
+        grid_reduce<true, EXACT, false>(inbox, nb, ++tag, EXACT ? zx : zr.sum(), mx,
+                                        [&](double tot, float m, bool ok) { residual_done(tot, m, ok, EXACT); });
+        if (EXACT && G.state == GRID_FAR) {
+            Sum far;
+            far.add_far(zs, r);
+            grid_reduce<true, false, true>(inbox, nb, ++tag, far, mx, [&](double tot, float m, bool ok) { residual_done(tot, m, ok, false); });
+        }
         if (G.state == GRID_STUCK) break;
         ++iters;
         beta = G.len;

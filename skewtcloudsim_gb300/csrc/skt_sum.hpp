@@ -66,15 +66,54 @@ struct Sum {
     // two lanes an SM for 48 cycles a warp.
     SKT_HD void add_prod(float a, float b) {
         const float p = rn_mul(a, b);
-        if ((float_bits(p) >> 23 & 0xffu) - 28u < 200u) {
-            float x, y, z;
-            two_sum(h, p, h, x);
-            two_sum(l, fmaf(a, b, -p), l, y);
-            two_sum(l, x, l, z);
-            t = rn_add(t, rn_add(y, z));
-        } else if (!(p == 0.0f && (a == 0.0f || b == 0.0f))) {
-            far = fma(double(a), double(b), far);
+        if (near(p) || zero(p, a, b)) add(p, fmaf(a, b, -p));
+        else far = fma(double(a), double(b), far);
+    }
+    // N products with one test of the largest: below 2^-90 (where what the small ones lose, 2^-149 each, could
+    // reach 2^-56 of it) or from 2^101 all of them go to FP64
+    template <int N>
+    SKT_HD void add_prods(const float (&a)[N], const float (&b)[N]) {
+        float p[N], most = 0.0f;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            p[i] = rn_mul(a[i], b[i]);
+            most = fmaxf(most, fabsf(p[i]));
         }
+        if (most >= 0x1p-90f && most < 0x1p101f) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) add(p[i], fmaf(a[i], b[i], -p[i]));
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (!zero(p[i], a[i], b[i])) far = fma(double(a[i]), double(b[i]), far);
+    }
+    // N products with no test: each loses up to 2^-149 where it is small, and one too large makes the sum not
+    // finite, so a grid's total stands where total_holds, and is taken again by add_far elsewhere
+    template <int N>
+    SKT_HD void add_near(const float (&a)[N], const float (&b)[N]) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float p = rn_mul(a[i], b[i]);
+            add(p, fmaf(a[i], b[i], -p));
+        }
+    }
+    // 2^31 terms lose 2^-118 at most, 2^-58 of such a total
+    static SKT_HD bool total_holds(double total) { return fabs(total) >= 0x1p-60 && fabs(total) < 0x1p120; }
+    template <int N>
+    SKT_HD void add_far(const float (&a)[N], const float (&b)[N]) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) far = fma(double(a[i]), double(b[i]), far);
+    }
+    static SKT_HD bool near(float p) { return (float_bits(p) >> 23 & 0xffu) - 28u < 200u; }
+    static SKT_HD bool zero(float p, float a, float b) { return p == 0.0f && (a == 0.0f || b == 0.0f); }  // not 0 * inf, not an underflow
+    // a product p with its rounding error e
+    SKT_HD void add(float p, float e) {
+        float x, y, z;
+        two_sum(h, p, h, x);
+        two_sum(l, e, l, y);
+        two_sum(l, x, l, z);
+        t = rn_add(t, rn_add(y, z));
     }
 };
 // a running sum s with its compensation c (the sum is s - c) as a Sum

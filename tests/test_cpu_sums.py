@@ -62,6 +62,21 @@ extern "C" double dot(const float* a, const float* b, int n) {
     for (int i = 0; i < n; ++i) v[i % 32].add_prod(a[i], b[i]);
     return warp(v, true);
 }
+extern "C" int holds(double t) { return Sum::total_holds(t); }
+extern "C" double dot16(const float* a, const float* b, int how) {  // the same 512 terms, a lane's 16 at a time
+    Sum v[32];
+    for (int i = 0; i < 32; ++i) {
+        float x[16], y[16];
+        for (int j = 0; j < 16; ++j) {
+            x[j] = a[i + 32 * j];
+            y[j] = b[i + 32 * j];
+        }
+        if (how == 0) v[i].add_prods(x, y);
+        else if (how == 1) v[i].add_near(x, y);
+        else v[i].add_far(x, y);
+    }
+    return warp(v, true);
+}
 extern "C" double total(const float* s, const float* c) {  // of 32 running sums with their compensations
     Sum v[32];
     for (int i = 0; i < 32; ++i) v[i] = sum_of(s[i], c[i]);
@@ -78,7 +93,9 @@ def lib(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-I", build.CSRC, str(d / "sums.cpp"), "-o", so], check=True)
     lb = ctypes.CDLL(so)
     p = ctypes.POINTER(ctypes.c_float)
-    lb.dot.restype = lb.total.restype = ctypes.c_double
+    lb.dot.restype = lb.dot16.restype = lb.total.restype = ctypes.c_double
+    lb.dot16.argtypes = [p, p, ctypes.c_int]
+    lb.holds.argtypes = [ctypes.c_double]
     lb.quot.restype = ctypes.c_float
     lb.quot.argtypes = [ctypes.c_double, ctypes.c_double]
     lb.lanes.restype = ctypes.c_double
@@ -198,3 +215,59 @@ def test_quotient_is_rounded_once(lib):
         with np.errstate(all="ignore"):
             want = np.float32(np.float64(a) / np.float64(b))
         assert np.float32(lib.quot(a, b)).tobytes() == want.tobytes() or (np.isnan(want) and np.isnan(lib.quot(a, b))), (a, b)
+
+
+@pytest.mark.parametrize("kind", ["one", "residual", "cancel", "gone", "tiny", "huge", "edge", "denormal", "spread"])
+@pytest.mark.parametrize("seed", range(8))
+def test_products_of_a_lane_together(lib, kind, seed):
+    """The bound of test_dot_is_no_worse_than_fp64, where a lane goes to FP64 when its largest product lies outside
+    2^-90 to 2^101; inside, a product too small for FP32 loses 2^-149, 16 of them 2^-55 of the largest."""
+    a, b = _terms(np.random.default_rng(seed), kind)
+    prods = [Fraction(float(x)) * Fraction(float(y)) for x, y in zip(a, b)]
+    exact, size, far, small = sum(prods), sum(abs(p) for p in prods), Fraction(0), Fraction(0)
+    for lane in range(32):
+        mine = [abs(p) for p in prods[lane::32]]
+        if not 2.0 ** -89 <= max(mine) < 2.0 ** 100:
+            far += sum(mine)
+        else:
+            small += sum(Fraction(1, 2 ** 149) for p in mine if p < 2.0 ** -98)
+    got = lib.dot16(_ptr(a), _ptr(b), 0)
+    assert abs(Fraction(got) - exact) <= abs(exact) / 2 ** 51 + size / 2 ** 60 + far / 2 ** 44 + small, (kind, seed, got, float(exact))
+
+
+def test_far_products_of_a_lane_together(lib):
+    one, z = np.ones(512, np.float32), np.zeros(512, np.float32)
+    for big in (1e25, 1e-25):
+        a = np.full(512, big, np.float32)
+        assert abs(lib.dot16(_ptr(a), _ptr(a), 0) / (512 * float(a[0]) ** 2) - 1) < 512 * 2.0 ** -53
+        for bad in (np.inf, np.nan):
+            b = a.copy()
+            b[37] = bad
+            for other in (a, one, z):
+                assert not np.isfinite(lib.dot16(_ptr(b), _ptr(other), 0))
+    assert lib.dot16(_ptr(z), _ptr(one), 0) == 0.0
+
+
+@pytest.mark.parametrize("kind", ["one", "residual", "cancel", "gone", "tiny", "huge", "edge", "denormal", "spread"])
+@pytest.mark.parametrize("seed", range(8))
+def test_untested_products_stand_where_the_total_holds(lib, kind, seed):
+    """Products without a test for their range, 2^-149 lost by each at most: where their total holds it meets the
+    bound of the tested ones, and where it does not (too small, too large, not finite) FP64's sum takes its
+    place, within FP64's own bound."""
+    a, b = _terms(np.random.default_rng(seed), kind)
+    prods = [Fraction(float(x)) * Fraction(float(y)) for x, y in zip(a, b)]
+    exact, size = sum(prods), sum(abs(p) for p in prods)
+    got = lib.dot16(_ptr(a), _ptr(b), 1)
+    if lib.holds(got):
+        assert abs(Fraction(got) - exact) <= abs(exact) / 2 ** 51 + size / 2 ** 60 + Fraction(512, 2 ** 149)
+    else:
+        assert kind not in ("one", "residual")
+        got = lib.dot16(_ptr(a), _ptr(b), 2)
+        assert abs(Fraction(got) - exact) <= size / 2 ** 44
+
+
+def test_totals_that_do_not_hold(lib):
+    for t in (0.0, 8e-19, 1.4e36, np.inf, np.nan):
+        assert not lib.holds(t) and not lib.holds(-t)
+    for t in (9e-19, 1.0, 1.3e36):
+        assert lib.holds(t) and lib.holds(-t)
