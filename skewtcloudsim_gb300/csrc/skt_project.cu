@@ -1607,9 +1607,10 @@ void launch_project(Env& e, float dtS) {
     const Runs MT = matvec_runs(g, e.num_sms);
     const dim3 mvb(32, MVY);
     const int gx = (g.X / 4 + 31) / 32, gy = (g.Y + MVY - 1) / MVY;
-    // about 6 blocks of 1024 threads per SM in the operator's grid (one resident at a time): at
-    // 512x512x256 the operator took 86.5 ms per step at 6, 87.0 at 8, 87.6 at 4, 89.1 at 12
-    int zc = std::max(1, std::min(g.Z, (e.num_sms * 6 + gx * gy - 1) / (gx * gy)));
+    // k_matvec4 (pcg_fused = 0): about 4 blocks of 1024 threads per SM (one resident at a time), 251 us a launch
+    // at 512x256x512 and 50.0 at 256x128x256; 6 blocks 256 and 51.8, 8 blocks 261 and 54.8, 12 blocks 266 and
+    // 54.6, all four 20.6 to 20.7 at 128x100x128
+    int zc = std::max(1, std::min(g.Z, (e.num_sms * 4 + gx * gy - 1) / (gx * gy)));
     while (gx * gy * zc > kMaxPartials && zc > 1) --zc;
     const int zlen = (g.Z + zc - 1) / zc;
     zc = (g.Z + zlen - 1) / zlen;
