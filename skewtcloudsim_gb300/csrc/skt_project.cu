@@ -1476,6 +1476,10 @@ void pcg_grid_shape(const Env& e, int& slot, int& nb) {
 
 // How the plain PCG runs: in one cooperative launch where the grid fits, else matrix-free in two
 // launches per iteration (X % 4 == 0), else from stored coefficients in three (any X; pcg_fused = 0).
+// Rows of less than 24 cells leave the matrix-free operator's warps, each across 128 cells of a row, too few
+// lanes to form coefficients with (us an iteration matrix-free and stored at 2.1M cells: X = 4 250 and 152, 8 146
+// and 100, 16 88 and 73; 1.8M cells, 20 68 and 64; 1.6M, 24 58 and 59; 1.9M, 48 47 and 53).
+constexpr int kFreeMinX = 24;
 enum class PcgPath { GRID, FREE, STORED };
 PcgPath pcg_path(Env& e, int& slot, int& nb, OpMaps* maps, float* const* dirs, const float* zbuf) {
     pcg_grid_shape(e, slot, nb);
@@ -1483,7 +1487,7 @@ PcgPath pcg_path(Env& e, int& slot, int& nb, OpMaps* maps, float* const* dirs, c
     if (nb > 0 && (slot == 0 ? pcg_grid_fits<2>(e, slot, nb) : slot == 1 ? pcg_grid_fits<4>(e, slot, nb)
                    : slot == 2 ? pcg_grid_fits<8>(e, slot, nb) : pcg_grid_fits<14>(e, slot, nb)))
         return PcgPath::GRID;
-    if (e.g.X % 4 != 0 || (long long)((e.g.X + 127) / 128) * ((e.g.Y + OPR - 1) / OPR) > kMaxPartials) return PcgPath::STORED;
+    if (e.g.X % 4 != 0 || e.g.X < kFreeMinX || (long long)((e.g.X + 127) / 128) * ((e.g.Y + OPR - 1) / OPR) > kMaxPartials) return PcgPath::STORED;
     // one set of tensor maps per direction buffer that an iteration reads; without an encoder: stored
     for (int j = 0; j < kDirs; ++j) {
         if (!field_tensor_map(e.g, zbuf, OPW, OPR + 2, &maps[j].z) || !field_tensor_map(e.g, dirs[j], OPW, OPR + 2, &maps[j].s) ||
