@@ -76,7 +76,7 @@ typedef struct {
     int pcg_max_iter;   /* 200 (Game/environment.cu:907) */
     int max_substeps;   /* Courant substep cap (100, Game/environment.cu:727) */
     int precision;      /* skt_precision */
-    float refine_tol;   /* MIXED: relative residual target of the FP64 refinement (1e-8) */
+    float refine_tol;   /* MIXED: relative residual target of the float-float refinement (1e-8) */
     int inner_max_iter; /* MIXED: FP32 iterations per refinement step */
     float inner_rtol;   /* MIXED: relative tolerance of each FP32 inner solve */
     int use_graph;      /* 1: each step is one launch of a CUDA graph captured at the first step (and
@@ -88,9 +88,10 @@ typedef struct {
                            issued stream-ordered, the loop counts read back by the host. */
     int mg_half;        /* MIXED: the V-cycle smooths with FP16 copies of the finest coefficients */
     int pcg_fused;      /* PLAIN: 1 the whole solve in one launch up to about a million cells, above that
-                           (nx % 4 == 0) two launches per iteration with the search step fused into a
-                           matrix-free operator and the pressure updated every fourth one; 0 three
-                           launches per iteration; same values up to the dot products' summation order */
+                           (nx % 4 == 0, nx >= 24) two launches per iteration with the search step fused
+                           into a matrix-free operator and the pressure updated every fourth one, else
+                           three; 0 three launches per iteration; same values up to the dot products'
+                           summation order */
 } skt_solver_cfg;
 
 typedef struct {

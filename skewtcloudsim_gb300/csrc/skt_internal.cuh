@@ -433,9 +433,10 @@ struct ProfScope {
 // at 64x32x64 (1.95 with ordinary launches), 2.08 at 128x64x128 (2.85), 7.6 at 256x128x256 (8.9) and 43.3
 // at 512x256x512 (44.6), the coarsest level's shorter solve included; a frame at 32^3 1.16 ms (1.37), three
 // substeps of one field's advection at 192x96x192 0.45 (0.55), 20 sweeps of theta at 256x128x256 0.34
-// (0.36). Inside a capture the launch is an ordinary one: programmatic edges gained a graph nothing (a
-// step at 64x32x64 1.386 ms with and without, eight members 11.51 and 11.36). A kernel that follows a copy or
-// a memset is launched in the ordinary way too.
+// (0.36; tiles of 14 rows). Inside a capture the launch is an ordinary one: programmatic edges gained a graph nothing (a
+// step at 64x32x64 1.386 ms with and without, eight members 11.51 and 11.36). Behind a copy or a memset the
+// attribute has nothing to overlap with and the wait still orders the kernel; the launchers set it there where
+// they cannot tell (a caller's copy, the tuner's).
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

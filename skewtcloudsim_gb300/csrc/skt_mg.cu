@@ -1,15 +1,15 @@
-// Mixed-precision pressure solve: FP64 iterative refinement around an FP32 conjugate gradient
+// Mixed-precision pressure solve: float-float iterative refinement around an FP32 conjugate gradient
 // preconditioned by a geometric multigrid V-cycle.
 //
 // The reference's projection (calculatePressureProject, Game/environment.cu:898-987) runs a
 // Jacobi-preconditioned CG for at most 200 iterations, which at 512x256x512 leaves the residual
 // far above any tight tolerance. This solver uses the textbook (symmetric) operator A of the
-// projection and solves it to a relative FP64 residual of refine_tol:
+// projection and solves it to a relative residual of refine_tol:
 //
-//   x64 = 0
-//   repeat: r = b - A x64 (FP64 arithmetic, FP64 norm)    until |r|/|b| <= refine_tol
+//   x = 0 (float-float: some 48 bits)
+//   repeat: r = b - A x (float-float arithmetic, FP64 norm)    until |r|/|b| <= refine_tol
 //           solve A e = r with MG-PCG in FP32 (FP64 reductions) to |r_inner| <= inner_rtol |r|
-//           x64 += e
+//           x += e
 //
 // Multigrid: cell-centred, the hierarchy of the full grid (ground cells inactive: diagonal 0).
 // Coarse face coefficient = 1/2 x (sum of the four fine coefficients of that face), the

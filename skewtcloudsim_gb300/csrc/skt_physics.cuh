@@ -89,7 +89,9 @@ struct Gammas {
 
 // ---- Process rates, Game/microPhysics.cu:67-685 -----------------------------------------------
 // What several processes of a cell share, formed once per cell that holds any condensate (each process
-// formed them again under its own condition), by the same calls: every rate keeps its bits.
+// formed them again under its own condition), by the same calls. Against the processes on their own, one stage
+// on 1.05M cells half of which hold each species: theta, vapour, cloud and snow bit for bit, 1.7 % of the rain
+// values and 0.08 % of the ice values off by a rounding of their rates (up to 9e-8 of the largest value).
 struct Air {
     float dQv;         // DQVair
     float Sc13, kvm;   // Sc^(1/3) and kv^(-1/2) of the ventilation terms, Sc = kv / dQv

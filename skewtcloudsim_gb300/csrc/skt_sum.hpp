@@ -62,8 +62,8 @@ struct Sum {
     // would leave FP32's range, below 2^-99 or from 2^101, goes to FP64. A warp's 512 products against exact
     // arithmetic, error over the terms' magnitudes: random terms 2.1e-18 on average and 1.1e-17 at most (FP64
     // products and tree 7.0e-18 and 3.7e-17), z.r over six decades 4.1e-17 and 9.5e-17 (6.4e-17 and 3.0e-16).
-    // 26 FP32 and integer instructions a product, where FP64's product and its two conversions hold a pipe of
-    // two lanes an SM for 48 cycles a warp.
+    // 22 FP32 instructions a product and the range's test, where FP64's product and its two conversions hold a
+    // pipe of two lanes an SM for 48 cycles a warp (k_update at 251x118x275 43 us so, 66 with FP64 products).
     SKT_HD void add_prod(float a, float b) {
         const float p = rn_mul(a, b);
         if (near(p) || zero(p, a, b)) add(p, fmaf(a, b, -p));
